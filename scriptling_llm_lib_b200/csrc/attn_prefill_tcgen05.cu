@@ -35,6 +35,15 @@
 // pair has its own issuing thread, softmax warps, barriers and 256 columns (one S buffer, two P
 // buffers, O); the two share the query/key/value fetches and the key/value ring, whose stage is
 // free when both have used it.
+//
+// Weights of 24 bits (PARTS = 3 of the pair kernel): for the layers that keep the softmax weights float32 into the product with
+// the values. A float is exactly the sum of three bfloat16 numbers (its mantissa cut into 8 + 8 + 8 bits), so P goes into tensor
+// memory as three bfloat16 matrices of 32 columns and O takes three products a page; Q, K and V are bfloat16 as they are stored.
+// O's 128 columns and P's 96 leave no room for a second S in a tile's 256, so P takes the place of the S it was made from and the
+// next page's S is issued behind P V; the other tile of the pair fills the tensor cores meanwhile. Keys go up to 192 here.
+// Bound by the chain S -> softmax and splitting -> P V of a page. Prompts of 2,048 tokens, 16 heads: keys 64, values 128, window
+// 1,024 on 4 key/value heads 55.6 us (1,827 on the kernel with a warp a row and head, attn_wide_value, 22 -> 175 TFLOP/s on the
+// pairs seen); keys 192, values 128, every earlier key 97.5 us (1,189 on the float32 tiles of attn_paged, 18 -> 220 TFLOP/s).
 #include "tcgen05.cuh"
 
 #define FT_BQ 128
@@ -144,6 +153,13 @@ __device__ __forceinline__ uint64_t ft_add2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+// two floats as the packed upper halves of their bits, and what that leaves of them (exactly): bfloat16 parts by truncation
+__device__ __forceinline__ uint32_t ft_cut_pair(float& u, float& v) {
+  const uint32_t a = __float_as_uint(u), b = __float_as_uint(v);
+  u -= __uint_as_float(a & 0xffff0000u);
+  v -= __uint_as_float(b & 0xffff0000u);
+  return __byte_perm(a, b, 0x7632);
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -536,8 +552,9 @@ __device__ __forceinline__ void ft_ld64(uint32_t taddr, uint32_t (&s)[64]) {
   tmem_ld32(taddr + 32, *(uint32_t(*)[32])&s[32]);
 }
 
-// Keys of up to KD and values of up to VD dims (64 or 128 either, not both 64: that is the kernel above), narrower heads as there.
-template <int KD, int VD, int FT_STAGES>
+// Keys of up to KD and values of up to VD dims (with rounded weights 64 or 128 either, not both 64: that is the kernel above),
+// narrower heads as there. PARTS: 1 rounds the weights to bfloat16, 3 keeps all their bits.
+template <int KD, int VD, int FT_STAGES, int PARTS>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, FtArgs p, uint32_t smem_bytes) {
@@ -546,8 +563,11 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   constexpr int NK = KD / 64, NV = VD / 64;                    // such blocks per key (query) head and per value head
   // tensor-memory columns of one tile of the pair (256): values of 64 have S0 0-63, S1 64-127, O 128-191, P0 192-223,
   // P1 224-255; values of 128, whose O takes 128-255, have one S buffer 0-63 and P0 64-95, P1 96-127
-  constexpr int NBUF = VD > 64 ? 1 : 2;          // S buffers; the next tile's S is issued while a tile's softmax runs
-  constexpr uint32_t P_COL0 = VD > 64 ? 64 : 192, P_STEP = 32, SUB_COLS = 256;
+  constexpr int NBUF = VD > 64 || PARTS == 3 ? 1 : 2;   // S buffers; the next tile's S is issued while a tile's softmax runs
+  // (P in three parts: 0-95, over the S it was made from; O 128-255)
+  constexpr bool P_OVER_S = PARTS == 3;
+  constexpr uint32_t P_COL0 = P_OVER_S ? 0 : VD > 64 ? 64 : 192, P_STEP = P_OVER_S ? 0 : 32, SUB_COLS = 256;
+  static_assert(PARTS == 1 || PARTS == 3, "weights in one part or in three");
   static_assert(FT_STAGES >= 3, "the key/value ring must hold the tile whose S is issued ahead");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -656,7 +676,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               const int Jg = J0 + fp_place(sub, t), sb = Jg % NBUF;
               // S(Jg) takes the place of S(Jg - NBUF), which the softmax threads have taken into their registers: with
               // two buffers their P(Jg - 2) was waited for; the single buffer has a barrier for it
-              if (NBUF == 1 && !mbar_wait(b_sub + SUB_BARS * x + B_SEMPTY + 8 * sb, ((Jg / NBUF) & 1) ^ 1, abort)) return false;
+              // (where P lies over S, this product is issued behind the one that read P)
+              if (NBUF == 1 && !P_OVER_S && !mbar_wait(b_sub + SUB_BARS * x + B_SEMPTY + 8 * sb, ((Jg / NBUF) & 1) ^ 1, abort)) return false;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
               for (int k = 0; k < KD / 16; k++)         // 16 dims a step: four steps in each 64-wide block
@@ -670,7 +691,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           };
           if (ok) ok = issue_s(0);
           for (int u = 0; u < n_union && ok; u++) {
-            if (u + 1 < n_union) { ok = issue_s(u + 1); if (!ok) break; }
+            if (!P_OVER_S && u + 1 < n_union) { ok = issue_s(u + 1); if (!ok) break; }
             const int JUg = JU0 + u, s = JUg % FT_STAGES, t = fp_union_tile(it, u);
             if (fp_active(sub, t)) {
               const int j = fp_place(sub, t), Jg = J0 + j, a = Jg & 1;
@@ -678,13 +699,16 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               if (!ok) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-              for (int k = 0; k < FT_BK / 16; k++)
-                umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + k * 8,
-                             umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k) ? 1u : 0u);
+              for (int part = 0; part < PARTS; part++)
+#pragma unroll
+                for (int k = 0; k < FT_BK / 16; k++)
+                  umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + part * 32 + k * 8,
+                               umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k | part) ? 1u : 0u);
               umma_commit(b_sub + SUB_BARS * x + B_OFULL + 8 * a);
             }
             if (!ok) break;
             umma_commit(b_kvempty + 8 * s);
+            if (P_OVER_S && u + 1 < n_union) ok = issue_s(u + 1);
           }
           JU0 += n_union;
           if (sub.valid) J0 += sub.n_tiles;
@@ -720,7 +744,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       ft_ld64(t_lane + bf * 64, s);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (NBUF == 1) {                             // the one S buffer may take the next tile's scores
+      if (NBUF == 1 && !P_OVER_S) {                // the one S buffer may take the next tile's scores
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(b_sempty + 8 * bf);
@@ -759,17 +783,39 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       const float msc = (m_ref == -INFINITY) ? 0.f : m_ref * sc;
       uint64_t rs2 = 0ull;                          // two partial sums side by side
       const uint64_t sc2 = ft_pack2(sc, sc), nm2 = ft_pack2(-msc, -msc);
-      uint32_t pk[32];                              // 64 probabilities as bfloat16 pairs: keys 2i, 2i+1
+      uint32_t pk[PARTS == 1 ? 32 : 1];             // 64 probabilities as bfloat16 pairs: keys 2i, 2i+1
+      if constexpr (PARTS == 1) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        float x0, x1, x2, x3;
-        ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nm2), x0, x1);
-        ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i + 2]), __uint_as_float(s[2 * i + 3])), sc2, nm2), x2, x3);
-        float e0 = ft_ex2(x0), e1 = ft_ex2(x1), e2 = ft_ex2(x2), e3 = ft_ex2(x3);
-        rs2 = ft_add2(rs2, ft_add2(ft_pack2(e0, e1), ft_pack2(e2, e3)));
-        __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
-        pk[i] = *(uint32_t*)&lo;
-        pk[i + 1] = *(uint32_t*)&hi;
+        for (int i = 0; i < 32; i += 2) {
+          float x0, x1, x2, x3;
+          ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nm2), x0, x1);
+          ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i + 2]), __uint_as_float(s[2 * i + 3])), sc2, nm2), x2, x3);
+          float e0 = ft_ex2(x0), e1 = ft_ex2(x1), e2 = ft_ex2(x2), e3 = ft_ex2(x3);
+          rs2 = ft_add2(rs2, ft_add2(ft_pack2(e0, e1), ft_pack2(e2, e3)));
+          __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
+          pk[i] = *(uint32_t*)&lo;
+          pk[i + 1] = *(uint32_t*)&hi;
+        }
+      } else {
+        // 32 keys at a time: their three parts go over the columns of S, which is in registers by now
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+          uint32_t p3[3][16];
+#pragma unroll
+          for (int i = 0; i < 16; i++) {
+            const int k0 = 32 * half + 2 * i;
+            float e0, e1;
+            ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[k0]), __uint_as_float(s[k0 + 1])), sc2, nm2), e0, e1);
+            e0 = ft_ex2(e0);
+            e1 = ft_ex2(e1);
+            rs2 = ft_add2(rs2, ft_pack2(e0, e1));
+            p3[0][i] = ft_cut_pair(e0, e1);
+            p3[1][i] = ft_cut_pair(e0, e1);
+            p3[2][i] = ft_cut_pair(e0, e1);
+          }
+#pragma unroll
+          for (int part = 0; part < 3; part++) tmem_st16(t_lane + part * 32 + half * 16, p3[part]);
+        }
       }
       {
         float ra, rb;
@@ -792,7 +838,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       }
       // ---- P into tensor memory. The product that read this buffer's last P, two tiles ago, is complete:
       // it was issued before S(Jg), and the commit that announced S(Jg) covers every product issued before it.
-      tmem_st32(t_lane + P_COL0 + a * P_STEP, pk);
+      if constexpr (PARTS == 1) tmem_st32(t_lane + P_COL0 + a * P_STEP, pk);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -855,7 +901,7 @@ static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   SLLM_RETURN_LAST();
 }
 
-template <int KD, int VD, int STAGES>
+template <int KD, int VD, int STAGES, int PARTS>
 static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FtArgs& a, dim3 grid,
                      cudaStream_t stream) {
   // what the kernel lays out after aligning to 1 KB; one block on an SM
@@ -865,23 +911,24 @@ static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   static_assert(need <= smem, "the block of this head width does not fit an SM");
   static bool raised = false;
   if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<KD, VD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<KD, VD, STAGES, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     raised = true;
   }
-  attn_prefill_pair_kernel<KD, VD, STAGES><<<grid, FP_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
+  attn_prefill_pair_kernel<KD, VD, STAGES, PARTS><<<grid, FP_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
   SLLM_RETURN_LAST();
 }
 
 // q: [T, q_ld] rotated queries (head h at columns h*hd); out: [T, H*vd]; kpages [n_pages][G][64][hd], vpages
-// [n_pages][G][64][vd] with n_pages the number of pages the storage holds; hd and vd multiples of 8 up to 128.
+// [n_pages][G][64][vd] with n_pages the number of pages the storage holds; hd and vd multiples of 8 up to 128, with weight_parts = 3
+// (the weights keep their 24 bits into the product with the values; 1 rounds them to bfloat16) hd up to 192.
 SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* out, const int* seq_start, const int* seq_pos0,
                                           const int* block_table, int max_pages, const void* kpages, const void* vpages,
                                           long long n_pages, int B, int max_new, int H, int G, int hd, int vd, int window, int keep, float scale,
-                                          float softcap, const float* sink, const void* gate, int gate_ld, int* err,
+                                          float softcap, const float* sink, const void* gate, int gate_ld, int weight_parts, int* err,
                                           cudaStream_t stream) {
   if (B <= 0 || max_new <= 0) return 0;
-  if (hd < 8 || hd > 128 || hd % 8 || vd < 8 || vd > 128 || vd % 8 || q_ld < H * hd || G < 1 || H % G != 0 || (q_ld & 7) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
+  if ((weight_parts != 1 && weight_parts != 3) || hd < 8 || hd > (weight_parts == 3 ? 192 : 128) || hd % 8 || vd < 8 || vd > 128 || vd % 8 || q_ld < H * hd || G < 1 || H % G != 0 || (q_ld & 7) || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
       ((uintptr_t)kpages & 15) || ((uintptr_t)vpages & 15) || keep < 0 ||
       (gate && (((uintptr_t)gate & 15) || (gate_ld & 7) || gate_ld < H * vd)))
     return SLLM_ERR_ARG;
@@ -904,7 +951,7 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
   }
-  if (hd <= 64 && vd <= 64) {
+  if (hd <= 64 && vd <= 64 && weight_parts == 1) {
     FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, 0, softcap, sink,
              (const bf16*)gate, gate_ld};
     dim3 grid((unsigned)(n_items < 2LL * sm_count ? n_items : 2LL * sm_count));     // two blocks per SM that stay
@@ -915,7 +962,17 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
   FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, pair_heads, softcap, sink,
            (const bf16*)gate, gate_ld};
   dim3 grid((unsigned)(n_items < (long long)sm_count ? n_items : (long long)sm_count));       // one block per SM that stays
-  if (vd <= 64) return fp_launch<128, 64, 5>(mq, mk, mv, a, grid, stream);
-  if (hd <= 64) return fp_launch<64, 128, 5>(mq, mk, mv, a, grid, stream);
-  return fp_launch<128, 128, 4>(mq, mk, mv, a, grid, stream);
+  if (weight_parts == 3) {
+    if (vd <= 64) {
+      if (hd <= 64) return fp_launch<64, 64, 5, 3>(mq, mk, mv, a, grid, stream);
+      if (hd <= 128) return fp_launch<128, 64, 5, 3>(mq, mk, mv, a, grid, stream);
+      return fp_launch<192, 64, 4, 3>(mq, mk, mv, a, grid, stream);
+    }
+    if (hd <= 64) return fp_launch<64, 128, 5, 3>(mq, mk, mv, a, grid, stream);
+    if (hd <= 128) return fp_launch<128, 128, 4, 3>(mq, mk, mv, a, grid, stream);
+    return fp_launch<192, 128, 3, 3>(mq, mk, mv, a, grid, stream);
+  }
+  if (vd <= 64) return fp_launch<128, 64, 5, 1>(mq, mk, mv, a, grid, stream);
+  if (hd <= 64) return fp_launch<64, 128, 5, 1>(mq, mk, mv, a, grid, stream);
+  return fp_launch<128, 128, 4, 1>(mq, mk, mv, a, grid, stream);
 }

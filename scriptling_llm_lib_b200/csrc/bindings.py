@@ -481,19 +481,20 @@ class TensorCoreGemm:
 
 class PrefillAttentionTC:
     """tcgen05 causal attention of a prompt step over the paged cache (bfloat16; keys and values of one width, 64 or 128, at
-    full speed, or any two multiples of 8 up to 128, filled up with zeros on the chip)."""
+    full speed, or any two multiples of 8 up to 128, filled up with zeros on the chip). With `exact_weights` the softmax weights
+    enter the product with the values in all their 24 bits (three products instead of one) and keys go up to 192."""
     HEAD_DIMS = (64, 128)
 
     @staticmethod
-    def takes(key_dim: int, value_dim: int) -> bool:
-        return all(w % 8 == 0 and 8 <= w <= 128 for w in (key_dim, value_dim))
+    def takes(key_dim: int, value_dim: int, exact_weights: bool = False) -> bool:
+        return key_dim % 8 == 0 and 8 <= key_dim <= (192 if exact_weights else 128) and value_dim % 8 == 0 and 8 <= value_dim <= 128
 
     def __init__(self):
         self.lib = load_library("attn_prefill_tcgen05")
         self.lib.sllm_attn_prefill_tc_bf16.restype = c_int
 
     def attn(self, q, out, seq_start, seq_pos0, block_table, kpages, vpages, n_seqs, max_new, n_heads, n_kv, head_dim,
-             window, scale, err_flag, softcap=None, sink=None, keep=0, gate=None, v_dim=None):
+             window, scale, err_flag, softcap=None, sink=None, keep=0, gate=None, v_dim=None, exact_weights=False):
         """`v_dim`: the values' width where it is not the keys'. `softcap`: a score s becomes softcap * tanh(s / softcap) before the softmax; `sink` float32 [n_heads]: exp(sink[h])
         joins head h's denominator with no key and no value; `keep`: the first positions of a sequence that stay visible behind
         the window; `gate`: bfloat16 [T, n_heads * v_dim] (a column slice), whose sigmoid multiplies the output."""
@@ -505,8 +506,8 @@ class PrefillAttentionTC:
             _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
             _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), c_longlong(kpages.shape[0]),
             c_int(n_seqs), c_int(max_new), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(v_dim), c_int(window or 0), c_int(keep),
-            c_float(scale), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, _ptr(err_flag, torch.int32, "err_flag"),
-            _stream()), "attn_prefill_tc")
+            c_float(scale), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, c_int(3 if exact_weights else 1),
+            _ptr(err_flag, torch.int32, "err_flag"), _stream()), "attn_prefill_tc")
 
 
 def _gate_args(gate, rows: int, cols: int):

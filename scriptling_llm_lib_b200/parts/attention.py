@@ -11,7 +11,8 @@ cache then keeps values that wide and the output product reads n_heads * v_dim c
 `value_norm_eps`: every value head is divided by its root mean square, sqrt(mean(v^2) + eps),
 before it is cached. Either sends the step's keys and values through a store kernel that does
 rotation, value norm and cache write in one pass (`kv_store`); values as wide as keys then still
-use the attention kernels below, other widths a kernel that takes both (`attn_wide_value`).
+use the attention kernels below, other widths kernels that take both (in a bfloat16 prompt step with widths in
+multiples of 8 the tcgen05 kernel with float32 weights, else `attn_wide_value`).
 
 Four more options, none in the reference. `chunk`: a query sees the earlier keys of its own chunk of that many
 positions only, chunks counted from position 0 of the sequence (not from where a step begins); the cache
@@ -71,19 +72,30 @@ from .linear import Linear
 from .norm import WithRowVector
 
 
+def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int) -> bool:
+    """Whether a layer that keeps its softmax weights in float32 runs this step's attention on the tcgen05 kernel that takes them
+    in three bfloat16 parts: a bfloat16 step that is no decode step, widths in multiples of 8 (keys up to 192, values up to 128).
+    Few rows are no worse off: 33 rows of 16 heads, keys 64 and values 128, take 8 us (70 with a warp a row). A decode step has one
+    query a sequence where the kernel works on 128, and keeps the kernels that split the keys."""
+    return dtype == torch.bfloat16 and not ctx.is_decode and PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True)
+
+
 def prompt_attention(q, gate, ctx, kpages, vpages, block_table, n_heads, n_kv, key_dim, value_dim, span, scale, tensor_cores=True,
                      **options):
     """Queries q [T, n_heads * key_dim] of a step that is no decode step over paged keys and values of two widths, on the
-    kernel that takes them: in bfloat16 (unless `tensor_cores` is off) the tcgen05 kernels or the mma.sync one, else the
+    kernel that takes them: in bfloat16 the tcgen05 kernels or the mma.sync one, else the generic one. With `tensor_cores` off the
+    softmax weights enter the product with the values as float32: on the tcgen05 kernel that takes them in three parts, else on the
     generic one. `options`: softcap, sink, keep. `gate`: logits per element [T, n_heads * value_dim] or None.
     Returns the output and whether the gate has been applied to it (some kernels do it on their way out)."""
     k = ctx.kernels
     attn = torch.empty((q.shape[0], n_heads * value_dim), dtype=q.dtype, device=q.device)
     fused = gate if gate is not None and q.dtype == torch.bfloat16 and gate_aligned(gate) else None
+    exact = not tensor_cores and exact_prompt_kernel(ctx, q.dtype, key_dim, value_dim)
     tensor_cores = tensor_cores and q.dtype == torch.bfloat16
-    if tensor_cores and PrefillAttentionTC.takes(key_dim, value_dim):
+    if exact or (tensor_cores and PrefillAttentionTC.takes(key_dim, value_dim)):
         k.prefill_attention_tc.attn(q, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs, ctx.max_new, n_heads,
-                                    n_kv, key_dim, span, scale, ctx.err_flag, gate=fused, v_dim=value_dim, **options)
+                                    n_kv, key_dim, span, scale, ctx.err_flag, gate=fused, v_dim=value_dim, exact_weights=exact,
+                                    **options)
     elif tensor_cores and PrefillAttentionMMA.takes(key_dim, value_dim):
         k.prefill_attention_mma.attn(q, key_dim, attn, value_dim, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs,
                                      ctx.max_new, n_heads, n_kv, key_dim, value_dim, span, scale, gate=fused, **options)
@@ -287,7 +299,12 @@ class Attention(Mixer):
     def _attend(self, qkv, x, ctx, kpages, vpages, block_table, fast_decode, fusion, writes):
         """The step's queries (the leading columns of `qkv`) over the cache -> [T, n_heads * v_dim]."""
         attn = torch.empty((x.shape[0], self.n_heads * self.v_dim), dtype=x.dtype, device=x.device)
-        if self.other_widths:
+        plain_widths = not self.other_widths and self.head_dim in PrefillAttentionTC.HEAD_DIMS
+        if not plain_widths and exact_prompt_kernel(ctx, x.dtype, self.head_dim, self.v_dim):
+            ctx.kernels.prefill_attention_tc.attn(qkv, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs,
+                                                  ctx.max_new, self.n_heads, self.n_kv_heads, self.head_dim, self.span, self.scale,
+                                                  ctx.err_flag, v_dim=self.v_dim, exact_weights=True)
+        elif self.other_widths:
             ctx.kernels.seq.attn_wide_value(qkv, attn, ctx.tok_pos, ctx.tok_seq, block_table, kpages, vpages, self.n_heads,
                                             self.n_kv_heads, self.head_dim, self.v_dim, self.span, self.scale)
         elif fast_decode:

@@ -26,8 +26,8 @@ turns dim i with dim i + rot / 2 instead of neighbours. `gate_name`: a matrix [n
 i's output is multiplied by the sigmoid of its logit before Wo (the logits ride in the down-projection's product);
 `gate_per="element"`: the matrix is [n_heads * v_dim, hidden] and every element has a logit of its own.
 `prompt_kernel="tensor"`: in bfloat16 the per-head form of a prompt runs on the tensor-core attention kernels that take keys
-and values of different widths instead of the float32 tiled kernel; the weights then enter the product with the values
-rounded to bfloat16. `window`: a query sees its own position and the window - 1 before it, and the cache gives old pages
+and values of different widths with weights rounded to bfloat16 (without it they stay float32 into the product with the values:
+on the tcgen05 kernel that takes them in three parts, or for other widths on the float32 tiled kernel). `window`: a query sees its own position and the window - 1 before it, and the cache gives old pages
 back. `sink_name`: a stored logit per head that joins the softmax's denominator once (not scaled, no key, no value).
 
 Where a kernel takes widths in steps (8 on the tensor cores, 4 otherwise), a head's keys are filled up with zeros as they are
@@ -42,7 +42,7 @@ import torch
 
 from ..cache.needs import PAGE, CacheNeed
 from ..weights.spec import TensorSpec
-from ..csrc.bindings import PrefillAttentionMMA
+from ..csrc.bindings import PrefillAttentionMMA, PrefillAttentionTC
 from .attention import prompt_attention
 from .base import MIXERS, POSITION_ENCODINGS, Mixer, PartSpec
 from .linear import Linear
@@ -123,7 +123,7 @@ class LatentAttention(Mixer):
         wide = lambda n, step: -(-n // step) * step             # noqa: E731
         self.kw, self.vw = wide(self.D + self.P, 8), wide(self.V, 8)
         self.tensor_cores = self.prompt_kernel == "tensor" and dtype == torch.bfloat16 and PrefillAttentionMMA.takes(self.kw, self.vw)
-        if not self.tensor_cores:
+        if not self.tensor_cores and not (dtype == torch.bfloat16 and PrefillAttentionTC.takes(self.kw, self.vw, exact_weights=True)):
             self.kw, self.vw = wide(self.D + self.P, 4), wide(self.V, 4)
         self.wuk, self.wuv = tensors[self.uk_name], self._value_rows(tensors[self.uv_name])
         self.kv_up = Linear([self.uk_name, self.uv_name], [self.H * self.D, self.H * self.vw], self.R)

@@ -530,6 +530,40 @@ def test_attn_prefill_tcgen05(kernel_sets, hd, H, G, window, lens, pos0):
     assert rel_err(out.cpu().float(), want) < 1.2e-2          # probabilities are rounded to bfloat16 before P V
 
 
+@pytest.mark.parametrize("lens, pos0", [([37, 1, 130, 64, 200, 128], [0, 250, 70, 64, 0, 300]), ([1], [700]), ([700], [0])])
+@pytest.mark.parametrize("kd, vd, H, G, window", [(64, 64, 4, 2, 0), (64, 128, 4, 1, 100), (128, 64, 3, 3, 0), (128, 128, 4, 4, -96),
+                                                  (192, 128, 3, 3, 0), (192, 64, 4, 2, 65), (136, 72, 6, 3, 0), (8, 8, 2, 1, 0),
+                                                  (80, 80, 2, 2, 1), (176, 120, 2, 1, 0)])
+def test_attn_prefill_tcgen05_with_float_weights(kernel_sets, kd, vd, H, G, window, lens, pos0):
+    """Softmax weights in three bfloat16 parts: what is left against 64 bits is the output's own rounding to 8 significant
+    bits (at most 2^-8 of an element) and float sums far below it. Unused cache memory is NaN; windows and (below 0) chunks."""
+    fa = kernel_sets[torch.bfloat16].prefill_attention_tc
+    assert fa.takes(kd, vd, exact_weights=True) and not fa.takes(200, 64, exact_weights=True) and not fa.takes(192, 64)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rnd = lambda t: t.bfloat16().float()
+    held = [p + n for p, n in zip(pos0, lens)]
+    kk = [rnd(rand(n, G, kd, seed=50 + 3 * b)) for b, n in enumerate(held)]
+    vv = [rnd(rand(n, G, vd, seed=51 + 3 * b)) for b, n in enumerate(held)]
+    qs = [rnd(rand(n, H, kd, seed=52 + 3 * b, scale=3.0)) for b, n in enumerate(lens)]
+    kp, _, bt = paged(kk, kk, held, dtype=torch.bfloat16)
+    vp, _, _ = paged(vv, vv, held, dtype=torch.bfloat16)
+    q = dev(torch.cat([t.reshape(t.shape[0], -1) for t in qs]), torch.bfloat16)
+    out = torch.full((sum(lens), H * vd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    seq_start = dev(np.concatenate([[0], np.cumsum(lens)]), torch.int32)
+    fa.attn(q, out, seq_start, dev(pos0, torch.int32), bt, kp, vp, len(lens), max(lens), H, G, kd, window, kd ** -0.5, err, v_dim=vd,
+            exact_weights=True)
+    want = []
+    for b, (n, p) in enumerate(zip(lens, pos0)):
+        at, key = torch.arange(p, p + n)[:, None], torch.arange(p + n)[None, :]
+        first = torch.zeros_like(at) if window == 0 else at - window + 1 if window > 0 else at - at % -window
+        k, v = (f64(t).repeat_interleave(H // G, 1) for t in (kk[b], vv[b]))
+        sc = torch.einsum("qhd,khd->hqk", f64(qs[b]), k) * kd ** -0.5
+        sc = sc.masked_fill((key > at) | (key < first), -math.inf).softmax(-1)
+        want.append(torch.einsum("hqk,khd->qhd", sc, v).reshape(n, -1))
+    assert int(err) == 0
+    assert rel_err(out.cpu().float(), torch.cat(want)) < 2.0 ** -8 + 2e-5
+
+
 @pytest.mark.parametrize("hd, H, G, window", [(64, 40, 40, None), (64, 24, 6, 700), (128, 24, 6, None), (128, 15, 15, None), (128, 9, 3, 900)])
 def test_attn_prefill_tcgen05_long_prompts_many_items(kernel_sets, hd, H, G, window):
     """Prompts of a few thousand tokens and more work items than resident blocks: every block walks several
