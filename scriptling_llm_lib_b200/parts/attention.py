@@ -75,7 +75,7 @@ from .norm import WithRowVector
 def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int) -> bool:
     """Whether a layer that keeps its softmax weights in float32 runs this step's attention on the tcgen05 kernel that takes them
     in three bfloat16 parts: a bfloat16 step that is no decode step, widths in multiples of 8 (keys up to 192, values up to 128).
-    Few rows are no worse off: 33 rows of 16 heads, keys 64 and values 128, take 8 us (70 with a warp a row). A decode step has one
+    Few rows are no worse off: 33 rows of 16 heads, keys 64 and values 128, take 8 us (14 with a warp a row). A decode step has one
     query a sequence where the kernel works on 128, and keeps the kernels that split the keys."""
     return dtype == torch.bfloat16 and not ctx.is_decode and PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True)
 
