@@ -909,6 +909,30 @@ class SequenceKernels:
                                       c_int(ctx.n_seqs), c_int(W), c_int(block_size), _stream()), "rglru_scan")
 
 
+class ChunkKernels:
+    """Linear recurrences with a matrix state over many rows, in chunks on tcgen05 (bfloat16 engines; see chunk_tcgen05.cu)."""
+    CHUNK = 128
+    # The longest run of a step from which on linear attention goes in chunks. One sequence, 16 heads of 128 x 128: 128 rows take 42 us
+    # in chunks and 40 in pieces of 32 rows (lin_attn_decay), 64 rows 37 and 26; a piece more is 8 us more, a chunk more is nothing
+    # while there are idle SMs.
+    LIN_MIN_ROWS = 144
+
+    def __init__(self):
+        self.lib = load_library("chunk_tcgen05")
+        self.lib.sllm_chunk_lin_attn_bf16.restype = c_int
+
+    def lin_attn(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
+        """As `MixKernels.lin_attn_decay`, keys up to 128 wide."""
+        n = proj.shape[0] // self.CHUNK + ctx.n_seqs
+        chunk_state = torch.empty((n, n_heads, dk, dv), dtype=torch.float32, device=o.device)
+        _check(self.lib.sllm_chunk_lin_attn_bf16(
+            _ptr(proj, torch.bfloat16, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
+            _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(ctx.max_new),
+            c_int(n_heads), c_int(dk), c_int(dv), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
+            "chunk_lin_attn")
+
+
 class MixKernels:
     """Launchers of mix_kernels.cuh: the norm without statistics fused with the residual sum, activations in
     place, linear attention with a decay per head, the gated read-out norm over a row, attention over a cached
@@ -924,6 +948,7 @@ class MixKernels:
         self.dtype, self.suffix = dtype, _SUFFIX[dtype]
         self.lib = load_library("mix_" + self.suffix)
         self._fns: dict[str, object] = {}
+        self._chunk = None
 
     _fn = SequenceKernels._fn
     _flag = SequenceKernels._flag
@@ -957,11 +982,20 @@ class MixKernels:
         applied on reading); decay float32 [H]; state float32 [slots, H, dk, dv] (read and advanced); o float32 [T, H dv]."""
         if tuple(state.shape[1:]) != (n_heads, dk, dv) or tuple(o.shape) != (proj.shape[0], n_heads * dv):
             raise KernelError(f"lin_attn_decay shapes: state {tuple(state.shape)}, o {tuple(o.shape)}")
+        if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.LIN_MIN_ROWS and dk <= ChunkKernels.CHUNK:
+            self.chunk.lin_attn(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
+            return
         _check(self._fn("lin_attn_decay")(
             _ptr(proj, self.dtype, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
             _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)),
             c_int(n_heads), c_int(dk), c_int(dv), c_int(ctx.engine.sm_count), _stream()), "lin_attn_decay")
+
+    @property
+    def chunk(self) -> "ChunkKernels":
+        if self._chunk is None:
+            self._chunk = ChunkKernels()
+        return self._chunk
 
     def gated_row_rms(self, o, gate, weight, y, eps, gate_act: str):
         _check(self._fn("gated_row_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), c_int(gate.stride(0)),

@@ -403,6 +403,40 @@ def test_linear_attention_in_pieces_against_the_recurrence():
     assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
 
 
+@pytest.mark.parametrize("H, D, V, pad", [(2, 128, 128, 0), (3, 24, 40, 0), (1, 64, 200, 8), (2, 50, 70, 3)])
+def test_linear_attention_in_chunks_against_the_recurrence(H, D, V, pad):
+    """Runs of one row to three chunks in one step, from states that are not zero, slots out of order; widths that fill the tiles, that
+    leave them partly empty, and that allow no 16-byte access; decays of 0, 1 and between. Float sums of up to 300 terms in three
+    bfloat16 parts: 1e-5 of the largest element."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k = KernelSet(torch.bfloat16).mix
+    g = torch.Generator().manual_seed(D)
+    lens = [1, 127, 128, 129, 300, 16]
+    T, slots = sum(lens), [5, 0, 3, 1, 6, 2]
+    proj = torch.randn(T, 2 * H * D + H * V + pad, generator=g).bfloat16()
+    decay = torch.tensor([[0.97], [0.0, 1.0], [0.3, 0.995, 1.0]][H - 1])
+    start = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    state0 = torch.randn(len(lens) + 2, H, D, V, generator=g)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(seq_start=torch.from_numpy(start).cuda(), slots=torch.tensor(slots, dtype=torch.int32).cuda(), err_flag=err,
+                          n_seqs=len(lens), max_new=max(lens), engine=SimpleNamespace(sm_count=148))
+    st = state0.clone().cuda()
+    o = torch.full((T, H * V), float("nan"), dtype=torch.float32, device="cuda")
+    k.chunk.lin_attn(proj.cuda(), 0, H * D, 2 * H * D, decay.cuda(), st, ctx, o, H, D, V)
+    q, kk, v = (plain.silu(t).view(T, H, -1) for t in proj[:, :2 * H * D + H * V].double().split([H * D, H * D, H * V], 1))
+    want, after = torch.empty((T, H, V), dtype=torch.float64), state0.double()
+    for b, slot in enumerate(slots):
+        S = state0[slot].double()
+        for t in range(start[b], start[b + 1]):
+            S = decay.double()[:, None, None] * S + kk[t, :, :, None] * v[t, :, None]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        after[slot] = S
+    assert int(err) == 0
+    assert float((o.cpu().double() - want.view(T, -1)).abs().max()) < 1e-5 * float(want.abs().max())
+    assert float((st.cpu().double() - after).abs().max()) < 1e-5 * float(after.abs().max())
+    assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
+
+
 def test_the_norm_adds_a_normed_addend_and_keeps_the_sum():
     from scriptling_llm_lib_b200.csrc.bindings import KernelSet
     for dtype in (torch.float32, torch.bfloat16):
