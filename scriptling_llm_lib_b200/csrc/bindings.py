@@ -1067,6 +1067,14 @@ class MixKernels:
                                          c_int(gate.stride(0) if gate is not None else 0), c_int(mode), _stream()), "latent_expand")
         LAUNCHES[0] += 1
 
+    SCAN_PIECES_MIN_ROWS = 112        # the longest run of a step from which on the selective scan goes in pieces
+
+    @staticmethod
+    def scan_piece_rows(rows: int, inner: int, sm_count: int) -> int:
+        """Rows of a piece: the fewest of 16, 32, 64 with which the blocks (128 channels of a piece) are about one wave, eight an SM;
+        shorter pieces for fewer rows, so that the walk over a piece, which nothing shortens, does not outlast the rest."""
+        return next((r for r in (16, 32) if -(-rows // r) * -(-inner // 128) <= 8 * sm_count), 64)
+
     def selective_scan(self, x, dt_raw, dt_bias, a_log, dskip, bc, b_col, c_col, z, state, ctx, out, inner, n_state):
         """x, z [T, I] views and bc [T, ...] of the element type (B at b_col, C at c_col), dt_raw float32 [T, I],
         dt_bias, a_log [I, N], dskip float32; state float32 [slots, I, N] (read and advanced); out [T, I]."""
@@ -1075,13 +1083,19 @@ class MixKernels:
         for t, name in ((x, "x"), (z, "z"), (bc, "bc"), (out, "out")):
             if t.dtype != self.dtype:
                 raise KernelError(f"selective_scan: {name} has dtype {t.dtype}, expected {self.dtype}")
-        _check(self._fn("selective_scan")(
-            self._view(x, "x"), c_int(x.stride(0)), _ptr(dt_raw, torch.float32, "dt_raw"), c_int(dt_raw.shape[1]),
-            _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"),
-            c_int(1), self._view(bc, "bc"), c_int(bc.stride(0)), c_int(b_col), c_int(c_col), self._view(z, "z"),
-            c_int(z.stride(0)), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), c_int(out.stride(0)), c_int(ctx.n_seqs),
-            c_int(max(1, ctx.max_new)), c_int(inner), c_int(n_state), _stream()), "selective_scan")
+        args = (self._view(x, "x"), c_int(x.stride(0)), _ptr(dt_raw, torch.float32, "dt_raw"), c_int(dt_raw.shape[1]),
+                _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"),
+                c_int(1), self._view(bc, "bc"), c_int(bc.stride(0)), c_int(b_col), c_int(c_col), self._view(z, "z"),
+                c_int(z.stride(0)), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+                _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), c_int(out.stride(0)))
+        tail = (c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)), c_int(inner), c_int(n_state), _stream())
+        if ctx.max_new >= self.SCAN_PIECES_MIN_ROWS and n_state <= 32:
+            T, rows = x.shape[0], self.scan_piece_rows(x.shape[0], inner, ctx.engine.sm_count)
+            n = T // rows + ctx.n_seqs
+            scratch = [torch.empty(shape, dtype=torch.float32, device=x.device) for shape in ((T, inner), (n, n_state, inner), (n, inner))]
+            _check(self._fn("selective_scan_pieces")(*args, *(_ptr(t) for t in scratch), c_int(rows), *tail), "selective_scan_pieces")
+            return
+        _check(self._fn("selective_scan")(*args, *tail), "selective_scan")
 
     ROUTERS = {"grouped_sigmoid": 0, "top_softmax": 1, "grouped_softmax": 2}
 

@@ -990,6 +990,232 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(ScanArgs p) {
   }
 }
 
+// The same over long runs, in pieces of R rows that run side by side: what a piece makes of a state of zeros and the sum of its
+// step sizes (scan_piece), the states in front of the pieces (scan_carry: a piece decays what it is given by exp(A times that
+// sum)), and the pieces' rows again from there with their outputs (scan_write). A thread has a channel with all its states in
+// registers, so a row needs no sums over lanes; B and C of the piece's rows are read from shared memory, the same for all threads.
+// Bound by the exponentials, one a row, channel and state in either walk (30 us a walk of 2,048 rows of 4,096 channels x 16
+// states at the rate of the special-function units alone), and the instructions around them. The first walk leaves the step
+// sizes behind their softplus for the second.
+//
+// A decay is 2^(dt a log2 e) on the special-function unit, whose error (2^-22 of the result at most) is what expf's bound allows as
+// well; states go two at a time through the paired float instructions. 2,048 rows of 4,096 channels x 16 states: 57 + 7 + 82 us
+// (the kernel above, one walk over all rows: 466); with expf instead of its own power of two 90 + 7 + 93. What a piece adds lies
+// channel after channel, so that a warp's accesses are whole lines.
+struct ScanPieces {
+  float* dt;            // [T][I] step sizes
+  float* end;           // [pieces][N][I]: what a piece adds, then the state in front of it
+  float* dt_sum;        // [pieces][I]
+  int R;
+};
+#define MIX_SCAN_BLOCK 128
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 parts_of(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul_pair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t exp2_pair(uint64_t x) {
+  float2 f = parts_of(x);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(f.x));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(f.y));
+  return pair_of(f.x, f.y);
+}
+// A log2 e of channel c's states (0 past the last one), A = -exp(a_log)
+template <int NP>
+__device__ __forceinline__ void scan_rates(uint64_t (&a)[NP / 2], const ScanArgs& p, int c) {
+  float l[NP];
+  const bool fours = p.w_f32 && (p.N & 3) == 0 && ((uintptr_t)p.a_log & 15) == 0;
+#pragma unroll
+  for (int i = 0; i < NP; i += 4) {
+    if (fours) {
+      const float4 q = i < p.N ? *(const float4*)((const float*)p.a_log + (size_t)c * p.N + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      l[i] = q.x; l[i + 1] = q.y; l[i + 2] = q.z; l[i + 3] = q.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) l[i + k] = i + k < p.N ? load_w(p.a_log, p.w_f32, (size_t)c * p.N + i + k) : 0.f;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NP; i += 2)
+    a[i / 2] = pair_of(i < p.N ? -1.4426950408889634f * expf(l[i]) : 0.f, i + 1 < p.N ? -1.4426950408889634f * expf(l[i + 1]) : 0.f);
+}
+// a sequence's pieces lie one behind the other from this one on (two sequences' never meet); at most T / R + sequences of them
+__device__ __forceinline__ size_t scan_first_piece(int start, int b, int R) { return (size_t)(start / R + b); }
+
+// B (and C) of n rows as floats, [row][NP] each, states from N on zero
+template <typename A, int NP, bool WITH_C>
+__device__ __forceinline__ void scan_stage(float* b_s, float* c_s, const ScanArgs& p, int row, int n) {
+  for (int i = threadIdx.x; i < n * NP; i += MIX_SCAN_BLOCK) {
+    const int r = i / NP, s = i % NP;
+    const A* src = (const A*)p.bc + (size_t)(row + r) * p.ldbc;
+    b_s[i] = s < p.N ? to_f32(src[p.b_col + s]) : 0.f;
+    if (WITH_C) c_s[i] = s < p.N ? to_f32(src[p.c_col + s]) : 0.f;
+  }
+}
+
+template <typename A, int NP>
+__global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_piece_kernel(ScanArgs p, ScanPieces w) {
+  extern __shared__ __align__(16) float sm[];
+  const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
+  if (r0 >= len) return;
+  const int n = min(w.R, len - r0), row = start + r0, ch = blockIdx.x * MIX_SCAN_BLOCK + threadIdx.x, c = min(ch, p.I - 1);
+  scan_stage<A, NP, false>(sm, nullptr, p, row, n);
+  uint64_t a[NP / 2], S[NP / 2];
+  scan_rates<NP>(a, p, c);
+#pragma unroll
+  for (int i = 0; i < NP / 2; i++) S[i] = 0ull;
+  const float bias = load_w(p.dt_bias, p.w_f32, c);
+  const float* dtr = p.dt_raw + (size_t)row * p.lddt + c;
+  const A* xs = (const A*)p.x + (size_t)row * p.ldx + c;
+  float* dts = w.dt + (size_t)row * p.I + c;
+  float sum = 0.f;
+  constexpr int U = 4;                   // rows whose loads are on their way together
+  float raw[U], xv[U];
+#pragma unroll
+  for (int k = 0; k < U; k++) { raw[k] = k < n ? dtr[(size_t)k * p.lddt] : 0.f; xv[k] = k < n ? to_f32(xs[(size_t)k * p.ldx]) : 0.f; }
+  __syncthreads();
+  for (int q0 = 0; q0 < n; q0 += U) {
+    float dt[U], dx[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) { dt[k] = softplus_f(raw[k] + bias); dx[k] = dt[k] * xv[k]; }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int r = q0 + U + k;
+      raw[k] = r < n ? dtr[(size_t)r * p.lddt] : 0.f;
+      xv[k] = r < n ? to_f32(xs[(size_t)r * p.ldx]) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int r = q0 + k;
+      if (r >= n) break;
+      if (ch < p.I) dts[(size_t)r * p.I] = dt[k];
+      sum += dt[k];
+      const ulonglong2* br = (const ulonglong2*)(sm + r * NP);
+      const uint64_t dt2 = pair_of(dt[k], dt[k]), dx2 = pair_of(dx[k], dx[k]);
+#pragma unroll
+      for (int i = 0; i < NP / 2; i += 2) {
+        const ulonglong2 bq = br[i / 2];
+        S[i] = fma_pair(exp2_pair(mul_pair(dt2, a[i])), S[i], mul_pair(dx2, bq.x));
+        S[i + 1] = fma_pair(exp2_pair(mul_pair(dt2, a[i + 1])), S[i + 1], mul_pair(dx2, bq.y));
+      }
+    }
+  }
+  if (ch >= p.I) return;
+  const size_t piece = scan_first_piece(start, b, w.R) + blockIdx.y;
+  w.dt_sum[piece * p.I + ch] = sum;
+  float* end = w.end + piece * p.I * p.N + ch;
+#pragma unroll
+  for (int i = 0; i < NP; i += 2) {
+    const float2 f = parts_of(S[i / 2]);
+    if (i < p.N) end[(size_t)i * p.I] = f.x;
+    if (i + 1 < p.N) end[(size_t)(i + 1) * p.I] = f.y;
+  }
+}
+
+// a thread a state of a channel: over the sequence's pieces in order, what a piece adds is replaced by the state in front of it
+__global__ void __launch_bounds__(256) selective_scan_carry_kernel(ScanArgs p, ScanPieces w) {
+  const int b = blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
+  const size_t e = (size_t)blockIdx.x * 256 + threadIdx.x, all = (size_t)p.I * p.N;
+  if (e >= all || len <= 0) return;
+  const int c = (int)(e % p.I), i = (int)(e / p.I), pieces = (len + w.R - 1) / w.R;
+  const size_t first = scan_first_piece(start, b, w.R), at = (size_t)c * p.N + i;
+  const float a = -expf(load_w(p.a_log, p.w_f32, at));
+  float* end = w.end + first * all + e;
+  const float* sums = w.dt_sum + first * p.I + c;
+  float* st = p.state + (size_t)p.slots[b] * all + at;
+  float S = *st;
+  constexpr int U = 8;
+  for (int q0 = 0; q0 < pieces; q0 += U) {
+    float add[U], d[U];
+#pragma unroll
+    for (int k = 0; k < U; k++)
+      if (q0 + k < pieces) { add[k] = end[(q0 + k) * all]; d[k] = sums[(size_t)(q0 + k) * p.I]; }
+#pragma unroll
+    for (int k = 0; k < U; k++)
+      if (q0 + k < pieces) {
+        end[(q0 + k) * all] = S;
+        S = fmaf(expf(d[k] * a), S, add[k]);
+      }
+  }
+  *st = S;
+}
+
+template <typename A, int NP>
+__global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_write_kernel(ScanArgs p, ScanPieces w) {
+  extern __shared__ __align__(16) float sm[];
+  const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
+  if (r0 >= len) return;
+  const int n = min(w.R, len - r0), row = start + r0, ch = blockIdx.x * MIX_SCAN_BLOCK + threadIdx.x, c = min(ch, p.I - 1);
+  float *b_s = sm, *c_s = sm + w.R * NP;
+  scan_stage<A, NP, true>(b_s, c_s, p, row, n);
+  const float* front = w.end + (scan_first_piece(start, b, w.R) + blockIdx.y) * p.I * p.N + c;
+  uint64_t a[NP / 2], S[NP / 2];
+  scan_rates<NP>(a, p, c);
+#pragma unroll
+  for (int i = 0; i < NP; i += 2)
+    S[i / 2] = pair_of(i < p.N ? front[(size_t)i * p.I] : 0.f, i + 1 < p.N ? front[(size_t)(i + 1) * p.I] : 0.f);
+  const float dsk = load_w(p.dskip, p.w_f32, c);
+  const float* dts = w.dt + (size_t)row * p.I + c;
+  const A* xs = (const A*)p.x + (size_t)row * p.ldx + c;
+  const A* zs = (const A*)p.z + (size_t)row * p.ldz + c;
+  A* out = (A*)p.out + (size_t)row * p.ldo + c;
+  constexpr int U = 4;
+  float dtv[U], xv[U], zv[U];
+#pragma unroll
+  for (int k = 0; k < U; k++) {
+    dtv[k] = k < n ? dts[(size_t)k * p.I] : 0.f;
+    xv[k] = k < n ? to_f32(xs[(size_t)k * p.ldx]) : 0.f;
+    zv[k] = k < n ? to_f32(zs[(size_t)k * p.ldz]) : 0.f;
+  }
+  __syncthreads();
+  for (int q0 = 0; q0 < n; q0 += U) {
+    float dt[U], x[U], z[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) { dt[k] = dtv[k]; x[k] = xv[k]; z[k] = zv[k]; }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int r = q0 + U + k;
+      dtv[k] = r < n ? dts[(size_t)r * p.I] : 0.f;
+      xv[k] = r < n ? to_f32(xs[(size_t)r * p.ldx]) : 0.f;
+      zv[k] = r < n ? to_f32(zs[(size_t)r * p.ldz]) : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int r = q0 + k;
+      if (r >= n) break;
+      const float dx = dt[k] * x[k];
+      const ulonglong2 *br = (const ulonglong2*)(b_s + r * NP), *cr = (const ulonglong2*)(c_s + r * NP);
+      const uint64_t dt2 = pair_of(dt[k], dt[k]), dx2 = pair_of(dx, dx);
+      uint64_t acc0 = 0ull, acc1 = 0ull;
+#pragma unroll
+      for (int i = 0; i < NP / 2; i += 2) {
+        const ulonglong2 bq = br[i / 2], cq = cr[i / 2];
+        S[i] = fma_pair(exp2_pair(mul_pair(dt2, a[i])), S[i], mul_pair(dx2, bq.x));
+        S[i + 1] = fma_pair(exp2_pair(mul_pair(dt2, a[i + 1])), S[i + 1], mul_pair(dx2, bq.y));
+        acc0 = fma_pair(S[i], cq.x, acc0);
+        acc1 = fma_pair(S[i + 1], cq.y, acc1);
+      }
+      const float2 f0 = parts_of(acc0), f1 = parts_of(acc1);
+      if (ch < p.I) out[(size_t)r * p.ldo] = from_f32<A>(fmaf(dsk, x[k], (f0.x + f0.y) + (f1.x + f1.y)) * silu_f(z[k]));
+    }
+  }
+}
+
 // ------------------------------------------------------------------ routed experts
 // router: a warp per token. z [T][E] float32 are the router's logits (a product of the library, float32 sums).
 // mode 2: s = softmax(z + bias) over all experts; runs of experts as in mode 0 but a run is rated by its best s alone; the

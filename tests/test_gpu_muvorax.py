@@ -403,6 +403,45 @@ def test_linear_attention_in_pieces_against_the_recurrence():
     assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("inner, N, lens", [(100, 16, [1, 63, 64, 65, 200]), (256, 5, [300]), (130, 17, [16, 33, 112]), (64, 32, [129, 2]),
+                                            (4096, 1, [2100])])
+def test_selective_scan_in_pieces_against_the_recurrence(dtype, inner, N, lens):
+    """Runs around the pieces' lengths (16, 32 and 64 rows by the size of the step), channels that fill no block, every built number of
+    states and ones between; states that are not zero, slots out of order; some decays near 1, some total. The states, float sums
+    decayed along the run, to 2e-6 sqrt(rows) of the largest; outputs to that and their own rounding."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k = KernelSet(dtype).mix
+    g = torch.Generator().manual_seed(inner + N)
+    T, K, slots = sum(lens), 3, list(range(len(lens)))[::-1]
+    xz = torch.randn(T, 2 * inner, generator=g).to(dtype)
+    bc = torch.randn(T, K + 2 * N, generator=g).to(dtype)
+    raw = torch.randn(T, inner, generator=g) * 2 - 3
+    bias, d = torch.randn(inner, generator=g), torch.randn(inner, generator=g)
+    a_log = torch.randn(inner, N, generator=g) * 2
+    start = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    state0 = torch.randn(len(lens) + 1, inner, N, generator=g)
+    ctx = SimpleNamespace(seq_start=torch.from_numpy(start).cuda(), slots=torch.tensor(slots, dtype=torch.int32).cuda(),
+                          n_seqs=len(lens), max_new=max(lens), engine=SimpleNamespace(sm_count=148))
+    assert max(lens) >= k.SCAN_PIECES_MIN_ROWS
+    st, xd = state0.clone().cuda(), xz.cuda()
+    out = torch.full((T, inner), float("nan"), dtype=dtype, device="cuda")
+    k.selective_scan(xd[:, :inner], raw.cuda(), bias.cuda(), a_log.cuda(), d.cuda(), bc.cuda(), K, K + N, xd[:, inner:], st, ctx, out, inner, N)
+    x, z, (_, B, C) = xz[:, :inner].double(), xz[:, inner:].double(), bc.double().split([K, N, N], 1)
+    dt = torch.nn.functional.softplus(raw.double() + bias.double(), threshold=1e9)
+    A, want, after = -torch.exp(a_log.double()), torch.empty(T, inner, dtype=torch.float64), state0.double()
+    for b, slot in enumerate(slots):
+        S = state0[slot].double()
+        for t in range(start[b], start[b + 1]):
+            S = torch.exp(dt[t, :, None] * A) * S + (dt[t] * x[t])[:, None] * B[t]
+            want[t] = (S @ C[t] + d.double() * x[t]) * plain.silu(z[t])
+        after[slot] = S
+    assert float((st.cpu().double() - after).abs().max()) < 2e-6 * max(lens) ** 0.5 * float(after.abs().max())
+    tol = 2e-6 * max(lens) ** 0.5 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+    assert float((out.cpu().double() - want).abs().max()) < tol * float(want.abs().max())
+    assert torch.equal(st[len(lens)].cpu(), state0[len(lens)])          # a slot no sequence of the step holds is left alone
+
+
 @pytest.mark.parametrize("H, D, V, pad", [(2, 128, 128, 0), (3, 24, 40, 0), (1, 64, 200, 8), (2, 50, 70, 3)])
 def test_linear_attention_in_chunks_against_the_recurrence(H, D, V, pad):
     """Runs of one row to three chunks in one step, from states that are not zero, slots out of order; widths that fill the tiles, that
