@@ -772,6 +772,13 @@ class SequenceKernels:
         self.dtype, self.suffix = dtype, _SUFFIX[dtype]
         self.lib = load_library("seq_" + self.suffix)
         self._fns: dict[str, object] = {}
+        self._chunk = None
+
+    @property
+    def chunk(self) -> "ChunkKernels":
+        if self._chunk is None:
+            self._chunk = ChunkKernels()
+        return self._chunk
 
     def _fn(self, name):
         fn = self._fns.get(name)
@@ -876,6 +883,9 @@ class SequenceKernels:
             raise KernelError(f"delta_rule: bd is {tuple(bd.shape)}, expected {(qk.shape[0], 2 * n_heads + n_kv)}")
         if qk.dtype != torch.float32 or v.dtype != torch.float32 or tuple(state.shape[1:]) != (n_heads, dk, dv):
             raise KernelError("delta_rule works on float32 queries, keys, values and state [slots, heads, dk, dv]")
+        if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.DELTA_MIN_ROWS and max(dk, dv) <= ChunkKernels.CHUNK:
+            self.chunk.delta(qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv)
+            return
         _check(self._fn("delta_rule")(self._view(qk, "qk"), c_int(qk.stride(0)), self._view(v, "v"), c_int(v.stride(0)),
                                       _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"),
                                       _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
@@ -916,10 +926,23 @@ class ChunkKernels:
     # in chunks and 40 in pieces of 32 rows (lin_attn_decay), 64 rows 37 and 26; a piece more is 8 us more, a chunk more is nothing
     # while there are idle SMs.
     LIN_MIN_ROWS = 144
+    # The same for the gated delta rule. One sequence, 16 heads of 128 x 128: 192 rows take 66 us in chunks and 70 walked row by row.
+    DELTA_MIN_ROWS = 192
 
     def __init__(self):
         self.lib = load_library("chunk_tcgen05")
-        self.lib.sllm_chunk_lin_attn_bf16.restype = c_int
+        self.lib.sllm_chunk_lin_attn_bf16.restype = self.lib.sllm_chunk_delta.restype = c_int
+
+    def delta(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
+        """As `SequenceKernels.delta_rule`, keys and values up to 128 wide."""
+        n = qk.shape[0] // self.CHUNK + ctx.n_seqs
+        scratch = torch.empty((n * n_heads * self.lib.sllm_chunk_delta_scratch(),), dtype=torch.uint8, device=o.device)
+        _check(self.lib.sllm_chunk_delta(
+            SequenceKernels._view(qk, "qk"), c_int(qk.stride(0)), SequenceKernels._view(v, "v"), c_int(v.stride(0)),
+            _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
+            c_int(ctx.max_new), c_int(n_heads), c_int(n_kv), c_int(dk), c_int(dv),
+            _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "chunk_delta")
 
     def lin_attn(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
         """As `MixKernels.lin_attn_decay`, keys up to 128 wide."""
@@ -991,11 +1014,7 @@ class MixKernels:
             _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)),
             c_int(n_heads), c_int(dk), c_int(dv), c_int(ctx.engine.sm_count), _stream()), "lin_attn_decay")
 
-    @property
-    def chunk(self) -> "ChunkKernels":
-        if self._chunk is None:
-            self._chunk = ChunkKernels()
-        return self._chunk
+    chunk = SequenceKernels.chunk
 
     def gated_row_rms(self, o, gate, weight, y, eps, gate_act: str):
         _check(self._fn("gated_row_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), c_int(gate.stride(0)),

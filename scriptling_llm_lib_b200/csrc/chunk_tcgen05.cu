@@ -14,6 +14,15 @@
 // loads or a product (256 threads a block: 155 + 84 us instead of 79 + 39). 3,001 rows, 16 heads of 128 x 128: 129 us for the
 // three kernels (760 in pieces of 32 rows on the FMA units, one piece after the other); the six products of three parts are
 // 0.29 of them at the tensor cores' rate. Eight sequences, 9,900 rows: 407 us (1,142).
+//
+// The gated delta rule: S_t = d_t S_{t-1} + k_t u_t^T with u_t = b_t (v_t - d_t S_{t-1}^T k_t), o_t = S_t^T q_t. With c_i the sum of
+// log d over a chunk's rows up to and with i, the rows' corrections of one another are a triangular system: L_ij = b_i e^(c_i - c_j)
+// (k_i . k_j) for j < i and T = (I + L)^-1 give U = U0 - W S with U0 = T diag(b) V, W = T diag(b e^c) K, S in front of the chunk.
+// With P_ij = e^(c_i - c_j) (q_i . k_j) for j <= i and K' = diag(e^(c_n - c)) K everything a chunk does is linear in S:
+//   O = (diag(e^c) Q - P W) S + P U0,      S <- (e^(c_n) I - K'^T W) S + K'^T U0 = M S + N.
+//   chunk_delta_parts   the four matrices of every chunk, side by side (they do not know S)
+//   chunk_delta_pass    S through the chunks one after the other, 32 of its columns a block
+//   chunk_delta_out     every chunk's outputs from the S in front of it
 #include "split_mma.cuh"
 
 namespace chunked {
@@ -293,6 +302,528 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   u.close(p.err);
 }
 
+// ------------------------------------------------------------------ the gated delta rule
+struct DeltaArgs {
+  const float* qk; int ld_qk;                         // rows [G dk queries | G dk keys]
+  const float* v; int ld_v;                           // [T][H dv]
+  const float* bd;                                    // [T][2 H + G]: b | d | (not read here)
+  float* state;                                       // [slots][H][dk][dv]
+  const int* seq_start; const int* slots;
+  uint8_t* m;                                         // [chunks][H]: M as the three planes of a tile
+  float *n, *qp, *o0;                                 // [chunks][H][32][128][4] each (see `quad`); n becomes the state in front of the chunk
+  float* o;                                           // [T][H dv]
+  int H, G, dk, dv;
+  int* err;
+};
+constexpr size_t MAT = (size_t)Q * Q;
+constexpr int LT = Q + 4;                             // padded row of a float matrix in shared memory
+constexpr uint32_t DELTA_SMEM = 2 * TILE_BYTES + 6 * Q * 4 + 16 + 1024;
+
+// A matrix that only these kernels read lies four columns at a time, all rows of a four side by side: a thread that has a row
+// (its lane of tensor memory) writes 16 bytes next to its neighbour's. Columns c (a multiple of 4) to c + 3 of row i:
+__device__ __forceinline__ size_t quad(int i, int c) { return ((size_t)(c >> 2) * Q + i) * 4; }
+__device__ __forceinline__ float4 four(const uint32_t (&v)[32], int k) {
+  return make_float4(__uint_as_float(v[k]), __uint_as_float(v[k + 1]), __uint_as_float(v[k + 2]), __uint_as_float(v[k + 3]));
+}
+__device__ __forceinline__ void store_quads(float* mat, int i, int c0, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) *(float4*)(mat + quad(i, c0 + k)) = four(v, k);
+}
+// such a matrix into a tile's planes: neighbouring threads have neighbouring rows
+__device__ __forceinline__ void fetch_quads(float (&f)[PIECES][8], const float* mat) {
+#pragma unroll
+  for (int u = 0; u < PIECES; u++) {
+    const int r = threadIdx.x & (Q - 1), c = ((threadIdx.x >> 7) + u * (NT >> 7)) * 8;
+    const float4 a = *(const float4*)(mat + quad(r, c)), b = *(const float4*)(mat + quad(r, c + 4));
+    f[u][0] = a.x; f[u][1] = a.y; f[u][2] = a.z; f[u][3] = a.w; f[u][4] = b.x; f[u][5] = b.y; f[u][6] = b.z; f[u][7] = b.w;
+  }
+}
+__device__ __forceinline__ void put_quads(uint8_t* tile, const float (&f)[PIECES][8]) {
+#pragma unroll
+  for (int u = 0; u < PIECES; u++) put8(tile, threadIdx.x & (Q - 1), ((threadIdx.x >> 7) + u * (NT >> 7)) * 8, f[u]);
+}
+// This thread's pieces of a float matrix of whole rows; rows from n and columns from `cols` on are zero. Fetching apart from what
+// follows, so that the loads are under way while a product runs.
+template <bool VEC>
+__device__ __forceinline__ void fetch_rows(float (&f)[PIECES][8], const float* src, size_t ld, int n, int cols) {
+#pragma unroll
+  for (int u = 0; u < PIECES; u++) {
+    const int i = u * NT + threadIdx.x, r = i >> 4, c = (i & 15) * 8;
+#pragma unroll
+    for (int k = 0; k < 8; k++) f[u][k] = 0.f;
+    if (r >= n || c >= cols) continue;
+    const float* p = src + (size_t)r * ld + c;
+    if constexpr (VEC) {
+      const float4 a = *(const float4*)p, b = *(const float4*)(p + 4);
+      f[u][0] = a.x; f[u][1] = a.y; f[u][2] = a.z; f[u][3] = a.w; f[u][4] = b.x; f[u][5] = b.y; f[u][6] = b.z; f[u][7] = b.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (c + k < cols) f[u][k] = p[k];
+    }
+  }
+}
+// the pieces, row r times scale[r], into the tile's planes
+template <bool SCALED>
+__device__ __forceinline__ void put_rows(uint8_t* tile, float (&f)[PIECES][8], const float* scale) {
+#pragma unroll
+  for (int u = 0; u < PIECES; u++) {
+    const int i = u * NT + threadIdx.x, r = i >> 4;
+    if constexpr (SCALED) {
+      const float w = scale[r];
+#pragma unroll
+      for (int k = 0; k < 8; k++) f[u][k] *= w;
+    }
+    put8(tile, r, (i & 15) * 8, f[u]);
+  }
+}
+// this thread's 32 floats of row i from column c0 on into a tile's planes
+__device__ __forceinline__ void put_lane(uint8_t* tile, int i, int c0, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int k = 0; k < 32; k += 8) {
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) f[e] = __uint_as_float(v[k + e]);
+    put8(tile, i, c0 + k, f);
+  }
+}
+// the same into three planes of 64 columns of tensor memory (an A operand)
+__device__ __forceinline__ void put_tmem(uint32_t t_lane, int c0, const uint32_t (&v)[32]) {
+  uint32_t part[3][16];
+#pragma unroll
+  for (int k = 0; k < 16; k++)
+    split_pair(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]), part[0][k], part[1][k], part[2][k]);
+#pragma unroll
+  for (int q = 0; q < 3; q++) tmem_st16(t_lane + q * 64 + c0 / 2, part[q]);
+}
+// the same into a float matrix in shared memory, and whole rows of that to memory
+__device__ __forceinline__ void stage_lane(float* t, int i, int c0, const uint32_t (&v)[32]) {
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) *(float4*)(t + i * LT + c0 + k) = four(v, k);
+}
+template <bool VEC>
+__device__ __forceinline__ void write_rows(const float* t, float* dst, size_t ld, int n, int cols) {
+  const int c = (threadIdx.x & 31) * 4;
+#pragma unroll 1
+  for (int r = threadIdx.x >> 5; r < n; r += NT / 32) {
+    const float4 f = *(const float4*)(t + r * LT + c);
+    float* d = dst + (size_t)r * ld + c;
+    if constexpr (VEC) {
+      if (c < cols) *(float4*)d = f;
+    } else {
+      if (c < cols) d[0] = f.x;
+      if (c + 1 < cols) d[1] = f.y;
+      if (c + 2 < cols) d[2] = f.z;
+      if (c + 3 < cols) d[3] = f.w;
+    }
+  }
+}
+__device__ __forceinline__ void take(uint32_t t_addr, uint32_t (&v)[32]) {
+  tmem_ld32(t_addr, v);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// One level of the inversion: pairs of neighbouring S x S blocks on the diagonal that are inverted already, T11 and T22, and L21
+// below the first become -T22 L21 T11 there. A warp has 16 x 16 elements of one pair's block, split on their way out of shared
+// memory; blocks this small would leave tcgen05's 128 rows empty, and on the FMA units their operands' reads from shared memory
+// took 24,000 of a block's 85,000 cycles (16,000 so).
+template <int S>
+__device__ __forceinline__ void merge_level(float* t) {
+  constexpr int SIDE = S / 16, TILES = SIDE * SIDE * (64 / S);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = (lane & 3) * 2;
+  const int o = warp / (SIDE * SIDE) * 2 * S, i0 = warp % (SIDE * SIDE) / SIDE * 16, j0 = warp % SIDE * 16;
+  const float *t11 = t + o * LT + o, *t22 = t + (o + S) * LT + o + S;
+  float* l21 = t + (o + S) * LT + o;
+#pragma unroll 1
+  for (int side = 0; side < 2; side++) {             // first L21 T11, then T22 times that
+    float acc[2][4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[0][e] = acc[1][e] = 0.f;
+    if (warp < TILES) {
+      const float *lhs = (side ? t22 : l21) + (i0 + g) * LT, *rhs = (side ? l21 : t11) + j0 + g;
+#pragma unroll 1
+      for (int k = 0; k < S; k += 16) {
+        uint32_t a[3][4], b[2][3][2];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float2 f = *(const float2*)(lhs + (e & 1) * 8 * LT + k + (e >> 1) * 8 + q);
+          split_pair(f.x, f.y, a[0][e], a[1][e], a[2][e]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const float* r = rhs + (k + e * 8 + q) * LT + n * 8;
+            split_pair(r[0], r[LT], b[n][0][e], b[n][1][e], b[n][2][e]);
+          }
+#pragma unroll
+        for (int n = 0; n < 2; n++) {
+          mma_bf16(acc[n], a[2], b[n][0]);
+          mma_bf16(acc[n], a[0], b[n][2]);
+          mma_bf16(acc[n], a[1], b[n][1]);
+          mma_bf16(acc[n], a[1], b[n][0]);
+          mma_bf16(acc[n], a[0], b[n][1]);
+          mma_bf16(acc[n], a[0], b[n][0]);
+        }
+      }
+    }
+    __syncthreads();
+    if (warp < TILES) {
+      const float sign = side ? -1.f : 1.f;
+#pragma unroll
+      for (int n = 0; n < 2; n++) {
+        float* d = l21 + (i0 + g) * LT + j0 + n * 8 + q;
+        *(float2*)d = make_float2(sign * acc[n][0], sign * acc[n][1]);
+        *(float2*)(d + 8 * LT) = make_float2(sign * acc[n][2], sign * acc[n][3]);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Tensor memory: k k^T in columns 0-127 and q k^T in 128-255, later T in three planes 0-191 and P in 192-383; sums in 384-511 (and,
+// once T is done with, in 0-127). VEC: 16-byte accesses are allowed everywhere.
+template <bool VEC>
+__global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
+  if (r0 >= len) return;
+  uint8_t* xa = aligned_smem(smem_raw);            // keys, then K', then M
+  uint8_t* ya = xa + TILE_BYTES;                   // queries, L and T as floats, scaled values, U0, scaled keys, W, scaled queries as floats
+  float* t = (float*)ya;
+  float *hi = (float*)(ya + TILE_BYTES), *lo = hi + Q, *beta = lo + Q, *front = beta + Q, *back = front + Q, *bfront = back + Q;
+  __shared__ double part_s[4];
+  const int n = min(Q, len - r0), row = start + r0, h = blockIdx.y, g = h / (p.H / p.G);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* qrow = p.qk + (size_t)row * p.ld_qk + (size_t)g * p.dk;
+  const float* krow = qrow + (size_t)p.G * p.dk;
+  const float* vrow = p.v + (size_t)row * p.ld_v + (size_t)h * p.dv;
+  float f[PIECES][8];
+  fetch_rows<VEC>(f, krow, p.ld_qk, n, p.dk);
+  Unit u;
+  u.open((uint8_t*)(bfront + Q));
+  // a thread a row: the running sum of log2 d, in double; a decay of 0 is far below what a float can hold from one row to the next
+  double c = 0.0;
+  float bt = 0.f;
+  if (tid < Q) {
+    if (tid < n) {
+      const float* e = p.bd + (size_t)(row + tid) * (2 * p.H + p.G) + h;
+      bt = e[0];
+      c = fmax(log2((double)e[p.H]), -1000.0);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double w = __shfl_up_sync(0xffffffffu, c, o);
+      if (lane >= o) c += w;
+    }
+    if (lane == 31) part_s[warp] = c;
+  }
+  put_rows<false>(xa, f, nullptr);
+  u.ready();
+  const int dsteps = (p.dk + 15) / 16;
+  if (tid == 0) {
+    product<false, false>(u.tmem, smem_u32(xa), smem_u32(xa), dsteps);
+    u.commit();
+  }
+  fetch_rows<VEC>(f, qrow, p.ld_qk, n, p.dk);
+  double last = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (k < warp && tid < Q) c += part_s[k];
+    last += part_s[k];
+  }
+  if (tid < Q) {
+    const float ch = (float)c;
+    hi[tid] = ch;
+    lo[tid] = (float)(c - (double)ch);
+    beta[tid] = bt;
+    front[tid] = exp2f(ch);
+    back[tid] = exp2f((float)(last - c));
+    bfront[tid] = bt * exp2f(ch);
+  }
+  const float whole = exp2f((float)last);
+  put_rows<false>(ya, f, nullptr);
+  u.done();
+  u.ready();
+  if (tid == 0) {
+    product<false, false>(u.tmem + 128, smem_u32(ya), smem_u32(xa), dsteps);
+    u.commit();
+  }
+  fetch_rows<VEC>(f, krow, p.ld_qk, n, p.dk);
+  u.done();
+  put_rows<true>(xa, f, back);
+  const int i = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;       // a warp has 32 rows (lanes) and 32 columns
+  const uint32_t t_lane = u.tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  {
+    uint32_t s1[32], s2[32];
+    tmem_ld32(t_lane + c0, s1);
+    take(t_lane + 128 + c0, s2);
+    const float hii = hi[i], loi = lo[i], bi = beta[i];
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+      const int j = c0 + k;
+      const float e = j <= i ? exp2f((hii - hi[j]) + (loi - lo[j])) : 0.f;
+      s2[k] = __float_as_uint(j <= i ? e * __uint_as_float(s2[k]) : 0.f);
+      s1[k] = __float_as_uint(j < i ? bi * (e * __uint_as_float(s1[k])) : 0.f);
+    }
+    stage_lane(t, i, c0, s1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();                               // every warp holds its scores: P may go over them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    put_tmem(t_lane + 192, c0, s2);
+  }
+  // T = (I + L)^-1 in place: 16 x 16 blocks on the diagonal, a thread a column, then neighbours merged three times
+  if (tid < Q) {
+    float* d = t + (tid & ~15) * LT + (tid & ~15);
+    const int j = tid & 15;
+    float x[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; k++)
+        if (k < r) acc = fmaf(d[r * LT + k], x[k], acc);
+      x[r] = r == j ? 1.f : -acc;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 16; r++) d[r * LT + j] = r < j ? 0.f : x[r];
+  }
+  __syncthreads();
+  merge_level<16>(t);
+  merge_level<32>(t);
+  fetch_rows<VEC>(f, vrow, p.ld_v, n, p.dv);
+  merge_level<64>(t);
+  uint32_t w[32];
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const float4 e = *(const float4*)(t + i * LT + c0 + k);
+    w[k] = __float_as_uint(e.x); w[k + 1] = __float_as_uint(e.y); w[k + 2] = __float_as_uint(e.z); w[k + 3] = __float_as_uint(e.w);
+  }
+  put_tmem(t_lane, c0, w);
+  __syncthreads();                                 // T has been read from where the scaled values go
+  const size_t unit = (first_chunk(start, b) + blockIdx.x) * p.H + h, mat = unit * MAT;
+  put_rows<true>(ya, f, beta);
+  u.ready();
+  if (tid == 0) {                                  // U0
+    product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
+    u.commit();
+  }
+  u.done();
+  take(t_lane + 384 + c0, w);
+  put_lane(ya, i, c0, w);
+  u.ready();
+  if (tid == 0) {                                  // P U0
+    product_ta<true>(u.tmem + 384, u.tmem + 192, smem_u32(ya), 8);
+    u.commit();
+  }
+  fetch_rows<VEC>(f, krow, p.ld_qk, n, p.dk);
+  u.done();
+  take(t_lane + 384 + c0, w);
+  u.ready();                                       // the sums have been read
+  if (tid == 0) {                                  // K'^T U0
+    product<true, true>(u.tmem + 384, smem_u32(xa), smem_u32(ya), 8);
+    u.commit();
+  }
+  store_quads(p.o0 + mat, i, c0, w);
+  u.done();
+  put_rows<true>(ya, f, bfront);
+  take(t_lane + 384 + c0, w);
+  u.ready();
+  if (tid == 0) {                                  // W
+    product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
+    u.commit();
+  }
+  store_quads(p.n + mat, i, c0, w);
+  u.done();
+  take(t_lane + 384 + c0, w);
+  put_lane(ya, i, c0, w);
+  u.ready();
+  if (tid == 0) {                                  // P W and K'^T W
+    product_ta<true>(u.tmem + 384, u.tmem + 192, smem_u32(ya), 8);
+    product<true, true>(u.tmem, smem_u32(xa), smem_u32(ya), 8);
+    u.commit();
+  }
+  fetch_rows<VEC>(f, qrow, p.ld_qk, n, p.dk);
+  u.done();
+#pragma unroll
+  for (int k = 0; k < PIECES; k++) {               // diag(e^c) Q, from whole rows to a row a thread
+    const int e = k * NT + tid, r = e >> 4, cc = (e & 15) * 8;
+    const float fr = front[r];
+    *(float4*)(t + r * LT + cc) = make_float4(fr * f[k][0], fr * f[k][1], fr * f[k][2], fr * f[k][3]);
+    *(float4*)(t + r * LT + cc + 4) = make_float4(fr * f[k][4], fr * f[k][5], fr * f[k][6], fr * f[k][7]);
+  }
+  take(t_lane + c0, w);
+#pragma unroll
+  for (int k = 0; k < 32; k++) w[k] = __float_as_uint((i == c0 + k ? whole : 0.f) - __uint_as_float(w[k]));
+  put_lane(xa, i, c0, w);
+  u.ready();
+  if (tid == 0) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(p.m + unit * TILE_BYTES), "r"(smem_u32(xa)), "r"(TILE_BYTES) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  take(t_lane + 384 + c0, w);
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const float4 e = *(const float4*)(t + i * LT + c0 + k);
+    w[k] = __float_as_uint(e.x - __uint_as_float(w[k]));
+    w[k + 1] = __float_as_uint(e.y - __uint_as_float(w[k + 1]));
+    w[k + 2] = __float_as_uint(e.z - __uint_as_float(w[k + 2]));
+    w[k + 3] = __float_as_uint(e.w - __uint_as_float(w[k + 3]));
+  }
+  store_quads(p.qp + mat, i, c0, w);
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  u.close(p.err);
+}
+
+// S <- M S + N through a sequence's chunks for 32 columns of a head's state. A thread has a row of 16 columns in registers; their
+// three planes, S^T, are the product's second operand (32 rows, two blocks of 64 columns), M's planes come by bulk copies two chunks
+// ahead. Bound by the chain of a chunk: split, product (48 steps that read 4 KB of M each), sums back to registers. On the FMA
+// units, 16 columns a block, reading M from shared memory took 73 us where this takes 50 (16 chunks).
+constexpr int PV = 32;
+constexpr uint32_t ST_BLOCK = PV * 128, ST_PLANE = 2 * ST_BLOCK, PASS_SMEM = 2 * TILE_BYTES + 3 * ST_PLANE + 32 + 1024;
+__global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ma = aligned_smem(smem_raw);
+  uint8_t* sa = ma + 2 * TILE_BYTES;
+  uint8_t* head = sa + 3 * ST_PLANE;
+  const int b = blockIdx.z, h = blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
+  if (len <= 0) return;
+  const int chunks = (len + Q - 1) / Q, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int d = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16, v0 = blockIdx.x * PV + j0;
+  const size_t first = first_chunk(start, b) * p.H + h;
+  float* st = p.state + (((size_t)p.slots[b] * p.H + h) * p.dk + d) * p.dv + v0;
+  float* nm = p.n + first * MAT + quad(d, v0);      // columns v0 .. v0 + 15: fours Q * 4 floats apart
+  const size_t stride = (size_t)p.H * MAT;
+  const uint32_t full = smem_u32(head + 16);        // two barriers of M's copies
+  if (tid == 0) { mbar_init(full, 1); mbar_init(full + 8, 1); }
+  Unit u;
+  u.open(head);
+  auto fetch_m = [&](int c) {
+    const uint32_t bar = full + 8 * (c & 1);
+    mbar_expect_tx(bar, TILE_BYTES);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(ma + (c & 1) * TILE_BYTES)), "l"(p.m + (first + (size_t)c * p.H) * TILE_BYTES), "r"(TILE_BYTES), "r"(bar) : "memory");
+  };
+  if (tid == 0) {
+    fetch_m(0);
+    if (chunks > 1) fetch_m(1);
+  }
+  float own[16];
+  float4 add[4];
+#pragma unroll
+  for (int e = 0; e < 16; e++) own[e] = d < p.dk && v0 + e < p.dv ? st[e] : 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; e++) add[e] = *(const float4*)(nm + e * Q * 4);
+  constexpr uint32_t id = umma_idesc_bf16(128, PV);
+  int fetched = min(chunks, 2);                     // copies of M asked for (thread 0's count)
+  for (int c = 0; c < chunks; c++) {
+    float* nc = nm + c * stride;
+    uint8_t* row = sa + (d >> 6) * ST_BLOCK + (d & 7) * 2;
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+      const int j = j0 + e;
+      uint32_t q[3];
+      split_pair(own[e], own[e + 1], q[0], q[1], q[2]);
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        *(uint16_t*)(row + k * ST_PLANE + j * 128 + ((((d >> 3) & 7) ^ (j & 7)) << 4)) = (uint16_t)q[k];
+        *(uint16_t*)(row + k * ST_PLANE + (j + 1) * 128 + ((((d >> 3) & 7) ^ ((j + 1) & 7)) << 4)) = (uint16_t)(q[k] >> 16);
+      }
+    }
+    u.ready();
+    if (tid == 0) {
+      if (!mbar_wait(full + 8 * (c & 1), (c >> 1) & 1, u.abort)) u.ok = false;
+      const uint32_t m = smem_u32(ma + (c & 1) * TILE_BYTES), s = smem_u32(sa);
+#pragma unroll 1
+      for (int t = 0; t < 6; t++) {
+        const uint32_t pa = m + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = s + (TERM_B >> 2 * t & 3) * ST_PLANE;
+#pragma unroll 2
+        for (int k = 0; k < 8; k++)
+          umma_bf16(u.tmem, desc_cols(pa, k), umma_desc_sw128(pb + (k >> 2) * ST_BLOCK + (k & 3) * 32), id, (t | k) ? 1u : 0u);
+      }
+      u.commit();
+    }
+    float4 next[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      next[e] = c + 1 < chunks ? *(const float4*)(nc + stride + e * Q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *(float4*)(nc + e * Q * 4) = make_float4(own[4 * e], own[4 * e + 1], own[4 * e + 2], own[4 * e + 3]);      // the state in front of the chunk
+    }
+    u.done();
+    if (tid == 0 && c + 2 < chunks && u.ok) {
+      fetch_m(c + 2);
+      fetched = c + 3;
+    }
+    uint32_t w[16];
+    tmem_ld16(u.tmem + ((uint32_t)((warp & 3) * 32) << 16) + j0, w);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      own[4 * e] = __uint_as_float(w[4 * e]) + add[e].x;
+      own[4 * e + 1] = __uint_as_float(w[4 * e + 1]) + add[e].y;
+      own[4 * e + 2] = __uint_as_float(w[4 * e + 2]) + add[e].z;
+      own[4 * e + 3] = __uint_as_float(w[4 * e + 3]) + add[e].w;
+      add[e] = next[e];
+    }
+  }
+  if (tid == 0 && !u.ok) {                           // a wait was given up: let the copies that are under way land
+    volatile int never = 0;
+    for (int c = max(0, fetched - 2); c < fetched; c++) mbar_wait(full + 8 * (c & 1), (c >> 1) & 1, &never);
+  }
+#pragma unroll
+  for (int e = 0; e < 16; e++)
+    if (d < p.dk && v0 + e < p.dv) st[e] = own[e];
+  u.close(p.err);
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(NT, 1) chunk_delta_out_kernel(DeltaArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
+  if (r0 >= len) return;
+  uint8_t* xa = aligned_smem(smem_raw);
+  uint8_t* ya = xa + TILE_BYTES;
+  const int n = min(Q, len - r0), h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t mat = ((first_chunk(start, b) + blockIdx.x) * p.H + h) * MAT;
+  float fq[PIECES][8], fs[PIECES][8];
+  fetch_quads(fq, p.qp + mat);
+  fetch_quads(fs, p.n + mat);
+  Unit u;
+  u.open(ya + TILE_BYTES);
+  put_quads(xa, fq);
+  put_quads(ya, fs);
+  u.ready();
+  if (threadIdx.x == 0) {
+    product<false, true>(u.tmem, smem_u32(xa), smem_u32(ya), (p.dk + 15) / 16);
+    u.commit();
+  }
+  const int i = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
+  float4 f[8];
+#pragma unroll
+  for (int k = 0; k < 8; k++) f[k] = *(const float4*)(p.o0 + mat + quad(i, c0 + 4 * k));
+  u.done();
+  uint32_t w[32];
+  take(u.tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0, w);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    w[4 * k] = __float_as_uint(__uint_as_float(w[4 * k]) + f[k].x);
+    w[4 * k + 1] = __float_as_uint(__uint_as_float(w[4 * k + 1]) + f[k].y);
+    w[4 * k + 2] = __float_as_uint(__uint_as_float(w[4 * k + 2]) + f[k].z);
+    w[4 * k + 3] = __float_as_uint(__uint_as_float(w[4 * k + 3]) + f[k].w);
+  }
+  float* t = (float*)xa;
+  stage_lane(t, i, c0, w);
+  __syncthreads();
+  write_rows<VEC>(t, p.o + ((size_t)(start + r0) * p.H + h) * p.dv, (size_t)p.H * p.dv, n, p.dv);
+  u.close(p.err);
+}
+
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t smem) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -319,5 +850,32 @@ SLLM_EXPORT int sllm_chunk_lin_attn_bf16(const void* proj, int ld, int q_col, in
   if (vec) chunked::chunk_lin_pass_kernel<4><<<dim3((DV / 4 + 255) / 256, H, n_seqs), 256, 0, stream>>>(p);
   else chunked::chunk_lin_pass_kernel<1><<<dim3((DV + 255) / 256, H, n_seqs), 256, 0, stream>>>(p);
   chunked::chunk_lin_scan_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
+  SLLM_RETURN_LAST();
+}
+
+// qk float rows [G dk | G dk], v float rows [H dv], bd float [T, 2 H + G] as the walk takes them; state float [slots][H][dk][dv], read
+// and advanced; scratch: sllm_chunk_delta_scratch() bytes for each head of each of `chunks_held` >= T / 128 + n_seqs chunks, 16-byte
+// aligned; o float [T, H dv]; dk and dv up to 128.
+SLLM_EXPORT int sllm_chunk_delta_scratch(void) { return (int)(chunked::TILE_BYTES + 3 * chunked::MAT * sizeof(float)); }
+SLLM_EXPORT int sllm_chunk_delta(const float* qk, int ld_qk, const float* v, int ld_v, const float* bd, float* state, const int* seq_start,
+                                 const int* slots, void* scratch, long long chunks_held, float* o, int n_seqs, int max_new, int H, int G,
+                                 int dk, int dv, int* err, cudaStream_t stream) {
+  using namespace chunked;
+  if (n_seqs <= 0 || max_new <= 0) return 0;
+  if (H < 1 || G < 1 || H % G || dk < 1 || dk > Q || dv < 1 || dv > Q || n_seqs > 65535 || H > 65535 || ((uintptr_t)scratch & 15)) return SLLM_ERR_ARG;
+  const size_t units = (size_t)chunks_held * H;
+  float* mats = (float*)((uint8_t*)scratch + units * TILE_BYTES);
+  const bool vec = !((ld_qk | ld_v | dk | dv) & 7) && !(((uintptr_t)qk | (uintptr_t)v | (uintptr_t)o) & 15);
+  DeltaArgs p{qk, ld_qk, v, ld_v, bd, state, seq_start, slots, (uint8_t*)scratch, mats, mats + units * MAT, mats + 2 * units * MAT, o, H, G, dk, dv, err};
+  const auto parts = vec ? chunk_delta_parts_kernel<true> : chunk_delta_parts_kernel<false>;
+  const auto out = vec ? chunk_delta_out_kernel<true> : chunk_delta_out_kernel<false>;
+  cudaError_t e = allow_smem(parts, DELTA_SMEM);
+  if (e == cudaSuccess) e = allow_smem(chunk_delta_pass_kernel, PASS_SMEM);
+  if (e == cudaSuccess) e = allow_smem(out, DELTA_SMEM);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid((max_new + Q - 1) / Q, H, n_seqs);
+  parts<<<grid, NT, DELTA_SMEM, stream>>>(p);
+  chunk_delta_pass_kernel<<<dim3((dv + PV - 1) / PV, H, n_seqs), 256, PASS_SMEM, stream>>>(p);
+  out<<<grid, NT, DELTA_SMEM, stream>>>(p);
   SLLM_RETURN_LAST();
 }

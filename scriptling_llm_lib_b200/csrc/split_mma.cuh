@@ -52,33 +52,33 @@ __device__ __forceinline__ uint64_t desc_rows(uint32_t plane, int k) {        //
 __host__ __device__ constexpr uint32_t idesc(bool a_rows, bool b_rows) {
   return umma_idesc_bf16(128, 128) | (a_rows ? 1u << 15 : 0u) | (b_rows ? 1u << 16 : 0u);
 }
-// D = A B (or D += A B), `steps` of 16 deep, both operands tiles in shared memory; one thread issues it
+// planes of the six terms' factors, smallest term first, two bits each
+constexpr uint32_t TERM_A = 2u | 0u << 2 | 1u << 4 | 1u << 6 | 0u << 8 | 0u << 10, TERM_B = 0u | 2u << 2 | 1u << 4 | 0u << 6 | 1u << 8 | 0u << 10;
+// D = A B, `steps` of 16 deep, both operands tiles in shared memory; one thread issues it. The loops stay loops: these kernels run
+// through their code once a block, so code is fetched, not found.
 template <bool A_ROWS, bool B_ROWS>
-__device__ __forceinline__ void product(uint32_t tmem_d, uint32_t a, uint32_t b, int steps, bool add = false) {
+__device__ __forceinline__ void product(uint32_t tmem_d, uint32_t a, uint32_t b, int steps) {
   constexpr uint32_t id = idesc(A_ROWS, B_ROWS);
-#pragma unroll
+#pragma unroll 1
   for (int t = 0; t < 6; t++) {
-    const int pa = t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0, pb = t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0;
-    for (int k = 0; k < steps; k++) {
-      const uint64_t da = A_ROWS ? desc_rows(a + pa * PLANE_BYTES, k) : desc_cols(a + pa * PLANE_BYTES, k);
-      const uint64_t db = B_ROWS ? desc_rows(b + pb * PLANE_BYTES, k) : desc_cols(b + pb * PLANE_BYTES, k);
-      umma_bf16(tmem_d, da, db, id, (add || t > 0 || k > 0) ? 1u : 0u);
-    }
+    const uint32_t pa = a + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
+#pragma unroll 1
+    for (int k = 0; k < steps; k++)
+      umma_bf16(tmem_d, A_ROWS ? desc_rows(pa, k) : desc_cols(pa, k), B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k), id, (t | k) ? 1u : 0u);
   }
 }
 // the same with A in tensor memory: three planes of 64 columns (two bfloat16 of K each)
 template <bool B_ROWS>
 __device__ __forceinline__ void product_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, int steps) {
   constexpr uint32_t id = idesc(false, B_ROWS);
-#pragma unroll
+#pragma unroll 1
   for (int t = 0; t < 6; t++) {
-    const int pa = t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0, pb = t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0;
-    for (int k = 0; k < steps; k++) {
-      const uint64_t db = B_ROWS ? desc_rows(b + pb * PLANE_BYTES, k) : desc_cols(b + pb * PLANE_BYTES, k);
+    const uint32_t pa = tmem_a + (TERM_A >> 2 * t & 3) * 64, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
+#pragma unroll 1
+    for (int k = 0; k < steps; k++)
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                    "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                   ::"r"(tmem_d), "r"(tmem_a + pa * 64 + k * 8), "l"(db), "r"(id), "r"((t > 0 || k > 0) ? 1u : 0u) : "memory");
-    }
+                   ::"r"(tmem_d), "r"(pa + k * 8), "l"(B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k)), "r"(id), "r"((t | k) ? 1u : 0u) : "memory");
   }
 }
 

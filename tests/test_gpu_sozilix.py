@@ -434,6 +434,47 @@ def test_the_delta_rule_forgets_by_its_decay_and_overwrites_along_a_key():
     assert float(state[:2].abs().max()) == 0.0 and float(state[2].abs().max()) > 0
 
 
+@pytest.mark.parametrize("H, G, dk, dv, alike", [(2, 1, 128, 128, 0.0), (3, 3, 24, 40, 3.0), (2, 2, 50, 70, 0.5), (4, 2, 64, 128, 30.0), (1, 1, 128, 8, 1.0)])
+def test_the_delta_rule_in_chunks_against_the_recurrence(H, G, dk, dv, alike):
+    """Runs of one row to three chunks in one step, from states that are not zero, slots out of order; widths that fill the tiles, leave
+    them partly empty, allow no 16-byte access; keys from independent to nearly the same one (`alike`: the part they share), decays
+    of 0, 1 and between. Float sums in three bfloat16 parts through a triangular inverse: 2e-5 of the largest element."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, dev = KernelSet(torch.bfloat16).seq, "cuda:0"
+    g = torch.Generator().manual_seed(dk)
+    lens, slots = [1, 127, 128, 129, 300, 16], [5, 0, 3, 1, 6, 2]
+    T = sum(lens)
+    keys = torch.randn(T, G, dk, generator=g) + alike * torch.randn(1, G, dk, generator=g)
+    q = torch.randn(T, G, dk, generator=g)
+    unit = lambda t: t / t.square().sum(-1, keepdim=True).sqrt()
+    q, keys = unit(q) * dk ** -0.5, unit(keys)
+    wide = torch.randn(T, 2 * G * dk + H * dv, generator=g)
+    wide[:, :2 * G * dk] = torch.cat([q.reshape(T, -1), keys.reshape(T, -1)], 1)
+    beta, decay = torch.rand(T, H, generator=g), torch.rand(T, H, generator=g) ** 0.05
+    beta[::7], decay[::11], decay[5::50] = 1.0, 1.0, 0.0
+    state0 = torch.randn(len(lens) + 2, H, dk, dv, generator=g)
+    st, wd = state0.clone().to(dev), wide.to(dev)
+    o = torch.full((T, H * dv), float("nan"), dtype=torch.float32, device=dev)
+    ctx = _Ctx(lens, slots, dev)
+    ctx.err_flag = torch.zeros(1, dtype=torch.int32, device=dev)
+    bd = torch.cat([beta, decay, (q * keys).sum(-1)], 1).to(dev)
+    k.chunk.delta(wd[:, :2 * G * dk], wd[:, 2 * G * dk:], bd, st, ctx, o, H, G, dk, dv)
+    q, keys = (t.double().repeat_interleave(H // G, 1) for t in (q, keys))
+    v, beta, decay = wide[:, 2 * G * dk:].double().view(T, H, dv), beta.double(), decay.double()
+    want, after, row = torch.empty(T, H, dv, dtype=torch.float64), state0.double(), 0
+    for n, slot in zip(lens, slots):
+        S = state0[slot].double()
+        for t in range(row, row + n):
+            S = S * decay[t, :, None, None]
+            S = S + keys[t, :, :, None] * (beta[t, :, None] * (v[t] - torch.einsum("hdv,hd->hv", S, keys[t])))[:, None]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        after[slot], row = S, row + n
+    assert int(ctx.err_flag) == 0
+    assert float((o.cpu().double() - want.view(T, -1)).abs().max()) < 2e-5 * float(want.abs().max())
+    assert float((st.cpu().double() - after).abs().max()) < 2e-5 * float(after.abs().max())
+    assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
+
+
 # ------------------------------------------------------------------ generation
 @pytest.mark.parametrize("cfg,seed", [(CFG_A, 21), (CFG_B, 22)])
 def test_greedy_generation_through_the_entry_point(tmp_path, cfg, seed):
