@@ -23,6 +23,10 @@
 //   chunk_delta_parts   the four matrices of every chunk, side by side (they do not know S)
 //   chunk_delta_pass    S through the chunks one after the other, 32 of its columns a block
 //   chunk_delta_out     every chunk's outputs from the S in front of it
+// 2,048 rows of 16 heads of 128 x 128: 100 + 50 + 20 us (640 walked row by row, a dependent chain a column of the state); eight
+// sequences, 9,900 rows: 420 + 137 + 103 (1,471). The first kernel is bound by its sixteen warps going through nine tiles and eight
+// products one after the other with nothing beside them on the SM; that its code is fetched once a block shows in it too (with
+// products and the inversion unrolled, and the paths without 16-byte accesses in the same kernel: 130 us, 597 for the eight).
 #include "split_mma.cuh"
 
 namespace chunked {
@@ -740,10 +744,10 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
     if (tid == 0) {
       if (!mbar_wait(full + 8 * (c & 1), (c >> 1) & 1, u.abort)) u.ok = false;
       const uint32_t m = smem_u32(ma + (c & 1) * TILE_BYTES), s = smem_u32(sa);
-#pragma unroll 1
+#pragma unroll
       for (int t = 0; t < 6; t++) {
         const uint32_t pa = m + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = s + (TERM_B >> 2 * t & 3) * ST_PLANE;
-#pragma unroll 2
+#pragma unroll
         for (int k = 0; k < 8; k++)
           umma_bf16(u.tmem, desc_cols(pa, k), umma_desc_sw128(pb + (k >> 2) * ST_BLOCK + (k & 3) * 32), id, (t | k) ? 1u : 0u);
       }

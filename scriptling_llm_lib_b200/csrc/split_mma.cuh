@@ -62,7 +62,7 @@ __device__ __forceinline__ void product(uint32_t tmem_d, uint32_t a, uint32_t b,
 #pragma unroll 1
   for (int t = 0; t < 6; t++) {
     const uint32_t pa = a + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
-#pragma unroll 1
+#pragma unroll 4
     for (int k = 0; k < steps; k++)
       umma_bf16(tmem_d, A_ROWS ? desc_rows(pa, k) : desc_cols(pa, k), B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k), id, (t | k) ? 1u : 0u);
   }
@@ -74,7 +74,7 @@ __device__ __forceinline__ void product_ta(uint32_t tmem_d, uint32_t tmem_a, uin
 #pragma unroll 1
   for (int t = 0; t < 6; t++) {
     const uint32_t pa = tmem_a + (TERM_A >> 2 * t & 3) * 64, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
-#pragma unroll 1
+#pragma unroll 4
     for (int k = 0; k < steps; k++)
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                    "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
