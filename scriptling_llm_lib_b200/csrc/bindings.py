@@ -956,6 +956,21 @@ class ChunkKernels:
             "chunk_lin_attn")
 
 
+class LatentKernels:
+    """Decode attention over a cached latent on mma.sync (bfloat16; see latent_mma.cu): the entries of `MixKernels` with the same
+    names, for widths in multiples of 8, latents up to 512 (576 with the rotated part) and heads of up to 256."""
+    HEADS = 16               # heads a block, and keys a step of its walk
+    KEYS = 64
+
+    def __init__(self):
+        self.lib = load_library("latent_mma")
+        for n in ("takes", "absorb_mma", "attn_mma", "expand_mma"):
+            getattr(self.lib, f"sllm_latent_{n}" if n != "takes" else "sllm_latent_mma_takes").restype = c_int
+
+    def takes(self, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:
+        return bool(self.lib.sllm_latent_mma_takes(dim, rot_dim, v_dim, rank))
+
+
 class MixKernels:
     """Launchers of mix_kernels.cuh: the norm without statistics fused with the residual sum, activations in
     place, linear attention with a decay per head, the gated read-out norm over a row, attention over a cached
@@ -971,7 +986,7 @@ class MixKernels:
         self.dtype, self.suffix = dtype, _SUFFIX[dtype]
         self.lib = load_library("mix_" + self.suffix)
         self._fns: dict[str, object] = {}
-        self._chunk = None
+        self._chunk = self._latent = None
 
     _fn = SequenceKernels._fn
     _flag = SequenceKernels._flag
@@ -1054,17 +1069,37 @@ class MixKernels:
                                         c_int(q.shape[0]), c_int(n_heads), c_int(dim), c_int(rot_dim), c_int(v_dim), c_int(kt.shape[-1]),
                                         c_int(vt.shape[-1]), _stream()), "latent_heads")
 
+    @property
+    def latent(self) -> "LatentKernels | None":
+        """The tensor-core kernels of latent attention's decode form (None in 32-bit)."""
+        if self._latent is None and self.dtype == torch.bfloat16:
+            self._latent = LatentKernels()
+        return self._latent
+
+    def latent_tile(self, dim, rot_dim, v_dim, rank):
+        """(heads a block, keys a step) of the kernel that `latent_attn` runs for these widths."""
+        lat = self.latent
+        return (lat.HEADS, lat.KEYS) if lat is not None and lat.takes(dim, rot_dim, v_dim, rank) else (8, 32)
+
     def latent_absorb(self, q, wuk, qa, n_heads, dim, rot_dim, rank, scale):
         """qa float32 [T, H, rank + rot_dim] = scale * [Wuk_h^T q_h[:dim] | q_h[dim:]] for every head."""
         if q.dtype != self.dtype:
             raise KernelError(f"latent_absorb: q has dtype {q.dtype}, expected {self.dtype}")
+        lat = self.latent
+        if lat is not None and lat.takes(dim, rot_dim, 8, rank) and q.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0:
+            _check(lat.lib.sllm_latent_absorb_mma(self._view(q, "q"), c_int(q.stride(0)), _ptr(wuk, self.dtype, "wuk"),
+                                                  _ptr(qa, torch.float32, "qa"), c_int(q.shape[0]), c_int(n_heads), c_int(dim),
+                                                  c_int(rot_dim), c_int(rank), c_float(scale), _stream()), "latent_absorb_mma")
+            return
         _check(self._fn("latent_absorb")(self._view(q, "q"), c_int(q.stride(0)), _ptr(wuk, self.dtype, "wuk"),
                                          _ptr(qa, torch.float32, "qa"), c_int(q.shape[0]), c_int(n_heads), c_int(dim),
                                          c_int(rot_dim), c_int(rank), c_float(scale), _stream()), "latent_absorb")
 
     def latent_attn(self, qa, pages, ctx, block_table, part, n_heads, rank, rot_dim, n_split, window=0):
         """`window` > 0: a row sees its own position and the window - 1 before it; 0: every earlier one."""
-        _check(self._fn("latent_attn")(
+        lat = self.latent
+        fn = lat.lib.sllm_latent_attn_mma if lat is not None and lat.takes(8, rot_dim, 8, rank) else self._fn("latent_attn")
+        _check(fn(
             _ptr(qa, torch.float32, "qa"), _ptr(pages, self.dtype, "pages"), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
             _ptr(part, torch.float32, "part"), c_int(qa.shape[0]), c_int(n_heads), c_int(rank), c_int(rot_dim), c_int(n_split),
@@ -1079,14 +1114,18 @@ class MixKernels:
             mode = 1 if gate.shape[1] == n_heads else 2
             if gate.dtype != self.dtype or tuple(gate.shape) != (out.shape[0], n_heads * (v_dim if mode == 2 else 1)):
                 raise KernelError(f"latent_expand: gate logits {tuple(gate.shape)} {gate.dtype} for {n_heads} heads of {v_dim}")
-        _check(self._fn("latent_expand")(_ptr(part, torch.float32, "part"), _ptr(olat, torch.float32, "olat"),
+        lat = self.latent
+        fn = lat.lib.sllm_latent_expand_mma if lat is not None and lat.takes(8, 0, v_dim, rank) and n_split <= 64 else self._fn("latent_expand")
+        _check(fn(_ptr(part, torch.float32, "part"), _ptr(olat, torch.float32, "olat"),
                                          _ptr(wuv, self.dtype, "wuv"), _ptr(out, self.dtype, "out"), c_int(out.shape[1]),
                                          c_int(out.shape[0]), c_int(n_heads), c_int(v_dim), c_int(rank), c_int(n_split),
                                          _ptr(sink, torch.float32, "sink"), self._view(gate, "gate") if gate is not None else c_void_p(0),
                                          c_int(gate.stride(0) if gate is not None else 0), c_int(mode), _stream()), "latent_expand")
         LAUNCHES[0] += 1
 
-    SCAN_PIECES_MIN_ROWS = 112        # the longest run of a step from which on the selective scan goes in pieces
+    # The longest run of a step from which on the selective scan goes in pieces. One sequence, 4,096 channels of 16 states: 112 rows
+    # take 24 us in pieces, 64 rows 24 (19 walked row by row), 300 rows 34 (74 walked).
+    SCAN_PIECES_MIN_ROWS = 96
 
     @staticmethod
     def scan_piece_rows(rows: int, inner: int, sm_count: int) -> int:

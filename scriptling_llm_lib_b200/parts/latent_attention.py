@@ -151,12 +151,15 @@ class LatentAttention(Mixer):
         return CacheNeed("window" if self.window else "full", 1, self.R + self.P, self.window, v_dim=0)
 
     def splits(self, ctx, unit) -> int:
-        """Over how many blocks a row's keys are split: one in a prompt step (its rows fill the GPU), in a
-        decode step enough for about two blocks per SM, at most one per 32 keys of the longest sequence."""
+        """Over how many blocks a row's keys are split: one in a prompt step (its rows fill the GPU), in a decode step enough for
+        about two blocks per SM (one of the tensor-core kernel, which fills an SM), at most one per step of the kernel's walk
+        over the longest sequence; no more than it takes to give every split as many steps as the fullest one has."""
         if not ctx.is_decode:
             return 1
-        blocks = ctx.n_seqs * -(-self.H // 8)
-        return max(1, min(-(-2 * ctx.engine.sm_count // blocks), ctx.pages_seen(unit) * PAGE // 32, 64))
+        heads, keys = ctx.kernels.mix.latent_tile(self.D, self.P, self.vw, self.R)
+        blocks, steps = ctx.n_seqs * -(-self.H // heads), ctx.pages_seen(unit) * PAGE // keys
+        n = max(1, min(-(-(2 if heads == 8 else 1) * ctx.engine.sm_count // blocks), steps, 64))
+        return n if heads == 8 else -(-steps // -(-steps // n))
 
     PER_HEAD_MIN_ROWS = 32       # prompts from position 0 with at least this many rows form keys and values per head
 

@@ -403,6 +403,58 @@ def test_linear_attention_in_pieces_against_the_recurrence():
     assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
 
 
+@pytest.mark.parametrize("H, D, P, V, R", [(16, 128, 64, 128, 512), (5, 40, 8, 24, 72), (20, 64, 0, 40, 256), (33, 8, 24, 8, 328), (4, 256, 16, 200, 120)])
+@pytest.mark.parametrize("window, n_split", [(0, 1), (0, 5), (100, 3)])
+def test_latent_decode_on_the_tensor_cores(H, D, P, V, R, window, n_split):
+    """The absorbed queries, scores and sums over the latent, merge and values against the formula, kernel by kernel on what the one
+    before left: one position to several pages, pages scattered, unused rows NaN, heads that leave a block partly empty, splits that
+    get no key, sink and gates. Float sums of products exact in their parts: 2e-6 sqrt(width) of the largest element; values rounded
+    to 8 bits."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k = KernelSet(torch.bfloat16).mix
+    assert k.latent.takes(D, P, V, R) and not k.latent.takes(D, P, V, 520) and not k.latent.takes(D + 4, P, V, R)
+    g = torch.Generator().manual_seed(R + H)
+    lens = [1, 64, 65, 200, 333, 130]
+    B, W = len(lens), R + P
+    need = [-(-n // 64) for n in lens]
+    table = torch.zeros(B, max(need), dtype=torch.int32)
+    order = torch.randperm(sum(need) + 2, generator=g).tolist()
+    pages = torch.full((sum(need) + 2, 1, 64, W), float("nan"))
+    rows = [torch.randn(n, W, generator=g).bfloat16() for n in lens]
+    for b, n in enumerate(lens):
+        for i in range(need[b]):
+            table[b, i] = order.pop()
+            part = rows[b][64 * i:64 * (i + 1)]
+            pages[table[b, i], 0, :len(part)] = part.float()
+    q = torch.randn(B, H * (D + P) + 8, generator=g).bfloat16()
+    wuk, wuv = torch.randn(H * D, R, generator=g).bfloat16(), torch.randn(H * V, R, generator=g).bfloat16()
+    sink, gate = torch.randn(H, generator=g), torch.randn(B, H * V, generator=g).bfloat16()
+    qd, scale = q.cuda()[:, :H * (D + P)], (D + P) ** -0.5 * R ** -0.5
+    qa = torch.full((B, H, W), float("nan"), device="cuda")
+    k.latent_absorb(qd, wuk.cuda(), qa, H, D, P, R, scale)
+    qh = q[:, :H * (D + P)].double().view(B, H, D + P)
+    want = torch.cat([torch.einsum("bhd,hdr->bhr", qh[..., :D], wuk.double().view(H, D, R)), qh[..., D:]], -1) * scale
+    assert float((qa.cpu().double() - want).abs().max()) < 2e-6 * D ** 0.5 * float(want.abs().max())
+    ctx = SimpleNamespace(tok_pos=torch.tensor(lens, dtype=torch.int32).cuda() - 1, tok_seq=torch.arange(B, dtype=torch.int32).cuda())
+    part = torch.full((B, H, n_split, R + 2), float("nan"), device="cuda")
+    k.latent_attn(qa, pages.bfloat16().cuda(), ctx, table.cuda(), part, H, R, P, n_split, window=window)
+    for mode, gt in ((0, None), (1, gate[:, :H]), (2, gate)):
+        out = torch.full((B, H * V), float("nan"), dtype=torch.bfloat16, device="cuda")
+        olat = torch.empty((B, H, R), device="cuda")
+        k.latent_expand(part, olat, wuv.cuda(), out, H, V, R, n_split, sink=sink.cuda() if mode else None, gate=gt.cuda() if mode else None)
+        lat = torch.empty(B, H, R, dtype=torch.float64)
+        for b, n in enumerate(lens):
+            seen = rows[b][max(0, n - window) if window else 0:].double()
+            s = qa[b].cpu().double() @ seen.T
+            w = torch.cat([s, sink.double()[:, None]], 1).softmax(-1)[:, :-1] if mode else s.softmax(-1)
+            lat[b] = w @ seen[:, :R]
+        assert float((olat.cpu().double() - lat).abs().max()) < 2e-6 * W ** 0.5 * float(lat.abs().max())
+        want = torch.einsum("bhr,hvr->bhv", olat.cpu().double(), wuv.double().view(H, V, R))
+        if mode:
+            want = want * torch.sigmoid(gt.double()).view(B, H, -1)
+        assert float((out.cpu().double() - want.reshape(B, -1)).abs().max()) < 2.0 ** -8 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner, N, lens", [(100, 16, [1, 63, 64, 65, 200]), (256, 5, [300]), (130, 17, [16, 33, 112]), (64, 32, [129, 2]),
                                             (4096, 1, [2100])])
