@@ -164,6 +164,22 @@ class KernelSet:
                                    c_int(K), c_int(a.stride(0)), c_int(w.stride(0)), c_int(N), c_int(out_f32),
                                    c_int(ksplit), _stream()), "gemm_nt")
 
+    def gemm_nt_blocks_take(self, a, w) -> bool:
+        """Whether `gemm_nt_blocks` runs these as one launch: more than 64 rows, 16-byte (float) or 8-byte (bfloat16) aligned pieces."""
+        nb, _, k = w.shape
+        return a.shape[0] > 64 and k % 4 == 0 and a.stride(0) % 4 == 0 and a.data_ptr() % (4 * a.element_size()) == 0
+
+    def gemm_nt_blocks(self, a, w, out):
+        """Block-diagonal product: out[b] = a[:, b K:(b + 1) K] @ w[b]^T for a [M, blocks K] (unit column stride), w [blocks, N, K] and
+        out [blocks, M, N], all of this set's dtype."""
+        nb, N, K = w.shape
+        M = a.shape[0]
+        if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or a.dtype != self.dtype or not a.is_cuda or a.stride(1) != 1:
+            raise KernelError(f"gemm_nt_blocks: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        _check(self._fn("gemm_nt_batched")(c_void_p(a.data_ptr()), _ptr(w, self.dtype, "w"), _ptr(out, self.dtype, "out"), c_int(M), c_int(N),
+                                           c_int(K), c_int(a.stride(0)), c_int(K), c_int(N), c_longlong(K), c_longlong(N * K),
+                                           c_longlong(M * N), c_int(nb), _stream()), "gemm_nt_batched")
+
     @staticmethod
     def gemm_nt_split(m: int, n_out: int, k: int, sm_count: int) -> int:
         """Into how many parts the generic product cuts K when its reader takes partial sums: none for

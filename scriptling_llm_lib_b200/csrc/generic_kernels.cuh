@@ -250,7 +250,7 @@ gemm_nt_tiled_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* __r
   }
 }
 
-// The same product for many rows with register tiles: a block of 256 threads owns a BM x 128 tile of
+// The same product for up to 64 rows with register tiles: a block of 256 threads owns a BM x 128 tile of
 // C, a thread (BM/16) x 8 outputs as (BM/64) x 2 groups of 4 x 4, 64 columns / rows apart so that its
 // operands are 16-byte shared-memory loads. A and B tiles of 16 k are fetched from global memory as
 // 16-byte vectors into registers while the previous tile is multiplied, then stored k-major
@@ -355,6 +355,146 @@ gemm_nt_regtile_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* _
 #pragma unroll
         for (int j = 0; j < 4; j++)
           if (gn + j < N) dst[j] = from_f32<TO>(acc[i][4 * g + j]);
+      }
+    }
+  }
+}
+
+// The same for many rows: a block of 256 threads owns a 128 x 128 tile of
+// C, a thread 8 x 8 outputs as 2 x 2 groups of 4 x 4, 64 columns / rows apart so that its
+// operands are 16-byte shared-memory loads. A and B tiles of 16 k are fetched from global memory as
+// 16-byte vectors into registers while the previous tile is multiplied, then stored k-major
+// (transposed) into the other of two shared buffers: one barrier per tile. Each output is still one
+// ascending-k chain of fused multiply-adds in float. Needs K, lda, ldb in multiples of 4 elements
+// and 16-byte (float) / 8-byte (bfloat16) aligned rows; the launcher falls back to the kernel above
+// otherwise. With several blocks along blockIdx.z, block z takes the z-th contiguous part of K
+// (k_per_split elements, a multiple of 16) and C receives float partial sums at C + z * M * ldc; with a
+// batch, it takes the z-th product (operands and result `batch` strides apart) over the whole of K.
+// Bound by issue slots: the multiply-adds go two to an instruction (outputs of neighbouring columns; the
+// chains and their roundings are the same), and four lanes read the 64 bytes of a row's tile, so that a load
+// touches 8 rows' lines and not 32. 2,778 rows: x W^T of 2,560 x 1,024, five blocks of 512 x 256 and 1,024 x 1,280 took 929 us
+// in seven launches, 621 in three (41 TFLOP/s; the tiles are one and a half waves). With tiles of 64 rows, where few blocks wait for
+// their loads, it was the slower one (64 rows of a decode step: 602 us of products against 547).
+struct GemmBatch { long long a, b, c; };      // strides in elements; all 0: no batch, blockIdx.z splits K
+__device__ __forceinline__ unsigned long long gemm_twice(float v) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(v));
+  return d;
+}
+__device__ __forceinline__ unsigned long long gemm_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(256, 2)
+gemm_nt_paired_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* __restrict__ C, int M, int N, int K,
+                       int lda, int ldb, int ldc, int k_per_split, GemmBatch batch) {
+  constexpr int BM = 128, BN = 128, BK = 16, TMG = BM / 64;   // TMG groups of 4 rows per thread
+  constexpr int A_VEC = BM * BK / 4 / 256;                 // 16-byte vectors of the A tile per thread (1 or 2)
+  constexpr int B_VEC = BN * BK / 4 / 256;                 // 2
+  constexpr int AP = BM + 4, BP = BN + 4;                  // padded rows: the transposing stores meet two to a bank, not four
+  __shared__ __align__(16) float As[2][BK][AP];
+  __shared__ __align__(16) float Bs[2][BK][BP];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const bool batched = batch.c != 0;
+  const int split = batched ? 0 : blockIdx.z;
+  if (batched) {
+    A += blockIdx.z * batch.a;
+    B += blockIdx.z * batch.b;
+  }
+  const int k_begin = split * k_per_split, k_end = min(K, k_begin + k_per_split);
+  TO* Cz = C + (batched ? blockIdx.z * batch.c : (long long)blockIdx.z * M * ldc);
+
+  unsigned long long acc[TMG * 4][4];                      // outputs of columns 2 j and 2 j + 1 of a group
+#pragma unroll
+  for (int i = 0; i < TMG * 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+
+  // vector v of this thread: row = (tid + 256 v) / 4, k quad = tid % 4
+  float4 ra[A_VEC], rb[B_VEC];
+  const int kq = (tid & 3) * 4;
+  auto fetch = [&](int k0) {
+    const int gk = k0 + kq;
+#pragma unroll
+    for (int v = 0; v < A_VEC; v++) {
+      const int gm = m0 + (tid >> 2) + 64 * v;
+      ra[v] = (gm < M && gk < k_end) ? ld4(A + (size_t)gm * lda + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int v = 0; v < B_VEC; v++) {
+      const int gn = n0 + (tid >> 2) + 64 * v;
+      rb[v] = (gn < N && gk < k_end) ? ld4(B + (size_t)gn * ldb + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto stash = [&](int buf) {
+#pragma unroll
+    for (int v = 0; v < A_VEC; v++) {
+      const int row = (tid >> 2) + 64 * v;
+      As[buf][kq + 0][row] = ra[v].x; As[buf][kq + 1][row] = ra[v].y;
+      As[buf][kq + 2][row] = ra[v].z; As[buf][kq + 3][row] = ra[v].w;
+    }
+#pragma unroll
+    for (int v = 0; v < B_VEC; v++) {
+      const int row = (tid >> 2) + 64 * v;
+      Bs[buf][kq + 0][row] = rb[v].x; Bs[buf][kq + 1][row] = rb[v].y;
+      Bs[buf][kq + 2][row] = rb[v].z; Bs[buf][kq + 3][row] = rb[v].w;
+    }
+  };
+
+  fetch(k_begin);
+  stash(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = k_begin; k0 < k_end; k0 += BK) {
+    const bool more = k0 + BK < k_end;
+    if (more) fetch(k0 + BK);
+#pragma unroll
+    for (int kk = 0; kk < BK; kk++) {
+      float a[TMG * 4];
+      unsigned long long b[4];
+#pragma unroll
+      for (int g = 0; g < TMG; g++) {
+        float4 t = *(const float4*)&As[buf][kk][g * 64 + ty * 4];
+        a[4 * g] = t.x; a[4 * g + 1] = t.y; a[4 * g + 2] = t.z; a[4 * g + 3] = t.w;
+      }
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        const ulonglong2 t = *(const ulonglong2*)&Bs[buf][kk][g * 64 + tx * 4];
+        b[2 * g] = t.x; b[2 * g + 1] = t.y;
+      }
+#pragma unroll
+      for (int i = 0; i < TMG * 4; i++) {
+        const unsigned long long a2 = gemm_twice(a[i]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = gemm_fma2(a2, b[j], acc[i][j]);
+      }
+    }
+    if (more) stash(buf ^ 1);
+    __syncthreads();
+    buf ^= 1;
+  }
+  const bool vec_out = (ldc & 3) == 0 && ((uintptr_t)Cz % (4 * sizeof(TO))) == 0;
+#pragma unroll
+  for (int i = 0; i < TMG * 4; i++) {
+    int gm = m0 + (i >> 2) * 64 + ty * 4 + (i & 3);
+    if (gm >= M) continue;
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+      int gn = n0 + g * 64 + tx * 4;
+      TO* dst = Cz + (size_t)gm * ldc + gn;
+      float f[4];
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(f[2 * j]), "=f"(f[2 * j + 1]) : "l"(acc[i][2 * g + j]));
+      if (vec_out && gn + 3 < N) {
+        st4(dst, make_float4(f[0], f[1], f[2], f[3]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (gn + j < N) dst[j] = from_f32<TO>(f[j]);
       }
     }
   }

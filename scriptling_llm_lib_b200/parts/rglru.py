@@ -73,8 +73,11 @@ class RGLRU(Mixer):
         u = self.conv.forward(yx[:, W:], st.get("conv"), ctx, torch.float32, in_bias=self.x_b, also=u_low)
         src = u if u_low is None else u_low
         gates = torch.empty((self.blocks, T, 2 * bs), dtype=torch.float32, device=x.device)
-        for b, lin in enumerate(self.gates):
-            lin.forward(src[:, b * bs:(b + 1) * bs], ctx, out_dtype=torch.float32, out=gates[b])
+        if src.dtype == torch.float32 == self.gate_w.dtype and ctx.kernels.gemm_nt_blocks_take(src, self.gate_w):
+            ctx.kernels.gemm_nt_blocks(src, self.gate_w, gates)                # every block's product in one launch
+        else:
+            for b, lin in enumerate(self.gates):
+                lin.forward(src[:, b * bs:(b + 1) * bs], ctx, out_dtype=torch.float32, out=gates[b])
         out = torch.empty((T, W), dtype=x.dtype, device=x.device)
         ctx.kernels.seq.rglru_scan(gates, u, yx[:, :W], self.ra_b, self.ri_b, self.lam, self.y_b, st["S"], ctx, out, bs)
         return self.out.forward(out, ctx)

@@ -416,6 +416,23 @@ def paged(k, v, lengths, n_extra=3, seed=0, dtype=torch.float32):
     return dev(kp, dtype), dev(vp, dtype), dev(bt)
 
 
+@pytest.mark.parametrize("blocks, M, N, K", [(5, 130, 512, 256), (3, 65, 20, 12), (2, 128, 7, 100), (10, 300, 130, 64)])
+def test_gemm_nt_blocks_is_every_block_by_itself(kernel_sets, blocks, M, N, K):
+    """One launch for a block-diagonal product, on a column slice: the same bits as a launch a block (each output is one chain of
+    multiply-adds in either)."""
+    ks = kernel_sets[torch.float32]
+    wide, w = dev(rand(M, blocks * K + 8, seed=3)), dev(rand(blocks, N, K, seed=4))
+    a = wide[:, 4:4 + blocks * K]
+    assert ks.gemm_nt_blocks_take(a, w) and not ks.gemm_nt_blocks_take(a[:64], w) and not ks.gemm_nt_blocks_take(wide[:, 1:1 + blocks * K], w)
+    out, each = (torch.full((blocks, M, N), float("nan"), device="cuda") for _ in range(2))
+    ks.gemm_nt_blocks(a, w, out)
+    for b in range(blocks):
+        ks.gemm_nt(a[:, b * K:(b + 1) * K], w[b], each[b])
+    assert torch.equal(out, each)
+    want = torch.einsum("mbk,bnk->bmn", f64(a).view(M, blocks, K), f64(w))
+    assert rel_err(out.cpu(), want) < TOL[torch.float32] * max(1.0, (K / 64) ** 0.5)
+
+
 # --------------------------------------------------------------------------- rotary + cache write
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H, G, hd, rot, pairing", [(4, 2, 16, 16, "interleaved"), (3, 1, 32, 16, "half"),
