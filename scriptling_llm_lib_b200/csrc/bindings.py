@@ -1255,6 +1255,9 @@ class SsdKernels:
     """Launchers of ssd_kernels.cuh: the state-space recurrence with one decay per head and token, and the norm over equal
     runs of columns behind it. `dtype` is the element type of activations; step sizes, decays, state and sums are float32."""
     CHUNK, CHUNK_MIN_ROWS, CHUNK_MAX_STATE = 128, 64, 256
+    # (sequence, head) pairs of a decode step from which on their states go through shared memory: about two for every block that stays
+    # (of 64 columns x 128 states: 512 pairs take 8.3 us, 9.3 in registers; with fewer there is no next pair to load meanwhile)
+    STEP_MIN_UNITS = 512
 
     def __init__(self, dtype: torch.dtype):
         if dtype not in _SUFFIX:
@@ -1262,9 +1265,16 @@ class SsdKernels:
         self.dtype, self.suffix = dtype, _SUFFIX[dtype]
         self.lib = load_library("ssd_" + self.suffix)
         self._fns: dict[str, object] = {}
+        self._sm_counts: dict = {}
 
     _fn = SequenceKernels._fn
     _view = staticmethod(SequenceKernels._view)
+
+    def _sms(self, device) -> int:
+        n = self._sm_counts.get(device)
+        if n is None:
+            n = self._sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+        return n
 
     def scan(self, xbc, dt, dt_bias, a_log, dskip, z, state, ctx, out, n_heads, n_groups, head_dim, n_state, weight=None, chunked=None):
         """xbc [T, H V + 2 G N] (x | B | C), dt [T, H] raw step sizes, z [T, H V]: views of the element type; dt_bias, a_log,
@@ -1281,6 +1291,15 @@ class SsdKernels:
         if chunked is None:
             chunked = self.dtype == torch.bfloat16 and ctx.max_new >= self.CHUNK_MIN_ROWS
         chunked = chunked and n_state <= self.CHUNK_MAX_STATE
+        if (not chunked and weight is None and ctx.max_new == 1 and T == ctx.n_seqs and T * n_heads >= self.STEP_MIN_UNITS
+                and state.data_ptr() % 16 == 0 and self._fn("ssd_step_takes")(c_int(head_dim), c_int(n_state))):
+            _check(self._fn("ssd_step")(
+                self._view(xbc, "xbc"), c_int(xbc.stride(0)), self._view(dt, "dt"), c_int(dt.stride(0)), _ptr(dt_bias, torch.float32, "dt_bias"),
+                _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), c_int(z.stride(0)),
+                _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
+                self._view(out, "out"), c_int(out.stride(0)), c_int(T), c_int(n_heads), c_int(n_groups), c_int(head_dim), c_int(n_state),
+                c_int(self._sms(out.device)), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "ssd_step")
+            return None
         states = decays = sums = sumsq = None
         if chunked:
             n = T // self.CHUNK + ctx.n_seqs

@@ -523,6 +523,29 @@ def test_the_recurrence_walked_and_in_chunks(dtype, H, G, V, N, lens, kw):
                 assert float((sq.sum(0).cpu().double() / (want * want).sum(-1) - 1.0).abs().max()) < 1e-4
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,V,N,B", [(64, 1, 64, 128, 9), (3, 3, 16, 5, 400), (8, 2, 128, 128, 64), (37, 1, 32, 250, 14)])
+def test_a_decode_step_with_its_states_through_shared_memory(dtype, H, G, V, N, B):
+    """One row a sequence: fewer pairs than blocks take at once and several a block, states of every part of a warp and of one block an
+    SM, on slots out of order. The states' arithmetic is the walk's, element by element: the same bits; outputs differ from it by the
+    order of N float terms, 1e-6 sqrt(N) of the largest, and by their rounding."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k = KernelSet(dtype).ssd
+    assert B * H >= k.STEP_MIN_UNITS
+    xbc, dt, z, dt_bias, a_log, dskip, state, slots = _scan_case(dtype, H, G, V, N, (1,) * B, 4)
+    ctx = SimpleNamespace(n_seqs=B, max_new=1, seq_start=torch.arange(B + 1, dtype=torch.int32).cuda(), slots=slots.cuda(),
+                          err_flag=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    got = []
+    for least in (1, 1 << 30):          # this kernel, then the walk
+        k.STEP_MIN_UNITS = least
+        st, out = state.cuda().contiguous(), torch.full((B, H * V), float("nan"), dtype=dtype, device="cuda")
+        k.scan(xbc.cuda(), dt.cuda(), dt_bias.cuda(), a_log.cuda(), dskip.cuda(), z.cuda(), st, ctx, out, H, G, V, N)
+        got.append((st, out.double()))
+    assert int(ctx.err_flag) == 0 and torch.equal(got[0][0], got[1][0])
+    tol = 1e-6 * N ** 0.5 + (2.0 ** -7 if dtype == torch.bfloat16 else 0.0)
+    assert float((got[0][1] - got[1][1]).abs().max()) < tol * float(got[1][1].abs().max())
+
+
 @pytest.mark.parametrize("taps,C", [(2, 12), (3, 520), (4, 64), (4, 516)])
 def test_the_convolution_over_many_rows(taps, C):
     """The kernel for steps of many rows: sequences that begin and end inside a thread's rows, runs shorter than the filter, past
