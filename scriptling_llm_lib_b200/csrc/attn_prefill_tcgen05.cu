@@ -43,7 +43,7 @@
 // next page's S is issued behind P V; the other tile of the pair fills the tensor cores meanwhile. Keys go up to 192 here.
 // Bound by the chain S -> softmax and splitting -> P V of a page. Prompts of 2,048 tokens, 16 heads: keys 64, values 128, window
 // 1,024 on 4 key/value heads 55.6 us (1,827 on the kernel with a warp a row and head, attn_wide_value, 22 -> 175 TFLOP/s on the
-// pairs seen); keys 192, values 128, every earlier key 97.5 us (1,189 on the float32 tiles of attn_paged, 18 -> 220 TFLOP/s).
+// pairs seen); keys 192, values 128, every earlier key 71.5 us (1,189 on the float32 tiles of attn_paged, 18 -> 300 TFLOP/s).
 #include "tcgen05.cuh"
 
 #define FT_BQ 128
@@ -61,7 +61,8 @@ struct FtArgs {
   float scale;
   int* err;
   int n_qt, n_seqs, n_items;   // query tiles per sequence (of the longest), sequences, work items
-  int pair_heads;              // pair kernel: 1: an item is heads 2i, 2i+1 on one query tile; 0: query tiles 2i, 2i+1 of one head
+  int pair_heads;              // pair kernel: 1: an item is heads 2i, 2i+1 on one query tile; 0: query tiles 2i, 2i+1 of one head; 2: tiles i and
+                               // n - 1 - i of one head
   float softcap;               // > 0: a score s (scaled) becomes softcap * tanh(s / softcap) before the softmax
   const float* sink;           // [H] or null: exp(sink[h]) joins head h's denominator, with no key and no value
   const bf16* gate;            // null, or [T, gate_ld]: output element (h, d) is multiplied by the sigmoid of column h * vd + d
@@ -486,7 +487,7 @@ __device__ __forceinline__ bool fp_item(const FtArgs& p, int round, FpItem& it) 
   int idx = round * G + ((round & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
   if (idx >= p.n_items) return false;
   int h0, h1, qt0, qt1, rest;
-  if (p.pair_heads) {
+  if (p.pair_heads == 1) {
     int H2 = p.H >> 1;
     h0 = 2 * (idx % H2);
     h1 = h0 + 1;
@@ -505,6 +506,11 @@ __device__ __forceinline__ bool fp_item(const FtArgs& p, int round, FpItem& it) 
   it.pos0 = p.seq_pos0[it.b];
   it.seq_end = it.pos0 + S - 1;
   it.g = h0 / (p.H / p.G);
+  if (p.pair_heads == 2) {       // the sequence's tiles from both ends: the i-th with the i-th from the last
+    const int n = (S + FT_BQ - 1) / FT_BQ, i = rest / p.n_seqs;
+    qt0 = 2 * i < n ? i : p.n_qt;                // past the sequence's end: nothing to do
+    qt1 = 2 * i < n - 1 ? n - 1 - i : p.n_qt;    // the middle tile is alone
+  }
   fp_tile(p, it.sub[0], h0, qt0, S, it.pos0);
   fp_tile(p, it.sub[1], h1, qt1, S, it.pos0);
   it.valid = it.sub[0].valid;                      // the second tile of a pair is never valid without the first
@@ -957,8 +963,14 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
     dim3 grid((unsigned)(n_items < 2LL * sm_count ? n_items : 2LL * sm_count));     // two blocks per SM that stay
     return ft_launch<64, 3>(mq, mk, mv, a, grid, stream);
   }
+  // A head by itself whose items are one wave (float weights, every earlier key seen): the wave lasts as long as its longest item,
+  // and neighbouring tiles at a prompt's end make that twice the average. Tiles from both ends make all items alike, though they
+  // share fewer pages. 16 heads of 192 / 128, one prompt of 2,048 tokens 97.5 -> 71.5 us, 1,100 tokens 50.7 -> 43.8, 500 tokens
+  // 27.3 -> 23.7, two of 900 tokens 48.5 -> 38.0. At five tiles a head both take 27; at three (15.9, 17.2 from both ends) the last tile is
+  // better alone. With several waves (three prompts of 900 tokens) the next item fills the gap, and neighbours share more.
   int pair_heads = ((H / G) % 2 == 0) ? 1 : 0;
-  n_items = pair_heads ? (long long)(H / 2) * n_qt * B : (long long)H * ((n_qt + 1) / 2) * B;
+  if (!pair_heads && weight_parts == 3 && window == 0 && n_qt >= 4 && (long long)H * ((n_qt + 1) / 2) * B <= sm_count) pair_heads = 2;
+  n_items = pair_heads == 1 ? (long long)(H / 2) * n_qt * B : (long long)H * ((n_qt + 1) / 2) * B;
   FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, pair_heads, softcap, sink,
            (const bf16*)gate, gate_ld};
   dim3 grid((unsigned)(n_items < (long long)sm_count ? n_items : (long long)sm_count));       // one block per SM that stays

@@ -547,7 +547,8 @@ def test_attn_prefill_tcgen05(kernel_sets, hd, H, G, window, lens, pos0):
     assert rel_err(out.cpu().float(), want) < 1.2e-2          # probabilities are rounded to bfloat16 before P V
 
 
-@pytest.mark.parametrize("lens, pos0", [([37, 1, 130, 64, 200, 128], [0, 250, 70, 64, 0, 300]), ([1], [700]), ([700], [0])])
+@pytest.mark.parametrize("lens, pos0", [([37, 1, 130, 64, 200, 128], [0, 250, 70, 64, 0, 300]), ([1], [700]), ([700], [0]),
+                                        ([300, 513, 1], [77, 0, 100])])
 @pytest.mark.parametrize("kd, vd, H, G, window", [(64, 64, 4, 2, 0), (64, 128, 4, 1, 100), (128, 64, 3, 3, 0), (128, 128, 4, 4, -96),
                                                   (192, 128, 3, 3, 0), (192, 64, 4, 2, 65), (136, 72, 6, 3, 0), (8, 8, 2, 1, 0),
                                                   (80, 80, 2, 2, 1), (176, 120, 2, 1, 0)])
