@@ -13,7 +13,7 @@
 // order of position) and find a sequence's state through slots[b]. State, sums, scores, norms, gates and decays are
 // float32 whatever the element type A of activations and weights.
 #pragma once
-#include "common.cuh"
+#include "state_step.cuh"
 
 namespace mix {
 
@@ -175,6 +175,33 @@ __device__ __forceinline__ void stage_silu_tile(float* __restrict__ dst, int dst
     }
   }
 }
+
+// A decode step of it as a walk over the states (state_step.cuh): b = silu(k), c = silu(q), x = silu(v), the head's decay.
+template <typename A>
+struct LinStepJob {
+  const A* proj; int ld, q_col, k_col, v_col;
+  const float* decay;
+  float* state;
+  const int* seq_start; const int* slots;
+  float* o;
+  int H, D, V;
+  __device__ __forceinline__ int heads() const { return H; }
+  __device__ __forceinline__ int rows() const { return D; }
+  __device__ __forceinline__ int cols() const { return V; }
+  __device__ __forceinline__ float* place(int b, int h) const { return state + ((size_t)slots[b] * H + h) * D * V; }
+  __device__ __forceinline__ void fetch(step::Row& r, int b, int h, int tid) const {
+    const A* row = proj + (size_t)seq_start[b] * ld;
+    if (tid < D) {
+      r.b = silu_f(to_f32(row[k_col + (size_t)h * D + tid]));
+      r.c = silu_f(to_f32(row[q_col + (size_t)h * D + tid]));
+    }
+    if (tid < V) r.x = silu_f(to_f32(row[v_col + (size_t)h * V + tid]));
+    if (tid == 0) { r.d = 1.f; r.dec = decay[h]; }
+  }
+  __device__ __forceinline__ void finish(int b, int h, int v, float s, float, float) const {
+    o[((size_t)seq_start[b] * H + h) * V + v] = s;
+  }
+};
 
 template <typename A>
 __global__ void __launch_bounds__(256) lin_attn_decay_kernel(const A* __restrict__ proj, int ld, int q_col, int k_col, int v_col,

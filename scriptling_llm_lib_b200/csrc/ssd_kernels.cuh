@@ -16,7 +16,7 @@
 // of squares of y silu(z) in front of that weight: the halves of an RMS norm over the whole row that the product behind it
 // can finish.
 #pragma once
-#include "tcgen05.cuh"
+#include "state_step.cuh"
 
 namespace ssd {
 
@@ -166,122 +166,37 @@ __global__ void __launch_bounds__(256) ssd_walk_kernel(Args p, int R) {
 }
 
 // ------------------------------------------------------------------ one row a sequence
-// A decode step reads and writes every sequence's states once and does little else, so the states are moved by bulk copies: a block
-// stays and walks (sequence, head) pairs, a ring of three tiles [N][V] in shared memory has the next pairs' states on their way in and
-// the last one's on its way out while a pair's row is worked on in place (V / 4 lanes a row of the state). What a row brings comes a
-// pair ahead through registers. Two blocks an SM. Bound by the copies: 64 sequences of 64 heads of 64 columns x 128 states, 268 MB,
-// take 49.9 us (5.4 TB/s; 69.6 with a block's states in registers, each block one load, one row and one store); 16 sequences 13.5 us
-// (16.1), 8 sequences 8.3 (9.3).
-#define SSD_RING 3
+// What the walk over states in state_step.cuh is told of this recurrence: b = B, c = C, x, the gate's z, step size and decay.
+// 64 sequences of 64 heads of 64 columns x 128 states, 268 MB, take 49.9 us (5.4 TB/s; 69.6 with a block's states in registers, each
+// block one load, one row and one store); 16 sequences 13.5 us (16.1), 8 sequences 8.3 (9.3).
 template <typename A>
-__global__ void __launch_bounds__(256) ssd_step_kernel(Args p, int units, int* err) {
-  extern __shared__ __align__(128) uint8_t smem_raw[];
-  const int N = p.N, V = p.V, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, HV = p.H * V;
-  const uint32_t tile_bytes = (uint32_t)N * V * 4;
-  float* tiles = (float*)smem_raw;                              // [ring][N][V]
-  float* red = tiles + (size_t)SSD_RING * N * V;                // [8][V]
-  float* rows = red + 8 * V;                                    // two of [x: V | z: V | step size, decay, -, - | b: N | c: N]
-  const int row_len = (2 * N + 2 * V + 7) & ~3, at_b = 2 * V + 4;
-  uint8_t* head = (uint8_t*)(rows + 2 * row_len);
-  const uint32_t full = smem_u32(head);
-  volatile int* abort = (volatile int*)(head + 8 * SSD_RING);
-  if (tid == 0) {
-    for (int s = 0; s < SSD_RING; s++) mbar_init(full + 8 * s, 1);
-    *abort = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  const int mine = ((int)blockIdx.x < units) ? (units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  auto place = [&](int i) {                                     // the states of this block's i-th pair
-    const int u = blockIdx.x + i * gridDim.x, b = u / p.H, h = u % p.H;
-    return p.state + ((size_t)p.slots[b] * p.H + h) * N * V;
-  };
-  auto load = [&](int i) {
-    const uint32_t bar = full + 8 * (i % SSD_RING);
-    mbar_expect_tx(bar, tile_bytes);
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(tiles + (size_t)(i % SSD_RING) * N * V)), "l"(place(i)), "r"(tile_bytes), "r"(bar) : "memory");
-  };
-  if (tid == 0)
-    for (int i = 0; i < min(mine, SSD_RING - 1); i++) load(i);
-  float nb = 0.f, nc = 0.f, nx = 0.f, nz = 0.f, nd = 0.f, ndec = 0.f;      // the next pair's row
-  auto fetch = [&](int i) {
-    const int u = blockIdx.x + i * gridDim.x, b = u / p.H, h = u % p.H, r = p.seq_start[b];
+struct StepJob {
+  Args p;
+  __device__ __forceinline__ int heads() const { return p.H; }
+  __device__ __forceinline__ int rows() const { return p.N; }
+  __device__ __forceinline__ int cols() const { return p.V; }
+  __device__ __forceinline__ float* place(int b, int h) const { return p.state + ((size_t)p.slots[b] * p.H + h) * p.N * p.V; }
+  __device__ __forceinline__ void fetch(step::Row& o, int b, int h, int tid) const {
+    const int N = p.N, V = p.V, r = p.seq_start[b];
     const A* xbc = (const A*)p.xbc + (size_t)r * p.ldx;
     if (tid < N) {
-      const A* e = xbc + HV + (size_t)(h / (p.H / p.G)) * N + tid;
-      nb = to_f32(e[0]);
-      nc = to_f32(e[(size_t)p.G * N]);
+      const A* e = xbc + p.H * V + (size_t)(h / (p.H / p.G)) * N + tid;
+      o.b = to_f32(e[0]);
+      o.c = to_f32(e[(size_t)p.G * N]);
     }
     if (tid < V) {
-      nx = to_f32(xbc[(size_t)h * V + tid]);
-      nz = to_f32(((const A*)p.z)[(size_t)r * p.ldz + (size_t)h * V + tid]);
+      o.x = to_f32(xbc[(size_t)h * V + tid]);
+      o.z = to_f32(((const A*)p.z)[(size_t)r * p.ldz + (size_t)h * V + tid]);
     }
     if (tid == 0) {
-      nd = softplus_f(to_f32(((const A*)p.dt)[(size_t)r * p.lddt + h]) + p.dt_bias[h]);
-      ndec = expf(-expf(p.a_log[h]) * nd);
+      o.d = softplus_f(to_f32(((const A*)p.dt)[(size_t)r * p.lddt + h]) + p.dt_bias[h]);
+      o.dec = expf(-expf(p.a_log[h]) * o.d);
     }
-  };
-  auto stash = [&](int i) {
-    float* d = rows + (i & 1) * row_len;
-    if (tid < N) { d[at_b + tid] = nb; d[at_b + N + tid] = nc; }
-    if (tid < V) { d[tid] = nx; d[V + tid] = nz; }
-    if (tid == 0) { d[2 * V] = nd; d[2 * V + 1] = ndec; }
-  };
-  if (mine > 0) {
-    fetch(0);
-    stash(0);
   }
-  __syncthreads();
-  const int per = V / 4, rows_at_once = 256 / per, c4 = (tid % per) * 4, r0 = tid / per;
-  bool ok = true;
-  for (int i = 0; i < mine; i++) {
-    if (!mbar_wait(full + 8 * (i % SSD_RING), (i / SSD_RING) & 1, abort)) ok = false;
-    if (i + 1 < mine) fetch(i + 1);
-    float* tile = tiles + (size_t)(i % SSD_RING) * N * V;
-    const float* row = rows + (i & 1) * row_len;
-    const float d = row[2 * V], dec = row[2 * V + 1];
-    float4 x = *(const float4*)(row + c4), y = make_float4(0.f, 0.f, 0.f, 0.f);
-    x.x *= d; x.y *= d; x.z *= d; x.w *= d;
-#pragma unroll 4
-    for (int n = r0; n < N; n += rows_at_once) {
-      float4 q = *(const float4*)(tile + n * V + c4);
-      const float b = row[at_b + n], c = row[at_b + N + n];
-      q.x = fmaf(dec, q.x, b * x.x); q.y = fmaf(dec, q.y, b * x.y); q.z = fmaf(dec, q.z, b * x.z); q.w = fmaf(dec, q.w, b * x.w);
-      *(float4*)(tile + n * V + c4) = q;
-      y.x = fmaf(c, q.x, y.x); y.y = fmaf(c, q.y, y.y); y.z = fmaf(c, q.z, y.z); y.w = fmaf(c, q.w, y.w);
-    }
-    for (int o = per; o < 32; o <<= 1) {                        // the rows that a warp's lanes share out
-      y.x += __shfl_xor_sync(0xffffffffu, y.x, o);
-      y.y += __shfl_xor_sync(0xffffffffu, y.y, o);
-      y.z += __shfl_xor_sync(0xffffffffu, y.z, o);
-      y.w += __shfl_xor_sync(0xffffffffu, y.w, o);
-    }
-    if (lane < per) *(float4*)(red + warp * V + c4) = y;
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();                                            // the states are done, and the warps' sums are there
-    if (tid == 0) {
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(place(i)), "r"(smem_u32(tile)), "r"(tile_bytes) : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-      if (i + SSD_RING - 1 < mine) {                            // its place was pair i - 1's: read out by now, or waited for
-        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        load(i + SSD_RING - 1);
-      }
-    }
-    if (tid < V) {
-      const int u = blockIdx.x + i * gridDim.x, b = u / p.H, h = u % p.H, r = p.seq_start[b];
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; w++) s += red[w * V + tid];
-      s = fmaf(p.dskip[h], row[tid], s) * silu_f(row[V + tid]);
-      ((A*)p.out)[(size_t)r * p.ldo + (size_t)h * V + tid] = from_f32<A>(s);
-    }
-    if (i + 1 < mine) stash(i + 1);
-    __syncthreads();
+  __device__ __forceinline__ void finish(int b, int h, int v, float s, float x, float z) const {
+    ((A*)p.out)[(size_t)p.seq_start[b] * p.ldo + (size_t)h * p.V + v] = from_f32<A>(fmaf(p.dskip[h], x, s) * silu_f(z));
   }
-  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-  if (!ok && err) atomicExch(err, 5);
-}
+};
 
 // ------------------------------------------------------------------ in chunks, on the tensor cores
 // A sequence's rows are cut into chunks of SSD_Q. With c_i the sum of a over the chunk's rows up to and with i:

@@ -456,6 +456,29 @@ def test_latent_decode_on_the_tensor_cores(H, D, P, V, R, window, n_split):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, D, V, B", [(16, 128, 128, 9), (3, 10, 16, 1), (2, 250, 64, 300), (5, 64, 32, 40)])
+def test_a_decode_step_of_linear_attention_walks_its_states(dtype, H, D, V, B):
+    """One row a sequence, fewer pairs than blocks and several a block, slots out of order: states to one rounding of their two terms
+    (1e-6 of the largest), outputs to float sums of D terms (1e-6 sqrt(D))."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k = KernelSet(dtype).mix
+    g = torch.Generator().manual_seed(D)
+    proj, state0 = torch.randn(B, 2 * H * D + H * V, generator=g).to(dtype), torch.randn(B + 2, H, D, V, generator=g)
+    decay, slots = torch.rand(H, generator=g), torch.randperm(B + 2, generator=g)[:B].to(torch.int32)
+    ctx = SimpleNamespace(seq_start=torch.arange(B + 1, dtype=torch.int32).cuda(), slots=slots.cuda(), n_seqs=B, max_new=1,
+                          engine=SimpleNamespace(sm_count=148), err_flag=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    st, o = state0.clone().cuda(), torch.full((B, H * V), float("nan"), device="cuda")
+    k.lin_attn_decay(proj.cuda(), 0, H * D, 2 * H * D, decay.cuda(), st, ctx, o, H, D, V)
+    q, kk, v = (plain.silu(t).view(B, H, -1) for t in proj.double().split([H * D, H * D, H * V], 1))
+    want, at = state0.double(), slots.long()
+    want[at] = decay.double()[:, None, None] * want[at] + kk[..., None] * v[:, :, None]
+    y = torch.einsum("bhdv,bhd->bhv", want[at], q).reshape(B, -1)
+    assert int(ctx.err_flag) == 0
+    assert float((st.cpu().double() - want).abs().max()) < 1e-6 * float(want.abs().max())
+    assert float((o.cpu().double() - y).abs().max()) < 1e-6 * D ** 0.5 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner, N, lens", [(100, 16, [1, 63, 64, 65, 200]), (256, 5, [300]), (130, 17, [16, 33, 112]), (64, 32, [129, 2]),
                                             (4096, 1, [2100])])
 def test_selective_scan_in_pieces_against_the_recurrence(dtype, inner, N, lens):
