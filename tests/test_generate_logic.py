@@ -1,4 +1,7 @@
 """The generation loop's decisions, driven by a scripted step function (no GPU)."""
+from array import array
+
+import numpy as np
 import pytest
 import torch
 
@@ -181,3 +184,19 @@ def test_sampling_options_and_params():
     assert p.shape == (2, 8) and p[0, 0] == 3 and p[0, 2] == 40
     assert p[0, 4] == 2 and p[0, 5] == 1 and p[0, 6] == 3 and p[1, 7] == 2
     assert p[:, 1].view("float32")[0] == 0.5 and p[:, 3].view("float32")[0] == 0.75
+
+
+@pytest.mark.parametrize("runs", [[[5, 0, 31999]], [[1], [2, 3], [4]], [(1, 2), [3]], [[np.int32(7), True, 2 ** 62]], [[1.9, 2]], [[1, None]],
+                                  [[1, 2 ** 70]], [np.array([4, 5])], [np.array([4.5])], [b"ab"], [array("i", [3, 4])], [["x"]], [[-1]]])
+def test_token_ids_are_what_an_iterator_would_read(runs):
+    """Lists of integers, and all else a step may be handed: the same values, or the same kind of error."""
+    from scriptling_llm_lib_b200.engine.step import _token_ids
+    total = sum(len(r) for r in runs)
+    try:
+        want = np.fromiter((t for r in runs for t in r), dtype=np.int64, count=total)
+    except Exception as e:
+        with pytest.raises(type(e)):
+            _token_ids(runs, total)
+    else:
+        got = _token_ids(runs, total)
+        assert got.dtype == np.int64 and got.tolist() == want.tolist()
