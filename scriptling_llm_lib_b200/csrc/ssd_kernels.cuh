@@ -5,7 +5,7 @@
 // Columns of a row of xbc: [x: H V | B: G N | C: G N] (element type). The state [slot][H][N][V] is float, read at a step's start
 // and left at its end. Step sizes, decays, exponentials, state and sums are float; out is of the element type.
 //
-//   ssd_step           a decode step of many sequences: one row each, the states through shared memory
+//   StepJob            a decode step of many sequences: one row each, the states through shared memory (state_step.cuh)
 //   ssd_walk           token by token with the state in registers: decode steps, short runs, and all of 32-bit
 //   ssd_chunk_states   bfloat16, long runs: what every chunk of SSD_Q rows adds to the state
 //   ssd_chunk_pass     the state in front of every chunk, and the state left at the end

@@ -14,7 +14,7 @@ the cached vectors with [Wuk_i^T q_i | q_rot] directly, sums the latents with th
 and applies Wuv_i once to that sum. All heads of a row read the same cached rows. That is the form
 of decode steps and of portions that land on a cache. A prompt step whose sequences all start at
 position 0 forms keys and values per head for its own rows instead (two products over the step's
-latents) and runs the library's attention kernel for keys and values of one width on them: fewer
+latents) and runs the library's prompt attention on them, with its softmax weights in float32: fewer
 products per query and key than asking the latent, which is wider than a head.
 
 A layer built with `shares_cache=True` has no Wdkv: it runs with `writes=False` on the unit another

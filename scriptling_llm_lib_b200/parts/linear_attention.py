@@ -7,10 +7,10 @@ model, no other scale). The heads' outputs side by side are divided by the root 
 whole row, sqrt(mean(o^2) + eps), multiplied by a weight [n_heads dv] and by sigmoid(Wg h), and Wo
 maps them back to the hidden width.
 
-The kernel works a step's rows in pieces: inside a piece the rows see each other through their
+The kernels work a step's rows in pieces: inside a piece the rows see each other through their
 decayed scores (q_i . k_j) g^(i-j), and the pieces before them through the state, so a prompt
-costs matrix products instead of one dependent update per row; a decode step is a piece of one
-row. State per sequence: S in float32. The projections run in the engine's dtype; SiLU, scores,
+costs matrix products instead of one dependent update per row; a decode step walks the states
+once. State per sequence: S in float32. The projections run in the engine's dtype; SiLU, scores,
 decay powers, state and the read-out norm are float32.
 """
 from __future__ import annotations
