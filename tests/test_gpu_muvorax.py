@@ -456,6 +456,23 @@ def test_latent_decode_on_the_tensor_cores(H, D, P, V, R, window, n_split):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("W, ld, off", [(8, 8, 0), (248, 504, 256), (2048, 4096, 2048), (4096, 4096, 0), (4104, 4104, 0), (2044, 2048, 0),
+                                        (256, 516, 4), (1024, 1030, 0)])
+@pytest.mark.parametrize("act", ["sigmoid", "silu"])
+def test_gated_row_rms_at_its_widths(dtype, W, ld, off, act):
+    """Eight elements a thread, and the widths and places that are not for it, against 64 bits: the output's rounding (2^-8 in
+    bfloat16) and float sums and functions (2e-6)."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    g = torch.Generator().manual_seed(W)
+    o, wide, w = torch.randn(5, W, generator=g), torch.randn(5, ld, generator=g).to(dtype), torch.rand(W, generator=g)
+    gate, y = wide.cuda()[:, off:off + W], torch.full((5, W), float("nan"), dtype=dtype, device="cuda")
+    KernelSet(dtype).mix.gated_row_rms(o.cuda(), gate, w.cuda(), y, 1e-6, act)
+    z = wide[:, off:off + W].double()
+    want = o.double() * torch.rsqrt((o.double() ** 2).mean(1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(z) * (z if act == "silu" else 1)
+    assert bool(((y.cpu().double() - want).abs() <= (2 ** -8 if dtype == torch.bfloat16 else 2e-6) * want.abs() + 2e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H, D, V, B", [(16, 128, 128, 9), (3, 10, 16, 1), (2, 250, 64, 300), (5, 64, 32, 40)])
 def test_a_decode_step_of_linear_attention_walks_its_states(dtype, H, D, V, B):
     """One row a sequence, fewer pairs than blocks and several a block, slots out of order: states to one rounding of their two terms
