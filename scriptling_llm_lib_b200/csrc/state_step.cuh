@@ -4,6 +4,9 @@
 // walks (sequence, head) pairs; a ring of three tiles [rows][cols] in shared memory has the next pairs' states on their way in and the
 // last one's on its way out while a pair's row is worked on in place (cols / 4 lanes a row of the state). What a row brings comes a
 // pair ahead through registers. Bound by the copies. A job says where states lie, what a row brings and what becomes of y.
+//
+// A block whose wait for a pair's states runs out stores nothing of that pair or of those behind it: it lets the copies that are under
+// way land, raises the error flag and leaves.
 #pragma once
 #include "tcgen05.cuh"
 
@@ -98,7 +101,13 @@ __global__ void __launch_bounds__(256) state_step_kernel(Job job, int units, int
     }
     if (lane < per) *(float4*)(red + warp * V + c4) = y;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();                                            // the states are done, and the warps' sums are there
+    if (!__syncthreads_and(ok)) {                               // the states are done, and the warps' sums are there, unless a wait ran out
+      volatile int never = 0;
+      if (tid == 0)
+        for (int j = i; j < min(mine, i + RING - 1); j++) mbar_wait(full + 8 * (j % RING), (j / RING) & 1, &never);
+      ok = false;
+      break;
+    }
     int b, h;
     pair(i, b, h);
     if (tid == 0) {

@@ -495,6 +495,52 @@ def test_a_decode_step_of_linear_attention_walks_its_states(dtype, H, D, V, B):
     assert float((o.cpu().double() - y).abs().max()) < 1e-6 * D ** 0.5 * float(y.abs().max())
 
 
+STEP_GIVES_UP = """
+#include "state_step.cuh"
+struct Job {
+  float *state, *y; int H, N, V;
+  __device__ int heads() const { return H; }
+  __device__ int rows() const { return N; }
+  __device__ int cols() const { return V; }
+  __device__ float* place(int b, int h) const { return state + (size_t)(b * H + h) * N * V; }
+  __device__ void fetch(step::Row& r, int, int, int) const { r.b = r.c = r.x = r.d = 1.f; r.dec = 0.5f; }
+  __device__ void finish(int b, int h, int v, float s, float, float) const { y[(b * H + h) * V + v] = s; }
+};
+extern "C" int run(float* state, float* y, int B, int H, int N, int V, int* err, cudaStream_t stream) {
+  return step::launch(Job{state, y, H, N, V}, N, V, B * H, 1, err, stream);      // "one SM": two blocks that stay
+}
+"""
+
+
+def test_a_state_whose_wait_runs_out_is_left_as_it_was(tmp_path):
+    """The walk over the states, built with one thread's wait for a block's third pair counted as run out: the two pairs in front of it
+    are advanced and stored, none behind it is, the error flag is raised and the stream goes on."""
+    import ctypes
+    import subprocess
+    from scriptling_llm_lib_b200.csrc import build
+    for f in ("common.cuh", "tcgen05.cuh"):
+        (tmp_path / f).write_text((build.CSRC / f).read_text())
+    wait = "if (!mbar_wait(full + 8 * (i % RING), (i / RING) & 1, abort)) ok = false;"
+    walk = (build.CSRC / "state_step.cuh").read_text()
+    assert walk.count(wait) == 1
+    (tmp_path / "state_step.cuh").write_text(walk.replace(wait, wait + " if (i == 2 && threadIdx.x == 7) ok = false;"))
+    (tmp_path / "t.cu").write_text(STEP_GIVES_UP)
+    subprocess.run([build.find_nvcc(), *build.ARCH_FLAGS, *build.NVCC_FLAGS, "-I", str(tmp_path), "-o", str(tmp_path / "t.so"), str(tmp_path / "t.cu")],
+                   check=True, capture_output=True, timeout=300)
+    lib = ctypes.CDLL(str(tmp_path / "t.so"))
+    B, H, N, V = 3, 5, 40, 64
+    state0 = torch.randn(B, H, N, V, generator=torch.Generator().manual_seed(1))
+    st, y, err = state0.cuda(), torch.zeros(B, H, V, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())      # noqa: E731
+    assert lib.run(p(st), p(y), B, H, N, V, p(err), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    want = state0.view(B * H, N, V).clone()
+    want[:4] = 0.5 * want[:4] + 1                    # two blocks: pairs 0, 2, ... and 1, 3, ...; the third of either gives up
+    assert int(err) == 5
+    assert torch.equal(st.view(B * H, N, V)[4:].cpu(), want[4:])
+    assert float((st.view(B * H, N, V)[:4].cpu() - want[:4]).abs().max()) < 1e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("inner, N, lens", [(100, 16, [1, 63, 64, 65, 200]), (256, 5, [300]), (130, 17, [16, 33, 112]), (64, 32, [129, 2]),
                                             (4096, 1, [2100])])
