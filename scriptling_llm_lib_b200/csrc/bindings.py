@@ -1039,8 +1039,9 @@ class MixKernels:
         if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.LIN_MIN_ROWS and dk <= ChunkKernels.CHUNK:
             self.chunk.lin_attn(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
             return
-        # One row a sequence: the walk over the states by bulk copies. 16 heads of 128 x 128 in bfloat16, 1 sequence 5.5 us (13.9 on the
-        # general kernel), 8 5.8 (20.0), 32 15.4 (63.0), in float32 32 17.4 (82.1): better at every size, so widths alone decide.
+        # One row a sequence: the walk over the states by bulk copies. 16 heads of 128 x 128 in bfloat16, 1 sequence 5.5 us (12.3 on the
+        # general kernel), 8 6.0 (19.6), 32 15.2 (62.6), 512 251 (1,062); of 16 x 16 1 sequence 4.3 (9.9), 512 59 (175); 8 heads of
+        # 256 x 64 1 sequence 5.6 (13.6); float32 the same. Better at every size of 1 x 16 to 256 x 64 and 128 x 128 measured: widths alone decide.
         if (ctx.max_new == 1 and proj.shape[0] == ctx.n_seqs and state.data_ptr() % 16 == 0
                 and self._fn("lin_attn_step_takes")(c_int(dk), c_int(dv))):
             _check(self._fn("lin_attn_step")(
@@ -1266,8 +1267,10 @@ class SsdKernels:
     runs of columns behind it. `dtype` is the element type of activations; step sizes, decays, state and sums are float32."""
     CHUNK, CHUNK_MIN_ROWS, CHUNK_MAX_STATE = 128, 64, 256
     # (sequence, head) pairs of a decode step from which on their states go through shared memory: about two for every block that stays
-    # (of 64 columns x 128 states: 512 pairs take 8.3 us, 9.3 in registers; with fewer there is no next pair to load meanwhile)
-    STEP_MIN_UNITS = 512
+    # (of 64 columns x 128 states: 512 pairs take 8.4 us, 9.2 in registers; with fewer there is no next pair to load meanwhile). A pair
+    # costs a block its barriers whatever its state: narrow ones, whose blocks of the walk are small, stay in registers. 4,096 pairs of
+    # 64 columns x 16 states 30.6 us (38.9 in registers), x 128 59.3 (77.5), 128 x 128 110 (146); 32 x 64 32.1 (22.5), 16 x 16 31.4 (20.9).
+    STEP_MIN_UNITS, STEP_MIN_COLS = 512, 64
 
     def __init__(self, dtype: torch.dtype):
         if dtype not in _SUFFIX:
@@ -1302,7 +1305,7 @@ class SsdKernels:
             chunked = self.dtype == torch.bfloat16 and ctx.max_new >= self.CHUNK_MIN_ROWS
         chunked = chunked and n_state <= self.CHUNK_MAX_STATE
         if (not chunked and weight is None and ctx.max_new == 1 and T == ctx.n_seqs and T * n_heads >= self.STEP_MIN_UNITS
-                and state.data_ptr() % 16 == 0 and self._fn("ssd_step_takes")(c_int(head_dim), c_int(n_state))):
+                and head_dim >= self.STEP_MIN_COLS and state.data_ptr() % 16 == 0 and self._fn("ssd_step_takes")(c_int(head_dim), c_int(n_state))):
             _check(self._fn("ssd_step")(
                 self._view(xbc, "xbc"), c_int(xbc.stride(0)), self._view(dt, "dt"), c_int(dt.stride(0)), _ptr(dt_bias, torch.float32, "dt_bias"),
                 _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), c_int(z.stride(0)),

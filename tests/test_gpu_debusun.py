@@ -537,13 +537,27 @@ def test_a_decode_step_with_its_states_through_shared_memory(dtype, H, G, V, N, 
                           err_flag=torch.zeros(1, dtype=torch.int32, device="cuda"))
     got = []
     for least in (1, 1 << 30):          # this kernel, then the walk
-        k.STEP_MIN_UNITS = least
+        k.STEP_MIN_UNITS, k.STEP_MIN_COLS = least, 1
         st, out = state.cuda().contiguous(), torch.full((B, H * V), float("nan"), dtype=dtype, device="cuda")
         k.scan(xbc.cuda(), dt.cuda(), dt_bias.cuda(), a_log.cuda(), dskip.cuda(), z.cuda(), st, ctx, out, H, G, V, N)
         got.append((st, out.double()))
     assert int(ctx.err_flag) == 0 and torch.equal(got[0][0], got[1][0])
     tol = 1e-6 * N ** 0.5 + (2.0 ** -7 if dtype == torch.bfloat16 else 0.0)
     assert float((got[0][1] - got[1][1]).abs().max()) < tol * float(got[1][1].abs().max())
+
+
+def test_a_decode_step_of_narrow_heads_stays_in_registers():
+    """From how many pairs, and of which widths, a decode step's states go through shared memory."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    for H, V, N, B, ring in ((64, 64, 16, 8, True), (64, 64, 16, 7, False), (128, 32, 64, 32, False), (128, 16, 16, 64, False), (16, 128, 128, 32, True)):
+        k, seen = KernelSet(torch.bfloat16).ssd, []
+        get = k._fn
+        k._fn = lambda name: seen.append(name) or get(name)
+        xbc, dt, z, dt_bias, a_log, dskip, state, slots = _scan_case(torch.bfloat16, H, 1, V, N, (1,) * B, 4)
+        ctx = SimpleNamespace(n_seqs=B, max_new=1, seq_start=torch.arange(B + 1, dtype=torch.int32).cuda(), slots=slots.cuda())
+        out = torch.empty((B, H * V), dtype=torch.bfloat16, device="cuda")
+        k.scan(xbc.cuda(), dt.cuda(), dt_bias.cuda(), a_log.cuda(), dskip.cuda(), z.cuda(), state.cuda().contiguous(), ctx, out, H, 1, V, N)
+        assert ("ssd_step" in seen, "ssd" in seen) == (ring, not ring), (H, V, B, seen)
 
 
 @pytest.mark.parametrize("taps,C", [(2, 12), (3, 520), (4, 64), (4, 516)])
