@@ -250,7 +250,7 @@ gemm_nt_tiled_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* __r
   }
 }
 
-// The same product for up to 64 rows with register tiles: a block of 256 threads owns a BM x 128 tile of
+// The same product for up to 64 rows (and 128 where blocks are few) with register tiles: a block of 256 threads owns a BM x 128 tile of
 // C, a thread (BM/16) x 8 outputs as (BM/64) x 2 groups of 4 x 4, 64 columns / rows apart so that its
 // operands are 16-byte shared-memory loads. A and B tiles of 16 k are fetched from global memory as
 // 16-byte vectors into registers while the previous tile is multiplied, then stored k-major
@@ -390,9 +390,8 @@ template <typename TI, typename TO>
 __global__ void __launch_bounds__(256, 2)
 gemm_nt_paired_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* __restrict__ C, int M, int N, int K,
                        int lda, int ldb, int ldc, int k_per_split, GemmBatch batch) {
-  constexpr int BM = 128, BN = 128, BK = 16, TMG = BM / 64;   // TMG groups of 4 rows per thread
-  constexpr int A_VEC = BM * BK / 4 / 256;                 // 16-byte vectors of the A tile per thread (1 or 2)
-  constexpr int B_VEC = BN * BK / 4 / 256;                 // 2
+  constexpr int BM = 128, BN = 128, BK = 16, TMG = 2;      // two groups of 4 rows per thread
+  constexpr int A_VEC = 2, B_VEC = 2;                      // 16-byte vectors of either tile per thread
   constexpr int AP = BM + 4, BP = BN + 4;                  // padded rows: the transposing stores meet two to a bank, not four
   __shared__ __align__(16) float As[2][BK][AP];
   __shared__ __align__(16) float Bs[2][BK][BP];

@@ -137,6 +137,13 @@ def test_gemm_nt_generic(kernel_sets, dtype, M, N, K):
             assert rel_err(parts.sum(0).cpu(), want) < tol32
 
 
+def test_gemm_nt_generic_kernel_choice(kernel_sets):
+    """One row of tiles on no more blocks than SMs keeps the kernel with a multiply-add an instruction."""
+    for M, N, ksplit, pairs in [(65, 16384, 1, False), (128, 148 * 128, 1, False), (128, 148 * 128 + 1, 1, True), (96, 2048, 8, False),
+                                (96, 6144, 6, True), (129, 128, 1, True), (2778, 1024, 1, True)]:
+        assert all(bool(ks._fn("gemm_nt_pairs")(M, N, ksplit)) == pairs for ks in kernel_sets.values()), (M, N, ksplit)
+
+
 def test_gemm_nt_generic_split_choice():
     from scriptling_llm_lib_b200.csrc.bindings import KernelSet
     assert KernelSet.gemm_nt_split(8, 2048, 8192, 148) == 1             # few rows: no cut
