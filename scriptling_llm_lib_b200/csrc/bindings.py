@@ -901,7 +901,11 @@ class SequenceKernels:
             raise KernelError("delta_rule works on float32 queries, keys, values and state [slots, heads, dk, dv]")
         if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.DELTA_MIN_ROWS and max(dk, dv) <= ChunkKernels.CHUNK:
             self.chunk.delta(qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv)
-            return
+        else:
+            self.delta_walk(qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv)
+
+    def delta_walk(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
+        """`delta_rule` row by row."""
         _check(self._fn("delta_rule")(self._view(qk, "qk"), c_int(qk.stride(0)), self._view(v, "v"), c_int(v.stride(0)),
                                       _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"),
                                       _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),

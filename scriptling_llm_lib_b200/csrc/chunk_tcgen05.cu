@@ -518,7 +518,8 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
     if (tid < n) {
       const float* e = p.bd + (size_t)(row + tid) * (2 * p.H + p.G) + h;
       bt = e[0];
-      c = fmax(log2((double)e[p.H]), -1000.0);
+      c = log2((double)e[p.H]);
+      if (c < -1000.0) c = -1000.0;                // not fmax, which would turn a decay that is no number into one of 0
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {

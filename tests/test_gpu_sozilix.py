@@ -475,6 +475,45 @@ def test_the_delta_rule_in_chunks_against_the_recurrence(H, G, dk, dv, alike):
     assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
 
 
+def _delta_case(lens, H, G, dk, dv, seed):
+    g = torch.Generator().manual_seed(seed)
+    T = sum(lens)
+    unit = lambda t: t / t.square().sum(-1, keepdim=True).sqrt()      # noqa: E731
+    q, keys = unit(torch.randn(T, G, dk, generator=g)) * dk ** -0.5, unit(torch.randn(T, G, dk, generator=g))
+    wide = torch.cat([q.reshape(T, -1), keys.reshape(T, -1), torch.randn(T, H * dv, generator=g)], 1)
+    bd = torch.cat([torch.rand(T, H, generator=g), torch.rand(T, H, generator=g) ** 0.05, (q * keys).sum(-1)], 1)
+    return wide, bd, torch.randn(len(lens) + 1, H, dk, dv, generator=g)
+
+
+def _delta_both(wide, bd, state0, lens, slots, H, G, dk, dv):
+    """Outputs and states of the walk over the rows and of the chunks, on the same inputs."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, got = KernelSet(torch.bfloat16).seq, []
+    ctx = _Ctx(lens, slots, "cuda:0")
+    ctx.err_flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for chunks in (False, True):
+        st, wd, o = state0.clone().cuda(), wide.cuda(), torch.zeros(sum(lens), H * dv, device="cuda")
+        run = k.chunk.delta if chunks else k.delta_walk
+        run(wd[:, :2 * G * dk], wd[:, 2 * G * dk:], bd.cuda(), st, ctx, o, H, G, dk, dv)
+        got.append((o.cpu(), st.cpu()))
+    assert int(ctx.err_flag) == 0
+    return got
+
+
+def test_a_decay_that_is_not_a_number_reaches_the_state_in_chunks():
+    """A NaN decay in the second of three chunks: the head's rows from there on and its state are NaN, as row by row; the other head's
+    are not, and a decay of 0 still forgets."""
+    lens, H, G, dk, dv = [300], 2, 1, 64, 32
+    wide, bd, state0 = _delta_case(lens, H, G, dk, dv, 3)
+    bd[190, H + 0] = float("nan")
+    bd[190, H + 1] = 0.0
+    (o, st), (oc, sc) = _delta_both(wide, bd, state0, lens, [1], H, G, dk, dv)
+    for a, b in ((o[128:].view(-1, H, dv)[:, 0][62:], oc[128:].view(-1, H, dv)[:, 0][62:]), (st[1, 0], sc[1, 0])):
+        assert bool(a.isnan().all()) and bool(b.isnan().all())
+    assert float((o.view(-1, H, dv)[:, 1] - oc.view(-1, H, dv)[:, 1]).abs().max()) < 2e-5 * float(o.view(-1, H, dv)[:, 1].abs().max())
+    assert float((st[1, 1] - sc[1, 1]).abs().max()) < 2e-5 * float(st[1, 1].abs().max())
+
+
 # ------------------------------------------------------------------ generation
 @pytest.mark.parametrize("cfg,seed", [(CFG_A, 21), (CFG_B, 22)])
 def test_greedy_generation_through_the_entry_point(tmp_path, cfg, seed):
