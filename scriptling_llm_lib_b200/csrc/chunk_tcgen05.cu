@@ -367,12 +367,59 @@ __device__ __forceinline__ void fetch_rows(float (&f)[PIECES][8], const float* s
     }
   }
 }
+// What is not finite in a row's key, value, step or decay may reach that row and those behind it, but a product over a chunk's rows
+// multiplies it by the zeros in front of it as well. So it is put into the tiles as 0, and the rows that it belongs to are made NaN
+// where they are stored: from `row` on, in column c from `col[c]` on (Q: none).
+struct Watch { int row, any, col[Q]; };
+__device__ __forceinline__ bool finite(float x) { return x * 0.f == 0.f; }
+__device__ __forceinline__ bool finite8(const float (&f)[8]) {
+  float t = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; k++) t = fmaf(f[k], 0.f, t);
+  return t == 0.f;
+}
+__device__ __forceinline__ void open_watch(Watch& w) {
+  if (threadIdx.x < Q) w.col[threadIdx.x] = Q;
+  if (threadIdx.x == 0) { w.row = Q; w.any = 0; }
+}
+__device__ __forceinline__ void clear_rows(float (&f)[PIECES][8]) {
+#pragma unroll
+  for (int u = 0; u < PIECES; u++)
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (!finite(f[u][k])) f[u][k] = 0.f;
+}
+__device__ __forceinline__ void watch_columns(Watch& w, float (&f)[8], int r, int c) {
+  if (finite8(f)) return;
+  w.any = 1;
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (!finite(f[k])) { atomicMin(&w.col[c + k], r); f[k] = 0.f; }
+}
+// row i of what is stored, columns c0 .. c0 + 31
+__device__ __forceinline__ void spoil(const Watch& w, uint32_t (&v)[32], int i, int c0) {
+  if (w.row == Q && !w.any) return;
+#pragma unroll
+  for (int k = 0; k < 32; k++)
+    if (i >= min(w.row, w.col[c0 + k])) v[k] = 0x7fc00000u;
+}
+
 // the pieces, row r times scale[r], into the tile's planes
-template <bool SCALED>
-__device__ __forceinline__ void put_rows(uint8_t* tile, float (&f)[PIECES][8], const float* scale) {
+enum { UNWATCHED, BY_ROW, BY_COLUMN };
+template <bool SCALED, int WATCHED = UNWATCHED>
+__device__ __forceinline__ void put_rows(uint8_t* tile, float (&f)[PIECES][8], const float* scale, Watch* watch = nullptr) {
 #pragma unroll
   for (int u = 0; u < PIECES; u++) {
     const int i = u * NT + threadIdx.x, r = i >> 4;
+    if constexpr (WATCHED == BY_COLUMN) watch_columns(*watch, f[u], r, (i & 15) * 8);
+    if constexpr (WATCHED == BY_ROW) {
+      if (!finite8(f[u])) {
+        atomicMin(&watch->row, r);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          if (!finite(f[u][k])) f[u][k] = 0.f;
+      }
+    }
     if constexpr (SCALED) {
       const float w = scale[r];
 #pragma unroll
@@ -502,6 +549,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   float* t = (float*)ya;
   float *hi = (float*)(ya + TILE_BYTES), *lo = hi + Q, *beta = lo + Q, *front = beta + Q, *back = front + Q, *bfront = back + Q;
   __shared__ double part_s[4];
+  __shared__ Watch watch;
   const int n = min(Q, len - r0), row = start + r0, h = blockIdx.y, g = h / (p.H / p.G);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* qrow = p.qk + (size_t)row * p.ld_qk + (size_t)g * p.dk;
@@ -509,6 +557,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   const float* vrow = p.v + (size_t)row * p.ld_v + (size_t)h * p.dv;
   float f[PIECES][8];
   fetch_rows<VEC>(f, krow, p.ld_qk, n, p.dk);
+  open_watch(watch);
   Unit u;
   u.open((uint8_t*)(bfront + Q));
   // a thread a row: the running sum of log2 d, in double; a decay of 0 is far below what a float can hold from one row to the next
@@ -519,7 +568,12 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
       const float* e = p.bd + (size_t)(row + tid) * (2 * p.H + p.G) + h;
       bt = e[0];
       c = log2((double)e[p.H]);
-      if (c < -1000.0) c = -1000.0;                // not fmax, which would turn a decay that is no number into one of 0
+      if (c < -1000.0) c = -1000.0;
+      if (!finite(bt) || !(c <= 1000.0)) {
+        atomicMin(&watch.row, tid);
+        bt = 0.f;
+        c = 0.0;
+      }
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -528,7 +582,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
     }
     if (lane == 31) part_s[warp] = c;
   }
-  put_rows<false>(xa, f, nullptr);
+  put_rows<false, BY_ROW>(xa, f, nullptr, &watch);
   u.ready();
   const int dsteps = (p.dk + 15) / 16;
   if (tid == 0) {
@@ -561,6 +615,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   }
   fetch_rows<VEC>(f, krow, p.ld_qk, n, p.dk);
   u.done();
+  if (watch.row < Q) clear_rows(f);
   put_rows<true>(xa, f, back);
   const int i = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;       // a warp has 32 rows (lanes) and 32 columns
   const uint32_t t_lane = u.tmem + ((uint32_t)((warp & 3) * 32) << 16);
@@ -613,7 +668,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   put_tmem(t_lane, c0, w);
   __syncthreads();                                 // T has been read from where the scaled values go
   const size_t unit = (first_chunk(start, b) + blockIdx.x) * p.H + h, mat = unit * MAT;
-  put_rows<true>(ya, f, beta);
+  put_rows<true, BY_COLUMN>(ya, f, beta, &watch);
   u.ready();
   if (tid == 0) {                                  // U0
     product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
@@ -635,8 +690,10 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
     product<true, true>(u.tmem + 384, smem_u32(xa), smem_u32(ya), 8);
     u.commit();
   }
+  spoil(watch, w, i, c0);
   store_quads(p.o0 + mat, i, c0, w);
   u.done();
+  if (watch.row < Q) clear_rows(f);
   put_rows<true>(ya, f, bfront);
   take(t_lane + 384 + c0, w);
   u.ready();
@@ -644,6 +701,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
     product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
     u.commit();
   }
+  spoil(watch, w, Q - 1, c0);                      // the state behind the chunk has seen all its rows
   store_quads(p.n + mat, i, c0, w);
   u.done();
   take(t_lane + 384 + c0, w);

@@ -514,6 +514,36 @@ def test_a_decay_that_is_not_a_number_reaches_the_state_in_chunks():
     assert float((st[1, 1] - sc[1, 1]).abs().max()) < 2e-5 * float(st[1, 1].abs().max())
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("where", ["key", "value", "beta", "decay", "query", "state"])
+def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
+    """One element that is not finite, in rows of the first, a middle and the last chunk of three runs: outputs and states that are not
+    finite are those of the walk row by row, element by element, and the others agree with it."""
+    lens, H, G, dk, dv = [300, 140, 257], 3, 1, 64, 40
+    for at in (5, 131, 299, 300 + 127, 440 + 200):
+        wide, bd, state0 = _delta_case(lens, H, G, dk, dv, 4)
+        if where == "key":
+            wide[at, G * dk + 7] = bad
+        elif where == "query":
+            wide[at, 7] = bad
+            bd[at, 2 * H] = bad                      # k . q
+        elif where == "value":
+            wide[at, 2 * G * dk + dv + 3] = bad
+        elif where == "beta":
+            bd[at, 1] = bad
+        elif where == "decay":
+            bd[at, H + 1] = abs(bad)                 # an exponential: never negative
+        else:
+            state0[2, 1, 3, 5] = bad
+        (o, st), (oc, sc) = _delta_both(wide, bd, state0, lens, [2, 0, 3], H, G, dk, dv)
+        assert not bool(o.isfinite().all())
+        for a, b in ((o, oc), (st, sc)):
+            same = a.isfinite() == b.isfinite()
+            assert bool(same.all()), (where, at, (~same).nonzero()[:4])
+            both = a.isfinite()
+            assert float((a[both] - b[both]).abs().max()) < 2e-5 * float(a[both].abs().max())
+
+
 # ------------------------------------------------------------------ generation
 @pytest.mark.parametrize("cfg,seed", [(CFG_A, 21), (CFG_B, 22)])
 def test_greedy_generation_through_the_entry_point(tmp_path, cfg, seed):
