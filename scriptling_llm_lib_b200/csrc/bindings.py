@@ -1054,6 +1054,10 @@ class MixKernels:
                 _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(n_heads), c_int(dk), c_int(dv),
                 c_int(ctx.engine.sm_count), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "lin_attn_step")
             return
+        self.lin_attn_walk(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
+
+    def lin_attn_walk(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
+        """`lin_attn_decay` in pieces of up to 32 rows one after the other."""
         _check(self._fn("lin_attn_decay")(
             _ptr(proj, self.dtype, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),

@@ -75,8 +75,38 @@ __device__ __forceinline__ void fetch(uint4 (&raw)[PIECES], const bf16* src, int
     }
   }
 }
+// What is not finite in a row's value (the delta rule: key, step or decay as well) may reach that row and those behind it, but a
+// product over a chunk's rows multiplies it by the zeros in front of it too. So it is put into the tile as 0, and the rows that it
+// belongs to are made NaN where they are stored: from `row` on, in column c from `col[c]` on (Q: none).
+struct Watch { int row, any, col[Q]; };
+__device__ __forceinline__ bool finite(float x) { return x * 0.f == 0.f; }
+__device__ __forceinline__ bool finite8(const float (&f)[8]) {
+  float t = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; k++) t = fmaf(f[k], 0.f, t);
+  return t == 0.f;
+}
+__device__ __forceinline__ void open_watch(Watch& w) {
+  if (threadIdx.x < Q) w.col[threadIdx.x] = Q;
+  if (threadIdx.x == 0) { w.row = Q; w.any = 0; }
+}
+__device__ __forceinline__ void watch_columns(Watch& w, float (&f)[8], int r, int c) {
+  if (finite8(f)) return;
+  w.any = 1;
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if (!finite(f[k])) { atomicMin(&w.col[c + k], r); f[k] = 0.f; }
+}
+// row i of what is stored, columns c0 .. c0 + 31
+__device__ __forceinline__ void spoil(const Watch& w, uint32_t (&v)[32], int i, int c0) {
+  if (w.row == Q && !w.any) return;
+#pragma unroll
+  for (int k = 0; k < 32; k++)
+    if (i >= min(w.row, w.col[c0 + k])) v[k] = 0x7fc00000u;
+}
+
 // silu of what was fetched, row r times scale[r] (null: 1), into the tile's planes
-__device__ __forceinline__ void put_silu(uint8_t* tile, const uint4 (&raw)[PIECES], const float* scale) {
+__device__ __forceinline__ void put_silu(uint8_t* tile, const uint4 (&raw)[PIECES], const float* scale, Watch* watch = nullptr) {
 #pragma unroll
   for (int u = 0; u < PIECES; u++) {
     const int i = u * NT + threadIdx.x, r = i >> 4, c = (i & 15) * 8;
@@ -88,6 +118,7 @@ __device__ __forceinline__ void put_silu(uint8_t* tile, const uint4 (&raw)[PIECE
       f[2 * k] = silu_f(__low2float(h[k])) * w;
       f[2 * k + 1] = silu_f(__high2float(h[k])) * w;
     }
+    if (watch) watch_columns(*watch, f, r, c);
     put8(tile, r, c, f);
   }
 }
@@ -241,12 +272,14 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   uint8_t* qa = aligned_smem(smem_raw);
   uint8_t* xa = qa + TILE_BYTES;                   // the state, then the keys, then the values
   float* pw = (float*)(xa + TILE_BYTES);
+  __shared__ Watch watch;
   const int n = min(Q, len - r0), vblocks = (p.V + Q - 1) / Q, h = blockIdx.y / vblocks, v0 = (blockIdx.y % vblocks) * Q;
   const int vn = min(Q, p.V - v0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bf16* row = p.proj + (size_t)(start + r0) * p.ld;
   uint4 raw[PIECES];
   fetch(raw, row + p.q_col + (size_t)h * p.D, p.ld, n, p.D, p.vec);
   fill_powers(pw, p.decay[h]);
+  open_watch(watch);
   Unit u;
   u.open((uint8_t*)(pw + 2 * (Q + 4)));
   put_silu(qa, raw, nullptr);
@@ -273,7 +306,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
     uint32_t s[32];
     tmem_ld32(t_lane + 128 + c0, s);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    put_silu(xa, raw, nullptr);                    // the keys have been read
+    put_silu(xa, raw, nullptr, &watch);            // the keys have been read
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();                               // every warp holds its scores: the planes may go over them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -302,6 +335,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int k = 0; k < 32; k++) c[k] = __float_as_uint(fmaf(f, __uint_as_float(a[k]), __uint_as_float(c[k])));
+  spoil(watch, c, i, c0);
   if (i < n) store_row(dst, c, c0, vn, p.vec);
   u.close(p.err);
 }
@@ -367,41 +401,12 @@ __device__ __forceinline__ void fetch_rows(float (&f)[PIECES][8], const float* s
     }
   }
 }
-// What is not finite in a row's key, value, step or decay may reach that row and those behind it, but a product over a chunk's rows
-// multiplies it by the zeros in front of it as well. So it is put into the tiles as 0, and the rows that it belongs to are made NaN
-// where they are stored: from `row` on, in column c from `col[c]` on (Q: none).
-struct Watch { int row, any, col[Q]; };
-__device__ __forceinline__ bool finite(float x) { return x * 0.f == 0.f; }
-__device__ __forceinline__ bool finite8(const float (&f)[8]) {
-  float t = 0.f;
-#pragma unroll
-  for (int k = 0; k < 8; k++) t = fmaf(f[k], 0.f, t);
-  return t == 0.f;
-}
-__device__ __forceinline__ void open_watch(Watch& w) {
-  if (threadIdx.x < Q) w.col[threadIdx.x] = Q;
-  if (threadIdx.x == 0) { w.row = Q; w.any = 0; }
-}
 __device__ __forceinline__ void clear_rows(float (&f)[PIECES][8]) {
 #pragma unroll
   for (int u = 0; u < PIECES; u++)
 #pragma unroll
     for (int k = 0; k < 8; k++)
       if (!finite(f[u][k])) f[u][k] = 0.f;
-}
-__device__ __forceinline__ void watch_columns(Watch& w, float (&f)[8], int r, int c) {
-  if (finite8(f)) return;
-  w.any = 1;
-#pragma unroll
-  for (int k = 0; k < 8; k++)
-    if (!finite(f[k])) { atomicMin(&w.col[c + k], r); f[k] = 0.f; }
-}
-// row i of what is stored, columns c0 .. c0 + 31
-__device__ __forceinline__ void spoil(const Watch& w, uint32_t (&v)[32], int i, int c0) {
-  if (w.row == Q && !w.any) return;
-#pragma unroll
-  for (int k = 0; k < 32; k++)
-    if (i >= min(w.row, w.col[c0 + k])) v[k] = 0x7fc00000u;
 }
 
 // the pieces, row r times scale[r], into the tile's planes

@@ -614,6 +614,40 @@ def test_linear_attention_in_chunks_against_the_recurrence(H, D, V, pad):
     assert torch.equal(st[4].cpu(), state0[4])          # a slot no sequence of the step holds is left alone
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["query", "key", "value", "state"])
+def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
+    """One element that is not finite, in rows of the first, a middle and the last chunk: what is not finite behind it is what the
+    recurrence in 64 bits leaves so, element by element, and the rest agrees with it."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, H, D, V, lens, slots = KernelSet(torch.bfloat16).mix, 2, 24, 40, [300, 140, 257], [2, 0, 3]
+    start, decay = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32), torch.tensor([0.9, 0.99])
+    for at in (5, 131, 299, 300 + 127, 440 + 200):
+        g = torch.Generator().manual_seed(at)
+        proj, state0 = torch.randn(sum(lens), 2 * H * D + H * V, generator=g).bfloat16(), torch.randn(4, H, D, V, generator=g)
+        if where == "state":
+            state0[2, 1, 3, 5] = bad
+        else:
+            proj[at, {"query": D + 7, "key": H * D + D + 7, "value": 2 * H * D + V + 3}[where]] = bad
+        ctx = SimpleNamespace(seq_start=torch.from_numpy(start).cuda(), slots=torch.tensor(slots, dtype=torch.int32).cuda(), n_seqs=len(lens),
+                              max_new=max(lens), err_flag=torch.zeros(1, dtype=torch.int32, device="cuda"))
+        st, o = state0.clone().cuda(), torch.zeros(sum(lens), H * V, device="cuda")
+        k.chunk.lin_attn(proj.cuda(), 0, H * D, 2 * H * D, decay.cuda(), st, ctx, o, H, D, V)
+        q, kk, v = (plain.silu(t).view(sum(lens), H, -1) for t in proj.double().split([H * D, H * D, H * V], 1))
+        want, after = torch.empty((sum(lens), H, V), dtype=torch.float64), state0.double()
+        for b, slot in enumerate(slots):
+            S = state0[slot].double()
+            for t in range(start[b], start[b + 1]):
+                S = decay.double()[:, None, None] * S + kk[t, :, :, None] * v[t, :, None]
+                want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+            after[slot] = S
+        assert int(ctx.err_flag) == 0 and not bool(want.isfinite().all())
+        for a, b in ((want.view(sum(lens), -1), o.cpu()), (after, st.cpu())):
+            both = a.isfinite()
+            assert torch.equal(both, b.isfinite()), (where, at, (both != b.isfinite()).nonzero()[:4])
+            assert float((a[both] - b[both]).abs().max()) < 1e-5 * float(a[both].abs().max())
+
+
 def test_the_norm_adds_a_normed_addend_and_keeps_the_sum():
     from scriptling_llm_lib_b200.csrc.bindings import KernelSet
     for dtype in (torch.float32, torch.bfloat16):
