@@ -67,6 +67,8 @@ struct FtArgs {
   const float* sink;           // [H] or null: exp(sink[h]) joins head h's denominator, with no key and no value
   const bf16* gate;            // null, or [T, gate_ld]: output element (h, d) is multiplied by the sigmoid of column h * vd + d
   int gate_ld;
+  const bf16 *q, *kpages, *vpages;   // what the maps describe
+  int q_ld;
 };
 
 // What a block works on in its r-th round.
@@ -558,12 +560,42 @@ __device__ __forceinline__ void ft_ld64(uint32_t taddr, uint32_t (&s)[64]) {
   tmem_ld32(taddr + 32, *(uint32_t(*)[32])&s[32]);
 }
 
+// One query's sums over columns c0 .. c0 + 31 of the values, key by key and over those alone that it sees. For a row whose sums are not
+// finite: on the tensor cores a page's values all enter them, with weights of zero, and 0 times what is not finite is NaN.
+__device__ __noinline__ void fp_sums_by_key(const FtArgs& p, const bf16* q, const int* bt, int g, int qpos, int qfirst, float msc, int c0, float (&acc)[32]) {
+  const float sc = p.scale * FT_LOG2E;
+#pragma unroll
+  for (int c = 0; c < 32; c++) acc[c] = 0.f;
+  for (int key = 0; key <= qpos; key++) {
+    if (!key_seen(key, qpos, qfirst, p.keep)) {          // between the kept positions and the window
+      key = qfirst - 1;
+      continue;
+    }
+    const size_t row = ((size_t)bt[key / FT_BK] * p.G + g) * FT_BK + key % FT_BK;
+    float s = 0.f;
+    for (int d = 0; d < p.hd; d += 8) {
+      const F8 a = ld8(q + d), b = ld8(p.kpages + row * p.hd + d);
+#pragma unroll
+      for (int e = 0; e < 8; e++) s = fmaf(a.f[e], b.f[e], s);
+    }
+    if (p.softcap > 0.f) s = __uint_as_float(ft_cap(__float_as_uint(s), p.softcap / p.scale, p.scale / p.softcap));
+    const float w = ft_ex2(fmaf(s, sc, -msc));
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+      if (c0 + c >= p.vd) break;
+      const F8 v = ld8(p.vpages + row * p.vd + c0 + c);
+#pragma unroll
+      for (int e = 0; e < 8; e++) acc[c + e] = fmaf(w, v.f[e], acc[c + e]);
+    }
+  }
+}
+
 // Keys of up to KD and values of up to VD dims (with rounded weights 64 or 128 either, not both 64: that is the kernel above),
 // narrower heads as there. PARTS: 1 rounds the weights to bfloat16, 3 keeps all their bits.
 template <int KD, int VD, int FT_STAGES, int PARTS>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                       const __grid_constant__ CUtensorMap map_v, FtArgs p, uint32_t smem_bytes) {
+                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FtArgs p, uint32_t smem_bytes) {
   constexpr uint32_t Q_BYTES = FT_BQ * KD * 2, K_BYTES = FT_BK * KD * 2, V_BYTES = FT_BK * VD * 2;
   constexpr uint32_t QA = FT_BQ * 128, KA = FT_BK * 128;       // bytes of one 64-wide block of Q and of a K or V page
   constexpr int NK = KD / 64, NV = VD / 64;                    // such blocks per key (query) head and per value head
@@ -861,6 +893,19 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         uint32_t v[32];
         tmem_ld32(t_lane + 128 + c0, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if constexpr (PARTS == 3) {                 // (a sum l that is not finite has seen a score that is not)
+          float t = 0.f;
+#pragma unroll
+          for (int k = 0; k < 32; k++) t = fmaf(__uint_as_float(v[k]), 0.f, t);
+          if (r < sb.nq && t != 0.f && l < INFINITY && c0 < p.vd) {
+            float acc[32];
+            fp_sums_by_key(p, p.q + (size_t)(it.row0 + sb.r0 + r) * p.q_ld + (size_t)sb.h * p.hd, p.block_table + (size_t)it.b * p.max_pages, it.g,
+                           qpos, qfirst, m_ref == -INFINITY ? 0.f : m_ref * sc, c0, acc);
+#pragma unroll
+            for (int k = 0; k < 32; k++) v[k] = __float_as_uint(acc[k]);
+          }
+          __syncwarp();
+        }
         if (r < sb.nq) {
           if (p.gate != nullptr) ft_gate(v, p.gate + (size_t)(it.row0 + sb.r0 + r) * p.gate_ld + (size_t)sb.h * p.vd + c0, p.vd - c0);
 #pragma unroll
@@ -959,7 +1004,7 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
   }
   if (hd <= 64 && vd <= 64 && weight_parts == 1) {
     FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, 0, softcap, sink,
-             (const bf16*)gate, gate_ld};
+             (const bf16*)gate, gate_ld, (const bf16*)q, (const bf16*)kpages, (const bf16*)vpages, q_ld};
     dim3 grid((unsigned)(n_items < 2LL * sm_count ? n_items : 2LL * sm_count));     // two blocks per SM that stay
     return ft_launch<64, 3>(mq, mk, mv, a, grid, stream);
   }
@@ -972,7 +1017,7 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
   if (!pair_heads && weight_parts == 3 && window == 0 && n_qt >= 4 && (long long)H * ((n_qt + 1) / 2) * B <= sm_count) pair_heads = 2;
   n_items = pair_heads == 1 ? (long long)(H / 2) * n_qt * B : (long long)H * ((n_qt + 1) / 2) * B;
   FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, pair_heads, softcap, sink,
-           (const bf16*)gate, gate_ld};
+           (const bf16*)gate, gate_ld, (const bf16*)q, (const bf16*)kpages, (const bf16*)vpages, q_ld};
   dim3 grid((unsigned)(n_items < (long long)sm_count ? n_items : (long long)sm_count));       // one block per SM that stays
   if (weight_parts == 3) {
     if (vd <= 64) {

@@ -952,3 +952,40 @@ def test_repeat_penalty_kernel():
         want = plain.apply_repeat_penalty(logits[i].numpy(), recent[i], p, last_n)
         assert rel_err(lg[i].cpu(), want) < 1e-6
     assert torch.equal(lg[2].cpu(), logits[2])                           # penalty 0: off
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("H, G, hd, vd, window, keep, softcap", [(4, 2, 64, 128, 0, 0, None), (3, 3, 80, 80, 100, 0, None), (2, 1, 16, 40, 90, 30, 5.0),
+                                                                 (2, 2, 192, 128, 0, 0, None)])
+def test_a_value_that_is_not_finite_is_seen_by_the_queries_that_see_it(kernel_sets, H, G, hd, vd, window, keep, softcap, bad):
+    """Prompt attention with float weights on tcgen05: one value of one key of either sequence is not finite, in the first, a middle and
+    the last page; the outputs that are not finite are those of the queries that see it, in its column, and the others are as they are
+    with an ordinary value there, to two roundings of the output."""
+    from types import SimpleNamespace
+    ks, lens, pos0 = kernel_sets[torch.bfloat16], [300, 130], [70, 0]
+    T, ends = sum(lens), [n + p for n, p in zip(lens, pos0)]
+    pages = [-(-e // 64) for e in ends]
+    table = torch.zeros(2, max(pages), dtype=torch.int32)
+    table[0, :pages[0]], table[1, :pages[1]] = torch.arange(pages[0]), torch.arange(pages[0], sum(pages))
+    kp, v0 = dev(rand(sum(pages), G, 64, hd, seed=1), torch.bfloat16), dev(rand(sum(pages), G, 64, vd, seed=2), torch.bfloat16)
+    q = dev(rand(T, H * hd, seed=3), torch.bfloat16)
+    i32 = lambda a: dev(a, torch.int32)      # noqa: E731
+    start, err, table = i32([0, lens[0], T]), torch.zeros(1, dtype=torch.int32, device="cuda"), table.cuda()
+
+    def run(v):
+        out = torch.full((T, H * vd), 7.0, dtype=torch.bfloat16, device="cuda")
+        ks.prefill_attention_tc.attn(q, out, start, i32(pos0), table, kp, v, 2, max(lens), H, G, hd, window, hd ** -0.5, err, softcap=softcap,
+                                     keep=keep, v_dim=vd, exact_weights=True)
+        return out.view(T, H, vd)
+    plain_out = run(v0)
+    for at in ((3, 5), (200, 64), (369, 129)):
+        v = v0.clone()
+        for b in range(2):
+            v[int(table[b, at[b] // 64]), G - 1, at[b] % 64, 9] = bad
+        out = run(v)
+        hit = torch.zeros(T, H, vd, dtype=torch.bool, device="cuda")
+        for b, row0 in ((0, 0), (1, lens[0])):
+            pos = pos0[b] + torch.arange(lens[b], device="cuda")
+            sees = (at[b] <= pos) & ((pos - at[b] < window) | (at[b] < keep) if window else True)
+            hit[row0:row0 + lens[b], (G - 1) * (H // G):, 9] = sees[:, None]
+        assert int(err) == 0 and bool(hit.any()) and torch.equal(~hit, out.isfinite())
+        assert float((out - plain_out)[~hit].abs().max()) <= 2.0 ** -7 * float(plain_out.abs().max())
