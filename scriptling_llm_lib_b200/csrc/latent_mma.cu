@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256) latent_merge_wide_kernel(const float* __r
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       ms[i] = ms[i] > -INFINITY ? expf(ms[i] - mx) : 0.f;
-      den += ms[i] > 0.f ? ms[i] * ls[i] : 0.f;
+      den += ms[i] * ls[i];                               // a sum that is no number shows, whatever its weight
     }
     den = warp_sum(den);
     if (sink) den += expf(snk - mx);

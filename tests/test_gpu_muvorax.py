@@ -455,6 +455,24 @@ def test_latent_decode_on_the_tensor_cores(H, D, P, V, R, window, n_split):
         assert float((out.cpu().double() - want.reshape(B, -1)).abs().max()) < 2.0 ** -8 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("sink", [False, True])
+def test_cached_latents_that_are_no_numbers_are_not_passed_over(sink):
+    """A page of a row's keys is NaN and falls to a split of its own: the row's output is NaN, as with one split, and the other row's is not."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, H, R, P, V = KernelSet(torch.bfloat16).mix, 3, 64, 16, 24
+    g = torch.Generator().manual_seed(1)
+    pages, table = torch.randn(10, 1, 64, R + P, generator=g).bfloat16(), torch.arange(10, dtype=torch.int32).view(2, 5)
+    pages[2] = float("nan")
+    qa, wuv = torch.randn(2, H, R + P, generator=g).cuda(), torch.randn(H * V, R, generator=g).bfloat16().cuda()
+    ctx = SimpleNamespace(tok_pos=torch.tensor([300, 250], dtype=torch.int32).cuda(), tok_seq=torch.arange(2, dtype=torch.int32).cuda())
+    for n_split in (1, 5):
+        part = torch.zeros((2, H, n_split, R + 2), device="cuda")
+        k.latent_attn(qa, pages.cuda(), ctx, table.cuda(), part, H, R, P, n_split)
+        olat, out = torch.empty((2, H, R), device="cuda"), torch.empty((2, H * V), dtype=torch.bfloat16, device="cuda")
+        k.latent_expand(part, olat, wuv, out, H, V, R, n_split, sink=torch.zeros(H, device="cuda") if sink else None)
+        assert bool(out[0].isnan().all()) and bool(out[1].isfinite().all()), n_split
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("W, ld, off", [(8, 8, 0), (248, 504, 256), (2048, 4096, 2048), (4096, 4096, 0), (4104, 4104, 0), (2044, 2048, 0),
                                         (256, 516, 4), (1024, 1030, 0)])
