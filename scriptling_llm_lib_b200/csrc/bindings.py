@@ -899,7 +899,7 @@ class SequenceKernels:
             raise KernelError(f"delta_rule: bd is {tuple(bd.shape)}, expected {(qk.shape[0], 2 * n_heads + n_kv)}")
         if qk.dtype != torch.float32 or v.dtype != torch.float32 or tuple(state.shape[1:]) != (n_heads, dk, dv):
             raise KernelError("delta_rule works on float32 queries, keys, values and state [slots, heads, dk, dv]")
-        if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.DELTA_MIN_ROWS and max(dk, dv) <= ChunkKernels.CHUNK:
+        if self.dtype == torch.bfloat16 and ChunkKernels.delta_pays(qk.shape[0], ctx.n_seqs, ctx.max_new, n_heads, dk, dv):
             self.chunk.delta(qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv)
         else:
             self.delta_walk(qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv)
@@ -942,12 +942,37 @@ class SequenceKernels:
 class ChunkKernels:
     """Linear recurrences with a matrix state over many rows, in chunks on tcgen05 (bfloat16 engines; see chunk_tcgen05.cu)."""
     CHUNK = 128
-    # The longest run of a step from which on linear attention goes in chunks. One sequence, 16 heads of 128 x 128: 128 rows take 42 us
-    # in chunks and 40 in pieces of 32 rows (lin_attn_decay), 64 rows 37 and 26; a piece more is 8 us more, a chunk more is nothing
-    # while there are idle SMs.
-    LIN_MIN_ROWS = 144
-    # The same for the gated delta rule. One sequence, 16 heads of 128 x 128: 192 rows take 66 us in chunks and 70 walked row by row.
-    DELTA_MIN_ROWS = 192
+
+    # Chunks or the kernels that walk a sequence's rows: by what either is about to take, in us, at the widths 128, 64 and 32 (and below;
+    # the wider of keys and values). In chunks a step has a floor, the longest run's hand-over, and what its blocks beyond the first wave
+    # take, one a chunk of a head whatever its rows and widths: short runs and narrow heads pay for 128 x 128 tiles. Walked, the longest
+    # run is one chain, and many runs share the SMs' rate. Chunks are counted by their bound, rows / 128 + sequences.
+    # Walked / in chunks, measured: delta rule, 16 heads of 128: 192 rows 69 / 65, 2,048 639 / 173, 8 runs of 200 261 / 167, one of 192
+    # and 100 of 16 504 / 1,036; 16 heads of 16: 2,048 rows 594 / 145, 8 of 200 67 / 108. Linear attention, 16 heads of 128: 144 rows
+    # 47 / 39, 2,048 459 / 78, one of 144 and 100 of 16 488 / 735; 16 heads of 16: 192 rows 27 / 29, 512 65 / 29, 8 of 200 34 / 53.
+    SMS = 148
+
+    @classmethod
+    def _shape(cls, rows, n_seqs, n_heads, width):
+        """(index of the width's figures, blocks beyond one wave)."""
+        blocks = (rows // cls.CHUNK + n_seqs) * n_heads
+        return (0 if width > 64 else 1 if width > 32 else 2), max(0, blocks - cls.SMS)
+
+    @classmethod
+    def delta_pays(cls, rows, n_seqs, longest, n_heads, dk, dv) -> bool:
+        if max(dk, dv) > cls.CHUNK:
+            return False
+        k, more = cls._shape(rows, n_seqs, n_heads, max(dk, dv))
+        chunks = (58, 55, 53)[k] + 2.5 * longest / cls.CHUNK + 0.5 * (n_seqs - 1) + (0.6, 0.44, 0.37)[k] * more
+        return chunks < 8 + max(0.29 * longest, 0.06e-3 * rows * n_heads * dv)
+
+    @classmethod
+    def lin_pays(cls, rows, n_seqs, longest, n_heads, dk, dv) -> bool:
+        if dk > cls.CHUNK:
+            return False
+        k, more = cls._shape(rows, n_seqs, n_heads * -(-dv // cls.CHUNK), max(dk, dv))
+        pieces, together = -(-longest // 32), (rows // 32 + n_seqs) * n_heads * -(-dv // cls.CHUNK)
+        return (38, 32, 30)[k] + (0.45, 0.22, 0.165)[k] * more < (10, 5.5, 5)[k] + max((7, 5.2, 4)[k] * pieces, (0.18, 0.045, 0.02)[k] * together)
 
     def __init__(self):
         self.lib = load_library("chunk_tcgen05")
@@ -1040,7 +1065,7 @@ class MixKernels:
         applied on reading); decay float32 [H]; state float32 [slots, H, dk, dv] (read and advanced); o float32 [T, H dv]."""
         if tuple(state.shape[1:]) != (n_heads, dk, dv) or tuple(o.shape) != (proj.shape[0], n_heads * dv):
             raise KernelError(f"lin_attn_decay shapes: state {tuple(state.shape)}, o {tuple(o.shape)}")
-        if self.dtype == torch.bfloat16 and ctx.max_new >= ChunkKernels.LIN_MIN_ROWS and dk <= ChunkKernels.CHUNK:
+        if self.dtype == torch.bfloat16 and ChunkKernels.lin_pays(proj.shape[0], ctx.n_seqs, ctx.max_new, n_heads, dk, dv):
             self.chunk.lin_attn(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
             return
         # One row a sequence: the walk over the states by bulk copies. 16 heads of 128 x 128 in bfloat16, 1 sequence 5.5 us (12.3 on the

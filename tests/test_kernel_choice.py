@@ -1,0 +1,64 @@
+"""Which kernel a step runs on, by its sizes (no GPU: the launches are recorded, not made)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from scriptling_llm_lib_b200.csrc.bindings import MixKernels, SequenceKernels
+
+
+def _recorded(cls, walk):
+    """A set of kernels whose chunked and walked forms only say which of them ran."""
+    k, ran = cls.__new__(cls), []
+    k.dtype, k._fns = torch.bfloat16, {}
+    k._chunk = SimpleNamespace(delta=lambda *a: ran.append("chunks"), lin_attn=lambda *a: ran.append("chunks"))
+    setattr(k, walk, lambda *a: ran.append("walk"))
+    return k, ran
+
+
+def _ctx(lens):
+    return SimpleNamespace(n_seqs=len(lens), max_new=max(lens), engine=SimpleNamespace(sm_count=148))
+
+
+# measured: walked / in chunks, us
+DELTA = [(16, 128, [2048], "chunks"),                    # 639 / 173
+         (16, 128, [200] * 8, "chunks"),                 # 261 / 167
+         (16, 128, [128], "walk"),                       # 49 / 63
+         (16, 128, [192] + [16] * 100, "walk"),          # 504 / 1,036
+         (16, 128, [1000] + [32] * 64, "walk"),          # 639 / 774
+         (2, 128, [1000] + [32] * 64, "chunks"),         # 308 / 116
+         (4, 128, [192] + [4] * 16, "walk"),             # 66 / 71
+         (16, 64, [192] + [32] * 200, "walk"),           # 536 / 1,407
+         (16, 16, [200] * 8, "walk"),                    # 67 / 108
+         (64, 16, [192] + [16] * 100, "walk"),           # 170 / 2,343
+         (64, 16, [2048], "chunks")]                     # 595 / 398
+
+
+@pytest.mark.parametrize("H, d, lens, want", DELTA)
+def test_the_delta_rule_goes_in_chunks_where_that_is_faster(H, d, lens, want):
+    k, ran = _recorded(SequenceKernels, "delta_walk")
+    T = sum(lens)
+    f = lambda *s: torch.empty(s, device="meta")      # noqa: E731
+    k.delta_rule(f(T, 2 * H * d), f(T, H * d), f(T, 3 * H), f(len(lens), H, d, d), _ctx(lens), f(T, H * d), H, H, d, d)
+    assert ran == [want]
+
+
+LINEAR = [(16, 128, [2048], "chunks"),                   # 459 / 78
+          (16, 128, [144], "chunks"),                    # 47 / 39
+          (16, 128, [144] + [16] * 100, "walk"),         # 488 / 735
+          (16, 128, [1000] + [32] * 64, "walk"),         # 444 / 542
+          (2, 128, [144] + [16] * 100, "walk"),          # 66 / 80
+          (16, 64, [144] + [4] * 16, "walk"),            # 50 / 63
+          (16, 16, [192], "walk"),                       # 27 / 29
+          (16, 16, [512], "chunks"),                     # 65 / 29
+          (16, 16, [200] * 8, "walk"),                   # 34 / 53
+          (64, 16, [1000] + [32] * 64, "walk")]          # 161 / 950
+
+
+@pytest.mark.parametrize("H, d, lens, want", LINEAR)
+def test_linear_attention_goes_in_chunks_where_that_is_faster(H, d, lens, want):
+    k, ran = _recorded(MixKernels, "lin_attn_walk")
+    T = sum(lens)
+    f = lambda *s: torch.empty(s, device="meta")      # noqa: E731
+    k.lin_attn_decay(f(T, 3 * H * d), 0, H * d, 2 * H * d, f(H), f(len(lens), H, d, d), _ctx(lens), f(T, H * d), H, d, d)
+    assert ran == [want]
