@@ -1183,15 +1183,25 @@ class MixKernels:
                                          c_int(gate.stride(0) if gate is not None else 0), c_int(mode), _stream()), "latent_expand")
         LAUNCHES[0] += 1
 
-    # The longest run of a step from which on the selective scan goes in pieces. One sequence, 4,096 channels of 16 states: 112 rows
-    # take 24 us in pieces, 64 rows 24 (19 walked row by row), 300 rows 34 (74 walked).
-    SCAN_PIECES_MIN_ROWS = 96
-
     @staticmethod
     def scan_piece_rows(rows: int, inner: int, sm_count: int) -> int:
         """Rows of a piece: the fewest of 16, 32, 64 with which the blocks (128 channels of a piece) are about one wave, eight an SM;
         shorter pieces for fewer rows, so that the walk over a piece, which nothing shortens, does not outlast the rest."""
         return next((r for r in (16, 32) if -(-rows // r) * -(-inner // 128) <= 8 * sm_count), 64)
+
+    @classmethod
+    def scan_pays(cls, rows, n_seqs, longest, inner, n_state, sm_count) -> bool:
+        """Whether the scan in pieces takes less than the walk over the rows, by what either is about to take (us). In pieces: its three
+        launches, blocks (most of which, in a step of unequal runs, find nothing to do) and a channel's states, which every run loads
+        and stores like ten rows. Walked: the longest run's chain, or all rows and runs at the SMs' rate. Measured, walked / in pieces, 16
+        states: one run of 96 rows 4,096 channels 27 / 23, 2,048 rows 466 / 143; of 96 and 16 of 4 rows 67 / 45, 1,024 channels 24 / 26; of
+        96 and 100 of 16, 64 channels 21 / 24, 1,024 132 / 70; 32 states, 1,024 channels, of 96 and 16 of 4 29 / 41."""
+        if n_state > 32:
+            return False
+        blocks = -(-inner // 128) * -(-longest // cls.scan_piece_rows(rows, inner, sm_count)) * n_seqs
+        work = 0.92e-6 * n_state * inner * (rows + 10 * n_seqs)
+        pieces = 14 + 0.35 * n_state + 0.03 * n_seqs + max(0, 1.7e-3 * blocks + work - 3)
+        return pieces < 4 + max(0.17 * longest, (3.2 * min(n_state, 16) + max(n_state - 16, 0)) * 1e-6 * inner * (rows + 8 * n_seqs))
 
     def selective_scan(self, x, dt_raw, dt_bias, a_log, dskip, bc, b_col, c_col, z, state, ctx, out, inner, n_state):
         """x, z [T, I] views and bc [T, ...] of the element type (B at b_col, C at c_col), dt_raw float32 [T, I],
@@ -1207,7 +1217,7 @@ class MixKernels:
                 c_int(z.stride(0)), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                 _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), c_int(out.stride(0)))
         tail = (c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)), c_int(inner), c_int(n_state), _stream())
-        if ctx.max_new >= self.SCAN_PIECES_MIN_ROWS and n_state <= 32:
+        if self.scan_pays(x.shape[0], ctx.n_seqs, ctx.max_new, inner, n_state, ctx.engine.sm_count):
             T, rows = x.shape[0], self.scan_piece_rows(x.shape[0], inner, ctx.engine.sm_count)
             n = T // rows + ctx.n_seqs
             scratch = [torch.empty(shape, dtype=torch.float32, device=x.device) for shape in ((T, inner), (n, n_state, inner), (n, inner))]

@@ -579,7 +579,7 @@ def test_selective_scan_in_pieces_against_the_recurrence(dtype, inner, N, lens):
     state0 = torch.randn(len(lens) + 1, inner, N, generator=g)
     ctx = SimpleNamespace(seq_start=torch.from_numpy(start).cuda(), slots=torch.tensor(slots, dtype=torch.int32).cuda(),
                           n_seqs=len(lens), max_new=max(lens), engine=SimpleNamespace(sm_count=148))
-    assert max(lens) >= k.SCAN_PIECES_MIN_ROWS
+    k.scan_pays = lambda *a: True
     st, xd = state0.clone().cuda(), xz.cuda()
     out = torch.full((T, inner), float("nan"), dtype=dtype, device="cuda")
     k.selective_scan(xd[:, :inner], raw.cuda(), bias.cuda(), a_log.cuda(), d.cuda(), bc.cuda(), K, K + N, xd[:, inner:], st, ctx, out, inner, N)

@@ -62,3 +62,33 @@ def test_linear_attention_goes_in_chunks_where_that_is_faster(H, d, lens, want):
     f = lambda *s: torch.empty(s, device="meta")      # noqa: E731
     k.lin_attn_decay(f(T, 3 * H * d), 0, H * d, 2 * H * d, f(H), f(len(lens), H, d, d), _ctx(lens), f(T, H * d), H, d, d)
     assert ran == [want]
+
+
+SCAN = [(4096, 16, [2048], "pieces"),                    # 466 / 143
+        (4096, 16, [64], "walk"),                        # 18 / 21
+        (256, 16, [300], "pieces"),                      # 56 / 21
+        (4096, 16, [96] + [4] * 16, "pieces"),           # 67 / 45
+        (1024, 16, [96] + [4] * 16, "walk"),             # 24 / 26
+        (1024, 32, [96] + [4] * 16, "walk"),             # 29 / 41
+        (64, 16, [96] + [16] * 100, "walk"),             # 21 / 24
+        (512, 4, [96] + [16] * 100, "walk"),             # 22 / 26
+        (1024, 16, [96] + [16] * 100, "pieces"),         # 132 / 70
+        (4096, 33, [2048], "walk")]                      # more states than it is built for
+
+
+@pytest.mark.parametrize("inner, N, lens, want", SCAN)
+def test_the_selective_scan_goes_in_pieces_where_that_is_faster(monkeypatch, inner, N, lens, want):
+    from scriptling_llm_lib_b200.csrc import bindings
+    k, ran = MixKernels.__new__(MixKernels), []
+    k.dtype = torch.bfloat16
+    k._fn = lambda name: lambda *a: ran.append(name) or 0
+    monkeypatch.setattr(bindings, "_ptr", lambda *a: None)
+    monkeypatch.setattr(bindings, "_stream", lambda: None)
+    k._view = lambda *a: None
+    T, ctx = sum(lens), _ctx(lens)
+    ctx.seq_start = ctx.slots = None
+    f = lambda *s, dt=torch.bfloat16: torch.empty(s, device="meta", dtype=dt)      # noqa: E731
+    f32 = torch.float32
+    k.selective_scan(f(T, inner), f(T, inner, dt=f32), f(inner), f(inner, N), f(inner), f(T, 2 * N), 0, N, f(T, inner),
+                     f(len(lens), inner, N, dt=f32), ctx, f(T, inner), inner, N)
+    assert ran == ["selective_scan_pieces" if want == "pieces" else "selective_scan"]
