@@ -75,8 +75,13 @@ from .norm import WithRowVector
 def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int) -> bool:
     """Whether a layer that keeps its softmax weights in float32 runs this step's attention on the tcgen05 kernel that takes them
     in three bfloat16 parts: a bfloat16 step that is no decode step, widths in multiples of 8 (keys up to 192, values up to 128).
-    Few rows are no worse off: 33 rows of 16 heads, keys 64 and values 128, take 8 us (14 with a warp a row). A decode step has one
-    query a sequence where the kernel works on 128, and keeps the kernels that split the keys."""
+    A portion on a cache, however short, is better off there (8 rows of 16 heads on 8,000 keys, keys 64 and values 128 306 us, 537 with
+    a warp a row; equal widths of 80 210, 1,310 on the float tiles), a prompt of very few rows is not: its fixed 7 to 9 us are more than
+    the others take for up to 16 rows of unequal widths (8 rows 8.5, 5.3; 20 rows 8.5 either way), or for one or two of a narrow
+    equal one (2 rows of 32 dims 6.9, 6.1; 4 rows 6.9, 8.0; one of 80 7.9, 8.1). A decode step has one query a sequence where the kernel
+    works on 128, and keeps the kernels that split the keys."""
+    if ctx.from_start and ctx.max_new * key_dim <= (16 * key_dim if value_dim != key_dim or key_dim % 16 else 96):
+        return False
     return dtype == torch.bfloat16 and not ctx.is_decode and PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True)
 
 

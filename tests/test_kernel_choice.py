@@ -92,3 +92,16 @@ def test_the_selective_scan_goes_in_pieces_where_that_is_faster(monkeypatch, inn
     k.selective_scan(f(T, inner), f(T, inner, dt=f32), f(inner), f(inner, N), f(inner), f(T, 2 * N), 0, N, f(T, inner),
                      f(len(lens), inner, N, dt=f32), ctx, f(T, inner), inner, N)
     assert ran == ["selective_scan_pieces" if want == "pieces" else "selective_scan"]
+
+
+@pytest.mark.parametrize("D, V, rows, from_start, want", [(64, 128, 8, True, False), (64, 128, 16, True, False), (64, 128, 17, True, True),
+                                                          (64, 128, 1, False, True), (32, 32, 2, True, False), (32, 32, 4, True, True),
+                                                          (80, 80, 1, True, False), (80, 80, 2, True, True), (80, 80, 2, False, True),
+                                                          (72, 72, 16, True, False), (200, 128, 500, True, False)])
+def test_a_prompt_of_very_few_rows_keeps_the_kernels_without_tiles(D, V, rows, from_start, want):
+    from scriptling_llm_lib_b200.parts.attention import exact_prompt_kernel
+    ctx = SimpleNamespace(is_decode=False, from_start=from_start, max_new=rows)
+    assert exact_prompt_kernel(ctx, torch.bfloat16, D, V) == want
+    assert not exact_prompt_kernel(ctx, torch.float32, D, V)
+    ctx.is_decode = True
+    assert not exact_prompt_kernel(ctx, torch.bfloat16, D, V)
