@@ -500,6 +500,7 @@ class PrefillAttentionTC:
     full speed, or any two multiples of 8 up to 128, filled up with zeros on the chip). With `exact_weights` the softmax weights
     enter the product with the values in all their 24 bits (three products instead of one) and keys go up to 192."""
     HEAD_DIMS = (64, 128)
+    MAX_ROWS = 2 ** 31 - 1               # rows of the key (or value) storage that a tensor map's coordinate reaches
 
     @staticmethod
     def takes(key_dim: int, value_dim: int, exact_weights: bool = False) -> bool:

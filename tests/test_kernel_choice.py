@@ -105,3 +105,18 @@ def test_a_prompt_of_very_few_rows_keeps_the_kernels_without_tiles(D, V, rows, f
     assert not exact_prompt_kernel(ctx, torch.float32, D, V)
     ctx.is_decode = True
     assert not exact_prompt_kernel(ctx, torch.bfloat16, D, V)
+
+
+def test_more_key_rows_than_a_tensor_map_reaches_keep_the_other_kernels():
+    """A cache of narrow heads can hold more rows than the tcgen05 launcher takes: such a prompt is not refused but runs as before."""
+    from scriptling_llm_lib_b200.parts.attention import Attention
+    ran, H, D = [], 8, 16
+    seen = lambda name: lambda *a, **k: ran.append(name)      # noqa: E731
+    layer = Attention(128, H, H, D, None, "q", "k", "v", "o")
+    ctx = SimpleNamespace(is_decode=False, from_start=True, max_new=100, n_seqs=1, seq_start=None, seq_pos0=None, err_flag=None,
+                          kernels=SimpleNamespace(attn_paged=seen("paged"), prefill_attention_tc=SimpleNamespace(attn=seen("tcgen05"))))
+    x = torch.empty((100, 128), dtype=torch.bfloat16, device="meta")
+    for pages in (2 ** 31 // (H * 64) - 1, 2 ** 31 // (H * 64)):
+        kp = torch.empty((pages, H, 64, D), dtype=torch.bfloat16, device="meta")
+        layer._attend(torch.empty((100, 3 * H * D), dtype=torch.bfloat16, device="meta"), x, ctx, kp, kp, None, False, None, True)
+    assert ran == ["tcgen05", "paged"]
