@@ -81,11 +81,10 @@ def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int, rows: int = 0)
     the others take for up to 16 rows of unequal widths (8 rows 8.5, 5.3; 20 rows 8.5 either way), or for one or two of a narrow
     equal one (2 rows of 32 dims 6.9, 6.1; 4 rows 6.9, 8.0; one of 80 7.9, 8.1). A decode step has one query a sequence where the kernel
     works on 128, and keeps the kernels that split the keys."""
-    if rows > PrefillAttentionTC.MAX_ROWS:
+    if dtype != torch.bfloat16 or ctx.is_decode or rows > PrefillAttentionTC.MAX_ROWS or not PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True):
         return False
-    if ctx.from_start and ctx.max_new * key_dim <= (16 * key_dim if value_dim != key_dim or key_dim % 16 else 96):
-        return False
-    return dtype == torch.bfloat16 and not ctx.is_decode and PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True)
+    few = 16 * key_dim if value_dim != key_dim or key_dim % 16 else 96
+    return ctx.max_new * key_dim > few or not getattr(ctx, "from_start", False)
 
 
 def prompt_attention(q, gate, ctx, kpages, vpages, block_table, n_heads, n_kv, key_dim, value_dim, span, scale, tensor_cores=True,
