@@ -2,7 +2,10 @@
 // cached rows, and the head's values. One query a sequence and sixteen heads that read the same cached rows are the sixteen rows of
 // an mma tile, which tcgen05's 128 would leave seven eighths empty. What is float stays float: a float operand enters a product as
 // the sum of three bfloat16 numbers (8 + 8 + 8 bits of mantissa), the other operand (weights, cached rows) is bfloat16 as it is
-// stored, sums are float. The float32 set and other widths have the kernels of mix_kernels.cuh.
+// stored, sums are float. The tensor cores cut what does not fit a sum's 24 bits off where FMA rounds, so a sum stays on them for a few
+// steps only (a page of keys, three steps of a score), smallest parts first, and is added to what came before as floats: against 64
+// bits the sums over 4,096 cached latents of 512 dims are 2.7e-7 off (3.7e-7 on the FMA units; 2.0e-6 while one sum ran through all
+// keys), the absorbed queries 1.1e-7 (1.7e-7). The float32 set and other widths have the kernels of mix_kernels.cuh.
 #include "common.cuh"
 
 namespace lat {
@@ -100,8 +103,8 @@ __global__ void __launch_bounds__(128) latent_absorb_mma_kernel(const bf16* __re
 // planes. Sums over the latent: a warp has an eighth of the columns. Keys first_seen(pos, window) .. pos are seen; rows of a page that
 // are not are zeros (what the page holds there may be anything). Each split leaves (max, sum, sums) as latent_attn does.
 // Bound by the chain of a page (three barriers, 204 products a warp) with one block an SM. Decode steps of 16 heads on 512 + 64 dims,
-// this kernel / with absorb, merge and expand: 8 rows of about 4,000 keys 22 / 35 us (106 / 147 on the FMA units), one row 9 / 25
-// (21 / 65), 32 rows of about 2,000 keys 51 / 69 (257 / 325).
+// this kernel / with absorb, merge and expand: 8 rows of about 4,000 keys 23.5 / 36 us (106 / 147 on the FMA units), one row 9 / 25
+// (21 / 65), 32 rows of about 2,000 keys 52 / 70 (257 / 325).
 #define LAT_KEYS SLLM_PAGE
 struct AttnArgs {
   const float* qa; const bf16* pages;
@@ -114,6 +117,7 @@ template <int NK, int NT>       // 16-dim steps of a score a warp, 8-column tile
 __global__ void __launch_bounds__(256) latent_attn_mma_kernel(AttnArgs p) {
   extern __shared__ __align__(16) bf16 smb[];
   __shared__ float corr_s[16];
+  constexpr int GROUP = 3;
   const int W = p.R + p.P, LD = W + 8;
   constexpr int SL = LAT_KEYS + 4, PL = LAT_KEYS + 8;
   bf16* tiles = smb;                                    // two of [64][LD], and 512 elements of slack behind them
@@ -178,18 +182,27 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(AttnArgs p) {
       for (int n = 0; n < 4; n++) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
       const bf16* kr = tile + (size_t)(half * 32 + (lane & 7) + (lane >> 4) * 8) * LD + ((lane >> 3) & 1) * 8;
 #pragma unroll
-      for (int st = 0; st < NK; st++) {
-        const int c = (kg + 4 * st) * 16;
-        if (c >= W) break;
+      for (int st = 0; st < NK; st += GROUP) {            // sums of a group of steps, smallest part first, added up as floats
+        if ((kg + 4 * st) * 16 >= W) break;
 #pragma unroll
         for (int n = 0; n < 4; n += 2) {
-          uint32_t b[4];
-          ldsm4(b, kr + (size_t)n * 8 * LD + c);
+          uint32_t b[GROUP][4];
+          float f[2][4];
 #pragma unroll
-          for (int part = 2; part >= 0; part--) {
-            mma(s[n], qf[st][part], b[0], b[1]);
-            mma(s[n + 1], qf[st][part], b[2], b[3]);
-          }
+          for (int e = 0; e < 4; e++) f[0][e] = f[1][e] = 0.f;
+#pragma unroll
+          for (int k = 0; k < GROUP; k++)
+            if (st + k < NK && (kg + 4 * (st + k)) * 16 < W) ldsm4(b[k], kr + (size_t)n * 8 * LD + (kg + 4 * (st + k)) * 16);
+#pragma unroll
+          for (int part = 2; part >= 0; part--)
+#pragma unroll
+            for (int k = 0; k < GROUP; k++)
+              if (st + k < NK && (kg + 4 * (st + k)) * 16 < W) {
+                mma(f[0], qf[st + k][part], b[k][0], b[k][1]);
+                mma(f[1], qf[st + k][part], b[k][2], b[k][3]);
+              }
+#pragma unroll
+          for (int e = 0; e < 4; e++) { s[n][e] += f[0][e]; s[n + 1][e] += f[1][e]; }
         }
       }
       float* d = ss + (kg * 16 + g) * SL + half * 32 + 2 * t;
@@ -233,24 +246,32 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(AttnArgs p) {
     __syncthreads();
     {
       const float ca = corr_s[g], cb = corr_s[g + 8];
-#pragma unroll
-      for (int n = 0; n < NT; n++) { o[n][0] *= ca; o[n][1] *= ca; o[n][2] *= cb; o[n][3] *= cb; }
       const bf16* vr = tile + (size_t)((lane & 7) + ((lane >> 3) & 1) * 8) * LD + warp * NT * 8 + (lane >> 4) * 8;
       const bf16* pr = pp + ((lane & 7) + ((lane >> 3) & 1) * 8) * PL + (lane >> 4) * 8;
+      uint32_t a[3][LAT_KEYS / 16][4];
 #pragma unroll
-      for (int k = 0; k < LAT_KEYS / 16; k++) {
-        uint32_t a[3][4];
+      for (int part = 0; part < 3; part++)
 #pragma unroll
-        for (int part = 0; part < 3; part++) ldsm4(a[part], pr + part * 16 * PL + k * 16);
+        for (int k = 0; k < LAT_KEYS / 16; k++) ldsm4(a[part][k], pr + part * 16 * PL + k * 16);
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-          uint32_t b[4];
-          ldsm4t(b, vr + (size_t)k * 16 * LD + n * 8);
+      for (int n = 0; n < NT; n += 2) {                   // the page's sums, smallest part first; what was there, as floats, behind them
+        float f[2][4];
 #pragma unroll
-          for (int part = 2; part >= 0; part--) {
-            mma(o[n], a[part], b[0], b[1]);
-            mma(o[n + 1], a[part], b[2], b[3]);
+        for (int e = 0; e < 4; e++) f[0][e] = f[1][e] = 0.f;
+        uint32_t b[LAT_KEYS / 16][4];
+#pragma unroll
+        for (int k = 0; k < LAT_KEYS / 16; k++) ldsm4t(b[k], vr + (size_t)k * 16 * LD + n * 8);
+#pragma unroll
+        for (int part = 2; part >= 0; part--)
+#pragma unroll
+          for (int k = 0; k < LAT_KEYS / 16; k++) {
+            mma(f[0], a[part][k], b[k][0], b[k][1]);
+            mma(f[1], a[part][k], b[k][2], b[k][3]);
           }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          o[n + e][0] = fmaf(o[n + e][0], ca, f[e][0]); o[n + e][1] = fmaf(o[n + e][1], ca, f[e][1]);
+          o[n + e][2] = fmaf(o[n + e][2], cb, f[e][2]); o[n + e][3] = fmaf(o[n + e][3], cb, f[e][3]);
         }
       }
     }
@@ -360,13 +381,20 @@ __global__ void __launch_bounds__(128) latent_expand_mma_kernel(const float* __r
     split3(b1.x, b1.y, f[1][0][1], f[1][1][1], f[1][2][1]);
     split3(a1.z, a1.w, f[1][0][2], f[1][1][2], f[1][2][2]);
     split3(b1.z, b1.w, f[1][0][3], f[1][1][3], f[1][2][3]);
+    float y[4][4];                                       // the step's sums, smallest part first, added up as floats
+#pragma unroll
+    for (int n = 0; n < 4; n++) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;
 #pragma unroll
     for (int part = 2; part >= 0; part--)
 #pragma unroll
       for (int n = 0; n < 4; n++) {
-        mma(acc[n], f[0][part], b[n].x, b[n].y);
-        mma(acc[n], f[1][part], b[n].z, b[n].w);
+        mma(y[n], f[0][part], b[n].x, b[n].y);
+        mma(y[n], f[1][part], b[n].z, b[n].w);
       }
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[n][e] += y[n][e];
   }
   if (warp > 0) {
 #pragma unroll

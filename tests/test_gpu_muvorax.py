@@ -473,6 +473,24 @@ def test_cached_latents_that_are_no_numbers_are_not_passed_over(sink):
         assert bool(out[0].isnan().all()) and bool(out[1].isfinite().all()), n_split
 
 
+def test_sums_over_cached_latents_are_rounded_as_floats():
+    """Many keys in one split: a sum that stayed on the tensor cores all the way, which cut where FMA rounds, would be 1.2e-5 off here.
+    A page's sum is cut up to 12 times and a score 9 times in three groups, each by up to 2^-24 of its size at that step: (12 + 3) / 2 of
+    them, 4.5e-7, and the roundings of the softmax."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, B, H, R, P, n = KernelSet(torch.bfloat16).mix, 2, 16, 512, 64, 4096
+    g = torch.Generator().manual_seed(2)
+    pages, qa = torch.randn(B * n // 64, 1, 64, R + P, generator=g).bfloat16(), torch.randn(B, H, R + P, generator=g) / (R + P) ** 0.5
+    table = torch.arange(B * n // 64, dtype=torch.int32).view(B, -1)
+    ctx = SimpleNamespace(tok_pos=torch.full((B,), n - 1, dtype=torch.int32).cuda(), tok_seq=torch.arange(B, dtype=torch.int32).cuda())
+    part, olat = torch.empty((B, H, 1, R + 2), device="cuda"), torch.empty((B, H, R), device="cuda")
+    k.latent_attn(qa.cuda(), pages.cuda(), ctx, table.cuda(), part, H, R, P, 1)
+    k.latent_expand(part, olat, torch.zeros(H * 8, R).bfloat16().cuda(), torch.empty((B, H * 8), dtype=torch.bfloat16, device="cuda"), H, 8, R, 1)
+    keys = pages.view(B, n, R + P).double()
+    want = torch.einsum("bhw,bnw->bhn", qa.double(), keys).softmax(-1) @ keys[..., :R]
+    assert float((olat.cpu().double() - want).norm() / want.norm()) < 6e-7
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("W, ld, off", [(8, 8, 0), (248, 504, 256), (2048, 4096, 2048), (4096, 4096, 0), (4104, 4104, 0), (2044, 2048, 0),
                                         (256, 516, 4), (1024, 1030, 0)])
