@@ -167,7 +167,8 @@ class KernelSet:
     def gemm_nt_blocks_take(self, a, w) -> bool:
         """Whether `gemm_nt_blocks` runs these as one launch: more than 64 rows, 16-byte (float) or 8-byte (bfloat16) aligned pieces."""
         nb, _, k = w.shape
-        return a.shape[0] > 64 and k % 4 == 0 and a.stride(0) % 4 == 0 and a.data_ptr() % (4 * a.element_size()) == 0
+        return (a.shape[0] > 64 and k % 4 == 0 and a.stride(0) % 4 == 0 and w.is_contiguous()
+                and all(t.data_ptr() % (4 * t.element_size()) == 0 for t in (a, w)))
 
     def gemm_nt_blocks(self, a, w, out):
         """Block-diagonal product: out[b] = a[:, b K:(b + 1) K] @ w[b]^T for a [M, blocks K] (unit column stride), w [blocks, N, K] and
@@ -1147,7 +1148,7 @@ class MixKernels:
         if q.dtype != self.dtype:
             raise KernelError(f"latent_absorb: q has dtype {q.dtype}, expected {self.dtype}")
         lat = self.latent
-        if lat is not None and lat.takes(dim, rot_dim, 8, rank) and q.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0:
+        if lat is not None and lat.takes(dim, rot_dim, 8, rank) and q.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0 and wuk.data_ptr() % 16 == 0:
             _check(lat.lib.sllm_latent_absorb_mma(self._view(q, "q"), c_int(q.stride(0)), _ptr(wuk, self.dtype, "wuk"),
                                                   _ptr(qa, torch.float32, "qa"), c_int(q.shape[0]), c_int(n_heads), c_int(dim),
                                                   c_int(rot_dim), c_int(rank), c_float(scale), _stream()), "latent_absorb_mma")
@@ -1159,7 +1160,7 @@ class MixKernels:
     def latent_attn(self, qa, pages, ctx, block_table, part, n_heads, rank, rot_dim, n_split, window=0):
         """`window` > 0: a row sees its own position and the window - 1 before it; 0: every earlier one."""
         lat = self.latent
-        fn = lat.lib.sllm_latent_attn_mma if lat is not None and lat.takes(8, rot_dim, 8, rank) else self._fn("latent_attn")
+        fn = lat.lib.sllm_latent_attn_mma if lat is not None and lat.takes(8, rot_dim, 8, rank) and pages.data_ptr() % 16 == 0 else self._fn("latent_attn")
         _check(fn(
             _ptr(qa, torch.float32, "qa"), _ptr(pages, self.dtype, "pages"), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
@@ -1176,7 +1177,8 @@ class MixKernels:
             if gate.dtype != self.dtype or tuple(gate.shape) != (out.shape[0], n_heads * (v_dim if mode == 2 else 1)):
                 raise KernelError(f"latent_expand: gate logits {tuple(gate.shape)} {gate.dtype} for {n_heads} heads of {v_dim}")
         lat = self.latent
-        fn = lat.lib.sllm_latent_expand_mma if lat is not None and lat.takes(8, 0, v_dim, rank) and n_split <= 64 else self._fn("latent_expand")
+        mma = lat is not None and lat.takes(8, 0, v_dim, rank) and n_split <= 64 and wuv.data_ptr() % 16 == 0
+        fn = lat.lib.sllm_latent_expand_mma if mma else self._fn("latent_expand")
         _check(fn(_ptr(part, torch.float32, "part"), _ptr(olat, torch.float32, "olat"),
                                          _ptr(wuv, self.dtype, "wuv"), _ptr(out, self.dtype, "out"), c_int(out.shape[1]),
                                          c_int(out.shape[0]), c_int(n_heads), c_int(v_dim), c_int(rank), c_int(n_split),

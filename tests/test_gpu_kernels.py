@@ -431,6 +431,7 @@ def test_gemm_nt_blocks_is_every_block_by_itself(kernel_sets, blocks, M, N, K):
     wide, w = dev(rand(M, blocks * K + 8, seed=3)), dev(rand(blocks, N, K, seed=4))
     a = wide[:, 4:4 + blocks * K]
     assert ks.gemm_nt_blocks_take(a, w) and not ks.gemm_nt_blocks_take(a[:64], w) and not ks.gemm_nt_blocks_take(wide[:, 1:1 + blocks * K], w)
+    assert not ks.gemm_nt_blocks_take(a, torch.empty(w.numel() + 1, dtype=w.dtype, device="cuda")[1:].view(w.shape))
     out, each = (torch.full((blocks, M, N), float("nan"), device="cuda") for _ in range(2))
     ks.gemm_nt_blocks(a, w, out)
     for b in range(blocks):

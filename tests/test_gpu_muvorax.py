@@ -491,6 +491,28 @@ def test_sums_over_cached_latents_are_rounded_as_floats():
     assert float((olat.cpu().double() - want).norm() / want.norm()) < 6e-7
 
 
+def test_latent_weights_and_pages_at_any_place():
+    """The decode form's matrices and pages two bytes off a multiple of 16: taken as before, by the kernels that ask for no alignment."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, H, D, P, V, R, n = KernelSet(torch.bfloat16).mix, 4, 16, 8, 24, 64, 130
+    g = torch.Generator().manual_seed(3)
+
+    def off(*shape):
+        t = torch.randn(math.prod(shape) + 1, generator=g).bfloat16().cuda()
+        return t[1:].view(shape), t[1:].view(shape).clone()
+    got = []
+    for wuk, wuv, pages in zip(off(H * D, R), off(H * V, R), off(3, 1, 64, R + P)):
+        q = torch.randn(1, H * (D + P), generator=torch.Generator().manual_seed(4)).bfloat16().cuda()
+        ctx = SimpleNamespace(tok_pos=torch.tensor([n - 1], dtype=torch.int32).cuda(), tok_seq=torch.zeros(1, dtype=torch.int32).cuda())
+        qa, part = torch.empty((1, H, R + P), device="cuda"), torch.empty((1, H, 2, R + 2), device="cuda")
+        k.latent_absorb(q, wuk, qa, H, D, P, R, 0.2)
+        k.latent_attn(qa, pages, ctx, torch.arange(3, dtype=torch.int32).view(1, 3).cuda(), part, H, R, P, 2)
+        olat, out = torch.empty((1, H, R), device="cuda"), torch.empty((1, H * V), dtype=torch.bfloat16, device="cuda")
+        k.latent_expand(part, olat, wuv, out, H, V, R, 2)
+        got.append(out.float())
+    assert float((got[0] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("W, ld, off", [(8, 8, 0), (248, 504, 256), (2048, 4096, 2048), (4096, 4096, 0), (4104, 4104, 0), (2044, 2048, 0),
                                         (256, 516, 4), (1024, 1030, 0)])
