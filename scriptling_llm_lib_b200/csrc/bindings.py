@@ -979,27 +979,46 @@ class ChunkKernels:
     def __init__(self):
         self.lib = load_library("chunk_tcgen05")
         self.lib.sllm_chunk_lin_attn_bf16.restype = self.lib.sllm_chunk_delta.restype = c_int
+        if self.lib.sllm_chunk_delta_scratch() != self.DELTA_BYTES:
+            raise KernelError("chunk_tcgen05 was built with another scratch per chunk than its launcher counts with")
+
+    # What a call's scratch may come to (one head's, where that is more): heads are gone through as many at a time as fit. 16,384 rows of
+    # 16 heads of the delta rule would take 600 MB at once; a third of the heads still fills the SMs several times.
+    SCRATCH_BYTES = 256 << 20
+    DELTA_BYTES = 294_912                # of a chunk of a head: M in three planes and three float matrices of 128 x 128
+
+    @classmethod
+    def heads_held(cls, chunks: int, n_heads: int, chunk_bytes: int) -> int:
+        passes = -(-n_heads // max(1, cls.SCRATCH_BYTES // (chunks * chunk_bytes)))
+        return -(-n_heads // passes)
+
+    @classmethod
+    def scratch_bytes(cls, rows: int, chunk_bytes: int) -> int:
+        """The most that a step of so many rows takes, whatever its runs."""
+        return max(cls.SCRATCH_BYTES, rows // cls.CHUNK * chunk_bytes)
 
     def delta(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
         """As `SequenceKernels.delta_rule`, keys and values up to 128 wide."""
         n = qk.shape[0] // self.CHUNK + ctx.n_seqs
-        scratch = torch.empty((n * n_heads * self.lib.sllm_chunk_delta_scratch(),), dtype=torch.uint8, device=o.device)
+        held = self.heads_held(n, n_heads, self.DELTA_BYTES)
+        scratch = torch.empty((n * held * self.DELTA_BYTES,), dtype=torch.uint8, device=o.device)
         _check(self.lib.sllm_chunk_delta(
             SequenceKernels._view(qk, "qk"), c_int(qk.stride(0)), SequenceKernels._view(v, "v"), c_int(v.stride(0)),
             _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), c_int(held), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
             c_int(ctx.max_new), c_int(n_heads), c_int(n_kv), c_int(dk), c_int(dv),
             _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "chunk_delta")
 
     def lin_attn(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
         """As `MixKernels.lin_attn_decay`, keys up to 128 wide."""
         n = proj.shape[0] // self.CHUNK + ctx.n_seqs
-        chunk_state = torch.empty((n, n_heads, dk, dv), dtype=torch.float32, device=o.device)
+        held = self.heads_held(n, n_heads, 4 * dk * dv)
+        chunk_state = torch.empty((n, held, dk, dv), dtype=torch.float32, device=o.device)
         _check(self.lib.sllm_chunk_lin_attn_bf16(
             _ptr(proj, torch.bfloat16, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(ctx.max_new),
-            c_int(n_heads), c_int(dk), c_int(dv), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), c_int(held), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
+            c_int(ctx.max_new), c_int(n_heads), c_int(dk), c_int(dv), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
             "chunk_lin_attn")
 
 
@@ -1193,13 +1212,18 @@ class MixKernels:
         return next((r for r in (16, 32) if -(-rows // r) * -(-inner // 128) <= 8 * sm_count), 64)
 
     @classmethod
+    def scan_scratch_bytes(cls, rows, n_seqs, inner, n_state, sm_count) -> int:
+        """Step sizes of all rows, and a piece's states and sum; runs that end within a piece come to one each."""
+        return 4 * inner * (rows + (rows // cls.scan_piece_rows(rows, inner, sm_count) + n_seqs) * (n_state + 1))
+
+    @classmethod
     def scan_pays(cls, rows, n_seqs, longest, inner, n_state, sm_count) -> bool:
         """Whether the scan in pieces takes less than the walk over the rows, by what either is about to take (us). In pieces: its three
         launches, blocks (most of which, in a step of unequal runs, find nothing to do) and a channel's states, which every run loads
         and stores like ten rows. Walked: the longest run's chain, or all rows and runs at the SMs' rate. Measured, walked / in pieces, 16
         states: one run of 96 rows 4,096 channels 27 / 23, 2,048 rows 466 / 143; of 96 and 16 of 4 rows 67 / 45, 1,024 channels 24 / 26; of
         96 and 100 of 16, 64 channels 21 / 24, 1,024 132 / 70; 32 states, 1,024 channels, of 96 and 16 of 4 29 / 41."""
-        if n_state > 32:
+        if n_state > 32 or cls.scan_scratch_bytes(0, n_seqs, inner, n_state, sm_count) > ChunkKernels.SCRATCH_BYTES:
             return False
         blocks = -(-inner // 128) * -(-longest // cls.scan_piece_rows(rows, inner, sm_count)) * n_seqs
         work = 0.92e-6 * n_state * inner * (rows + 10 * n_seqs)

@@ -48,9 +48,10 @@ struct LinArgs {
   const float* decay;                                 // [H]
   float* state;                                       // [slots][H][D][V]
   const int* seq_start; const int* slots;
-  float* chunk_state;                                 // [chunks][H][D][V]
+  float* chunk_state;                                 // [chunks][hs][D][V]
   float* o;                                           // [T][H V]
   int H, D, V;
+  int h0, hs;                                         // the launch's heads: the first, and how many
   int* err;
   int vec;                                            // rows, columns and widths allow 16-byte accesses
 };
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
   uint8_t* va = ka + TILE_BYTES;
   float* pw = (float*)(va + TILE_BYTES);
   float* scale = pw + Q + 4;
-  const int n = min(Q, len - r0), vblocks = (p.V + Q - 1) / Q, h = blockIdx.y / vblocks, v0 = (blockIdx.y % vblocks) * Q;
+  const int n = min(Q, len - r0), vblocks = (p.V + Q - 1) / Q, hl = blockIdx.y / vblocks, h = p.h0 + hl, v0 = (blockIdx.y % vblocks) * Q;
   const int vn = min(Q, p.V - v0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bf16* row = p.proj + (size_t)(start + r0) * p.ld;
   uint4 kr[PIECES], vr[PIECES];
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
   }
   u.done();
   const int d = (warp & 3) * 32 + lane;
-  float* dst = p.chunk_state + (((first_chunk(start, b) + blockIdx.x) * p.H + h) * p.D + d) * (size_t)p.V + v0;
+  float* dst = p.chunk_state + (((first_chunk(start, b) + blockIdx.x) * p.hs + hl) * p.D + d) * (size_t)p.V + v0;
   const int c0 = (warp >> 2) * 32;                 // a warp reads 32 lanes (rows) of 32 columns
   uint32_t v[32];
   tmem_ld32(u.tmem + ((uint32_t)((warp & 3) * 32) << 16) + c0, v);
@@ -221,12 +222,12 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
 // a thread (4 where they come in fours).
 template <int E>
 __global__ void __launch_bounds__(256) chunk_lin_pass_kernel(LinArgs p) {
-  const int b = blockIdx.z, h = blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
+  const int b = blockIdx.z, h = p.h0 + blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
   const int DV = p.D * p.V, e0 = (blockIdx.x * 256 + threadIdx.x) * E;
   if (e0 >= DV || len <= 0) return;
   const int chunks = (len + Q - 1) / Q;
-  const size_t stride = (size_t)p.H * DV;
-  float* u = p.chunk_state + (first_chunk(start, b) * p.H + h) * (size_t)DV + e0;
+  const size_t stride = (size_t)p.hs * DV;
+  float* u = p.chunk_state + (first_chunk(start, b) * p.hs + blockIdx.y) * (size_t)DV + e0;
   float* st = p.state + ((size_t)p.slots[b] * p.H + h) * DV + e0;
   const float g = p.decay[h], whole = power(g, Q), last = power(g, len - (chunks - 1) * Q);
   float s[E];
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   uint8_t* xa = qa + TILE_BYTES;                   // the state, then the keys, then the values
   float* pw = (float*)(xa + TILE_BYTES);
   __shared__ Watch watch;
-  const int n = min(Q, len - r0), vblocks = (p.V + Q - 1) / Q, h = blockIdx.y / vblocks, v0 = (blockIdx.y % vblocks) * Q;
+  const int n = min(Q, len - r0), vblocks = (p.V + Q - 1) / Q, hl = blockIdx.y / vblocks, h = p.h0 + hl, v0 = (blockIdx.y % vblocks) * Q;
   const int vn = min(Q, p.V - v0), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bf16* row = p.proj + (size_t)(start + r0) * p.ld;
   uint4 raw[PIECES];
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   Unit u;
   u.open((uint8_t*)(pw + 2 * (Q + 4)));
   put_silu(qa, raw, nullptr);
-  put_floats(xa, p.chunk_state + ((first_chunk(start, b) + blockIdx.x) * p.H + h) * (size_t)p.D * p.V + v0, p.V, p.D, vn, p.vec);
+  put_floats(xa, p.chunk_state + ((first_chunk(start, b) + blockIdx.x) * p.hs + hl) * (size_t)p.D * p.V + v0, p.V, p.D, vn, p.vec);
   u.ready();
   const int dsteps = (p.D + 15) / 16, rsteps = (n + 15) / 16;
   if (tid == 0) {
@@ -347,10 +348,11 @@ struct DeltaArgs {
   const float* bd;                                    // [T][2 H + G]: b | d | (not read here)
   float* state;                                       // [slots][H][dk][dv]
   const int* seq_start; const int* slots;
-  uint8_t* m;                                         // [chunks][H]: M as the three planes of a tile
-  float *n, *qp, *o0;                                 // [chunks][H][32][128][4] each (see `quad`); n becomes the state in front of the chunk
+  uint8_t* m;                                         // [chunks][hs]: M as the three planes of a tile
+  float *n, *qp, *o0;                                 // [chunks][hs][32][128][4] each (see `quad`); n becomes the state in front of the chunk
   float* o;                                           // [T][H dv]
   int H, G, dk, dv;
+  int h0, hs;                                         // the launch's heads: the first, and how many
   int* err;
 };
 constexpr size_t MAT = (size_t)Q * Q;
@@ -555,7 +557,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   float *hi = (float*)(ya + TILE_BYTES), *lo = hi + Q, *beta = lo + Q, *front = beta + Q, *back = front + Q, *bfront = back + Q;
   __shared__ double part_s[4];
   __shared__ Watch watch;
-  const int n = min(Q, len - r0), row = start + r0, h = blockIdx.y, g = h / (p.H / p.G);
+  const int n = min(Q, len - r0), row = start + r0, h = p.h0 + blockIdx.y, g = h / (p.H / p.G);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* qrow = p.qk + (size_t)row * p.ld_qk + (size_t)g * p.dk;
   const float* krow = qrow + (size_t)p.G * p.dk;
@@ -672,7 +674,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   }
   put_tmem(t_lane, c0, w);
   __syncthreads();                                 // T has been read from where the scaled values go
-  const size_t unit = (first_chunk(start, b) + blockIdx.x) * p.H + h, mat = unit * MAT;
+  const size_t unit = (first_chunk(start, b) + blockIdx.x) * p.hs + blockIdx.y, mat = unit * MAT;
   put_rows<true, BY_COLUMN>(ya, f, beta, &watch);
   u.ready();
   if (tid == 0) {                                  // U0
@@ -760,14 +762,14 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
   uint8_t* ma = aligned_smem(smem_raw);
   uint8_t* sa = ma + 2 * TILE_BYTES;
   uint8_t* head = sa + 3 * ST_PLANE;
-  const int b = blockIdx.z, h = blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
+  const int b = blockIdx.z, h = p.h0 + blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
   if (len <= 0) return;
   const int chunks = (len + Q - 1) / Q, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int d = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16, v0 = blockIdx.x * PV + j0;
-  const size_t first = first_chunk(start, b) * p.H + h;
+  const size_t first = first_chunk(start, b) * p.hs + blockIdx.y;
   float* st = p.state + (((size_t)p.slots[b] * p.H + h) * p.dk + d) * p.dv + v0;
   float* nm = p.n + first * MAT + quad(d, v0);      // columns v0 .. v0 + 15: fours Q * 4 floats apart
-  const size_t stride = (size_t)p.H * MAT;
+  const size_t stride = (size_t)p.hs * MAT;
   const uint32_t full = smem_u32(head + 16);        // two barriers of M's copies
   if (tid == 0) { mbar_init(full, 1); mbar_init(full + 8, 1); }
   Unit u;
@@ -776,7 +778,7 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
     const uint32_t bar = full + 8 * (c & 1);
     mbar_expect_tx(bar, TILE_BYTES);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(ma + (c & 1) * TILE_BYTES)), "l"(p.m + (first + (size_t)c * p.H) * TILE_BYTES), "r"(TILE_BYTES), "r"(bar) : "memory");
+                 ::"r"(smem_u32(ma + (c & 1) * TILE_BYTES)), "l"(p.m + (first + (size_t)c * p.hs) * TILE_BYTES), "r"(TILE_BYTES), "r"(bar) : "memory");
   };
   if (tid == 0) {
     fetch_m(0);
@@ -857,8 +859,8 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_out_kernel(DeltaArgs p) {
   if (r0 >= len) return;
   uint8_t* xa = aligned_smem(smem_raw);
   uint8_t* ya = xa + TILE_BYTES;
-  const int n = min(Q, len - r0), h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t mat = ((first_chunk(start, b) + blockIdx.x) * p.H + h) * MAT;
+  const int n = min(Q, len - r0), h = p.h0 + blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t mat = ((first_chunk(start, b) + blockIdx.x) * p.hs + blockIdx.y) * MAT;
   float fq[PIECES][8], fs[PIECES][8];
   fetch_quads(fq, p.qp + mat);
   fetch_quads(fs, p.n + mat);
@@ -900,50 +902,59 @@ static cudaError_t allow_smem(K kernel, size_t smem) {
 }  // namespace chunked
 
 // proj [T, ld]: raw q, k, v of the heads from columns q_col, k_col, v_col; decay float [H]; state float [slots][H][D][V], read and
-// advanced; chunk_state float [T / 128 + n_seqs][H][D][V]; o float [T, H V]; err int or null.
+// advanced; chunk_state float [T / 128 + n_seqs][heads_held][D][V]: heads_held heads are gone through at a time; o float [T, H V]; err
+// int or null.
 SLLM_EXPORT int sllm_chunk_lin_attn_bf16(const void* proj, int ld, int q_col, int k_col, int v_col, const float* decay, float* state,
-                                         const int* seq_start, const int* slots, float* chunk_state, float* o, int n_seqs, int max_new,
-                                         int H, int D, int V, int* err, cudaStream_t stream) {
+                                         const int* seq_start, const int* slots, float* chunk_state, int heads_held, float* o, int n_seqs,
+                                         int max_new, int H, int D, int V, int* err, cudaStream_t stream) {
   if (n_seqs <= 0 || max_new <= 0) return 0;
   const int vblocks = (V + chunked::Q - 1) / chunked::Q;
-  if (H < 1 || D < 1 || D > chunked::Q || V < 1 || n_seqs > 65535 || (long long)H * vblocks > 65535) return SLLM_ERR_ARG;
+  if (H < 1 || heads_held < 1 || D < 1 || D > chunked::Q || V < 1 || n_seqs > 65535 || (long long)H * vblocks > 65535) return SLLM_ERR_ARG;
   const int vec = !((ld | q_col | k_col | v_col | D | V) & 7) && !(((uintptr_t)proj | (uintptr_t)state | (uintptr_t)chunk_state | (uintptr_t)o) & 15);
-  chunked::LinArgs p{(const bf16*)proj, ld, q_col, k_col, v_col, decay, state, seq_start, slots, chunk_state, o, H, D, V, err, vec};
   cudaError_t e = chunked::allow_smem(chunked::chunk_lin_states_kernel, chunked::LIN_SMEM);
   if (e == cudaSuccess) e = chunked::allow_smem(chunked::chunk_lin_scan_kernel, chunked::LIN_SMEM);
   if (e != cudaSuccess) return (int)e;
   const int chunks = (max_new + chunked::Q - 1) / chunked::Q, DV = D * V;
-  const dim3 grid(chunks, H * vblocks, n_seqs);
-  chunked::chunk_lin_states_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
-  if (vec) chunked::chunk_lin_pass_kernel<4><<<dim3((DV / 4 + 255) / 256, H, n_seqs), 256, 0, stream>>>(p);
-  else chunked::chunk_lin_pass_kernel<1><<<dim3((DV + 255) / 256, H, n_seqs), 256, 0, stream>>>(p);
-  chunked::chunk_lin_scan_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
+  for (int h0 = 0; h0 < H; h0 += heads_held) {
+    const int hs = H - h0 < heads_held ? H - h0 : heads_held;
+    chunked::LinArgs p{(const bf16*)proj, ld, q_col, k_col, v_col, decay, state, seq_start, slots, chunk_state, o, H, D, V, h0, hs, err, vec};
+    const dim3 grid(chunks, hs * vblocks, n_seqs);
+    chunked::chunk_lin_states_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
+    if (vec) chunked::chunk_lin_pass_kernel<4><<<dim3((DV / 4 + 255) / 256, hs, n_seqs), 256, 0, stream>>>(p);
+    else chunked::chunk_lin_pass_kernel<1><<<dim3((DV + 255) / 256, hs, n_seqs), 256, 0, stream>>>(p);
+    chunked::chunk_lin_scan_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
+  }
   SLLM_RETURN_LAST();
 }
 
 // qk float rows [G dk | G dk], v float rows [H dv], bd float [T, 2 H + G] as the walk takes them; state float [slots][H][dk][dv], read
-// and advanced; scratch: sllm_chunk_delta_scratch() bytes for each head of each of `chunks_held` >= T / 128 + n_seqs chunks, 16-byte
-// aligned; o float [T, H dv]; dk and dv up to 128.
+// and advanced; scratch: sllm_chunk_delta_scratch() bytes for each of `heads_held` heads (gone through that many at a time) of each of
+// `chunks_held` >= T / 128 + n_seqs chunks, 16-byte aligned; o float [T, H dv]; dk and dv up to 128.
 SLLM_EXPORT int sllm_chunk_delta_scratch(void) { return (int)(chunked::TILE_BYTES + 3 * chunked::MAT * sizeof(float)); }
 SLLM_EXPORT int sllm_chunk_delta(const float* qk, int ld_qk, const float* v, int ld_v, const float* bd, float* state, const int* seq_start,
-                                 const int* slots, void* scratch, long long chunks_held, float* o, int n_seqs, int max_new, int H, int G,
-                                 int dk, int dv, int* err, cudaStream_t stream) {
+                                 const int* slots, void* scratch, long long chunks_held, int heads_held, float* o, int n_seqs, int max_new,
+                                 int H, int G, int dk, int dv, int* err, cudaStream_t stream) {
   using namespace chunked;
   if (n_seqs <= 0 || max_new <= 0) return 0;
-  if (H < 1 || G < 1 || H % G || dk < 1 || dk > Q || dv < 1 || dv > Q || n_seqs > 65535 || H > 65535 || ((uintptr_t)scratch & 15)) return SLLM_ERR_ARG;
-  const size_t units = (size_t)chunks_held * H;
-  float* mats = (float*)((uint8_t*)scratch + units * TILE_BYTES);
+  if (H < 1 || heads_held < 1 || G < 1 || H % G || dk < 1 || dk > Q || dv < 1 || dv > Q || n_seqs > 65535 || H > 65535 || ((uintptr_t)scratch & 15))
+    return SLLM_ERR_ARG;
   const bool vec = !((ld_qk | ld_v | dk | dv) & 7) && !(((uintptr_t)qk | (uintptr_t)v | (uintptr_t)o) & 15);
-  DeltaArgs p{qk, ld_qk, v, ld_v, bd, state, seq_start, slots, (uint8_t*)scratch, mats, mats + units * MAT, mats + 2 * units * MAT, o, H, G, dk, dv, err};
   const auto parts = vec ? chunk_delta_parts_kernel<true> : chunk_delta_parts_kernel<false>;
   const auto out = vec ? chunk_delta_out_kernel<true> : chunk_delta_out_kernel<false>;
   cudaError_t e = allow_smem(parts, DELTA_SMEM);
   if (e == cudaSuccess) e = allow_smem(chunk_delta_pass_kernel, PASS_SMEM);
   if (e == cudaSuccess) e = allow_smem(out, DELTA_SMEM);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid((max_new + Q - 1) / Q, H, n_seqs);
-  parts<<<grid, NT, DELTA_SMEM, stream>>>(p);
-  chunk_delta_pass_kernel<<<dim3((dv + PV - 1) / PV, H, n_seqs), 256, PASS_SMEM, stream>>>(p);
-  out<<<grid, NT, DELTA_SMEM, stream>>>(p);
+  for (int h0 = 0; h0 < H; h0 += heads_held) {
+    const int hs = H - h0 < heads_held ? H - h0 : heads_held;
+    const size_t units = (size_t)chunks_held * hs;
+    float* mats = (float*)((uint8_t*)scratch + units * TILE_BYTES);
+    DeltaArgs p{qk, ld_qk, v, ld_v, bd, state, seq_start, slots, (uint8_t*)scratch, mats, mats + units * MAT, mats + 2 * units * MAT, o, H, G, dk, dv,
+                h0, hs, err};
+    const dim3 grid((max_new + Q - 1) / Q, hs, n_seqs);
+    parts<<<grid, NT, DELTA_SMEM, stream>>>(p);
+    chunk_delta_pass_kernel<<<dim3((dv + PV - 1) / PV, hs, n_seqs), 256, PASS_SMEM, stream>>>(p);
+    out<<<grid, NT, DELTA_SMEM, stream>>>(p);
+  }
   SLLM_RETURN_LAST();
 }

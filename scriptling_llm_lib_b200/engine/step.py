@@ -19,6 +19,7 @@ import torch
 from ..cache import PAGE, SequenceCache, pages_for
 from ..config.registry import architecture_for, architecture_name, load_config
 from ..csrc.bindings import CastKernels, KernelSet
+from ..parts.base import Part
 from ..weights.loader import load_weights, stored_to_kept
 from .graphs import DecodeGraphs
 from .layout import ModelLayout
@@ -354,7 +355,8 @@ class Engine:
         weights and cache (residual, products' outputs), plus the logits of the captured decode steps:
         what the cache must leave free."""
         width = 64 * self.layout.hidden_size                        # bytes a row, all buffers of a layer alive at once
-        return self.PROMPT_TOKENS_PER_STEP * width + 4 * self.layout.vocab_size * 4 * 1024
+        scratch = max(p.scratch_bytes(self.PROMPT_TOKENS_PER_STEP) for p in self.model.parts() if isinstance(p, Part))
+        return self.PROMPT_TOKENS_PER_STEP * width + scratch + 4 * self.layout.vocab_size * 4 * 1024
 
     def check_errors(self) -> None:
         """Raises if a kernel of an earlier step reported an error (a wait on the device that ran out

@@ -78,6 +78,10 @@ class Part:
     def prepare(self, max_positions: int, device) -> None:
         """Build host-made tables once the engine knows its longest sequence."""
 
+    def scratch_bytes(self, rows: int) -> int:
+        """Device memory that the part's kernels take in a prompt step of that many rows beside what enters and leaves them."""
+        return 0
+
 
 @dataclass
 class FoldRequest:

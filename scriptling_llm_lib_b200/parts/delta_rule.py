@@ -20,6 +20,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.needs import StateNeed
+from ..csrc.bindings import ChunkKernels
 from ..weights.spec import TensorSpec
 from .base import MIXERS, Mixer
 from .conv import CausalConv
@@ -61,6 +62,9 @@ class GatedDeltaRule(Mixer):
         if pad:
             self.small.weight = torch.cat([w, torch.zeros((pad, w.shape[1]), dtype=w.dtype, device=w.device)]).contiguous()
         self.a_log, self.dt_bias, self.norm_w = tensors[self.a_log_name], tensors[self.dt_bias_name], tensors[self.norm_name]
+
+    def scratch_bytes(self, rows: int) -> int:
+        return ChunkKernels.scratch_bytes(rows, ChunkKernels.DELTA_BYTES)
 
     def state_need(self):
         need = {"S": StateNeed((self.H, self.dk, self.dv), torch.float32)}

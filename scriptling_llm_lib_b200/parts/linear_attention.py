@@ -18,6 +18,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.needs import StateNeed
+from ..csrc.bindings import ChunkKernels
 from ..weights.spec import TensorSpec
 from .base import MIXERS, Mixer
 from .linear import Linear
@@ -48,6 +49,9 @@ class DecayLinearAttention(Mixer):
         self.out.bind(tensors, dtype, device)
         self.norm_w = tensors[self.norm_name].float().contiguous()
         self.decay = torch.tensor(self.decay_values, dtype=torch.float64).to(torch.float32).to(device)
+
+    def scratch_bytes(self, rows: int) -> int:
+        return ChunkKernels.scratch_bytes(rows, 4 * self.dk * self.dv)
 
     def state_need(self):
         return {"S": StateNeed((self.H, self.dk, self.dv), torch.float32)}

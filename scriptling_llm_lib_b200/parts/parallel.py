@@ -37,6 +37,9 @@ class ParallelMixer(Mixer):
         for m in self.mixers:
             m.prepare(max_positions, device)
 
+    def scratch_bytes(self, rows: int) -> int:
+        return max(m.scratch_bytes(rows) for m in self.mixers)
+
     def cache_need(self):
         for m in self.mixers:
             if m.cache_need() is not None:

@@ -17,6 +17,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.needs import StateNeed
+from ..csrc.bindings import ChunkKernels, MixKernels
 from ..weights.spec import TensorSpec
 from .base import MIXERS, Mixer
 from .conv import CausalConv
@@ -53,6 +54,9 @@ class SelectiveScan(Mixer):
             p.bind(tensors, dtype, device)
         n = self.names
         self.dt_b, self.a_log, self.d = (tensors[n[k]].float().contiguous() for k in ("dt_b", "a_log", "d"))
+
+    def scratch_bytes(self, rows: int) -> int:
+        return MixKernels.scan_scratch_bytes(rows, 0, self.I, self.N, ChunkKernels.SMS) + ChunkKernels.SCRATCH_BYTES
 
     def state_need(self):
         need = {"S": StateNeed((self.I, self.N), torch.float32)}

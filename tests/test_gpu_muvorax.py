@@ -706,6 +706,23 @@ def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
             assert float((a[both] - b[both]).abs().max()) < 1e-5 * float(a[both].abs().max())
 
 
+def test_heads_of_linear_attention_in_several_passes(monkeypatch):
+    """As many heads at a time as the scratch's bound holds: three, then two; the bits of all five at once."""
+    from scriptling_llm_lib_b200.csrc.bindings import ChunkKernels, KernelSet
+    k, H, D, V, lens = KernelSet(torch.bfloat16).mix, 5, 24, 136, [300, 140]
+    g = torch.Generator().manual_seed(6)
+    proj, decay = torch.randn(sum(lens), 2 * H * D + H * V, generator=g).bfloat16().cuda(), torch.rand(H, generator=g).cuda()
+    state0, got = torch.randn(2, H, D, V, generator=g), []
+    ctx = SimpleNamespace(seq_start=torch.tensor([0, 300, 440], dtype=torch.int32).cuda(), slots=torch.tensor([1, 0], dtype=torch.int32).cuda(), n_seqs=2,
+                          max_new=300)
+    for bound in (ChunkKernels.SCRATCH_BYTES, (sum(lens) // 128 + 2) * 3 * 4 * D * V):
+        monkeypatch.setattr(ChunkKernels, "SCRATCH_BYTES", bound)
+        st, o = state0.clone().cuda(), torch.full((sum(lens), H * V), float("nan"), device="cuda")
+        k.chunk.lin_attn(proj, 0, H * D, 2 * H * D, decay, st, ctx, o, H, D, V)
+        got.append((st, o))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_the_norm_adds_a_normed_addend_and_keeps_the_sum():
     from scriptling_llm_lib_b200.csrc.bindings import KernelSet
     for dtype in (torch.float32, torch.bfloat16):

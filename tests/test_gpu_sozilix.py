@@ -544,6 +544,17 @@ def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
             assert float((a[both] - b[both]).abs().max()) < 2e-5 * float(a[both].abs().max())
 
 
+def test_heads_of_the_delta_rule_in_several_passes(monkeypatch):
+    """As many heads at a time as the scratch's bound holds: three, then two; the bits of all five at once."""
+    from scriptling_llm_lib_b200.csrc.bindings import ChunkKernels
+    lens, H, G, dk, dv = [300, 140], 5, 5, 40, 24
+    case = _delta_case(lens, H, G, dk, dv, 5)
+    _, want = _delta_both(*case, lens, [2, 0], H, G, dk, dv)
+    monkeypatch.setattr(ChunkKernels, "SCRATCH_BYTES", (sum(lens) // 128 + 2) * 3 * ChunkKernels.DELTA_BYTES)
+    _, got = _delta_both(*case, lens, [2, 0], H, G, dk, dv)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
 # ------------------------------------------------------------------ generation
 @pytest.mark.parametrize("cfg,seed", [(CFG_A, 21), (CFG_B, 22)])
 def test_greedy_generation_through_the_entry_point(tmp_path, cfg, seed):

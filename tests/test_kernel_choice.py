@@ -4,7 +4,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-from scriptling_llm_lib_b200.csrc.bindings import MixKernels, SequenceKernels
+from scriptling_llm_lib_b200.csrc.bindings import ChunkKernels, MixKernels, SequenceKernels
 
 
 def _recorded(cls, walk):
@@ -73,7 +73,8 @@ SCAN = [(4096, 16, [2048], "pieces"),                    # 466 / 143
         (64, 16, [96] + [16] * 100, "walk"),             # 21 / 24
         (512, 4, [96] + [16] * 100, "walk"),             # 22 / 26
         (1024, 16, [96] + [16] * 100, "pieces"),         # 132 / 70
-        (4096, 33, [2048], "walk")]                      # more states than it is built for
+        (4096, 33, [2048], "walk"),                      # more states than it is built for
+        (4096, 16, [96] + [16] * 2000, "walk")]          # a state for each of so many runs would take 550 MB
 
 
 @pytest.mark.parametrize("inner, N, lens, want", SCAN)
@@ -120,3 +121,33 @@ def test_more_key_rows_than_a_tensor_map_reaches_keep_the_other_kernels():
         kp = torch.empty((pages, H, 64, D), dtype=torch.bfloat16, device="meta")
         layer._attend(torch.empty((100, 3 * H * D), dtype=torch.bfloat16, device="meta"), x, ctx, kp, kp, None, False, None, True)
     assert ran == ["tcgen05", "paged"]
+
+
+@pytest.mark.parametrize("rows, n_seqs, H", [(2048, 1, 16), (16384, 1, 16), (16384, 8, 64), (12992, 401, 16), (16384, 1, 1), (130000, 1000, 32)])
+def test_scratch_of_the_chunks_is_bounded(rows, n_seqs, H):
+    """Heads are gone through as many at a time as the bound holds, evenly; one at least."""
+    n, per = rows // ChunkKernels.CHUNK + n_seqs, ChunkKernels.DELTA_BYTES
+    held = ChunkKernels.heads_held(n, H, per)
+    passes = -(-H // held)
+    assert 1 <= held <= H and (n * held * per <= ChunkKernels.SCRATCH_BYTES or held == 1)
+    assert passes == 1 or n * -(-H // (passes - 1)) * per > ChunkKernels.SCRATCH_BYTES       # no pass more than it takes
+
+
+def test_the_reserve_counts_what_a_recurrence_takes_beside_its_rows():
+    """What the cache leaves free for a prompt step holds the chunks' scratch, alone and inside a parallel mixer."""
+    from scriptling_llm_lib_b200.engine import Engine
+    from scriptling_llm_lib_b200.parts.base import MIXERS, Norm, PartSpec
+    delta = PartSpec("gated_delta_rule", dict(hidden=1024, n_heads=64, n_kv_heads=64, key_dim=16, value_dim=16, conv_taps=4, norm_eps=1e-6,
+                                              **{n: n for n in ("q_name", "k_name", "v_name", "q_conv_name", "k_conv_name", "v_conv_name", "beta_name",
+                                                                "decay_name", "a_log_name", "dt_bias_name", "gate_name", "norm_name", "o_name")}))
+    eng = lambda parts: SimpleNamespace(layout=SimpleNamespace(hidden_size=1024, vocab_size=512), model=SimpleNamespace(parts=lambda: parts),      # noqa: E731
+                                        PROMPT_TOKENS_PER_STEP=Engine.PROMPT_TOKENS_PER_STEP)
+    plain = Engine.activation_reserve_bytes(eng([Norm(), object()]))
+    for part in (MIXERS.build(delta), MIXERS.build(PartSpec("parallel", dict(branches=[("a", delta, 1.0)])))):
+        assert Engine.activation_reserve_bytes(eng([Norm(), part])) == plain + ChunkKernels.SCRATCH_BYTES
+    scan = PartSpec("selective_scan", dict(hidden=1024, inner=2048, n_state=16, dt_rank=64, conv_taps=4, **{n: n for n in (
+        "in_name", "conv_name", "conv_bias_name", "x_name", "dt_name", "dt_bias_name", "a_log_name", "d_name", "o_name")}))
+    rows = Engine.PROMPT_TOKENS_PER_STEP
+    need = 4 * 2048 * (rows + (rows // 64 + 50) * 17)
+    assert Engine.activation_reserve_bytes(eng([MIXERS.build(scan)])) >= plain + need
+    assert MixKernels.scan_scratch_bytes(rows, 50, 2048, 16, 148) == need
