@@ -165,14 +165,13 @@ class KernelSet:
                                    c_int(ksplit), _stream()), "gemm_nt")
 
     def gemm_nt_blocks_take(self, a, w) -> bool:
-        """Whether `gemm_nt_blocks` runs these as one launch: more than 64 rows, 16-byte (float) or 8-byte (bfloat16) aligned pieces."""
-        nb, _, k = w.shape
-        return (a.shape[0] > 64 and k % 4 == 0 and a.stride(0) % 4 == 0 and w.is_contiguous()
-                and all(t.data_ptr() % (4 * t.element_size()) == 0 for t in (a, w)))
+        """Whether `gemm_nt_blocks` runs these as one launch: the 32-bit set, more than 64 rows, 16-byte aligned pieces."""
+        return (self.dtype == torch.float32 and a.shape[0] > 64 and w.shape[2] % 4 == 0 and a.stride(0) % 4 == 0 and w.is_contiguous()
+                and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
     def gemm_nt_blocks(self, a, w, out):
         """Block-diagonal product: out[b] = a[:, b K:(b + 1) K] @ w[b]^T for a [M, blocks K] (unit column stride), w [blocks, N, K] and
-        out [blocks, M, N], all of this set's dtype."""
+        out [blocks, M, N], all float32."""
         nb, N, K = w.shape
         M = a.shape[0]
         if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or a.dtype != self.dtype or not a.is_cuda or a.stride(1) != 1:

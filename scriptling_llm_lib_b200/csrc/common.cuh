@@ -170,6 +170,20 @@ __device__ __forceinline__ void st4(bf16* p, float4 v) {
   r.y = *(uint32_t*)&hi;
   *(uint2*)p = r;
 }
+// two neighbouring floats as three packed pairs of bfloat16 that add up to them
+__device__ __forceinline__ void split_pair(float u, float v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(u, v);
+  p0 = *(const uint32_t*)&a;
+  u -= __uint_as_float(p0 << 16);
+  v -= __uint_as_float(p0 & 0xffff0000u);
+  const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
+  p1 = *(const uint32_t*)&b;
+  u -= __uint_as_float(p1 << 16);
+  v -= __uint_as_float(p1 & 0xffff0000u);
+  const __nv_bfloat162 c = __floats2bfloat162_rn(u, v);
+  p2 = *(const uint32_t*)&c;
+}
+
 struct F8 { float f[8]; };
 __device__ __forceinline__ F8 ld8(const float* p) {
   F8 r;

@@ -30,19 +30,6 @@ __device__ __forceinline__ void cp16(bf16* dst, const bf16* src, bool there) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
-// two neighbouring floats as three packed pairs of bfloat16 that add up to them
-__device__ __forceinline__ void split3(float u, float v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(u, v);
-  p0 = *(const uint32_t*)&a;
-  u -= __uint_as_float(p0 << 16);
-  v -= __uint_as_float(p0 & 0xffff0000u);
-  const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
-  p1 = *(const uint32_t*)&b;
-  u -= __uint_as_float(p1 << 16);
-  v -= __uint_as_float(p1 & 0xffff0000u);
-  const __nv_bfloat162 c = __floats2bfloat162_rn(u, v);
-  p2 = *(const uint32_t*)&c;
-}
 
 // ------------------------------------------------------------------ the queries
 // qa[t][h] = scale * [Wuk_h^T q_unrot | q_rot]. A block has 16 rows, one head and 64 of the latent's columns: the matrix's part comes
@@ -158,10 +145,10 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(AttnArgs p) {
       const float2 z = make_float2(0.f, 0.f);
       const float2 f0 = ha < p.H && c < W ? *(const float2*)(qr_a + c) : z, f1 = hb < p.H && c < W ? *(const float2*)(qr_b + c) : z;
       const float2 f2 = ha < p.H && c + 8 < W ? *(const float2*)(qr_a + c + 8) : z, f3 = hb < p.H && c + 8 < W ? *(const float2*)(qr_b + c + 8) : z;
-      split3(f0.x, f0.y, qf[s][0][0], qf[s][1][0], qf[s][2][0]);
-      split3(f1.x, f1.y, qf[s][0][1], qf[s][1][1], qf[s][2][1]);
-      split3(f2.x, f2.y, qf[s][0][2], qf[s][1][2], qf[s][2][2]);
-      split3(f3.x, f3.y, qf[s][0][3], qf[s][1][3], qf[s][2][3]);
+      split_pair(f0.x, f0.y, qf[s][0][0], qf[s][1][0], qf[s][2][0]);
+      split_pair(f1.x, f1.y, qf[s][0][1], qf[s][1][1], qf[s][2][1]);
+      split_pair(f2.x, f2.y, qf[s][0][2], qf[s][1][2], qf[s][2][2]);
+      split_pair(f3.x, f3.y, qf[s][0][3], qf[s][1][3], qf[s][2][3]);
     }
   }
   float o[NT][4];
@@ -237,8 +224,8 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(AttnArgs p) {
       l = l * cor + sum;
       m = mn;
       uint2 q[3];
-      split3(v[0], v[1], q[0].x, q[1].x, q[2].x);
-      split3(v[2], v[3], q[0].y, q[1].y, q[2].y);
+      split_pair(v[0], v[1], q[0].x, q[1].x, q[2].x);
+      split_pair(v[2], v[3], q[0].y, q[1].y, q[2].y);
 #pragma unroll
       for (int k = 0; k < 3; k++) *(uint2*)(pp + (k * 16 + srow) * PL + skey) = q[k];
       if ((lane & 15) == 0) corr_s[srow] = cor;
@@ -373,14 +360,14 @@ __global__ void __launch_bounds__(128) latent_expand_mma_kernel(const float* __r
     const float4 a0 = in && ra < T ? *(const float4*)(xa + c) : z, a1 = in && ra < T ? *(const float4*)(xa + c + 4) : z;
     const float4 b0 = in && rb < T ? *(const float4*)(xb + c) : z, b1 = in && rb < T ? *(const float4*)(xb + c + 4) : z;
     uint32_t f[2][3][4];
-    split3(a0.x, a0.y, f[0][0][0], f[0][1][0], f[0][2][0]);
-    split3(b0.x, b0.y, f[0][0][1], f[0][1][1], f[0][2][1]);
-    split3(a0.z, a0.w, f[0][0][2], f[0][1][2], f[0][2][2]);
-    split3(b0.z, b0.w, f[0][0][3], f[0][1][3], f[0][2][3]);
-    split3(a1.x, a1.y, f[1][0][0], f[1][1][0], f[1][2][0]);
-    split3(b1.x, b1.y, f[1][0][1], f[1][1][1], f[1][2][1]);
-    split3(a1.z, a1.w, f[1][0][2], f[1][1][2], f[1][2][2]);
-    split3(b1.z, b1.w, f[1][0][3], f[1][1][3], f[1][2][3]);
+    split_pair(a0.x, a0.y, f[0][0][0], f[0][1][0], f[0][2][0]);
+    split_pair(b0.x, b0.y, f[0][0][1], f[0][1][1], f[0][2][1]);
+    split_pair(a0.z, a0.w, f[0][0][2], f[0][1][2], f[0][2][2]);
+    split_pair(b0.z, b0.w, f[0][0][3], f[0][1][3], f[0][2][3]);
+    split_pair(a1.x, a1.y, f[1][0][0], f[1][1][0], f[1][2][0]);
+    split_pair(b1.x, b1.y, f[1][0][1], f[1][1][1], f[1][2][1]);
+    split_pair(a1.z, a1.w, f[1][0][2], f[1][1][2], f[1][2][2]);
+    split_pair(b1.z, b1.w, f[1][0][3], f[1][1][3], f[1][2][3]);
     float y[4][4];                                       // the step's sums, smallest part first, added up as floats
 #pragma unroll
     for (int n = 0; n < 4; n++) y[n][0] = y[n][1] = y[n][2] = y[n][3] = 0.f;

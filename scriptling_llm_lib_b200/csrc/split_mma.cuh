@@ -16,19 +16,6 @@ namespace sm3 {
 constexpr int TILE = 128;
 constexpr uint32_t BLOCK_BYTES = TILE * 128, PLANE_BYTES = 2 * BLOCK_BYTES, TILE_BYTES = 3 * PLANE_BYTES;
 
-// two neighbouring floats as three packed pairs of bfloat16 that add up to them
-__device__ __forceinline__ void split_pair(float u, float v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  const __nv_bfloat162 a = __floats2bfloat162_rn(u, v);
-  p0 = *(const uint32_t*)&a;
-  u -= __uint_as_float(p0 << 16);
-  v -= __uint_as_float(p0 & 0xffff0000u);
-  const __nv_bfloat162 b = __floats2bfloat162_rn(u, v);
-  p1 = *(const uint32_t*)&b;
-  u -= __uint_as_float(p1 << 16);
-  v -= __uint_as_float(p1 & 0xffff0000u);
-  const __nv_bfloat162 c = __floats2bfloat162_rn(u, v);
-  p2 = *(const uint32_t*)&c;
-}
 // eight columns from c (a multiple of 8) of row r into the tile's three planes
 __device__ __forceinline__ void put8(uint8_t* tile, int r, int c, const float (&f)[8]) {
   uint4 q[3];
