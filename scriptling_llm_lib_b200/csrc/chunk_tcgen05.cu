@@ -34,13 +34,14 @@ using namespace sm3;
 
 constexpr int Q = TILE, NT = 512, PIECES = Q * Q / 8 / NT;      // rows of a chunk, threads, 8-column pieces of a tile a thread makes
 
-// z / (1 + exp(-z)); the reciprocal is the hardware's with one Newton step (its error is then a float's last place), and the
-// exponential is held below where that step would meet an infinity
+// z / (1 + exp(-z)); the reciprocal is the hardware's with one Newton step (its error is then a float's last place), which is left out
+// where it would meet a product beyond float's range
 __device__ __forceinline__ float silu_f(float z) {
-  const float d = 1.0f + fminf(expf(-z), 1e36f);
+  const float d = 1.0f + expf(-z);
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return z * fmaf(r, fmaf(-d, r, 1.0f), r);
+  const float near = fmaf(r, fmaf(-d, r, 1.0f), r);
+  return z * (d < 1e36f ? near : r);
 }
 
 struct LinArgs {

@@ -706,6 +706,48 @@ def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
             assert float((a[both] - b[both]).abs().max()) < 1e-5 * float(a[both].abs().max())
 
 
+def test_linear_attention_in_chunks_over_long_runs():
+    """Runs of up to eleven chunks, past the eight that the hand-over asks for at a time, beside one of a row: 1e-5 of the largest element
+    as for short runs."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, H, D, V, lens, slots = KernelSet(torch.bfloat16).mix, 2, 24, 40, [1, 1025, 1300, 640], [3, 0, 4, 1]
+    g, T = torch.Generator().manual_seed(8), sum(lens)
+    proj, decay, state0 = torch.randn(T, 2 * H * D + H * V, generator=g).bfloat16(), torch.tensor([0.9995, 0.97]), torch.randn(5, H, D, V, generator=g)
+    start = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ctx = SimpleNamespace(seq_start=torch.from_numpy(start).cuda(), slots=torch.tensor(slots, dtype=torch.int32).cuda(), n_seqs=4, max_new=1300)
+    st, o = state0.clone().cuda(), torch.full((T, H * V), float("nan"), device="cuda")
+    k.chunk.lin_attn(proj.cuda(), 0, H * D, 2 * H * D, decay.cuda(), st, ctx, o, H, D, V)
+    q, kk, v = (plain.silu(t).view(T, H, -1) for t in proj.double().split([H * D, H * D, H * V], 1))
+    want, after = torch.empty((T, H, V), dtype=torch.float64), state0.double()
+    for b, slot in enumerate(slots):
+        S = state0[slot].double()
+        for t in range(start[b], start[b + 1]):
+            S = decay.double()[:, None, None] * S + kk[t, :, :, None] * v[t, :, None]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        after[slot] = S
+    assert float((o.cpu().double() - want.view(T, -1)).abs().max()) < 1e-5 * float(want.abs().max())
+    assert float((st.cpu().double() - after).abs().max()) < 1e-5 * float(after.abs().max())
+
+
+def test_silu_of_every_bfloat16_in_the_chunks():
+    """One row, values of every finite bfloat16 there is: the state silu(k) silu(v) to a float's few last places (its parts, down to where
+    they leave float's range: 1e-4 below 1e-30), and what silu makes 0 is 0."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    k, D = KernelSet(torch.bfloat16).mix, 8
+    v = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    v = v[v.isfinite() & (v.abs() < 1e30)]
+    v = v[:len(v) // 8 * 8]
+    V, key = len(v), torch.tensor(1.28).bfloat16()
+    proj = torch.cat([torch.ones(D).bfloat16(), key.expand(D), v])[None].cuda()
+    ctx = SimpleNamespace(seq_start=torch.tensor([0, 1], dtype=torch.int32).cuda(), slots=torch.zeros(1, dtype=torch.int32).cuda(), n_seqs=1, max_new=1)
+    st, o = torch.zeros(1, 1, D, V, device="cuda"), torch.empty(1, V, device="cuda")
+    k.chunk.lin_attn(proj, 0, D, 2 * D, torch.ones(1, device="cuda"), st, ctx, o, 1, D, V)
+    want = plain.silu(key.double()) * torch.where(v.double() < -700, torch.zeros(V, dtype=torch.float64), plain.silu(v.double().clamp(min=-700)))
+    err = (st[0, 0, 0].cpu().double() - want).abs()
+    tol = torch.where(want.abs() > 1e-30, 1e-6, 1e-4) * want.abs() + 1e-36
+    assert bool((err <= tol).all()), (v[err > tol][:8], err[err > tol][:8])
+
+
 def test_heads_of_linear_attention_in_several_passes(monkeypatch):
     """As many heads at a time as the scratch's bound holds: three, then two; the bits of all five at once."""
     from scriptling_llm_lib_b200.csrc.bindings import ChunkKernels, KernelSet

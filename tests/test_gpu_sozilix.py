@@ -544,6 +544,30 @@ def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
             assert float((a[both] - b[both]).abs().max()) < 2e-5 * float(a[both].abs().max())
 
 
+def test_the_delta_rule_in_chunks_over_long_runs():
+    """Runs of up to ten chunks beside one of a row: the hand-over's buffers and barriers come round several times. Against the recurrence in
+    64 bits, 2e-5 of the largest element as for short runs; nearer the walk's error than five times."""
+    lens, H, G, dk, dv = [1, 1025, 1153, 640], 2, 1, 48, 40
+    wide, bd, state0 = _delta_case(lens, H, G, dk, dv, 7)
+    bd[:, H:2 * H] = bd[:, H:2 * H] ** 0.1           # what comes from chunks back still counts
+    (o, st), (oc, sc) = _delta_both(wide, bd, state0, lens, [3, 0, 4, 1], H, G, dk, dv)
+    T = sum(lens)
+    q, keys = (t.double().view(T, G, dk).repeat_interleave(H // G, 1) for t in (wide[:, :G * dk], wide[:, G * dk:2 * G * dk]))
+    v, beta, decay = wide[:, 2 * G * dk:].double().view(T, H, dv), bd[:, :H].double(), bd[:, H:2 * H].double()
+    want, after, row = torch.empty(T, H, dv, dtype=torch.float64), state0.double(), 0
+    for n, slot in zip(lens, [3, 0, 4, 1]):
+        S = state0[slot].double()
+        for t in range(row, row + n):
+            S = S * decay[t, :, None, None]
+            S = S + keys[t, :, :, None] * (beta[t, :, None] * (v[t] - torch.einsum("hdv,hd->hv", S, keys[t])))[:, None]
+            want[t] = torch.einsum("hdv,hd->hv", S, q[t])
+        after[slot], row = S, row + n
+    want = want.view(T, -1)
+    off = lambda a, b: float((a.double() - b).norm() / b.norm())      # noqa: E731
+    assert float((oc.double() - want).abs().max()) < 2e-5 * float(want.abs().max())
+    assert off(oc, want) < 5 * off(o, want) and off(sc, after) < 5 * off(st, after)
+
+
 def test_heads_of_the_delta_rule_in_several_passes(monkeypatch):
     """As many heads at a time as the scratch's bound holds: three, then two; the bits of all five at once."""
     from scriptling_llm_lib_b200.csrc.bindings import ChunkKernels
