@@ -24,7 +24,7 @@
 //   chunk_delta_pass    S through the chunks one after the other, 32 of its columns a block
 //   chunk_delta_out     every chunk's outputs from the S in front of it
 // 2,048 rows of 16 heads of 128 x 128: 100 + 50 + 20 us (640 walked row by row, a dependent chain a column of the state); eight
-// sequences, 9,900 rows: 420 + 137 + 103 (1,471). The first kernel is bound by its sixteen warps going through nine tiles and eight
+// sequences, 9,900 rows: 420 + 137 + 103 (1,471). The first kernel has taken 4 us more since it watches for what is not finite. The first kernel is bound by its sixteen warps going through nine tiles and eight
 // products one after the other with nothing beside them on the SM; that its code is fetched once a block shows in it too (with
 // products and the inversion unrolled, and the paths without 16-byte accesses in the same kernel: 130 us, 597 for the eight).
 #include "split_mma.cuh"

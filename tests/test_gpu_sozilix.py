@@ -546,7 +546,8 @@ def test_what_is_not_finite_in_a_row_stays_behind_it_in_chunks(where, bad):
 
 def test_the_delta_rule_in_chunks_over_long_runs():
     """Runs of up to ten chunks beside one of a row: the hand-over's buffers and barriers come round several times. Against the recurrence in
-    64 bits, 2e-5 of the largest element as for short runs; nearer the walk's error than five times."""
+    64 bits, 2e-5 of the largest element as for short runs; and all in all: three products behind one another, each of eight steps that
+    cut half of 2^-24 on average, 7e-7."""
     lens, H, G, dk, dv = [1, 1025, 1153, 640], 2, 1, 48, 40
     wide, bd, state0 = _delta_case(lens, H, G, dk, dv, 7)
     bd[:, H:2 * H] = bd[:, H:2 * H] ** 0.1           # what comes from chunks back still counts
@@ -565,7 +566,7 @@ def test_the_delta_rule_in_chunks_over_long_runs():
     want = want.view(T, -1)
     off = lambda a, b: float((a.double() - b).norm() / b.norm())      # noqa: E731
     assert float((oc.double() - want).abs().max()) < 2e-5 * float(want.abs().max())
-    assert off(oc, want) < 5 * off(o, want) and off(sc, after) < 5 * off(st, after)
+    assert max(off(o, want), off(st, after)) < 7e-7 and max(off(oc, want), off(sc, after)) < 7e-7
 
 
 def test_heads_of_the_delta_rule_in_several_passes(monkeypatch):
