@@ -517,14 +517,14 @@ class PrefillAttentionTC:
         the window; `gate`: bfloat16 [T, n_heads * v_dim] (a column slice), whose sigmoid multiplies the output."""
         v_dim = v_dim or head_dim
         gp, gl = _gate_args(gate, q.shape[0], n_heads * v_dim)
+        # (a Python int goes to C as it is: a c_int made for each would cost a short prompt's launch another microsecond or two)
         _check(self.lib.sllm_attn_prefill_tc_bf16(
-            _ptr(q, torch.bfloat16, "q"), c_int(q.shape[1]), c_int(q.shape[0]), _ptr(out, torch.bfloat16, "out"),
+            _ptr(q, torch.bfloat16, "q"), q.shape[1], q.shape[0], _ptr(out, torch.bfloat16, "out"),
             _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
-            _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
+            _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
             _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), c_longlong(kpages.shape[0]),
-            c_int(n_seqs), c_int(max_new), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(v_dim), c_int(window or 0), c_int(keep),
-            c_float(scale), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, c_int(3 if exact_weights else 1),
-            _ptr(err_flag, torch.int32, "err_flag"), _stream()), "attn_prefill_tc")
+            n_seqs, max_new, n_heads, n_kv, head_dim, v_dim, window or 0, keep, c_float(scale), c_float(softcap or 0.0),
+            _ptr(sink, torch.float32, "sink"), gp, gl, 3 if exact_weights else 1, _ptr(err_flag, torch.int32, "err_flag"), _stream()), "attn_prefill_tc")
 
 
 def _gate_args(gate, rows: int, cols: int):

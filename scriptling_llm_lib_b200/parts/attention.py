@@ -72,16 +72,16 @@ from .linear import Linear
 from .norm import WithRowVector
 
 
-def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int, rows: int = 0) -> bool:
+def exact_prompt_kernel(ctx, dtype, key_dim: int, value_dim: int, key_elements: int = 0) -> bool:
     """Whether a layer that keeps its softmax weights in float32 runs this step's attention on the tcgen05 kernel that takes them
-    in three bfloat16 parts: a bfloat16 step that is no decode step, widths in multiples of 8 (keys up to 192, values up to 128), `rows`
-    of key storage that its tensor maps reach (narrow heads can have more in memory).
+    in three bfloat16 parts: a bfloat16 step that is no decode step, widths in multiples of 8 (keys up to 192, values up to 128), key
+    storage of no more rows than its tensor maps reach (narrow heads can have more in memory).
     A portion on a cache, however short, is better off there (8 rows of 16 heads on 8,000 keys, keys 64 and values 128 306 us, 537 with
     a warp a row; equal widths of 80 210, 1,310 on the float tiles), a prompt of very few rows is not: its fixed 7 to 9 us are more than
     the others take for up to 16 rows of unequal widths (8 rows 8.5, 5.3; 20 rows 8.5 either way), or for one or two of a narrow
     equal one (2 rows of 32 dims 6.9, 6.1; 4 rows 6.9, 8.0; one of 80 7.9, 8.1). A decode step has one query a sequence where the kernel
     works on 128, and keeps the kernels that split the keys."""
-    if dtype != torch.bfloat16 or ctx.is_decode or rows > PrefillAttentionTC.MAX_ROWS or not PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True):
+    if dtype != torch.bfloat16 or ctx.is_decode or key_elements > PrefillAttentionTC.MAX_ROWS * key_dim or not PrefillAttentionTC.takes(key_dim, value_dim, exact_weights=True):
         return False
     few = 16 * key_dim if value_dim != key_dim or key_dim % 16 else 96
     return ctx.max_new * key_dim > few or not getattr(ctx, "from_start", False)
@@ -97,7 +97,7 @@ def prompt_attention(q, gate, ctx, kpages, vpages, block_table, n_heads, n_kv, k
     k = ctx.kernels
     attn = torch.empty((q.shape[0], n_heads * value_dim), dtype=q.dtype, device=q.device)
     fused = gate if gate is not None and q.dtype == torch.bfloat16 and gate_aligned(gate) else None
-    exact = not tensor_cores and exact_prompt_kernel(ctx, q.dtype, key_dim, value_dim, kpages.shape[:-1].numel())
+    exact = not tensor_cores and exact_prompt_kernel(ctx, q.dtype, key_dim, value_dim, kpages.numel())
     tensor_cores = tensor_cores and q.dtype == torch.bfloat16
     if exact or (tensor_cores and PrefillAttentionTC.takes(key_dim, value_dim)):
         k.prefill_attention_tc.attn(q, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs, ctx.max_new, n_heads,
@@ -307,7 +307,7 @@ class Attention(Mixer):
         """The step's queries (the leading columns of `qkv`) over the cache -> [T, n_heads * v_dim]."""
         attn = torch.empty((x.shape[0], self.n_heads * self.v_dim), dtype=x.dtype, device=x.device)
         plain_widths = not self.other_widths and self.head_dim in PrefillAttentionTC.HEAD_DIMS
-        if not plain_widths and exact_prompt_kernel(ctx, x.dtype, self.head_dim, self.v_dim, kpages.shape[:-1].numel()):
+        if not plain_widths and exact_prompt_kernel(ctx, x.dtype, self.head_dim, self.v_dim, kpages.numel()):
             ctx.kernels.prefill_attention_tc.attn(qkv, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs,
                                                   ctx.max_new, self.n_heads, self.n_kv_heads, self.head_dim, self.span, self.scale,
                                                   ctx.err_flag, v_dim=self.v_dim, exact_weights=True)
