@@ -864,12 +864,12 @@ class SequenceKernels:
         """Rotate queries (in place) and keys by the table, store keys and values (divided by their root
         mean square when v_eps is not None) at the rows' places in the cache pages."""
         T, ld = qkv.shape
-        _check(self._fn("kv_store")(_ptr(qkv, self.dtype, "qkv"), c_int(ld), _ptr(tok_pos, torch.int32, "tok_pos"),
+        _check(self._fn("kv_store")(_ptr(qkv, self.dtype, "qkv"), ld, _ptr(tok_pos, torch.int32, "tok_pos"),
                                     _ptr(tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"),
-                                    c_int(block_table.shape[1]), _ptr(cos_sin, torch.float32, "cos_sin"),
+                                    block_table.shape[1], _ptr(cos_sin, torch.float32, "cos_sin"),
                                     _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-                                    _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c_int(T), c_int(n_heads),
-                                    c_int(n_kv), c_int(head_dim), c_int(v_dim), c_int(rot), c_int(1 if interleaved else 0),
+                                    _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, n_heads,
+                                    n_kv, head_dim, v_dim, rot, (1 if interleaved else 0),
                                     c_float(-1.0 if v_eps is None else v_eps), _stream()), "kv_store")
 
     def attn_wide_value(self, q, out, tok_pos, tok_seq, block_table, kpages, vpages, n_heads, n_kv, head_dim, v_dim, window, scale):
@@ -887,10 +887,10 @@ class SequenceKernels:
         dt_bias)) and k . q per query/key head."""
         if tuple(bd.shape) != (qk.shape[0], 2 * n_heads + n_kv):
             raise KernelError(f"delta_prepare: bd is {tuple(bd.shape)}, expected {(qk.shape[0], 2 * n_heads + n_kv)}")
-        _check(self._fn("delta_prepare")(self._view(qk, "qk"), c_int(qk.stride(0)), self._view(ba, "ba"), c_int(ba.stride(0)),
+        _check(self._fn("delta_prepare")(self._view(qk, "qk"), qk.stride(0), self._view(ba, "ba"), ba.stride(0),
                                          _ptr(a_log, None, "a_log"), _ptr(dt_bias, None, "dt_bias"),
-                                         c_int(self._flag(a_log, "a_log")), _ptr(bd, torch.float32, "bd"), c_int(qk.shape[0]),
-                                         c_int(n_heads), c_int(n_kv), c_int(dk), _stream()), "delta_prepare")
+                                         self._flag(a_log, "a_log"), _ptr(bd, torch.float32, "bd"), qk.shape[0],
+                                         n_heads, n_kv, dk, _stream()), "delta_prepare")
 
     def delta_rule(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
         """qk float32 rows [G dk queries | G dk keys] (unit vectors), v float32 [T, H dv], bd float32 [T, 2H + G]
@@ -907,11 +907,11 @@ class SequenceKernels:
 
     def delta_walk(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
         """`delta_rule` row by row."""
-        _check(self._fn("delta_rule")(self._view(qk, "qk"), c_int(qk.stride(0)), self._view(v, "v"), c_int(v.stride(0)),
+        _check(self._fn("delta_rule")(self._view(qk, "qk"), qk.stride(0), self._view(v, "v"), v.stride(0),
                                       _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"),
                                       _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
-                                      _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)), c_int(n_heads),
-                                      c_int(n_kv), c_int(dk), c_int(dv), _stream()), "delta_rule")
+                                      _ptr(o, torch.float32, "o"), ctx.n_seqs, max(1, ctx.max_new), n_heads,
+                                      n_kv, dk, dv, _stream()), "delta_rule")
 
     def gated_unit_rms(self, o, gate, weight, y, n_heads, dv, eps):
         _check(self._fn("gated_unit_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), c_int(gate.stride(0)),
@@ -961,7 +961,7 @@ class ChunkKernels:
 
     @classmethod
     def delta_pays(cls, rows, n_seqs, longest, n_heads, dk, dv) -> bool:
-        if max(dk, dv) > cls.CHUNK:
+        if max(dk, dv) > cls.CHUNK or (longest < 160 and rows * n_heads * dv < 750_000):      # less than any chunk takes
             return False
         k, more = cls._shape(rows, n_seqs, n_heads, max(dk, dv))
         chunks = (58, 55, 53)[k] + 2.5 * longest / cls.CHUNK + 0.5 * (n_seqs - 1) + (0.6, 0.44, 0.37)[k] * more
