@@ -259,6 +259,15 @@ class KernelSet:
         _check(self._fn("swiglu")(_ptr(gate_up, self.dtype, "gate_up"), _ptr(out, self.dtype, "out"), c_int(T), c_int(F),
                                   c_int(1 if tiled else 0), _stream()), "swiglu")
 
+    @property
+    def split(self) -> "SplitGemm":
+        """The 32-bit products on the tensor cores (their own library, loaded on first use)."""
+        if self.dtype != torch.float32:
+            raise KernelError("products in three parts are the 32-bit set's")
+        if getattr(self, "_split", None) is None:
+            self._split = SplitGemm()
+        return self._split
+
     # ------------------------------------------------------------------ fast bfloat16 kernels
     @property
     def tensor_core(self) -> "TensorCoreGemm":
@@ -320,6 +329,57 @@ class KernelSet:
         if getattr(self, "_decode", None) is None:
             self._decode = DecodeKernels()
         return self._decode
+
+
+class SplitGemm:
+    """float32 products on the tcgen05 tensor cores, operands in three bfloat16 parts (see gemm_split_tcgen05.cu)."""
+
+    SCRATCH_BYTES = 256 << 20        # the most that the planes of a product's operands take at a time; larger ones go in portions
+
+    def __init__(self):
+        self.lib = load_library("gemm_split")
+        self.lib.sllm_gemm_split_f32.restype = c_int
+
+    FEW_ROWS_BYTES = 64 << 20        # and in products of up to 64 rows, whose planes a captured decode step would keep
+
+    @classmethod
+    def takes(cls, a, w, parts: int = 1) -> bool:
+        """Whether a product of `a` [M, K] with `w` [N, K], or with blocks [b, N, K] of a's columns, goes here and not to the FMA kernels:
+        widths and places that the copies take, sums of at least 64 terms (shorter ones can come out less exact than a chain of FMA: 48
+        terms of very unequal rows 1.11e-7, 1.10e-7), and sizes where it is faster, which is from 65 rows on everywhere (weights out
+        of memory, FMA / here, us: 65 rows 2,048 x 8,192 909 / 202, in 16 parts 103 / 71; 6,144 x 2,048 234 / 67; 2,048 x 64 9.4 / 8.2) and
+        from 17 on where K is one part and not tiny (17 rows 1,024 x 1,024 76 / 27, 64 x 2,048 129 / 45; but 2,048 x 64 6.4 / 7.8, 6,144 x
+        2,048 in 6 parts 50 / 51)."""
+        M, K, N = a.shape[0], w.shape[-1], w.numel() // w.shape[-1]
+        if not (M > 64 or (M > 16 and K >= 128 and parts == 1 and 6 * K * N + 6 * M * a.shape[1] <= cls.FEW_ROWS_BYTES)):
+            return False
+        return (a.dtype == w.dtype == torch.float32 and K % 8 == 0 and 64 <= K <= 32768 and 6 * a.shape[1] * 512 <= cls.SCRATCH_BYTES
+                and (w.dim() == 2 or 12 * K * N <= cls.SCRATCH_BYTES) and a.stride(0) % 4 == 0 and a.stride(1) == 1
+                and a.data_ptr() % 16 == 0 and w.is_contiguous() and w.data_ptr() % 16 == 0)
+
+    def _run(self, a, w, out, M, N, K, ldb, parts, batch, apart, err_flag):
+        scratch = torch.empty((min(6 * K * batch * (M + N), self.SCRATCH_BYTES),), dtype=torch.uint8, device=a.device)
+        _check(self.lib.sllm_gemm_split_f32(
+            c_void_p(a.data_ptr()), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), c_int(M), c_int(N), c_int(K),
+            c_int(a.stride(0)), c_int(ldb), c_int(N), c_int(parts), c_int(batch), c_longlong(apart), _ptr(scratch),
+            c_longlong(scratch.numel()), _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_split")
+
+    def gemm(self, a, w, out, err_flag):
+        """As `KernelSet.gemm_nt` of the 32-bit set: out[M,N] = a[M,K] @ w[N,K]^T, or its partial sums [P,M,N]."""
+        M, K = a.shape
+        N = w.shape[0]
+        parts = out.shape[0] if out.dim() == 3 else 1
+        if w.shape[1] != K or tuple(out.shape[-2:]) != (M, N) or a.dtype != torch.float32 or not a.is_cuda or a.stride(1) != 1:
+            raise KernelError(f"gemm_split shapes: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        self._run(a, w, out, M, N, K, w.stride(0), parts, 1, M * N, err_flag)
+
+    def blocks(self, a, w, out, err_flag):
+        """As `KernelSet.gemm_nt_blocks`: out[b] = a[:, b K:(b + 1) K] @ w[b]^T."""
+        nb, N, K = w.shape
+        M = a.shape[0]
+        if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or a.dtype != torch.float32 or not a.is_cuda or a.stride(1) != 1:
+            raise KernelError(f"gemm_split blocks: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        self._run(a, w, out, M, N, K, K, 1, nb, M * N, err_flag)
 
 
 class TensorCoreGemm:

@@ -32,6 +32,7 @@ LIBRARIES: dict[str, tuple[str, tuple[str, ...]]] = {
     "random": ("lib_random.cu", ("common.cuh", "philox.cuh")),
     "probe": ("lib_probe.cu", ("common.cuh",)),
     "decode_bf16": ("decode_bf16.cu", ("common.cuh", "attn_decode_noalloc.h")),
+    "gemm_split": ("gemm_split_tcgen05.cu", ("common.cuh", "tcgen05.cuh")),
     "gemm_tcgen05": ("gemm_tcgen05.cu", ("common.cuh", "tcgen05.cuh")),
     "attn_prefill_tcgen05": ("attn_prefill_tcgen05.cu", ("common.cuh", "tcgen05.cuh")),
     "attn_prefill_mma": ("attn_prefill_mma.cu", ("common.cuh",)),

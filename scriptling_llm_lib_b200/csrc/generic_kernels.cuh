@@ -372,9 +372,10 @@ gemm_nt_regtile_kernel(const TI* __restrict__ A, const TI* __restrict__ B, TO* _
 // batch, it takes the z-th product (operands and result `batch` strides apart) over the whole of K.
 // Bound by issue slots: the multiply-adds go two to an instruction (outputs of neighbouring columns; the
 // chains and their roundings are the same), and four lanes read the 64 bytes of a row's tile, so that a load
-// touches 8 rows' lines and not 32. 2,778 rows: x W^T of 2,560 x 1,024, five blocks of 512 x 256 and 1,024 x 1,280 took 929 us
-// in seven launches, 621 in three (41 TFLOP/s; the tiles are one and a half waves). With tiles of 64 rows, where few blocks wait for
-// their loads, it was the slower one (64 rows of a decode step: 602 us of products against 547).
+// touches 8 rows' lines and not 32. 2,778 rows: x W^T of 2,560 x 1,024, five blocks of 512 x 256 and 1,024 x 1,280 take 621 us in
+// three launches (41 TFLOP/s). Floats of widths in multiples of 8 go to the tensor cores (gemm_split_tcgen05.cu: 170 us for those); what
+// stays here are other widths, sums of fewer than 64 terms, and bfloat16 operands that the tensor-core kernels refuse. With tiles of
+// 64 rows, where few blocks wait for their loads, it was the slower one (64 rows of a decode step: 602 us of products against 547).
 struct GemmBatch { long long a, b, c; };      // strides in elements; all 0: no batch, blockIdx.z splits K
 __device__ __forceinline__ unsigned long long gemm_twice(float v) {
   unsigned long long d;

@@ -8,8 +8,8 @@
 // linear attention's state 1.1e-7 / 1.2e-6 off (whose chain there is the longer one), the delta rule's outputs and state 2.1e-7 and
 // 1.2e-7 / 9.7e-8 and 6.6e-8 (128 dims; of 32 dims 1.5e-7 and 1.1e-7 / 1.0e-7 and 7.9e-8; with decays near 1 2.8e-7 and 2.3e-7 /
 // 2.0e-7 and 1.9e-7). Ending a sum half way and adding the halves as floats took the outputs to 1.7e-7, left the state where it was
-// and cost a seventh of the kernels' time. Long sums do lose by it: 9.1e-6 against 1.6e-6 over 8,192 terms, so products of
-// weights are not made this way.
+// and cost a seventh of the kernels' time. Long sums do lose by it: 9.1e-6 against 1.6e-6 over 8,192 terms, so the products of
+// weights (gemm_split_tcgen05.cu) end a sum after 64.
 //
 // A tile is 128 rows of 128 columns: three planes of 32 KB, a plane two blocks of 64 columns, a block 128 rows of 128 bytes with
 // the 128-byte swizzle. The same bytes are an operand whose contraction runs along the columns (K-major) or along the rows

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc.bindings import SplitGemm
 from ..weights.spec import TensorSpec
 from .base import Folded, FoldRequest
 
@@ -116,14 +117,20 @@ class Linear:
             split = ctx.kernels.gemm_nt_split(x.shape[0], w.shape[0], w.shape[1], ctx.engine.sm_count) if partials_ok else 1
             shape = (split, x.shape[0], w.shape[0]) if split > 1 else (x.shape[0], w.shape[0])
             out = torch_empty(shape, torch.float32 if split > 1 else out_dtype, x.device)
-            ctx.kernels.gemm_nt(x, w, out)
+            if x.dtype == torch.float32 and SplitGemm.takes(x, w, split):
+                ctx.kernels.split.gemm(x, w, out, ctx.err_flag)
+            else:
+                ctx.kernels.gemm_nt(x, w, out)
             return out
         if w.dtype == torch.float32 and x.dtype == torch.bfloat16:
             # a matrix kept in 32-bit inside a bfloat16 model: widen the rows, multiply in 32-bit
             x32 = torch.empty(x.shape, dtype=torch.float32, device=x.device)
             ctx.casts.to_f32(x, x32)
             out32 = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
-            ctx.kernels_f32.gemm_nt(x32, w, out32)
+            if SplitGemm.takes(x32, w):
+                ctx.kernels_f32.split.gemm(x32, w, out32, ctx.err_flag)
+            else:
+                ctx.kernels_f32.gemm_nt(x32, w, out32)
             if out_dtype == torch.float32:
                 return out32
             out = torch.empty(out32.shape, dtype=torch.bfloat16, device=x.device)

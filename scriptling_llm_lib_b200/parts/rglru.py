@@ -16,6 +16,7 @@ from __future__ import annotations
 import torch
 
 from ..cache.needs import StateNeed
+from ..csrc.bindings import SplitGemm
 from ..weights.spec import TensorSpec
 from .base import MIXERS, Mixer
 from .conv import CausalConv
@@ -73,8 +74,10 @@ class RGLRU(Mixer):
         u = self.conv.forward(yx[:, W:], st.get("conv"), ctx, torch.float32, in_bias=self.x_b, also=u_low)
         src = u if u_low is None else u_low
         gates = torch.empty((self.blocks, T, 2 * bs), dtype=torch.float32, device=x.device)
-        if src.dtype == torch.float32 == self.gate_w.dtype and ctx.kernels.gemm_nt_blocks_take(src, self.gate_w):
-            ctx.kernels.gemm_nt_blocks(src, self.gate_w, gates)                # every block's product in one launch
+        if src.dtype == torch.float32 == self.gate_w.dtype and SplitGemm.takes(src, self.gate_w):
+            ctx.kernels.split.blocks(src, self.gate_w, gates, ctx.err_flag)    # every block's product in one launch
+        elif src.dtype == torch.float32 == self.gate_w.dtype and ctx.kernels.gemm_nt_blocks_take(src, self.gate_w):
+            ctx.kernels.gemm_nt_blocks(src, self.gate_w, gates)
         else:
             for b, lin in enumerate(self.gates):
                 lin.forward(src[:, b * bs:(b + 1) * bs], ctx, out_dtype=torch.float32, out=gates[b])

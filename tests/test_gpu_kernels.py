@@ -8,6 +8,7 @@ import torch
 
 import plain_llama as plain
 from helpers import rel_err
+from scriptling_llm_lib_b200.csrc.bindings import SplitGemm
 
 pytestmark = pytest.mark.gpu
 
@@ -439,6 +440,54 @@ def test_gemm_nt_blocks_is_every_block_by_itself(kernel_sets, blocks, M, N, K):
     assert torch.equal(out, each)
     want = torch.einsum("mbk,bnk->bmn", f64(a).view(M, blocks, K), f64(w))
     assert rel_err(out.cpu(), want) < TOL[torch.float32] * max(1.0, (K / 64) ** 0.5)
+
+
+@pytest.mark.parametrize("M, N, K", [(17, 1, 128), (65, 7, 64), (128, 256, 72), (129, 129, 1000), (256, 128, 264), (257, 300, 4096), (700, 520, 136)])
+def test_gemm_split_is_at_least_as_exact_as_the_chain(kernel_sets, M, N, K):
+    """Products in three bfloat16 parts on the tensor cores: ragged tiles and k-blocks, K in parts (more than there are k-blocks among
+    them), planes in portions. Sums end after 64 terms, so the error grows with sqrt(K / 64) from 2^-23, the terms left out and the
+    last places cut within one sum; and it is no larger than that of the chains of multiply-adds."""
+    ks = kernel_sets[torch.float32]
+    wide, w = dev(rand(M, K + 8, seed=3)), dev(rand(N, K, seed=4))
+    a, flag = wide[:, 4:4 + K], torch.zeros(1, dtype=torch.int32, device="cuda")
+    want, tol = f64(a) @ f64(w).T, 2.0 ** -23 * (1 + 0.25 * math.sqrt(K / 64))
+    off = lambda got: ((got.cpu().double() - want).norm() / want.norm()).item()                  # noqa: E731
+    assert SplitGemm.takes(a, w) and not SplitGemm.takes(wide[:, 1:1 + K], w) and not SplitGemm.takes(a[:16], w)
+    out, chain = (torch.full((M, N), float("nan"), device="cuda") for _ in range(2))
+    ks.split.gemm(a, w, out, flag)
+    ks.gemm_nt(a, w, chain)
+    assert off(out) < min(tol, 1.05 * off(chain))
+    for split in (2, 5):
+        parts = torch.full((split, M, N), float("nan"), device="cuda")
+        ks.split.gemm(a, w, parts, flag)
+        assert off(parts.sum(0)) < 2 * tol
+    class Portions(SplitGemm):
+        SCRATCH_BYTES = 6 * K * 513                                      # 256 rows and columns at a time, or all of one of them
+    again = torch.full((M, N), float("nan"), device="cuda")
+    Portions().gemm(a, w, again, flag)
+    assert torch.equal(again, out) and int(flag) == 0
+
+
+def test_gemm_split_blocks_and_what_is_not_finite(kernel_sets):
+    """A block-diagonal product in one launch; infinities, NaN and values whose first part rounds up to an infinity come out as the
+    chain of multiply-adds has them."""
+    ks, flag = kernel_sets[torch.float32], torch.zeros(1, dtype=torch.int32, device="cuda")
+    blocks, M, N, K = 5, 300, 72, 72
+    a, w = dev(rand(M, blocks * K, seed=3)), dev(rand(blocks, N, K, seed=4))
+    for row, col, v in ((5, 3, math.inf), (7, 2, math.nan), (9, 1, 3.4e38), (11, 2 * K + 5, -math.inf)):
+        a[row, col] = v
+    w[1, 4, 6], w[3, 70, 71], a[12, K + 6] = -math.inf, 3.395e38, 0.0
+    a[:, 4 * K - 1] = a[:, 4 * K - 1].clamp(-0.5, 0.5)                   # 3.395e38 times it stays finite
+    out, chain = (torch.full((blocks, M, N), 7.0, device="cuda") for _ in range(2))
+    ks.split.blocks(a, w, out, flag)
+    ks.gemm_nt_blocks(a, w, chain)
+    bad = ~chain.isfinite()
+    assert bad.sum() > 4 * N and torch.equal(bad, ~out.isfinite()) and int(flag) == 0
+    assert torch.equal(chain[bad].nan_to_num(1.5, 2.5, 3.5), out[bad].nan_to_num(1.5, 2.5, 3.5))
+    large = chain.abs() > 1e30
+    assert ((out - chain)[large & ~bad] / chain[large & ~bad]).abs().max() < 1e-6
+    rest = ~(bad | large)
+    assert rel_err(out[rest].cpu(), f64(chain[rest])) < 4e-7
 
 
 # --------------------------------------------------------------------------- rotary + cache write
