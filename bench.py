@@ -927,9 +927,7 @@ def mix_kernels_alone(args):
             report(f"moe_pairs {pairs} pairs, experts {W} x {F} ({label})", T, us, nbytes=pairs * 2 * F * W * esz)
         elif dt == torch.bfloat16:
             rows = -(-(pairs + E * 127) // 128) * 128
-            counts = torch.zeros(E, dtype=torch.int32, device=dev)
             offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
-            por = torch.empty(rows, dtype=torch.int32, device=dev)
             rop = torch.empty(pairs, dtype=torch.int32, device=dev)
             tg = torch.empty(rows // 128, dtype=torch.int32, device=dev)
             xs2 = torch.empty(rows, W, dtype=dt, device=dev)
@@ -938,8 +936,8 @@ def mix_kernels_alone(args):
             out = torch.empty(T, W, device=dev)
             err = torch.zeros(1, dtype=torch.int32, device=dev)
             tc = ks.tensor_core
-            us = timed(lambda i: (k.moe_group_rows(idx, counts, offsets, por, rop, tg, pad=128), k.moe_gather_rows(h, por, top, xs2)), 1)
-            report(f"moe_group_rows + moe_gather_rows ({label})", T, us, nbytes=rows * W * esz * 2)
+            us = timed(lambda i: (k.moe_group_rows(idx, E, offsets, None, rop, tg, pad=128), k.moe_gather_rows(h, rop, top, xs2)), 1)
+            report(f"moe_group_rows + moe_gather_rows ({label})", T, us, nbytes=(T + pairs) * W * esz)
             us = timed(lambda i: tc.gemm_grouped(xs2, w_up, hid, tg, err, act="relu_squared", rows_used=offsets[E:]), 1)
             report(f"gemm_grouped up, {rows} rows for {pairs} pairs ({label})", T, us, flops=2 * pairs * F * W, tensor=True)
             us = timed(lambda i: tc.gemm_grouped(hid, w_down, ys2, tg, err, rows_used=offsets[E:]), 1)
@@ -1086,9 +1084,7 @@ def gate_kernels_alone(args):
             report(f"moe_pairs relu^2 ({label})", T, us, nbytes=pairs * 2 * F * W * esz, like="moe_pairs clamped gate")
         else:
             rows = -(-(pairs + E * 127) // 128) * 128
-            counts = torch.zeros(E, dtype=torch.int32, device=dev)
             offsets = torch.empty(E + 1, dtype=torch.int32, device=dev)
-            por = torch.empty(rows, dtype=torch.int32, device=dev)
             rop = torch.empty(pairs, dtype=torch.int32, device=dev)
             tg = torch.empty(rows // 128, dtype=torch.int32, device=dev)
             xs2 = torch.empty(rows, W, dtype=dt, device=dev)
@@ -1097,8 +1093,8 @@ def gate_kernels_alone(args):
             ys2 = torch.empty(rows, W, device=dev)
             out = torch.empty(T, W, device=dev)
             tc = ks.tensor_core
-            ks.mix.moe_group_rows(idx, counts, offsets, por, rop, tg, pad=128)
-            ks.mix.moe_gather_rows(h, por, top, xs2)
+            ks.mix.moe_group_rows(idx, E, offsets, None, rop, tg, pad=128)
+            ks.mix.moe_gather_rows(h, rop, top, xs2)
             us = timed(lambda i: tc.gemm_grouped(xs2, w_gu, hid, tg, err, rows_used=offsets[E:], glu=(7.0, 1.702)), 1)
             report(f"gemm_grouped gate|up with the clamped gate, {rows} rows for {pairs} pairs ({label})", T, us, flops=4 * pairs * F * W)
             us = timed(lambda i: (tc.gemm_grouped(xs2, w_gu, raw, tg, err, rows_used=offsets[E:]),

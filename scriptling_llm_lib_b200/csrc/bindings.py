@@ -477,9 +477,9 @@ class TensorCoreGemm:
 
     ACTS = {None: 0, "gelu_tanh": 1, "relu_squared": 2, "silu": 3}
 
-    def gemm_grouped(self, a, w, out, tile_group, err_flag, act=None, rows_used=None, glu=None):
-        """out[M, N] = act(a[M, K] @ w[g]^T) with w [G, N, K] and the 128 rows of `a` from row 128 t on multiplied by
-        matrix tile_group[t] (int32 on the device, M / 128 entries): rows laid out so that no 128 hold two groups.
+    def gemm_grouped(self, a, w, out, tile_group, err_flag, act=None, rows_used=None, glu=None, tile_rows=128):
+        """out[M, N] = act(a[M, K] @ w[g]^T) with w [G, N, K] and the `tile_rows` (128, or 256 for N > 128) rows of `a` from
+        row tile_rows * t on multiplied by matrix tile_group[t] (int32 on the device): rows laid out so that no tile holds two groups.
         rows_used: an int32 on the device (one element), how many of the M rows hold anything; the rest is not worked.
         `glu` = (limit, alpha): every matrix's N rows are tiles of 8 gate rows and their 8 up rows, and out [M, N / 2]
         (bfloat16) receives the clamped gate of each pair of sums, g' * sigmoid(alpha g') * (u' + 1); a limit of 0 stands
@@ -490,13 +490,13 @@ class TensorCoreGemm:
             raise KernelError(f"gemm_grouped with a gate: {N} stacked rows a matrix, out {out.dtype}, act {act}, limit {glu[0]}")
         if (w.dim() != 3 or w.shape[2] != K or tuple(out.shape) != (M, N // 2 if glu is not None else N)
                 or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16
-                or out.dtype not in (torch.bfloat16, torch.float32) or tile_group.shape[0] * 128 < M):
+                or out.dtype not in (torch.bfloat16, torch.float32) or tile_group.shape[0] * tile_rows < M):
             raise KernelError(f"gemm_grouped shapes: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}")
         fn = self.lib.sllm_gemm_tc_grouped_bf16
         fn.restype = c_int
         _check(fn(_ptr(a, torch.bfloat16, "a"), _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), c_int(M), c_int(N), c_int(K),
                   c_int(K), c_int(K), c_int(out.shape[1]), c_int(1 if out.dtype == torch.float32 else 0),
-                  _ptr(tile_group, torch.int32, "tile_group"), c_int(G), c_int(self.ACTS[act]), _ptr(rows_used, torch.int32, "rows_used"),
+                  _ptr(tile_group, torch.int32, "tile_group"), c_int(tile_rows), c_int(G), c_int(self.ACTS[act]), _ptr(rows_used, torch.int32, "rows_used"),
                   c_int(0 if glu is None else 1), c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]),
                   _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_grouped")
 
@@ -1348,18 +1348,18 @@ class MixKernels:
                                      c_int(out.shape[1]), c_float(limit), c_float(alpha), _ptr(rows_used, torch.int32, "rows_used"),
                                      c_int(1 if tiled else 0), _stream()), "glu_clamp")
 
-    def moe_group_rows(self, idx, counts, offsets, pair_of_row, row_of_pair=None, tile_group=None, pad=1):
-        """Groups the (token, expert) pairs of idx [T, top] by expert. counts int32 [E] must be zero and is left
-        zero; offsets int32 [E + 1] the experts' first rows; pair_of_row int32 [rows] (-1: no pair); row_of_pair
-        int32 [T * top] the inverse. pad > 1: every expert's rows start at a multiple of pad, and
-        tile_group int32 [rows / pad] names the expert of every pad rows."""
+    def moe_group_rows(self, idx, n_experts, offsets, pair_of_row=None, row_of_pair=None, tile_group=None, pad=1):
+        """Groups the (token, expert) pairs of idx [T, top] by expert. offsets int32 [E + 1]: the experts' first rows; pair_of_row
+        int32 [rows] (rows that pad are not written) and row_of_pair int32 [T * top], the inverse, where given. pad > 1:
+        every expert's rows start at a multiple of pad, and tile_group int32 [rows / pad] names the expert of every pad rows."""
         T, top = idx.shape
-        _check(self._fn("moe_group_rows")(_ptr(idx, torch.int32, "idx"), _ptr(counts, torch.int32, "counts"),
-                                          _ptr(offsets, torch.int32, "offsets"), _ptr(pair_of_row, torch.int32, "pair_of_row"),
-                                          _ptr(row_of_pair, torch.int32, "row_of_pair"), _ptr(tile_group, torch.int32, "tile_group"),
-                                          c_int(T), c_int(top), c_int(counts.shape[0]), c_int(pad), c_int(pair_of_row.shape[0]),
-                                          _stream()), "moe_group_rows")
-        LAUNCHES[0] += 4
+        rows = T * top if pad == 1 else tile_group.shape[0] * pad
+        if offsets.numel() != n_experts + 1 or (pair_of_row is not None and pair_of_row.numel() < rows):
+            raise KernelError(f"moe_group_rows: offsets {tuple(offsets.shape)} for {n_experts} experts, {rows} rows")
+        _check(self._fn("moe_group_rows")(_ptr(idx, torch.int32, "idx"), _ptr(offsets, torch.int32, "offsets"),
+                                          _ptr(pair_of_row, torch.int32, "pair_of_row"), _ptr(row_of_pair, torch.int32, "row_of_pair"),
+                                          _ptr(tile_group, torch.int32, "tile_group"), c_int(T), c_int(top), c_int(n_experts), c_int(pad),
+                                          c_int(rows), _stream()), "moe_group_rows")
 
     def moe_grouped(self, h, wup, wdown, wgt, offsets, pair_of_row, hid, out, glu=None, raw=None, tiled=False):
         """The experts' products over rows grouped without padding (`moe_group_rows` with pad 1), float32 sums on
@@ -1377,10 +1377,12 @@ class MixKernels:
                "moe_grouped")
         LAUNCHES[0] += 1
 
-    def moe_gather_rows(self, h, pair_of_row, top, xs):
-        """xs[row] = h[pair_of_row[row] // top], zeros where a row holds no pair."""
-        _check(self._fn("moe_gather_rows")(self._view(h, "h"), c_int(h.stride(0)), _ptr(pair_of_row, torch.int32, "pair_of_row"),
-                                           c_int(top), _ptr(xs, self.dtype, "xs"), c_int(xs.shape[0]), c_int(xs.shape[1]), _stream()),
+    def moe_gather_rows(self, h, row_of_pair, top, xs):
+        """xs[row_of_pair[t * top + k]] = h[t]; other rows of xs stay."""
+        if row_of_pair.numel() != h.shape[0] * top:
+            raise KernelError(f"moe_gather_rows: {row_of_pair.numel()} pairs of {h.shape[0]} rows, {top} each")
+        _check(self._fn("moe_gather_rows")(self._view(h, "h"), c_int(h.stride(0)), _ptr(row_of_pair, torch.int32, "row_of_pair"),
+                                           c_int(top), _ptr(xs, self.dtype, "xs"), c_int(h.shape[0]), c_int(xs.shape[1]), _stream()),
                "moe_gather_rows")
 
     def moe_combine(self, ys, row_of_pair, wgt, out):

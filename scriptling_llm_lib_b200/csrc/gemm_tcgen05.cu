@@ -45,8 +45,8 @@ struct TcFold {
   const float* norm_w;
   bf16* xb;
   float* sumsq_out;
-  // grouped rows (the one-SM kernel only): B holds `group_rows`-row matrices one under the other, and the 128 rows
-  // of A from row 128 t on are multiplied by matrix tile_group[t]. Null: one matrix for all rows.
+  // grouped rows: B holds `group_rows`-row matrices one under the other, and the rows of A of row tile t (128 rows in
+  // the one-SM kernel, 256 in the two-SM kernel) are multiplied by matrix tile_group[t]. Null: one matrix for all rows.
   const int* tile_group;
   int group_rows;
   const int* m_used;      // (or null) on the device: the rows of A that hold anything; tiles behind them are not worked
@@ -100,6 +100,16 @@ __device__ __forceinline__ float bf16_round(uint32_t f32_bits) {
   return __bfloat162float(__float2bfloat16_rn(__uint_as_float(f32_bits)));
 }
 
+// 32 bytes of one row in one store: a lane's row lies in lines of its own, so a store of 16 bytes would fill half a sector
+__device__ __forceinline__ void tc_store_sector(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f, uint32_t g, uint32_t h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
+}
+__device__ __forceinline__ uint32_t tc_pack(uint32_t lo, uint32_t hi) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(lo), __uint_as_float(hi));
+  return *(const uint32_t*)&p;
+}
+
 // 32 consecutive columns of one row, already final: to C (a query head), or to the row's place in
 // the key or value pages.
 __device__ __forceinline__ void qkv_store32(const TcRope& rp, void* C, int ldc, int row, int col, size_t cache_row,
@@ -109,13 +119,15 @@ __device__ __forceinline__ void qkv_store32(const TcRope& rp, void* C, int ldc, 
   if (hidx < rp.H) dst = (bf16*)C + (size_t)row * ldc + col;
   else if (hidx < rp.H + rp.G) dst = rp.kpages + (cache_row + (size_t)(hidx - rp.H) * SLLM_PAGE) * rp.hd + d0;
   else dst = rp.vpages + (cache_row + (size_t)(hidx - rp.H - rp.G) * SLLM_PAGE) * rp.hd + d0;
+  uint32_t o[16];
 #pragma unroll
-  for (int j = 0; j < 32; j += 8) {
-    uint4 o;
-    __nv_bfloat162 p0 = __floats2bfloat162_rn(v[j], v[j + 1]), p1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-    __nv_bfloat162 p2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]), p3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-    o.x = *(uint32_t*)&p0; o.y = *(uint32_t*)&p1; o.z = *(uint32_t*)&p2; o.w = *(uint32_t*)&p3;
-    *(uint4*)(dst + j) = o;
+  for (int j = 0; j < 16; j++) o[j] = tc_pack(__float_as_uint(v[2 * j]), __float_as_uint(v[2 * j + 1]));
+  if (((uintptr_t)dst & 31) == 0) {
+    tc_store_sector(dst, o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]);
+    tc_store_sector(dst + 16, o[8], o[9], o[10], o[11], o[12], o[13], o[14], o[15]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) *(uint4*)(dst + 2 * j) = make_uint4(o[j], o[j + 1], o[j + 2], o[j + 3]);
   }
 }
 
@@ -128,7 +140,10 @@ __device__ __forceinline__ void tc_store_row(void* C, int row, int col, int N, i
   if (EPI == TC_EPI_STORE) {
     if (out_f32) {
       float* dst = (float*)C + (size_t)row * ldc + col;
-      if (col + 32 <= N && ((uintptr_t)dst & 15) == 0) {
+      if (col + 32 <= N && ((uintptr_t)dst & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) tc_store_sector(dst + j, r[j], r[j + 1], r[j + 2], r[j + 3], r[j + 4], r[j + 5], r[j + 6], r[j + 7]);
+      } else if (col + 32 <= N && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           *(float4*)(dst + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
@@ -138,7 +153,12 @@ __device__ __forceinline__ void tc_store_row(void* C, int row, int col, int N, i
       }
     } else {
       bf16* dst = (bf16*)C + (size_t)row * ldc + col;
-      if (col + 32 <= N && ((uintptr_t)dst & 15) == 0) {
+      if (col + 32 <= N && ((uintptr_t)dst & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 16)
+          tc_store_sector(dst + j, tc_pack(r[j], r[j + 1]), tc_pack(r[j + 2], r[j + 3]), tc_pack(r[j + 4], r[j + 5]), tc_pack(r[j + 6], r[j + 7]),
+                          tc_pack(r[j + 8], r[j + 9]), tc_pack(r[j + 10], r[j + 11]), tc_pack(r[j + 12], r[j + 13]), tc_pack(r[j + 14], r[j + 15]));
+      } else if (col + 32 <= N && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
         for (int j = 0; j < 32; j += 8) {
           uint4 v;
@@ -172,13 +192,14 @@ __device__ __forceinline__ void tc_store_row(void* C, int row, int col, int N, i
         }
       }
     if (ocol + 16 <= n_out && ((uintptr_t)dst & 15) == 0) {
+      uint32_t v[8];
 #pragma unroll
-      for (int j = 0; j < 16; j += 8) {
-        uint4 v;
-        __nv_bfloat162 p0 = __floats2bfloat162_rn(h[j], h[j + 1]), p1 = __floats2bfloat162_rn(h[j + 2], h[j + 3]);
-        __nv_bfloat162 p2 = __floats2bfloat162_rn(h[j + 4], h[j + 5]), p3 = __floats2bfloat162_rn(h[j + 6], h[j + 7]);
-        v.x = *(uint32_t*)&p0; v.y = *(uint32_t*)&p1; v.z = *(uint32_t*)&p2; v.w = *(uint32_t*)&p3;
-        *(uint4*)(dst + j) = v;
+      for (int j = 0; j < 8; j++) v[j] = tc_pack(__float_as_uint(h[2 * j]), __float_as_uint(h[2 * j + 1]));
+      if (((uintptr_t)dst & 31) == 0) {
+        tc_store_sector(dst, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+      } else {
+        *(uint4*)dst = make_uint4(v[0], v[1], v[2], v[3]);
+        *(uint4*)(dst + 8) = make_uint4(v[4], v[5], v[6], v[7]);
       }
     } else {
 #pragma unroll
@@ -541,6 +562,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  if (fd.m_used) M = min(M, *fd.m_used);     // the same number for every thread of every block: all walk the same tiles
   const int tiles_m = (M + TC2_BM - 1) / TC2_BM, tiles_n = (N + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
   const int nkb = (K + TC_BK - 1) / TC_BK;
   // A read of tensor memory waits behind the products already queued, some thousands of clocks
@@ -575,7 +597,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         int tm, tn;
         tc2_tile_origin(tile, tiles_m, tiles_n, tm, tn);
-        const int m0 = tm * TC2_BM + (int)rank * 128, n0 = tn * BN + (int)rank * 128;
+        const int m0 = tm * TC2_BM + (int)rank * 128;
+        const int b_row = tn * BN + (int)rank * 128 + (fd.tile_group ? fd.tile_group[tm] * fd.group_rows : 0);     // the row tile's own matrix
         for (int kb = 0; kb < nkb; kb++, it++) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
@@ -585,7 +608,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           uint32_t full_lead = mapa_shared(full0 + 8 * s, 0);
           uint32_t a_dst = smem_base + s * STAGE_BYTES;
           tma_load_2d_pair(a_dst, &map_a, kb * TC_BK, m0, full_lead);
-          tma_load_2d_pair(a_dst + A_BYTES, &map_b, kb * TC_BK, n0, full_lead);
+          tma_load_2d_pair(a_dst + A_BYTES, &map_b, kb * TC_BK, b_row, full_lead);
         }
       }
       if (*abort) {
@@ -732,40 +755,43 @@ SLLM_EXPORT int sllm_gemm_tc_fold_bf16(const void* A, const void* B, void* C, in
              : tc_launch<128, 6, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd);
 }
 
-// Grouped rows: C[M,N] = A[M,K] B_g^T with B [n_groups * N, K] holding one [N, K] matrix per group and the 128 rows
-// of A from row 128 t on multiplied by matrix tile_group[t] (int32 on the device, ceil(M / 128) entries, each in
-// 0 .. n_groups - 1). The caller lays the rows of A out so that no tile holds rows of two groups. The one-SM kernel
-// (tiles of 128 rows); a tile's columns beyond N read the next group's rows and are not written. m_used (or null): an
+// Grouped rows: C[M,N] = A[M,K] B_g^T with B [n_groups * N, K] holding one [N, K] matrix per group and the tile_rows (128:
+// the one-SM kernel; 256: the two-SM kernel, N > 128) rows of A from row tile_rows t on multiplied by matrix tile_group[t]
+// (int32 on the device, ceil(M / tile_rows) entries, each in 0 .. n_groups - 1). The caller lays the rows of A out so that no
+// tile holds rows of two groups. A tile's columns beyond N read the next group's rows and are not written. m_used (or null): an
 // int on the device, the rows of A in use; the tiles behind them are left alone (their number is known on the device only).
 // gated (act 0, bfloat16 out, N a multiple of 16): every matrix's rows come in tiles of 16 (8 gate rows, 8 up
 // rows) and C[M, N/2] receives the gate of each pair: the clamped one with glu_limit > 0 (see TcFold), else silu(g) * u.
 SLLM_EXPORT int sllm_gemm_tc_grouped_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                                          int out_f32, const int* tile_group, int n_groups, int act, const int* m_used,
+                                          int out_f32, const int* tile_group, int tile_rows, int n_groups, int act, const int* m_used,
                                           int gated, float glu_limit, float glu_alpha, int* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || (K & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || !tile_group || n_groups < 1)
     return SLLM_ERR_ARG;
   if ((long long)n_groups * N > 0x7fffffffLL) return SLLM_ERR_ARG;
+  if (tile_rows != 128 && (tile_rows != 256 || N <= 128)) return SLLM_ERR_ARG;
   TcFold fd{};
   if (act < 0 || act > 3) return SLLM_ERR_ARG;
+  if (gated && (act || out_f32 || (N & 15))) return SLLM_ERR_ARG;
   fd.tile_group = tile_group;
   fd.group_rows = N;
   fd.act = act;
   fd.m_used = m_used;
+  fd.glu_limit = gated && glu_limit > 0.f ? glu_limit : 0.f;
+  fd.glu_alpha = gated ? glu_alpha : 0.f;
   const TcRope rp{};
   CUtensorMap ma, mb;
   int big = N > 128;
   int rc = tc_make_map(&ma, A, M, K, lda, TC_BM);
   if (rc) return rc;
-  rc = tc_make_map(&mb, B, n_groups * N, K, ldb, big ? 256 : 128);
+  rc = tc_make_map(&mb, B, n_groups * N, K, ldb, big && tile_rows == 128 ? 256 : 128);
   if (rc) return rc;
-  if (gated) {
-    if (act || out_f32 || (N & 15)) return SLLM_ERR_ARG;
-    fd.glu_limit = glu_limit > 0.f ? glu_limit : 0.f;
-    fd.glu_alpha = glu_alpha;
+  if (tile_rows == 256)
+    return gated ? tc_pair_launch<6, TC_EPI_SWIGLU>(ma, mb, C, M, N, K, ldc, 0, err, stream, rp, fd)
+                 : tc_pair_launch<6, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd);
+  if (gated)
     return big ? tc_launch<256, 4, TC_EPI_SWIGLU>(ma, mb, C, M, N, K, ldc, 0, err, stream, rp, fd)
                : tc_launch<128, 6, TC_EPI_SWIGLU>(ma, mb, C, M, N, K, ldc, 0, err, stream, rp, fd);
-  }
   return big ? tc_launch<256, 4, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd)
              : tc_launch<128, 6, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd);
 }

@@ -41,6 +41,7 @@ from __future__ import annotations
 
 import torch
 
+from ..csrc.bindings import TensorCoreGemm
 from ..weights.spec import TensorSpec
 from .base import FEED_FORWARDS, FeedForward
 from .linear import Linear
@@ -159,7 +160,6 @@ class RoutedExperts(FeedForward):
         else:
             self.w_up = torch.stack([tensors[n] for n in self.up_names]).contiguous()    # [E, F, hidden]
         self.w_down = torch.stack([tensors[n] for n in self.down_names]).contiguous()    # [E, hidden, F]
-        self.counts = torch.zeros((self.E,), dtype=torch.int32, device=device)
         if self.w_up.dtype != dtype:
             raise ValueError(f"the experts' matrices are {self.w_up.dtype}, the engine runs in {dtype}")
 
@@ -167,6 +167,14 @@ class RoutedExperts(FeedForward):
         """The grouped products can run on the tensor-core kernel: bfloat16, and the contraction widths (hidden for the
         experts' first product, their own width for the second) multiples of 8 elements (16 bytes for its copies)."""
         return x.dtype == torch.bfloat16 and self.hidden % 8 == 0 and self.F % 8 == 0 and x.data_ptr() % 16 == 0
+
+    def _tile_rows(self, pairs: int) -> int:
+        """Rows of a tile of the grouped products: 256 on two SMs where the experts have more than 112 rows on average, so that most
+        fill more than one tile of 128, which one SM works at three quarters of the rate; with fewer most of a wide tile would be
+        padding. Both products, 128 / 256, us: 64 experts of 1,408 x 2,048, 192 rows each 359 / 247, 94 353 / 379 (of the whole
+        sublayer), 47 337 / 373; 32 of 704 x 1,024, 256 rows 167 / 159, 125 164 / 160. (The two-SM tile is wider than 128 columns.)"""
+        wide = pairs > 112 * self.E and self.hidden > 128 and (self.F if self.glu is None else 2 * self.F) > 128
+        return 256 if wide and not TensorCoreGemm.ONE_SM_FORCED else 128
 
     def forward(self, x, ctx):
         routed = self._routed(x, ctx)
@@ -190,29 +198,28 @@ class RoutedExperts(FeedForward):
         offsets = torch.empty((self.E + 1,), dtype=torch.int32, device=dev)
         if not self._on_tensor_cores(x):
             pair_of_row = torch.empty((pairs,), dtype=torch.int32, device=dev)
-            k.moe_group_rows(idx, self.counts, offsets, pair_of_row)
+            k.moe_group_rows(idx, self.E, offsets, pair_of_row)
             hid = torch.empty((pairs, self.F), dtype=x.dtype, device=dev)
             out = torch.empty((self.top, T, self.hidden), dtype=torch.float32, device=dev)
             raw = torch.empty((pairs, 2 * self.F), dtype=x.dtype, device=dev) if self.glu is not None else None
             k.moe_grouped(x, self.w_up, self.w_down, wgt, offsets, pair_of_row, hid, out, glu=self.glu, raw=raw, tiled=self.tiled)
             return out
-        # every expert's rows from a multiple of 128 on, so that a tile of the tensor-core product has one expert
-        tile = 128
+        # every expert's rows from a multiple of a tile on, so that a tile of the tensor-core product has one expert
+        tile = self._tile_rows(pairs)
         rows = -(-(pairs + self.E * (tile - 1)) // tile) * tile
-        pair_of_row = torch.empty((rows,), dtype=torch.int32, device=dev)
         row_of_pair = torch.empty((pairs,), dtype=torch.int32, device=dev)
         tile_group = torch.empty((rows // tile,), dtype=torch.int32, device=dev)
-        k.moe_group_rows(idx, self.counts, offsets, pair_of_row, row_of_pair, tile_group, pad=tile)
+        k.moe_group_rows(idx, self.E, offsets, None, row_of_pair, tile_group, pad=tile)
         xs = torch.empty((rows, self.hidden), dtype=x.dtype, device=dev)
-        k.moe_gather_rows(x, pair_of_row, self.top, xs)
+        k.moe_gather_rows(x, row_of_pair, self.top, xs)
         tc = ctx.kernels.tensor_core
         hid = torch.empty((rows, self.F), dtype=x.dtype, device=dev)
         if self.glu is not None:      # `tiled` holds here: its conditions are those of the tensor-core path
-            tc.gemm_grouped(xs, self.w_up, hid, tile_group, ctx.err_flag, rows_used=offsets[self.E:], glu=self.glu)
+            tc.gemm_grouped(xs, self.w_up, hid, tile_group, ctx.err_flag, rows_used=offsets[self.E:], glu=self.glu, tile_rows=tile)
         else:
-            tc.gemm_grouped(xs, self.w_up, hid, tile_group, ctx.err_flag, act="relu_squared", rows_used=offsets[self.E:])
+            tc.gemm_grouped(xs, self.w_up, hid, tile_group, ctx.err_flag, act="relu_squared", rows_used=offsets[self.E:], tile_rows=tile)
         ys = torch.empty((rows, self.hidden), dtype=torch.float32, device=dev)
-        tc.gemm_grouped(hid, self.w_down, ys, tile_group, ctx.err_flag, rows_used=offsets[self.E:])
+        tc.gemm_grouped(hid, self.w_down, ys, tile_group, ctx.err_flag, rows_used=offsets[self.E:], tile_rows=tile)
         out = torch.empty((T, self.hidden), dtype=torch.float32, device=dev)
         k.moe_combine(ys, row_of_pair, wgt, out)
         return out

@@ -46,6 +46,9 @@ class RMSNorm(Norm):
     def forward(self, residual, delta, ctx, rows=None):
         if isinstance(delta, Folded):          # the product before this norm has done its work already
             return delta
+        if isinstance(delta, (list, tuple)) and len(delta) == 1 and rows is None and delta[0].shape == residual.shape:
+            # one addend after all: it passes with the norm, float32 as a sum of one part
+            delta = delta[0].unsqueeze(0) if delta[0].dtype == torch.float32 else delta[0]
         n = residual.shape[0] if rows is None else rows.shape[0]
         y = torch.empty((n, self.width), dtype=ctx.dtype, device=residual.device)
         if isinstance(delta, RmsNormedAddend):  # the addend's own norm, the sum and this norm in one pass

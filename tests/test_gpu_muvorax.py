@@ -13,6 +13,7 @@ import pytest
 import torch
 
 import plain_muvorax as plain
+from scriptling_llm_lib_b200.csrc.bindings import KernelSet
 
 pytestmark = pytest.mark.gpu
 
@@ -788,6 +789,42 @@ def test_the_norm_adds_a_normed_addend_and_keeps_the_sum():
         want2 = torch.tanh(1.3 * (x.double() + one.double())[[7, 2]]) * w.double() + b.double()
         assert torch.equal(x2.cpu(), x)                  # picked rows: the stream is left as it was
         assert float((out2.cpu().double() - want2).abs().max()) < (1e-5 if dtype == torch.float32 else 3e-2)
+
+
+@pytest.mark.parametrize("T, top, E, pad", [(1, 1, 1, 1), (5, 3, 7, 256), (2048, 6, 64, 256), (700, 4, 1500, 1), (333, 8, 1025, 128), (900, 2, 8192, 1)])
+def test_moe_grouping_gives_every_pair_its_row(T, top, E, pad):
+    """Offsets, tiles and rows of the grouped pairs, a share of the pairs a block of the cluster: few pairs, more experts than threads,
+    experts without a pair; then the rows that gathering by them leaves, and their products on either tile."""
+    k = KernelSet(torch.bfloat16)
+    g = torch.Generator().manual_seed(T)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] if E < 2000 else torch.randint(0, E, (top,), generator=g) for _ in range(T)]).int()
+    idx[:, 0] = torch.where(torch.rand(T, generator=g) < 0.3, idx[0, 0], idx[:, 0])
+    pairs, counts = T * top, torch.bincount(idx.flatten().long(), minlength=E)
+    rows = pairs if pad == 1 else -(-(pairs + E * (pad - 1)) // pad) * pad
+    offsets, rop = torch.full((E + 1,), -7, dtype=torch.int32, device="cuda"), torch.full((pairs,), -7, dtype=torch.int32, device="cuda")
+    por, tiles = torch.full((rows,), -7, dtype=torch.int32, device="cuda"), torch.full((max(1, rows // pad),), -7, dtype=torch.int32, device="cuda")
+    k.mix.moe_group_rows(idx.cuda(), E, offsets, por, rop, tiles if pad > 1 else None, pad=pad)
+    want = torch.cat([torch.zeros(1, dtype=torch.long), ((counts + pad - 1) // pad * pad).cumsum(0)])
+    assert torch.equal(offsets.cpu().long(), want)
+    row, experts = rop.cpu().long(), idx.flatten().long()
+    assert torch.equal(por.cpu().long()[row], torch.arange(pairs)) and row.unique().numel() == pairs
+    assert bool(((row >= want[experts]) & (row < want[experts] + counts[experts])).all())
+    if pad > 1:
+        first = torch.arange(rows // pad) * pad
+        assert torch.equal(tiles.cpu().long(), (torch.searchsorted(want[1:], first, right=True)).clamp(max=E - 1))
+    if pad == 1 or E > 100:
+        return
+    K, N, tc, flag = 72, 264, k.tensor_core, torch.zeros(1, dtype=torch.int32, device="cuda")
+    h, w = torch.randn(T, K, generator=g).bfloat16().cuda(), (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().cuda()
+    xs = torch.full((rows, K), float("nan"), dtype=torch.bfloat16, device="cuda")
+    k.mix.moe_gather_rows(h, rop, top, xs)
+    assert torch.equal(xs[rop.long()], h.repeat_interleave(top, 0))
+    out = torch.full((rows, N), 7.0, device="cuda")
+    tc.gemm_grouped(xs, w, out, tiles, flag, rows_used=offsets[E:], tile_rows=pad)
+    exact = torch.einsum("pk,pnk->pn", xs[rop.long()].double(), w.double()[experts.cuda()])
+    got = out[rop.long()].double()
+    assert ((got - exact).norm() / exact.norm()).item() < 2e-6 and int(flag) == 0       # products of bfloat16, float sums of 72 terms
+    assert bool((out[int(want[-1]):] == 7.0).all())                                     # tiles behind the rows in use are left alone
 
 
 def test_experts_one_by_one_and_grouped_agree(folders):

@@ -151,3 +151,13 @@ def test_the_reserve_counts_what_a_recurrence_takes_beside_its_rows():
     need = 4 * 2048 * (rows + (rows // 64 + 50) * 17)
     assert Engine.activation_reserve_bytes(eng([MIXERS.build(scan)])) >= plain + need
     assert MixKernels.scan_scratch_bytes(rows, 50, 2048, 16, 148) == need
+
+
+@pytest.mark.parametrize("pairs, E, F, hidden, want", [(12288, 64, 1408, 2048, 256), (7168, 64, 1408, 2048, 128), (7169, 64, 1408, 2048, 256), (9000, 8, 64, 2048, 128),
+                                                       (9000, 8, 65, 2048, 256), (9000, 8, 1408, 128, 128)])
+def test_rows_of_a_tile_of_the_grouped_products(pairs, E, F, hidden, want):
+    """256 rows on two SMs from more than 112 rows an expert on, where both products have more than 128 columns (gated: 2 F and hidden)."""
+    from scriptling_llm_lib_b200.parts.experts import RoutedExperts
+    part = RoutedExperts(hidden, F, E, 1, 1, 1, 1.0, "r", "c", [f"u{j}" for j in range(E)], [f"d{j}" for j in range(E)], act="silu_glu",
+                         gate_names=[f"g{j}" for j in range(E)])
+    assert part._tile_rows(pairs) == want
