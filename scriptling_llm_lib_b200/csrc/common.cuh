@@ -211,6 +211,10 @@ __device__ __forceinline__ void st8(bf16* p, const F8& r) {
   *(uint4*)p = v;
 }
 
+static inline bool sllm_pdl_off() {            // launch the ordinary, fully serialised way
+  static const bool off = getenv("SLLM_NO_PDL") != nullptr;
+  return off;
+}
 template <typename... KArgs, typename... Args>
 static inline cudaError_t sllm_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                       Args... args) {
@@ -219,11 +223,10 @@ static inline cudaError_t sllm_launch(void (*kernel)(KArgs...), dim3 grid, dim3 
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  static const bool off = getenv("SLLM_NO_PDL") != nullptr;   // launch the ordinary, fully serialised way
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = off ? 0 : 1;
+  cfg.numAttrs = sllm_pdl_off() ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }

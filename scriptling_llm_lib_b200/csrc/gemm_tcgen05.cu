@@ -710,10 +710,244 @@ static int tc_pair_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C,
 }
 
 // whether the two-SM kernel takes a product: more than one block's rows and wide enough for its tile
-static bool tc_use_pair(int M, int N) {
+static bool tc_one_sm_forced() {
   static int off = -1;
   if (off < 0) { const char* e = getenv("SLLM_GEMM_ONE_SM"); off = e && *e && *e != '0'; }
-  return !off && M > 128 && N > 128;
+  return off;
+}
+static bool tc_use_pair(int M, int N) { return !tc_one_sm_forced() && M > 128 && N > 128; }
+
+// ------------------------------------------------------------------ few tiles: a cluster along K
+// Products whose output is a handful of tiles (a router's 64 columns, step sizes and decays, low ranks, short prompts) leave most SMs
+// idle and walk all of K on the others, a serial chain of copies and products. Here a cluster of 2, 4 or 8 blocks takes one tile of 128 x
+// BN outputs (BN a multiple of 16 up to 256, as the host cuts N), each block its share of K; the accumulators meet in shared memory,
+// where every block adds up its share of the tile's rows, the blocks' sums in their order, and stores whole rows. Weights are fetched
+// before the kernel in front has finished. Bound by latency: a copy's way, the cluster's two barriers. 2,048 rows by 64 x 2,048 13.8 us
+// on 16 one-SM tiles, 6.6 here; by 160 x 4,096 24.2 on 8 two-SM tiles, 11.9 here.
+__device__ __forceinline__ float4 tc_cluster_float4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+  return v;
+}
+template <int SPLIT>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, void* __restrict__ C, int M,
+                       int N, int K, int ldc, int out_f32, int BN, int stages, int act, int* __restrict__ err) {
+  const uint32_t A_BYTES = TC_BM * TC_BK * 2, STAGE_BYTES = A_BYTES + BN * TC_BK * 2;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ uint64_t bars[2 * 8 + 1];                 // full[stages], empty[stages], acc_full
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  volatile int* abort = &abort_flag;
+  const uint32_t smem_base = smem_u32(smem), full0 = smem_u32(bars), empty0 = full0 + 8 * stages, acc_full = empty0 + 8 * stages;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int tile = blockIdx.x / SPLIT, tiles_m = (M + TC_BM - 1) / TC_BM;
+  const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;
+  const int nkb_all = (K + TC_BK - 1) / TC_BK, kb0 = (int)rank * nkb_all / SPLIT, nkb = ((int)rank + 1) * nkb_all / SPLIT - kb0;
+  uint32_t cols = 32;
+  while (cols < (uint32_t)BN) cols <<= 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
+    mbar_init(acc_full, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
+  const uint32_t tmem_base = tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int pre = min(nkb, stages);
+      for (int i = 0; i < pre; i++) {
+        mbar_expect_tx(full0 + 8 * i, STAGE_BYTES);
+        tma_load_2d(smem_base + i * STAGE_BYTES + A_BYTES, &map_b, (kb0 + i) * TC_BK, n0, full0 + 8 * i);
+      }
+      pdl_wait();
+      for (int i = 0; i < pre; i++) tma_load_2d(smem_base + i * STAGE_BYTES, &map_a, (kb0 + i) * TC_BK, m0, full0 + 8 * i);
+      int it = pre, s = 0;
+      for (uint32_t ph = 0; it < nkb; it++) {
+        if (!mbar_wait(empty0 + 8 * s, ph, abort)) break;
+        mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
+        tma_load_2d(smem_base + s * STAGE_BYTES, &map_a, (kb0 + it) * TC_BK, m0, full0 + 8 * s);
+        tma_load_2d(smem_base + s * STAGE_BYTES + A_BYTES, &map_b, (kb0 + it) * TC_BK, n0, full0 + 8 * s);
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
+      if (*abort) {
+        // copies already issued still land in this block's shared memory: wait for them (bounded)
+        volatile int never = 0;
+        for (int j = max(0, it - stages); j < it; j++) mbar_wait(full0 + 8 * (j % stages), (j / stages) & 1, &never);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
+      bool ok = true;
+      uint32_t ph = 0;
+      for (int it = 0, s = 0; it < nkb; it++) {
+        ok = mbar_wait(full0 + 8 * s, ph, abort);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a_addr = smem_base + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
+#pragma unroll
+        for (int k = 0; k < TC_BK / 16; k++)
+          umma_bf16(tmem_base, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (it | k) ? 1u : 0u);
+        umma_commit(empty0 + 8 * s);
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
+      if (ok) umma_commit(acc_full);
+    }
+  } else if (mbar_wait(acc_full, 0, abort)) {
+    // every product has read its operands: the ring's space takes the sums, a row's columns together (rows 16 bytes apart modulo
+    // the banks: eight lanes store to eight groups of four)
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int q = warp & 3;
+    float* row = (float*)smem + (size_t)(q * 32 + lane) * (BN + 4);
+    for (int c0 = 0; c0 < BN; c0 += 16) {
+      uint32_t r[16];
+      tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 16; j += 4)
+        *(float4*)(row + c0 + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync_all();
+  pdl_wait();                            // before C is written: the kernel in front may still read what lies there
+  constexpr int ROWS = TC_BM / SPLIT;
+  const bool vec = out_f32 ? ((ldc & 3) == 0 && ((uintptr_t)C & 15) == 0) : ((ldc & 3) == 0 && ((uintptr_t)C & 7) == 0);
+  uint32_t peer[SPLIT];
+#pragma unroll
+  for (int p = 0; p < SPLIT; p++) peer[p] = mapa_shared(smem_base, p) + (rank * ROWS * (BN + 4) << 2);
+  // a warp takes whole rows of 128 columns or more, else as many rows at a time as it has lanes for (lanes a row: a power of two)
+  int lanes = 32;
+  while (lanes * 4 >= 2 * BN && lanes > 4) lanes >>= 1;
+  const int at_once = 32 / lanes;
+#pragma unroll 2
+  for (int r = warp * at_once + lane / lanes; r < ROWS; r += TC_THREADS / 32 * at_once) {
+    const int row = m0 + (int)rank * ROWS + r;
+    if (row >= M) break;
+#pragma unroll 2
+    for (int c = (lane & (lanes - 1)) << 2; c < BN && n0 + c < N; c += lanes << 2) {
+      const uint32_t at = (uint32_t)(r * (BN + 4) + c) << 2;
+      float4 t[SPLIT];
+#pragma unroll
+      for (int p = 0; p < SPLIT; p++) t[p] = tc_cluster_float4(peer[p] + at);
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int p = 0; p < SPLIT; p++) { v[0] += t[p].x; v[1] += t[p].y; v[2] += t[p].z; v[3] += t[p].w; }
+      if (act) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = act_of(act, v[j]);
+      }
+      const int col = n0 + c;
+      if (out_f32) {
+        float* dst = (float*)C + (size_t)row * ldc + col;
+        if (vec && col + 4 <= N) *(float4*)dst = make_float4(v[0], v[1], v[2], v[3]);
+        else
+          for (int j = 0; j < 4; j++) if (col + j < N) dst[j] = v[j];
+      } else {
+        bf16* dst = (bf16*)C + (size_t)row * ldc + col;
+        if (vec && col + 4 <= N) {
+          const __nv_bfloat162 p0 = __floats2bfloat162_rn(v[0], v[1]), p1 = __floats2bfloat162_rn(v[2], v[3]);
+          *(uint2*)dst = make_uint2(*(const uint32_t*)&p0, *(const uint32_t*)&p1);
+        } else
+          for (int j = 0; j < 4; j++) if (col + j < N) dst[j] = __float2bfloat16_rn(v[j]);
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                    // nobody leaves while its sums may be read
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(cols) : "memory");
+  }
+  if (threadIdx.x == 0 && *abort) atomicExch(err, 2);
+}
+
+// How many blocks share a tile's K (1: not this kernel), and the tile's columns: N cut evenly into runs of up to 256, a multiple of 16.
+// Both sides' time in us, fitted to 13 shapes (32 to 6,144 columns, K 128 to 4,096) of 65 to 2,048 rows, one wave each: here a base that
+// grows with the columns that a block stores, and 0.31 a k-block; a kernel that walks all of K starts at `start` (one-SM tiles 3.6 at up to
+// 128 columns and 4.7 beyond, two-SM tiles 6.2) and takes 0.28 a k-block. Measured, there / here: 300 rows by 64 x 1,024 8.1 / 4.6, 300 by
+// 1,024 x 1,024 11.2 / 8.9, 300 by 2,048 x 2,048 15.8 / 10.9, 2,048 by 576 x 2,048 15.7 / 15.0 (the seventh asked of two blocks); but
+// 512 by 2,560 x 1,024 11.0 / 12.5, 300 by 4,096 x 128 7.0 / 10.1. Clusters beyond the first wave double it (512 rows by 1,024 x 1,024
+// on 16 clusters of 8 17.2, on 4 9.0): 14 of 8, 32 of 4 and 72 of 2 stand side by side, twice as many where two blocks fit an SM.
+static int tc_cluster_split(int M, int N, int K, float start, int* tile_n) {
+  const int nkb = (K + TC_BK - 1) / TC_BK, tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + 255) / 256;
+  *tile_n = ((N + tiles_n - 1) / tiles_n + 15) / 16 * 16;
+  const long long tiles = (long long)tiles_m * tiles_n;
+  const float there = start + 0.28f * nkb;
+  for (int split = 8; split > 1; split >>= 1) {
+    const int per = (nkb + split - 1) / split;
+    const bool two = (per < 8 ? per : 8) * (TC_BM + *tile_n) * TC_BK * 2 <= 104 * 1024 && *tile_n <= 128;
+    const int room = (split == 8 ? 14 : split == 4 ? 32 : 72) * (two ? 2 : 1);
+    if (tiles > room || nkb < 2 * split) continue;
+    const float here = 3.5f + (split == 2 ? 5.7f : 3.8f) / 256.f * *tile_n + 0.31f * nkb / split;
+    if (here * (split == 2 ? 1.15f : 1.f) < there) return split;
+  }
+  return 1;
+}
+
+static int tc_cluster_choice(int M, int N, int K, int* tile_n) {
+  if (tc_one_sm_forced()) return 1;
+  return tc_cluster_split(M, N, K, tc_use_pair(M, N) ? 6.2f : N > 128 ? 4.7f : 3.6f, tile_n);
+}
+// the blocks that the plain product of these sizes puts on a tile's K (1: a kernel that walks all of it)
+SLLM_EXPORT int sllm_gemm_tc_cluster_split(int M, int N, int K) {
+  int tile_n;
+  return tc_cluster_choice(M, N, K, &tile_n);
+}
+
+template <int SPLIT>
+static int tc_cluster_run(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int out_f32, int act,
+                          int tile_n, int* err, cudaStream_t stream) {
+  CUtensorMap ma, mb;
+  int rc = tc_make_map(&ma, A, M, K, lda, TC_BM);
+  if (!rc) rc = tc_make_map(&mb, B, N, K, ldb, tile_n);
+  if (rc) return rc;
+  const int stage = TC_BM * TC_BK * 2 + tile_n * TC_BK * 2, per = ((K + TC_BK - 1) / TC_BK + SPLIT - 1) / SPLIT;
+  int stages = (tile_n <= 128 ? 104 : 200) * 1024 / stage;      // (two blocks an SM where a tile is narrow: no less in flight)
+  stages = stages < 8 ? stages : 8;
+  stages = stages < per ? stages : per;
+  const int sums = TC_BM * (tile_n + 4) * 4;
+  const int smem = (stages * stage > sums ? stages * stage : sums) + 1024;
+  static bool raised = false;
+  if (!raised) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_cluster_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    raised = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(SPLIT * ((M + TC_BM - 1) / TC_BM) * ((N + tile_n - 1) / tile_n));
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLIT;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = sllm_pdl_off() ? 1 : 2;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<SPLIT>, ma, mb, C, M, N, K, ldc, out_f32, tile_n, stages, act, err);
+}
+static int tc_cluster_launch(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int out_f32, int act,
+                             int split, int tile_n, int* err, cudaStream_t stream) {
+  return split == 8   ? tc_cluster_run<8>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream)
+         : split == 4 ? tc_cluster_run<4>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream)
+                      : tc_cluster_run<2>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream);
 }
 
 // C[M,N] = A[M,K] B[N,K]^T. epilogue 0: C bfloat16 (or float when out_f32), row stride ldc;
@@ -735,6 +969,11 @@ SLLM_EXPORT int sllm_gemm_tc_fold_bf16(const void* A, const void* B, void* C, in
   if (sumsq_in && (n_in < 1 || width_in < 1)) return SLLM_ERR_ARG;
   const TcFold fd{sumsq_in, n_in, sumsq_in ? 1.0f / (float)width_in : 0.f, eps_in, norm_w, (bf16*)xb, sumsq_out};
   const TcRope rp{};
+  if (epilogue == TC_EPI_STORE && !sumsq_in) {
+    int tile_n;
+    const int split = tc_cluster_choice(M, N, K, &tile_n);
+    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, err, stream);
+  }
   CUtensorMap ma, mb;
   int big = N > 128;
   int rc = tc_make_map(&ma, A, M, K, lda, TC_BM);
@@ -802,6 +1041,9 @@ SLLM_EXPORT int sllm_gemm_tc_act_bf16(const void* A, const void* B, void* C, int
                                       int out_f32, int act, int* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || (K & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || act < 1 || act > 3) return SLLM_ERR_ARG;
+  int tile_n;
+  const int split = tc_cluster_choice(M, N, K, &tile_n);
+  if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, split, tile_n, err, stream);
   TcFold fd{};
   fd.act = act;
   const TcRope rp{};
@@ -894,7 +1136,6 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   const int nkb_all = (K + TC_BK - 1) / TC_BK, per = (nkb_all + gridDim.y - 1) / gridDim.y;
   const int kb0 = blockIdx.y * per, kb1 = min(nkb_all, kb0 + per), nkb = max(0, kb1 - kb0);
 
-  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     mbar_init(acc_full, 1);
@@ -909,6 +1150,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -1030,6 +1272,11 @@ SLLM_EXPORT int sllm_gemm_tc_skinny_bf16(const void* A, const void* B, void* C, 
   if (epilogue != TC_EPI_STORE && epilogue != TC_EPI_SWIGLU) return SLLM_ERR_ARG;
   if (epilogue == TC_EPI_SWIGLU && ((N & 15) || out_f32 || ksplit != 1)) return SLLM_ERR_ARG;
   if (ksplit < 1 || ksplit > (K + TC_BK - 1) / TC_BK || (ksplit > 1 && !out_f32)) return SLLM_ERR_ARG;
+  if (epilogue == TC_EPI_STORE && ksplit == 1 && M > 32 && !tc_one_sm_forced()) {
+    int tile_n;
+    const int split = tc_cluster_split(M, N, K, 3.6f, &tile_n);
+    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, err, stream);
+  }
   int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   CUtensorMap mw, mx;
   int rc = tc_make_map(&mw, B, N, K, ldb, 128);
