@@ -1280,7 +1280,7 @@ class MixKernels:
         """Whether the scan in pieces takes less than the walk over the rows, by what either is about to take (us). In pieces: its three
         launches, blocks (most of which, in a step of unequal runs, find nothing to do) and a channel's states, which every run loads
         and stores like ten rows. Walked: the longest run's chain, or all rows and runs at the SMs' rate. Measured, walked / in pieces, 16
-        states: one run of 96 rows 4,096 channels 27 / 23, 2,048 rows 466 / 143; of 96 and 16 of 4 rows 67 / 45, 1,024 channels 24 / 26; of
+        states: one run of 96 rows 4,096 channels 27 / 23, 2,048 rows 466 / 115; of 96 and 16 of 4 rows 67 / 45, 1,024 channels 24 / 26; of
         96 and 100 of 16, 64 channels 21 / 24, 1,024 132 / 70; 32 states, 1,024 channels, of 96 and 16 of 4 29 / 41."""
         if n_state > 32 or cls.scan_scratch_bytes(0, n_seqs, inner, n_state, sm_count) > ChunkKernels.SCRATCH_BYTES:
             return False

@@ -1054,9 +1054,12 @@ __global__ void __launch_bounds__(256) selective_scan_kernel(ScanArgs p) {
 // sizes behind their softplus for the second.
 //
 // A decay is 2^(dt a log2 e) on the special-function unit, whose error (2^-22 of the result at most) is what expf's bound allows as
-// well; states go two at a time through the paired float instructions. 2,048 rows of 4,096 channels x 16 states: 57 + 7 + 82 us
-// (the kernel above, one walk over all rows: 466); with expf instead of its own power of two 90 + 7 + 93. What a piece adds lies
-// channel after channel, so that a warp's accesses are whole lines.
+// well; states go two at a time through the paired float instructions. Rows come through a ring in shared memory: fetched into registers
+// four rows ahead, their way was a third of the walks' time, and the write walk's registers held it to five blocks an SM besides. 2,048
+// rows of 4,096 channels x 16 states: 50 + 7 + 57 us (from registers 57 + 7 + 82; the kernel above, one walk over all rows, 466; with
+// expf instead of its own power of two 90 + 7 + 93). The special-function units are at 0.62 of their rate in either walk; six or seven
+// blocks an SM in the second, with fewer registers, take 59 to 61. What a piece adds lies channel after channel, so that a warp's
+// accesses are whole lines.
 struct ScanPieces {
   float* dt;            // [T][I] step sizes
   float* end;           // [pieces][N][I]: what a piece adds, then the state in front of it
@@ -1115,6 +1118,7 @@ __device__ __forceinline__ size_t scan_first_piece(int start, int b, int R) { re
 // B (and C) of n rows as floats, [row][NP] each, states from N on zero
 template <typename A, int NP, bool WITH_C>
 __device__ __forceinline__ void scan_stage(float* b_s, float* c_s, const ScanArgs& p, int row, int n) {
+#pragma unroll 4
   for (int i = threadIdx.x; i < n * NP; i += MIX_SCAN_BLOCK) {
     const int r = i / NP, s = i % NP;
     const A* src = (const A*)p.bc + (size_t)(row + r) * p.ldbc;
@@ -1123,45 +1127,96 @@ __device__ __forceinline__ void scan_stage(float* b_s, float* c_s, const ScanArg
   }
 }
 
+// A block's rows of step sizes (raw, or behind their softplus), inputs and, for the second walk, gates: MIX_SCAN_ROWS rows of its 128
+// channels at a time through a ring in shared memory, two stages on their way while one is walked. Copies are 16 bytes and asynchronous
+// where every row starts on such a boundary, else the threads' own loads. Channels past the last one and rows past the piece are zeros.
+#define MIX_SCAN_ROWS 8
+#define MIX_SCAN_STAGES 3
+template <typename A, bool WITH_Z>
+struct ScanRing {
+  static constexpr int DT_BYTES = MIX_SCAN_ROWS * MIX_SCAN_BLOCK * 4, X_BYTES = MIX_SCAN_ROWS * MIX_SCAN_BLOCK * (int)sizeof(A);
+  static constexpr int STAGE = DT_BYTES + X_BYTES * (WITH_Z ? 2 : 1), BYTES = MIX_SCAN_STAGES * STAGE;
+  uint8_t* at;
+  const float* dt; int lddt;
+  const A* x; int ldx;
+  const A* z; int ldz;
+  int n, left;              // rows; channels from the block's first one on
+  bool vec;
+  template <typename T>
+  __device__ __forceinline__ void rows(T* dst, const T* src, int ld, int r0) const {
+    constexpr int PER = 16 / (int)sizeof(T), VECS = MIX_SCAN_BLOCK / PER;
+    if (vec) {
+#pragma unroll
+      for (int i = threadIdx.x; i < MIX_SCAN_ROWS * VECS; i += MIX_SCAN_BLOCK) {
+        const int r = i / VECS, c = i % VECS * PER;
+        const int there = r0 + r < n ? max(0, min(PER, left - c)) : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * MIX_SCAN_BLOCK + c)), "l"(src + (there ? (size_t)(r0 + r) * ld + c : 0)),
+                     "r"(there * (int)sizeof(T)) : "memory");
+      }
+    } else {
+      for (int r = 0; r < MIX_SCAN_ROWS; r++)
+        dst[r * MIX_SCAN_BLOCK + threadIdx.x] = r0 + r < n && (int)threadIdx.x < left ? src[(size_t)(r0 + r) * ld + threadIdx.x] : from_f32<T>(0.f);
+    }
+  }
+  // asks for rows r0 .. of the piece (a multiple of MIX_SCAN_ROWS); beyond the last nothing is asked, but the group counts
+  __device__ __forceinline__ void fetch(int r0) const {
+    if (r0 < n) {
+      uint8_t* s = at + (r0 / MIX_SCAN_ROWS) % MIX_SCAN_STAGES * STAGE;
+      rows((float*)s, dt, lddt, r0);
+      rows((A*)(s + DT_BYTES), x, ldx, r0);
+      if (WITH_Z) rows((A*)(s + DT_BYTES + X_BYTES), z, ldz, r0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  __device__ __forceinline__ void open() const {
+#pragma unroll
+    for (int k = 0; k < MIX_SCAN_STAGES - 1; k++) fetch(k * MIX_SCAN_ROWS);
+  }
+  // rows r0 .. are there, and the stage before them is free: its place takes the rows after next
+  __device__ __forceinline__ const uint8_t* next(int r0) const {
+    asm volatile("cp.async.wait_group %0;" ::"n"(MIX_SCAN_STAGES - 2) : "memory");
+    __syncthreads();
+    fetch(r0 + (MIX_SCAN_STAGES - 1) * MIX_SCAN_ROWS);
+    return at + (r0 / MIX_SCAN_ROWS) % MIX_SCAN_STAGES * STAGE;
+  }
+};
+__device__ __forceinline__ bool scan_aligned(const void* p, size_t row_bytes) { return ((uintptr_t)p & 15) == 0 && (row_bytes & 15) == 0; }
+
 template <typename A, int NP>
 __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_piece_kernel(ScanArgs p, ScanPieces w) {
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
   if (r0 >= len) return;
-  const int n = min(w.R, len - r0), row = start + r0, ch = blockIdx.x * MIX_SCAN_BLOCK + threadIdx.x, c = min(ch, p.I - 1);
+  const int n = min(w.R, len - r0), row = start + r0, ch0 = blockIdx.x * MIX_SCAN_BLOCK, ch = ch0 + threadIdx.x, c = min(ch, p.I - 1);
+  typedef ScanRing<A, false> Ring;
+  Ring ring;
+  ring.at = (uint8_t*)(sm + w.R * NP);
+  ring.dt = p.dt_raw + (size_t)row * p.lddt + ch0; ring.lddt = p.lddt;
+  ring.x = (const A*)p.x + (size_t)row * p.ldx + ch0; ring.ldx = p.ldx;
+  ring.n = n; ring.left = p.I - ch0;
+  ring.vec = scan_aligned(p.dt_raw, (size_t)p.lddt * 4) && scan_aligned(p.x, (size_t)p.ldx * sizeof(A));
+  ring.open();
   scan_stage<A, NP, false>(sm, nullptr, p, row, n);
   uint64_t a[NP / 2], S[NP / 2];
   scan_rates<NP>(a, p, c);
 #pragma unroll
   for (int i = 0; i < NP / 2; i++) S[i] = 0ull;
   const float bias = load_w(p.dt_bias, p.w_f32, c);
-  const float* dtr = p.dt_raw + (size_t)row * p.lddt + c;
-  const A* xs = (const A*)p.x + (size_t)row * p.ldx + c;
   float* dts = w.dt + (size_t)row * p.I + c;
   float sum = 0.f;
-  constexpr int U = 4;                   // rows whose loads are on their way together
-  float raw[U], xv[U];
-#pragma unroll
-  for (int k = 0; k < U; k++) { raw[k] = k < n ? dtr[(size_t)k * p.lddt] : 0.f; xv[k] = k < n ? to_f32(xs[(size_t)k * p.ldx]) : 0.f; }
-  __syncthreads();
-  for (int q0 = 0; q0 < n; q0 += U) {
-    float dt[U], dx[U];
-#pragma unroll
-    for (int k = 0; k < U; k++) { dt[k] = softplus_f(raw[k] + bias); dx[k] = dt[k] * xv[k]; }
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const int r = q0 + U + k;
-      raw[k] = r < n ? dtr[(size_t)r * p.lddt] : 0.f;
-      xv[k] = r < n ? to_f32(xs[(size_t)r * p.ldx]) : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const int r = q0 + k;
-      if (r >= n) break;
-      if (ch < p.I) dts[(size_t)r * p.I] = dt[k];
-      sum += dt[k];
-      const ulonglong2* br = (const ulonglong2*)(sm + r * NP);
-      const uint64_t dt2 = pair_of(dt[k], dt[k]), dx2 = pair_of(dx[k], dx[k]);
+  for (int q0 = 0; q0 < n; q0 += MIX_SCAN_ROWS) {
+    const uint8_t* s = ring.next(q0);
+    const float* dt_s = (const float*)s + threadIdx.x;
+    const A* x_s = (const A*)(s + Ring::DT_BYTES) + threadIdx.x;
+    const int m = min(MIX_SCAN_ROWS, n - q0);
+#pragma unroll 4
+    for (int r = 0; r < m; r++) {
+      const float dt = softplus_f(dt_s[r * MIX_SCAN_BLOCK] + bias), dx = dt * to_f32(x_s[r * MIX_SCAN_BLOCK]);
+      if (ch < p.I) dts[(size_t)(q0 + r) * p.I] = dt;
+      sum += dt;
+      const ulonglong2* br = (const ulonglong2*)(sm + (q0 + r) * NP);
+      const uint64_t dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
 #pragma unroll
       for (int i = 0; i < NP / 2; i += 2) {
         const ulonglong2 bq = br[i / 2];
@@ -1215,8 +1270,17 @@ __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_write_kernel(Sc
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
   if (r0 >= len) return;
-  const int n = min(w.R, len - r0), row = start + r0, ch = blockIdx.x * MIX_SCAN_BLOCK + threadIdx.x, c = min(ch, p.I - 1);
+  const int n = min(w.R, len - r0), row = start + r0, ch0 = blockIdx.x * MIX_SCAN_BLOCK, ch = ch0 + threadIdx.x, c = min(ch, p.I - 1);
+  typedef ScanRing<A, true> Ring;
   float *b_s = sm, *c_s = sm + w.R * NP;
+  Ring ring;
+  ring.at = (uint8_t*)(c_s + w.R * NP);
+  ring.dt = w.dt + (size_t)row * p.I + ch0; ring.lddt = p.I;
+  ring.x = (const A*)p.x + (size_t)row * p.ldx + ch0; ring.ldx = p.ldx;
+  ring.z = (const A*)p.z + (size_t)row * p.ldz + ch0; ring.ldz = p.ldz;
+  ring.n = n; ring.left = p.I - ch0;
+  ring.vec = scan_aligned(w.dt, (size_t)p.I * 4) && scan_aligned(p.x, (size_t)p.ldx * sizeof(A)) && scan_aligned(p.z, (size_t)p.ldz * sizeof(A));
+  ring.open();
   scan_stage<A, NP, true>(b_s, c_s, p, row, n);
   const float* front = w.end + (scan_first_piece(start, b, w.R) + blockIdx.y) * p.I * p.N + c;
   uint64_t a[NP / 2], S[NP / 2];
@@ -1225,37 +1289,17 @@ __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_write_kernel(Sc
   for (int i = 0; i < NP; i += 2)
     S[i / 2] = pair_of(i < p.N ? front[(size_t)i * p.I] : 0.f, i + 1 < p.N ? front[(size_t)(i + 1) * p.I] : 0.f);
   const float dsk = load_w(p.dskip, p.w_f32, c);
-  const float* dts = w.dt + (size_t)row * p.I + c;
-  const A* xs = (const A*)p.x + (size_t)row * p.ldx + c;
-  const A* zs = (const A*)p.z + (size_t)row * p.ldz + c;
   A* out = (A*)p.out + (size_t)row * p.ldo + c;
-  constexpr int U = 4;
-  float dtv[U], xv[U], zv[U];
-#pragma unroll
-  for (int k = 0; k < U; k++) {
-    dtv[k] = k < n ? dts[(size_t)k * p.I] : 0.f;
-    xv[k] = k < n ? to_f32(xs[(size_t)k * p.ldx]) : 0.f;
-    zv[k] = k < n ? to_f32(zs[(size_t)k * p.ldz]) : 0.f;
-  }
-  __syncthreads();
-  for (int q0 = 0; q0 < n; q0 += U) {
-    float dt[U], x[U], z[U];
-#pragma unroll
-    for (int k = 0; k < U; k++) { dt[k] = dtv[k]; x[k] = xv[k]; z[k] = zv[k]; }
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const int r = q0 + U + k;
-      dtv[k] = r < n ? dts[(size_t)r * p.I] : 0.f;
-      xv[k] = r < n ? to_f32(xs[(size_t)r * p.ldx]) : 0.f;
-      zv[k] = r < n ? to_f32(zs[(size_t)r * p.ldz]) : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < U; k++) {
-      const int r = q0 + k;
-      if (r >= n) break;
-      const float dx = dt[k] * x[k];
-      const ulonglong2 *br = (const ulonglong2*)(b_s + r * NP), *cr = (const ulonglong2*)(c_s + r * NP);
-      const uint64_t dt2 = pair_of(dt[k], dt[k]), dx2 = pair_of(dx, dx);
+  for (int q0 = 0; q0 < n; q0 += MIX_SCAN_ROWS) {
+    const uint8_t* s = ring.next(q0);
+    const float* dt_s = (const float*)s + threadIdx.x;
+    const A *x_s = (const A*)(s + Ring::DT_BYTES) + threadIdx.x, *z_s = x_s + MIX_SCAN_ROWS * MIX_SCAN_BLOCK;
+    const int m = min(MIX_SCAN_ROWS, n - q0);
+#pragma unroll 2
+    for (int r = 0; r < m; r++) {
+      const float dt = dt_s[r * MIX_SCAN_BLOCK], x = to_f32(x_s[r * MIX_SCAN_BLOCK]), dx = dt * x;
+      const ulonglong2 *br = (const ulonglong2*)(b_s + (q0 + r) * NP), *cr = (const ulonglong2*)(c_s + (q0 + r) * NP);
+      const uint64_t dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
       uint64_t acc0 = 0ull, acc1 = 0ull;
 #pragma unroll
       for (int i = 0; i < NP / 2; i += 2) {
@@ -1266,7 +1310,7 @@ __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_write_kernel(Sc
         acc1 = fma_pair(S[i + 1], cq.y, acc1);
       }
       const float2 f0 = parts_of(acc0), f1 = parts_of(acc1);
-      if (ch < p.I) out[(size_t)r * p.ldo] = from_f32<A>(fmaf(dsk, x[k], (f0.x + f0.y) + (f1.x + f1.y)) * silu_f(z[k]));
+      if (ch < p.I) out[(size_t)(q0 + r) * p.ldo] = from_f32<A>(fmaf(dsk, x, (f0.x + f0.y) + (f1.x + f1.y)) * silu_f(to_f32(z_s[r * MIX_SCAN_BLOCK])));
     }
   }
 }
