@@ -982,8 +982,8 @@ class SequenceKernels:
     SCAN_WALK_MAX = 4     # rows of a sequence in one step up to which a thread walks them one after the other
 
     def rglru_scan(self, gates, u, yraw, ra_b, ri_b, lam, y_b, state, ctx, out, block_size):
-        """gates float32 [blocks, T, 2 * block_size], u float32 [T, W], yraw [T, W] view of the element type,
-        state float32 [slots, W] (read and advanced), out [T, W] of the element type."""
+        """gates float32 [blocks, T, 2 * block_size] (a long portion leaves the recurrence's terms there), u float32 [T, W], yraw
+        [T, W] view of the element type, state float32 [slots, W] (read and advanced), out [T, W] of the element type."""
         T, W = u.shape
         if gates.dtype != torch.float32 or tuple(gates.shape) != (W // block_size, T, 2 * block_size) or yraw.dtype != self.dtype:
             raise KernelError(f"rglru_scan shapes: gates {tuple(gates.shape)} {gates.dtype}, u {tuple(u.shape)}")

@@ -192,6 +192,63 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const void* __restrict
   }
 }
 
+// The same for the many rows of a prompt: PER accesses of four elements a thread, a row's block as wide as that takes, the row in registers from its
+// loads to its store. Bound by what the rows weigh and the launch: the two norms of a sublayer of 2,048 rows of 2,048, without and with a
+// bfloat16 addend, 15.0 us; through shared memory, with 73 registers a thread and so two and a half waves, 19.2. Kernels of fewer rows
+// keep the one above, whose blocks are as wide as a row allows.
+template <typename A, int PER>
+__global__ void __launch_bounds__(1024) add_rmsnorm_rows_kernel(float* __restrict__ x, const void* __restrict__ delta, int n_parts,
+                                                                size_t part_stride, const int* __restrict__ rows, const void* __restrict__ w,
+                                                                int w_f32, A* __restrict__ y, int d, float eps) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int r = blockIdx.x, step = blockDim.x * 4, j0 = threadIdx.x * 4;
+  const size_t in = rows ? (size_t)rows[r] : (size_t)r;
+  float* xr = x + in * d;
+  float4 v[PER];
+#pragma unroll
+  for (int u = 0; u < PER; u++) v[u] = j0 + u * step < d ? *(const float4*)(xr + j0 + u * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (delta && n_parts == 0) {
+    const A* dr = (const A*)delta + in * d;
+    float4 a[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) a[u] = j0 + u * step < d ? ld_dep4(dr + j0 + u * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < PER; u++) { v[u].x += a[u].x; v[u].y += a[u].y; v[u].z += a[u].z; v[u].w += a[u].w; }
+  } else if (delta) {
+    const float* pr = (const float*)delta + in * d;
+    float4 a[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < n_parts; q++) {
+#pragma unroll
+      for (int u = 0; u < PER; u++)
+        if (j0 + u * step < d) {
+          const float4 b = ld_dep4(pr + (size_t)q * part_stride + j0 + u * step);
+          a[u].x += b.x; a[u].y += b.y; a[u].z += b.z; a[u].w += b.w;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) { v[u].x += a[u].x; v[u].y += a[u].y; v[u].z += a[u].z; v[u].w += a[u].w; }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int u = 0; u < PER; u++) ss += v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+  ss = block_sum(ss, red);
+  const float inv = 1.0f / sqrtf(ss / (float)d + eps);
+  const bool update = rows == nullptr && delta != nullptr;
+  A* yr = y + (size_t)r * d;
+#pragma unroll
+  for (int u = 0; u < PER; u++) {
+    const int j = j0 + u * step;
+    if (j >= d) break;
+    if (update) *(float4*)(xr + j) = v[u];
+    const float4 wv = w_f32 ? ld4((const float*)w + j) : ld4((const bf16*)w + j);
+    st4(yr + j, make_float4((v[u].x * inv) * wv.x, (v[u].y * inv) * wv.y, (v[u].z * inv) * wv.z, (v[u].w * inv) * wv.w));
+  }
+}
+
 // ------------------------------------------------------------------ C = A * B^T, tiled, FP32 FMA
 // A [M,K] (row stride lda), B [N,K] (row stride ldb: weights are [out, in]), C [M,N].
 // Each output is one ascending-k chain of fused multiply-adds in float.

@@ -191,8 +191,10 @@ __global__ void causal_conv_vec_kernel(ConvArgs p) {
 }
 
 // The same for steps of many rows: four neighbouring channels and ROWS rows a thread, whose inputs it reads once (all asked for
-// before the first is used) with the channels' filters in registers. TAPS: the number of taps.
-template <typename A, int TAPS, int ROWS>
+// before the first is used) with the channels' filters in registers. TAPS: the number of taps. 2,048 rows of 4,096 channels, bfloat16 to
+// bfloat16 14.0 us, to floats 16.5 (types told at run time 15.5 and 18.0; two or eight rows a thread 21 and 15; a thread that walks down
+// 16 rows with four on their way 22: it waits more than it saves).
+template <typename A, int TAPS, int ROWS, bool XF, bool YF>      // inputs, results: floats or of type A
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T) {
   constexpr int HIST = TAPS - 1;
   const int t0 = blockIdx.x * ROWS, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T
 #pragma unroll
   for (int k = 0; k < HIST + ROWS; k++) {
     const int s = t0 - HIST + k;
-    v[k] = s >= 0 && s < T ? ld4_flag<A>(p.x, p.x_f32, (size_t)s * p.ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[k] = s >= 0 && s < T ? (XF ? ld4((const float*)p.x + (size_t)s * p.ldx + c) : ld4((const A*)p.x + (size_t)s * p.ldx + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const int b0 = p.tok_seq[t0], first0 = p.seq_start[b0], end0 = p.seq_start[b0 + 1];
   float w[4 * TAPS];                            // the four channels' taps lie one behind the other
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T
       acc.x += q.x; acc.y += q.y; acc.z += q.z; acc.w += q.w;
     }
     if (p.act == 1) {
-      if (sizeof(A) == 2 && !p.y_f32) {         // on its way into a 16-bit number
+      if (sizeof(A) == 2 && !YF) {         // on its way into a 16-bit number
         acc.x = __fdividef(acc.x, 1.0f + __expf(-acc.x));
         acc.y = __fdividef(acc.y, 1.0f + __expf(-acc.y));
         acc.z = __fdividef(acc.z, 1.0f + __expf(-acc.z));
@@ -258,7 +260,8 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T
         acc.x = silu_f(acc.x); acc.y = silu_f(acc.y); acc.z = silu_f(acc.z); acc.w = silu_f(acc.w);
       }
     }
-    st4_flag<A>(p.y, p.y_f32, (size_t)t * p.ldy + c, acc);
+    if (YF) st4((float*)p.y + (size_t)t * p.ldy + c, acc);
+    else st4((A*)p.y + (size_t)t * p.ldy + c, acc);
     if (p.y2) st4((A*)p.y2 + (size_t)t * p.ldy2 + c, acc);
   }
 }
@@ -478,7 +481,7 @@ __global__ void __launch_bounds__(128) attn_wide_value_kernel(const A* __restric
 template <typename A>
 __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld_qk, const float* __restrict__ ba, int ld_ba,
                                      const void* __restrict__ a_log, const void* __restrict__ dt_bias, int w_f32,
-                                     float* __restrict__ bd, int H, int G, int dk) {
+                                     float* __restrict__ bd, int H, int G, int dk, int vec) {
   int t = blockIdx.x;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float qmult = rsqrtf((float)dk);
@@ -486,6 +489,17 @@ __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld_qk, const fl
   for (int gg = wid; gg < G; gg += nw) {
     float* qv = qk + (size_t)t * ld_qk + (size_t)gg * dk;
     float* kv = qv + (size_t)G * dk;
+    if (vec) {                                   // heads of up to 128, four elements a lane, read once
+      const bool in = lane * 4 < dk;
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), q = in ? ld4(qv + lane * 4) : z, k = in ? ld4(kv + lane * 4) : z;
+      const float sq = warp_sum(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w), sk = warp_sum(k.x * k.x + k.y * k.y + k.z * k.z + k.w * k.w);
+      const float iq = qmult / sqrtf(sq + 1e-6f), ik = 1.0f / sqrtf(sk + 1e-6f);
+      const float4 a = make_float4(q.x * iq, q.y * iq, q.z * iq, q.w * iq), b = make_float4(k.x * ik, k.y * ik, k.z * ik, k.w * ik);
+      if (in) { st4(qv + lane * 4, a); st4(kv + lane * 4, b); }
+      const float kq = warp_sum(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w);
+      if (lane == 0) brow[2 * H + gg] = kq;
+      continue;
+    }
     float sq = 0.f, sk = 0.f;
     for (int j = lane; j < dk; j += 32) { sq += qv[j] * qv[j]; sk += kv[j] * kv[j]; }
     sq = warp_sum(sq);
@@ -736,6 +750,24 @@ __global__ void gated_unit_rms_kernel(const float* __restrict__ o, const A* __re
   }
 }
 
+// The same for heads of up to 128 values, four elements a lane, read once. 2,048 rows of 16 heads of 128: 11.5 us (an element at a time
+// 15.3; two or four pairs a warp, their loads asked for together, 12.5 and 14.2: more warps hide more than more loads a warp).
+template <typename A>
+__global__ void __launch_bounds__(128) gated_unit_rms_vec_kernel(const float* __restrict__ o, const A* __restrict__ gate, int ld_gate,
+                                                                 const void* __restrict__ w, int w_f32, A* __restrict__ y, int T, int H, int dv,
+                                                                 float eps) {
+  const int j = (threadIdx.x & 31) * 4;
+  const size_t i = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (i >= (size_t)T * H) return;
+  const bool in = j < dv;
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), v = in ? ld4(o + i * dv + j) : z, g = in ? ld4(gate + (i / H) * ld_gate + (i % H) * dv + j) : z;
+  const float4 wv = in ? ld4_w(w, w_f32, j) : z;
+  const float ss = warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+  const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+  if (in) st4(y + i * dv + j, make_float4(v.x * inv * wv.x * silu_f(g.x), v.y * inv * wv.y * silu_f(g.y), v.z * inv * wv.z * silu_f(g.z),
+                                          v.w * inv * wv.w * silu_f(g.w)));
+}
+
 // ------------------------------------------------------------------ real-gated linear recurrence
 // Channel c of width W lies in block c / bs of the gates; gates[block][t][0..bs) is the raw recurrence gate,
 // [bs..2bs) the raw input gate (block-diagonal products of u, float). r = sigmoid(. + ra_b), i = sigmoid(. + ri_b),
@@ -763,13 +795,13 @@ __device__ __forceinline__ LruChannel lru_channel(const LruArgs& p, int c) {
   return ch;
 }
 
-// a_t and b_t of S_t = a_t S_{t-1} + b_t for row t
-__device__ __forceinline__ void lru_terms(const LruArgs& p, const LruChannel& ch, int t, float& a, float& bt) {
-  float r = sigmoid_f(ch.gb[(size_t)t * 2 * ch.bs + ch.cc] + ch.rb);
-  float i = sigmoid_f(ch.gb[(size_t)t * 2 * ch.bs + ch.bs + ch.cc] + ch.ib);
+// a_t and b_t of S_t = a_t S_{t-1} + b_t for a row's raw gates and input
+__device__ __forceinline__ void lru_terms(const LruChannel& ch, float raw_r, float raw_i, float u, float& a, float& bt) {
+  float r = sigmoid_f(raw_r + ch.rb);
+  float i = sigmoid_f(raw_i + ch.ib);
   float log_a = -8.0f * r * ch.sp;
   a = expf(log_a);
-  bt = sqrtf(-expm1f(2.0f * log_a)) * (i * p.u[(size_t)t * p.W + ch.c]);      // 1 - a^2 without cancellation
+  bt = sqrtf(-expm1f(2.0f * log_a)) * (i * u);      // 1 - a^2 without cancellation
 }
 
 // A thread per (sequence, channel) walks the sequence's rows: the decode step, and short portions.
@@ -784,7 +816,7 @@ __global__ void rglru_scan_kernel(LruArgs p) {
   int t0 = p.seq_start[b], t1 = p.seq_start[b + 1];
   for (int t = t0; t < t1; t++) {
     float a, bt;
-    lru_terms(p, ch, t, a, bt);
+    lru_terms(ch, ch.gb[(size_t)t * 2 * ch.bs + ch.cc], ch.gb[(size_t)t * 2 * ch.bs + ch.bs + ch.cc], p.u[(size_t)t * p.W + c], a, bt);
     S = a * S + bt;
     ((A*)p.out)[(size_t)t * p.W + c] = from_f32<A>(S * gelu_tanh_f(to_f32(((const A*)p.yraw)[(size_t)t * p.ld_y + c]) + ch.yb));
   }
@@ -793,10 +825,14 @@ __global__ void rglru_scan_kernel(LruArgs p) {
 
 // Long portions, in three kernels. The rows of a sequence are cut into pieces of LRU_PIECE. (1) A thread per
 // (piece, channel) runs its piece from S = 0 and leaves the piece's product of a and its end value:
-// S_end = prod * S_start + end. (2) A thread per (sequence, channel) carries the state from piece to piece
-// and leaves every piece's S_start (the sequence's state is advanced here). (3) A thread per (piece, channel)
-// runs its piece again from S_start and writes the rows. `pieces` = most pieces of any sequence.
+// S_end = prod * S_start + end, and every row's a and b where its gates were. (2) A thread per (sequence, channel) carries
+// the state from piece to piece and leaves every piece's S_start (the sequence's state is advanced here). (3) A thread per
+// (piece, channel) runs its piece again from S_start, over the a and b kept, and writes the rows. `pieces` = most pieces of any sequence.
+// Bound by the gate terms' arithmetic (two sigmoids, two exponentials, a root a row and channel: once, in (1)) and by waiting for rows, of
+// which LRU_ROWS are asked for at a time. 2,778 rows of 1,280 channels in 32-bit: 24 + 8 + 12 us; with the terms computed in (1) and again in
+// (3), a row asked for at a time, 26 + 8 + 32.
 #define LRU_PIECE 16
+#define LRU_ROWS 4
 template <typename A>
 __global__ void rglru_piece_kernel(LruArgs p, float* __restrict__ prod, float* __restrict__ end, int pieces) {
   int b = blockIdx.x / pieces, k = blockIdx.x % pieces;
@@ -804,12 +840,27 @@ __global__ void rglru_piece_kernel(LruArgs p, float* __restrict__ prod, float* _
   int t0 = p.seq_start[b] + k * LRU_PIECE, t1 = min(p.seq_start[b + 1], t0 + LRU_PIECE);
   if (c >= p.W || t0 >= t1) return;
   LruChannel ch = lru_channel(p, c);
+  float* terms = const_cast<float*>(ch.gb) + ch.cc;
   float P = 1.f, S = 0.f;
-  for (int t = t0; t < t1; t++) {
-    float a, bt;
-    lru_terms(p, ch, t, a, bt);
-    S = a * S + bt;
-    P *= a;
+  for (int t = t0; t < t1; t += LRU_ROWS) {
+    float r[LRU_ROWS], i[LRU_ROWS], u[LRU_ROWS];
+#pragma unroll
+    for (int j = 0; j < LRU_ROWS; j++) {
+      const size_t row = min(t + j, t1 - 1);
+      r[j] = terms[row * 2 * ch.bs];
+      i[j] = terms[row * 2 * ch.bs + ch.bs];
+      u[j] = p.u[row * p.W + c];
+    }
+#pragma unroll
+    for (int j = 0; j < LRU_ROWS; j++) {
+      if (t + j >= t1) break;
+      float a, bt;
+      lru_terms(ch, r[j], i[j], u[j], a, bt);
+      terms[(size_t)(t + j) * 2 * ch.bs] = a;
+      terms[(size_t)(t + j) * 2 * ch.bs + ch.bs] = bt;
+      S = a * S + bt;
+      P *= a;
+    }
   }
   prod[(size_t)blockIdx.x * p.W + c] = P;
   end[(size_t)blockIdx.x * p.W + c] = S;
@@ -823,16 +874,17 @@ __global__ void rglru_carry_kernel(LruArgs p, const float* __restrict__ prod, fl
   float S = *sp_state;
   int n = p.seq_start[b + 1] - p.seq_start[b];
   int used = (n + LRU_PIECE - 1) / LRU_PIECE;
-  for (int k0 = 0; k0 < used; k0 += 8) {        // eight pieces' terms fetched together, then chained
-    float P[8], E[8];
+  constexpr int U = 16;                         // pieces' terms fetched together, then chained
+  for (int k0 = 0; k0 < used; k0 += U) {
+    float P[U], E[U];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < U; i++) {
       size_t at = ((size_t)b * pieces + min(k0 + i, used - 1)) * p.W + c;
       P[i] = prod[at];
       E[i] = end[at];
     }
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < U; i++) {
       if (k0 + i < used) {
         end[((size_t)b * pieces + k0 + i) * p.W + c] = S;      // from here on: the piece's start value
         S = P[i] * S + E[i];
@@ -848,12 +900,24 @@ __global__ void rglru_write_kernel(LruArgs p, const float* __restrict__ start, i
   int c = blockIdx.y * blockDim.x + threadIdx.x;
   int t0 = p.seq_start[b] + k * LRU_PIECE, t1 = min(p.seq_start[b + 1], t0 + LRU_PIECE);
   if (c >= p.W || t0 >= t1) return;
-  LruChannel ch = lru_channel(p, c);
+  const int cc = c % p.bs;
+  const float* terms = p.gates + (size_t)(c / p.bs) * p.T * 2 * p.bs + cc;
+  const float yb = load_w(p.y_b, p.w_f32, c);
   float S = start[(size_t)blockIdx.x * p.W + c];
-  for (int t = t0; t < t1; t++) {
-    float a, bt;
-    lru_terms(p, ch, t, a, bt);
-    S = a * S + bt;
-    ((A*)p.out)[(size_t)t * p.W + c] = from_f32<A>(S * gelu_tanh_f(to_f32(((const A*)p.yraw)[(size_t)t * p.ld_y + c]) + ch.yb));
+  for (int t = t0; t < t1; t += LRU_ROWS) {
+    float a[LRU_ROWS], bt[LRU_ROWS], y[LRU_ROWS];
+#pragma unroll
+    for (int j = 0; j < LRU_ROWS; j++) {
+      const size_t row = min(t + j, t1 - 1);
+      a[j] = terms[row * 2 * p.bs];
+      bt[j] = terms[row * 2 * p.bs + p.bs];
+      y[j] = to_f32(((const A*)p.yraw)[row * p.ld_y + c]);
+    }
+#pragma unroll
+    for (int j = 0; j < LRU_ROWS; j++) {
+      if (t + j >= t1) break;
+      S = a[j] * S + bt[j];
+      ((A*)p.out)[(size_t)(t + j) * p.W + c] = from_f32<A>(S * gelu_tanh_f(y[j] + yb));
+    }
   }
 }

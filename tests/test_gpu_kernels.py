@@ -108,6 +108,43 @@ def test_add_rmsnorm_many_rows(kernel_sets, dtype, d, w32):
     assert torch.equal(xs, x) and rel_err(y.cpu().float(), plain.rms_norm(f64(x), f64(w), eps)) < TOL[dtype]
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [512, 516, 2000, 2052, 8192, 16384])
+def test_add_rmsnorm_many_rows_of_any_width(kernel_sets, dtype, d):
+    """Rows in registers: widths that fill no access, partial sums as the addend, and rows picked out of the stream, which stays."""
+    ks, T, eps = kernel_sets[dtype], 600, 1e-5
+    x, w = dev(rand(T, d, seed=1, scale=2.0)), dev(rand(d, seed=3) + 1.0, dtype)
+    parts = dev(rand(3, T, d, seed=4))
+    y, xs = torch.full((T, d), float("nan"), dtype=dtype, device="cuda"), x.clone()
+    ks.add_rmsnorm(xs, parts, None, w, y, eps)
+    want = f64(x) + f64(parts).sum(0)
+    assert rel_err(xs.cpu(), want) < 4e-7 and rel_err(y.cpu().float(), plain.rms_norm(want, f64(w), eps)) < TOL[dtype]
+    rows, xs = dev(torch.arange(T - 1, -1, -1, dtype=torch.int32)), x.clone()
+    ks.add_rmsnorm(xs, parts[:1], rows, w, y, eps)
+    assert torch.equal(xs, x) and rel_err(y.cpu().float(), plain.rms_norm((f64(x) + f64(parts[0])).flip(0), f64(w), eps)) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dv", [4, 100, 127, 128, 132])
+def test_unit_norms_of_heads(kernel_sets, dtype, dv):
+    """The gated norm behind the delta rule and the unit keys and queries in front of it: heads of up to 128 by four elements, others."""
+    seq, T, H, G = kernel_sets[dtype].seq, 37, 5, 3
+    o, gate, w = dev(rand(T, H, dv, seed=1)), dev(rand(T, 8 + H * dv, seed=2), dtype), dev(rand(dv, seed=3) + 1.0, dtype)
+    y = torch.full((T, H * dv), float("nan"), dtype=dtype, device="cuda")
+    g = gate[:, 8:] if dtype == torch.bfloat16 or dv != 127 else gate[:, 7:7 + H * dv]
+    seq.gated_unit_rms(o.view(T, H * dv), g, w, y, H, dv, 1e-6)
+    od, gd = f64(o), f64(g.reshape(T, H, dv))
+    want = od / torch.sqrt(od.square().mean(-1, keepdim=True) + 1e-6) * f64(w) * gd * torch.sigmoid(gd)
+    assert rel_err(y.cpu().float(), want.reshape(T, H * dv)) < TOL[dtype]
+    qk, ba, a_log, bias = dev(rand(T, 2 * G * dv, seed=5)), dev(rand(T, 2 * H, seed=6)), dev(rand(H, seed=7)), dev(rand(H, seed=8))
+    bd, before = torch.full((T, 2 * H + G), float("nan"), device="cuda"), f64(qk).view(T, 2, G, dv)
+    seq.delta_prepare(qk, ba, a_log, bias, bd, H, G, dv)
+    unit = before / torch.sqrt(before.square().sum(-1, keepdim=True) + 1e-6)
+    unit[:, 0] *= dv ** -0.5
+    assert rel_err(qk.cpu(), unit.reshape(T, -1)) < 2e-6 and rel_err(bd[:, 2 * H:].cpu(), (unit[:, 0] * unit[:, 1]).sum(-1)) < 4e-6
+
+
+
 # --------------------------------------------------------------------------- matrix products
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M, N, K", [(1, 33, 19), (3, 100, 72), (8, 64, 1000), (9, 130, 65), (70, 257, 136), (200, 96, 520),
