@@ -12,7 +12,8 @@ cache then keeps values that wide and the output product reads n_heads * v_dim c
 before it is cached. Either sends the step's keys and values through a store kernel that does
 rotation, value norm and cache write in one pass (`kv_store`); values as wide as keys then still
 use the attention kernels below, other widths kernels that take both (in a bfloat16 prompt step with widths in
-multiples of 8 the tcgen05 kernel with float32 weights, else `attn_wide_value`).
+multiples of 8 the tcgen05 kernel with float32 weights, in a decode step with widths in multiples of 4 the one that
+splits the keys over blocks, else `attn_wide_value`).
 
 Four more options, none in the reference. `chunk`: a query sees the earlier keys of its own chunk of that many
 positions only, chunks counted from position 0 of the sequence (not from where a step begins); the cache
@@ -303,7 +304,7 @@ class Attention(Mixer):
         path = self.out.fold_path(ctx, rows, ctx.dtype, finishing=True)
         return path is not None and (ctx.is_decode or path == "tiles")
 
-    def _attend(self, qkv, x, ctx, kpages, vpages, block_table, fast_decode, fusion, writes):
+    def _attend(self, qkv, x, ctx, kpages, vpages, block_table, fast_decode, fusion, writes, unit=None):
         """The step's queries (the leading columns of `qkv`) over the cache -> [T, n_heads * v_dim]."""
         attn = torch.empty((x.shape[0], self.n_heads * self.v_dim), dtype=x.dtype, device=x.device)
         plain_widths = not self.other_widths and self.head_dim in PrefillAttentionTC.HEAD_DIMS
@@ -311,6 +312,14 @@ class Attention(Mixer):
             ctx.kernels.prefill_attention_tc.attn(qkv, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs,
                                                   ctx.max_new, self.n_heads, self.n_kv_heads, self.head_dim, self.span, self.scale,
                                                   ctx.err_flag, v_dim=self.v_dim, exact_weights=True)
+        elif self.other_widths and ctx.is_decode and ctx.kernels.attn_decode_split_takes(self.head_dim, qkv.stride(0), self.v_dim):
+            # keys split over blocks, read once for up to four of a group's heads (8 sequences of 16 heads, keys 64 and values 128, 500
+            # keys each: 12.9 us with the merge, 36.4 with a block a row and head)
+            n_split = ctx.kernels.attn_decode_splits(ctx.n_seqs, self.n_heads, self.n_kv_heads, ctx.pages_seen(unit), ctx.engine.sm_count)
+            part = torch.empty((ctx.n_seqs * self.n_heads * n_split * (self.v_dim + 2),), dtype=torch.float32,
+                               device=x.device) if n_split > 1 else None
+            ctx.kernels.attn_decode_split(qkv, attn, ctx.seq_pos0, block_table, kpages, vpages, part, ctx.n_seqs, self.n_heads,
+                                          self.n_kv_heads, self.head_dim, self.span, self.scale, n_split, v_dim=self.v_dim)
         elif self.other_widths:
             ctx.kernels.seq.attn_wide_value(qkv, attn, ctx.tok_pos, ctx.tok_seq, block_table, kpages, vpages, self.n_heads,
                                             self.n_kv_heads, self.head_dim, self.v_dim, self.span, self.scale)
@@ -420,7 +429,7 @@ class Attention(Mixer):
         else:
             fast_decode = (ctx.is_decode and x.dtype == torch.bfloat16 and self.head_dim in DecodeKernels.HEAD_DIMS
                            and not self.other_widths)
-            attn = self._attend(q, x, ctx, kpages, vpages, block_table, fast_decode, None, writes)
+            attn = self._attend(q, x, ctx, kpages, vpages, block_table, fast_decode, None, writes, unit)
             if gate is not None and self.gate_per == "element":
                 k.head_gate(attn, gate, self.n_heads * self.v_dim, 1)
         if gate is not None and self.gate_per == "head":
@@ -462,7 +471,7 @@ class Attention(Mixer):
             if fusion is None:
                 self._store(qkv, ctx, rotation, self.n_kv_heads if writes else 0, kpages if writes else None,
                             vpages if writes else None, block_table)
-        attn = self._attend(qkv, x, ctx, kpages, vpages, block_table, fast_decode, fusion, writes)
+        attn = self._attend(qkv, x, ctx, kpages, vpages, block_table, fast_decode, fusion, writes, unit)
         if fold is not None:
             return self.out.forward_folded(attn, ctx, fold=fold)
         return self.out.forward(attn, ctx, partials_ok=True)

@@ -161,3 +161,22 @@ def test_rows_of_a_tile_of_the_grouped_products(pairs, E, F, hidden, want):
     part = RoutedExperts(hidden, F, E, 1, 1, 1, 1.0, "r", "c", [f"u{j}" for j in range(E)], [f"d{j}" for j in range(E)], act="silu_glu",
                          gate_names=[f"g{j}" for j in range(E)])
     assert part._tile_rows(pairs) == want
+
+
+@pytest.mark.parametrize("D, V, decode, want", [(64, 128, True, "split"), (12, 20, True, "split"), (64, 126, True, "wide"), (64, 128, False, "wide"),
+                                                (80, 80, True, "paged"), (24, 24, True, "split")])
+def test_a_decode_step_of_unequal_widths_splits_its_keys(D, V, decode, want):
+    """Widths in multiples of four: keys split over blocks; others, and the few rows of a portion, a block a row and head."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    from scriptling_llm_lib_b200.parts.attention import Attention
+    ran, H, G = [], 8, 2
+    seen = lambda name: lambda *a, **k: ran.append(name)      # noqa: E731
+    layer = Attention(128, H, G, D, None, "q", "k", "v", "o", v_dim=V)
+    kernels = SimpleNamespace(attn_paged=seen("paged"), attn_decode_split=seen("split"), seq=SimpleNamespace(attn_wide_value=seen("wide")),
+                              attn_decode_split_takes=KernelSet.attn_decode_split_takes if D != 80 else lambda *a: False,
+                              attn_decode_splits=KernelSet.attn_decode_splits)
+    ctx = SimpleNamespace(is_decode=decode, from_start=False, max_new=1 if decode else 3, n_seqs=3, seq_pos0=None, seq_start=None, tok_pos=None,
+                          tok_seq=None, kernels=kernels, pages_seen=lambda unit: 9, engine=SimpleNamespace(sm_count=148))
+    x, kp = torch.empty((3, 128), dtype=torch.float32, device="meta"), torch.empty((9, G, 64, D), dtype=torch.float32, device="meta")
+    layer._attend(torch.empty((3, H * D + G * (D + V)), dtype=torch.float32, device="meta"), x, ctx, kp, kp, None, False, None, True, 0)
+    assert ran == [want]
