@@ -36,14 +36,17 @@
 // buffers, O); the two share the query/key/value fetches and the key/value ring, whose stage is
 // free when both have used it.
 //
-// Weights of 24 bits (PARTS = 3 of the pair kernel): for the layers that keep the softmax weights float32 into the product with
+// Weights of 24 bits (attn_prefill_exact_kernel): for the layers that keep the softmax weights float32 into the product with
 // the values. A float is exactly the sum of three bfloat16 numbers (its mantissa cut into 8 + 8 + 8 bits), so P goes into tensor
 // memory as three bfloat16 matrices of 32 columns and O takes three products a page; Q, K and V are bfloat16 as they are stored.
-// O's 128 columns and P's 96 leave no room for a second S in a tile's 256, so P takes the place of the S it was made from and the
-// next page's S is issued behind P V; the other tile of the pair fills the tensor cores meanwhile. Keys go up to 192 here.
-// Bound by the chain S -> softmax and splitting -> P V of a page. Prompts of 2,048 tokens, 16 heads: keys 64, values 128, window
-// 1,024 on 4 key/value heads 55.6 us (1,827 on the kernel with a warp a row and head, attn_wide_value, 22 -> 175 TFLOP/s on the
-// pairs seen); keys 192, values 128, every earlier key 71.5 us (1,189 on the float32 tiles of attn_paged, 18 -> 300 TFLOP/s).
+// One query tile a block, one block an SM, items dealt as for width 64: two S (128 columns), O (128) and two P (192) fit its 512
+// columns, so the scores of the next two pages are made while a page's softmax runs. Eight softmax warps: two threads a query row, each
+// with half of a page's keys and half of O's columns, that meet over the row's maximum in shared memory, so that the chain of a
+// page, which bounds narrow keys, is half as long. The products are issued by a whole warp through one elected lane: with the
+// loop in a branch of one lane each took 85 clocks to issue, here 61 to 64, their time on the tensor cores. Keys go up to 192 here.
+// Prompts of 2,048 tokens, 16 heads: keys 64, values 128, window 1,024 on 4 key/value heads 36.9 us (a page of two query tiles a block
+// with one S each, four softmax warps a tile: 52.5); keys 192, values 128, every earlier key 40.8 (70.8); 400 tokens behind 4,000
+// 24 and 73 (55 and 196); 48 tokens 6.6 (8.7). Scores read ahead of announcing P, or weights made while the maxima meet: 5% slower.
 #include "tcgen05.cuh"
 
 #define FT_BQ 128
@@ -61,8 +64,7 @@ struct FtArgs {
   float scale;
   int* err;
   int n_qt, n_seqs, n_items;   // query tiles per sequence (of the longest), sequences, work items
-  int pair_heads;              // pair kernel: 1: an item is heads 2i, 2i+1 on one query tile; 0: query tiles 2i, 2i+1 of one head; 2: tiles i and
-                               // n - 1 - i of one head
+  int pair_heads;              // pair kernel: 1: an item is heads 2i, 2i+1 on one query tile; 0: query tiles 2i, 2i+1 of one head
   float softcap;               // > 0: a score s (scaled) becomes softcap * tanh(s / softcap) before the softmax
   const float* sink;           // [H] or null: exp(sink[h]) joins head h's denominator, with no key and no value
   const bf16* gate;            // null, or [T, gate_ld]: output element (h, d) is multiplied by the sigmoid of column h * vd + d
@@ -508,11 +510,6 @@ __device__ __forceinline__ bool fp_item(const FtArgs& p, int round, FpItem& it) 
   it.pos0 = p.seq_pos0[it.b];
   it.seq_end = it.pos0 + S - 1;
   it.g = h0 / (p.H / p.G);
-  if (p.pair_heads == 2) {       // the sequence's tiles from both ends: the i-th with the i-th from the last
-    const int n = (S + FT_BQ - 1) / FT_BQ, i = rest / p.n_seqs;
-    qt0 = 2 * i < n ? i : p.n_qt;                // past the sequence's end: nothing to do
-    qt1 = 2 * i < n - 1 ? n - 1 - i : p.n_qt;    // the middle tile is alone
-  }
   fp_tile(p, it.sub[0], h0, qt0, S, it.pos0);
   fp_tile(p, it.sub[1], h1, qt1, S, it.pos0);
   it.valid = it.sub[0].valid;                      // the second tile of a pair is never valid without the first
@@ -590,9 +587,8 @@ __device__ __noinline__ void fp_sums_by_key(const FtArgs& p, const bf16* q, cons
   }
 }
 
-// Keys of up to KD and values of up to VD dims (with rounded weights 64 or 128 either, not both 64: that is the kernel above),
-// narrower heads as there. PARTS: 1 rounds the weights to bfloat16, 3 keeps all their bits.
-template <int KD, int VD, int FT_STAGES, int PARTS>
+// Keys of up to KD and values of up to VD dims (64 or 128 either, not both 64: that is the kernel above), narrower heads as there.
+template <int KD, int VD, int FT_STAGES>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FtArgs p, uint32_t smem_bytes) {
@@ -601,11 +597,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   constexpr int NK = KD / 64, NV = VD / 64;                    // such blocks per key (query) head and per value head
   // tensor-memory columns of one tile of the pair (256): values of 64 have S0 0-63, S1 64-127, O 128-191, P0 192-223,
   // P1 224-255; values of 128, whose O takes 128-255, have one S buffer 0-63 and P0 64-95, P1 96-127
-  constexpr int NBUF = VD > 64 || PARTS == 3 ? 1 : 2;   // S buffers; the next tile's S is issued while a tile's softmax runs
-  // (P in three parts: 0-95, over the S it was made from; O 128-255)
-  constexpr bool P_OVER_S = PARTS == 3;
-  constexpr uint32_t P_COL0 = P_OVER_S ? 0 : VD > 64 ? 64 : 192, P_STEP = P_OVER_S ? 0 : 32, SUB_COLS = 256;
-  static_assert(PARTS == 1 || PARTS == 3, "weights in one part or in three");
+  constexpr int NBUF = VD > 64 ? 1 : 2;   // S buffers; the next tile's S is issued while a tile's softmax runs
+  constexpr uint32_t P_COL0 = VD > 64 ? 64 : 192, P_STEP = 32, SUB_COLS = 256;
   static_assert(FT_STAGES >= 3, "the key/value ring must hold the tile whose S is issued ahead");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -714,8 +707,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               const int Jg = J0 + fp_place(sub, t), sb = Jg % NBUF;
               // S(Jg) takes the place of S(Jg - NBUF), which the softmax threads have taken into their registers: with
               // two buffers their P(Jg - 2) was waited for; the single buffer has a barrier for it
-              // (where P lies over S, this product is issued behind the one that read P)
-              if (NBUF == 1 && !P_OVER_S && !mbar_wait(b_sub + SUB_BARS * x + B_SEMPTY + 8 * sb, ((Jg / NBUF) & 1) ^ 1, abort)) return false;
+              if (NBUF == 1 && !mbar_wait(b_sub + SUB_BARS * x + B_SEMPTY + 8 * sb, ((Jg / NBUF) & 1) ^ 1, abort)) return false;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
               for (int k = 0; k < KD / 16; k++)         // 16 dims a step: four steps in each 64-wide block
@@ -729,7 +721,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
           };
           if (ok) ok = issue_s(0);
           for (int u = 0; u < n_union && ok; u++) {
-            if (!P_OVER_S && u + 1 < n_union) { ok = issue_s(u + 1); if (!ok) break; }
+            if (u + 1 < n_union) { ok = issue_s(u + 1); if (!ok) break; }
             const int JUg = JU0 + u, s = JUg % FT_STAGES, t = fp_union_tile(it, u);
             if (fp_active(sub, t)) {
               const int j = fp_place(sub, t), Jg = J0 + j, a = Jg & 1;
@@ -737,16 +729,13 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               if (!ok) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-              for (int part = 0; part < PARTS; part++)
-#pragma unroll
-                for (int k = 0; k < FT_BK / 16; k++)
-                  umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + part * 32 + k * 8,
-                               umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k | part) ? 1u : 0u);
+              for (int k = 0; k < FT_BK / 16; k++)
+                umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + k * 8,
+                             umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k) ? 1u : 0u);
               umma_commit(b_sub + SUB_BARS * x + B_OFULL + 8 * a);
             }
             if (!ok) break;
             umma_commit(b_kvempty + 8 * s);
-            if (P_OVER_S && u + 1 < n_union) ok = issue_s(u + 1);
           }
           JU0 += n_union;
           if (sub.valid) J0 += sub.n_tiles;
@@ -782,7 +771,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       ft_ld64(t_lane + bf * 64, s);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (NBUF == 1 && !P_OVER_S) {                // the one S buffer may take the next tile's scores
+      if (NBUF == 1) {                // the one S buffer may take the next tile's scores
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(b_sempty + 8 * bf);
@@ -821,39 +810,17 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       const float msc = (m_ref == -INFINITY) ? 0.f : m_ref * sc;
       uint64_t rs2 = 0ull;                          // two partial sums side by side
       const uint64_t sc2 = ft_pack2(sc, sc), nm2 = ft_pack2(-msc, -msc);
-      uint32_t pk[PARTS == 1 ? 32 : 1];             // 64 probabilities as bfloat16 pairs: keys 2i, 2i+1
-      if constexpr (PARTS == 1) {
+      uint32_t pk[32];                              // 64 probabilities as bfloat16 pairs: keys 2i, 2i+1
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float x0, x1, x2, x3;
-          ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nm2), x0, x1);
-          ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i + 2]), __uint_as_float(s[2 * i + 3])), sc2, nm2), x2, x3);
-          float e0 = ft_ex2(x0), e1 = ft_ex2(x1), e2 = ft_ex2(x2), e3 = ft_ex2(x3);
-          rs2 = ft_add2(rs2, ft_add2(ft_pack2(e0, e1), ft_pack2(e2, e3)));
-          __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
-          pk[i] = *(uint32_t*)&lo;
-          pk[i + 1] = *(uint32_t*)&hi;
-        }
-      } else {
-        // 32 keys at a time: their three parts go over the columns of S, which is in registers by now
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-          uint32_t p3[3][16];
-#pragma unroll
-          for (int i = 0; i < 16; i++) {
-            const int k0 = 32 * half + 2 * i;
-            float e0, e1;
-            ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[k0]), __uint_as_float(s[k0 + 1])), sc2, nm2), e0, e1);
-            e0 = ft_ex2(e0);
-            e1 = ft_ex2(e1);
-            rs2 = ft_add2(rs2, ft_pack2(e0, e1));
-            p3[0][i] = ft_cut_pair(e0, e1);
-            p3[1][i] = ft_cut_pair(e0, e1);
-            p3[2][i] = ft_cut_pair(e0, e1);
-          }
-#pragma unroll
-          for (int part = 0; part < 3; part++) tmem_st16(t_lane + part * 32 + half * 16, p3[part]);
-        }
+      for (int i = 0; i < 32; i += 2) {
+        float x0, x1, x2, x3;
+        ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nm2), x0, x1);
+        ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i + 2]), __uint_as_float(s[2 * i + 3])), sc2, nm2), x2, x3);
+        float e0 = ft_ex2(x0), e1 = ft_ex2(x1), e2 = ft_ex2(x2), e3 = ft_ex2(x3);
+        rs2 = ft_add2(rs2, ft_add2(ft_pack2(e0, e1), ft_pack2(e2, e3)));
+        __nv_bfloat162 lo = __floats2bfloat162_rn(e0, e1), hi = __floats2bfloat162_rn(e2, e3);
+        pk[i] = *(uint32_t*)&lo;
+        pk[i + 1] = *(uint32_t*)&hi;
       }
       {
         float ra, rb;
@@ -876,7 +843,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
       }
       // ---- P into tensor memory. The product that read this buffer's last P, two tiles ago, is complete:
       // it was issued before S(Jg), and the commit that announced S(Jg) covers every product issued before it.
-      if constexpr (PARTS == 1) tmem_st32(t_lane + P_COL0 + a * P_STEP, pk);
+      tmem_st32(t_lane + P_COL0 + a * P_STEP, pk);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -893,19 +860,6 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         uint32_t v[32];
         tmem_ld32(t_lane + 128 + c0, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if constexpr (PARTS == 3) {                 // (a sum l that is not finite has seen a score that is not)
-          float t = 0.f;
-#pragma unroll
-          for (int k = 0; k < 32; k++) t = fmaf(__uint_as_float(v[k]), 0.f, t);
-          if (r < sb.nq && t != 0.f && l < INFINITY && c0 < p.vd) {
-            float acc[32];
-            fp_sums_by_key(p, p.q + (size_t)(it.row0 + sb.r0 + r) * p.q_ld + (size_t)sb.h * p.hd, p.block_table + (size_t)it.b * p.max_pages, it.g,
-                           qpos, qfirst, m_ref == -INFINITY ? 0.f : m_ref * sc, c0, acc);
-#pragma unroll
-            for (int k = 0; k < 32; k++) v[k] = __float_as_uint(acc[k]);
-          }
-          __syncwarp();
-        }
         if (r < sb.nq) {
           if (p.gate != nullptr) ft_gate(v, p.gate + (size_t)(it.row0 + sb.r0 + r) * p.gate_ld + (size_t)sb.h * p.vd + c0, p.vd - c0);
 #pragma unroll
@@ -934,6 +888,336 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   if (threadIdx.x == 0 && *abort) atomicExch(p.err, 1000 * (int)blockIdx.x + *abort);
 }
 
+// ------------------------------------------------------------------ weights of 24 bits
+#define FE_THREADS 320       // warp 0: TMA, warp 1: the products, warps 2-9: softmax, two threads a query row
+
+// scores of keys the query at qpos does not see become -inf: 32 keys from k0 on
+__device__ __forceinline__ void fe_mask(uint32_t (&s)[32], int k0, int qpos, int qfirst, int keep) {
+  if (k0 + 31 <= qpos && (k0 >= qfirst || k0 + 32 <= keep)) return;
+#pragma unroll
+  for (int i = 0; i < 32; i++)
+    if (!key_seen(k0 + i, qpos, qfirst, keep)) s[i] = 0xff800000u;   // -inf
+}
+__device__ __forceinline__ float fe_rowmax(const uint32_t (&s)[32]) {
+  float m[4];
+#pragma unroll
+  for (int c = 0; c < 4; c++) m[c] = ft_max3(__uint_as_float(s[8 * c]), __uint_as_float(s[8 * c + 1]), __uint_as_float(s[8 * c + 2]));
+#pragma unroll
+  for (int i = 3; i < 7; i += 2)
+#pragma unroll
+    for (int c = 0; c < 4; c++) m[c] = ft_max3(m[c], __uint_as_float(s[8 * c + i]), __uint_as_float(s[8 * c + i + 1]));
+#pragma unroll
+  for (int c = 0; c < 4; c++) m[c] = fmaxf(m[c], __uint_as_float(s[8 * c + 7]));
+  return fmaxf(ft_max3(m[0], m[1], m[2]), m[3]);
+}
+
+// Keys of up to KD and values of up to VD dims, narrower heads as above; the weights enter the product with the values in three parts.
+template <int KD, int VD, int FT_STAGES>
+__global__ void __launch_bounds__(FE_THREADS, 1)
+attn_prefill_exact_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                          const __grid_constant__ CUtensorMap map_v, const __grid_constant__ FtArgs p, uint32_t smem_bytes) {
+  constexpr uint32_t Q_BYTES = FT_BQ * KD * 2, K_BYTES = FT_BK * KD * 2, V_BYTES = FT_BK * VD * 2;
+  constexpr uint32_t QA = FT_BQ * 128, KA = FT_BK * 128;       // bytes of one 64-wide block of Q and of a K or V page
+  constexpr int NK = KD / 64, NV = VD / 64;
+  // tensor-memory columns: S of either parity 0-63, 64-127; O 128-255; P of either parity 256-351, 352-447
+  constexpr uint32_t O_COL = 128, P_COL = 256, P_STEP = 96;
+  static_assert(FT_STAGES >= 4, "the key/value ring must hold the two tiles whose S is issued ahead, the one worked on, and one on its way");
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  // [Q][K stages][V stages][barriers][row maxima of either parity and half][row sums of either half]
+  const uint32_t sQ = smem_u32(smem), sK = sQ + Q_BYTES, sV = sK + FT_STAGES * K_BYTES;
+  uint64_t* bars = (uint64_t*)(smem + Q_BYTES + FT_STAGES * (K_BYTES + V_BYTES));
+  // q_full, q_empty, kv_full[ST], kv_empty[ST], s_full[2], p_full[2], o_full[2], max_full[4][2], sum_full[4]
+  const uint32_t b_qfull = smem_u32(bars), b_qempty = b_qfull + 8, b_kvfull = b_qempty + 8, b_kvempty = b_kvfull + 8 * FT_STAGES,
+                 b_sfull = b_kvempty + 8 * FT_STAGES, b_pfull = b_sfull + 16, b_ofull = b_pfull + 16, b_max = b_ofull + 16, b_sum = b_max + 64;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 + 2 * FT_STAGES + 18);
+  volatile int* abort = (volatile int*)(tmem_slot + 1);
+  volatile float* row_max = (volatile float*)(tmem_slot + 2);  // [parity][half][128]
+  volatile float* row_sum = row_max + 4 * FT_BQ;               // [half][128]
+  if ((uint8_t*)(row_sum + 2 * FT_BQ) > smem_raw + smem_bytes) {      // the 1 KB alignment took more than the launch left room for
+    if (threadIdx.x == 0) atomicExch(p.err, 3);
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    mbar_init(b_qfull, 1);
+    mbar_init(b_qempty, 1);
+    for (int s = 0; s < FT_STAGES; s++) { mbar_init(b_kvfull + 8 * s, 1); mbar_init(b_kvempty + 8 * s, 1); }
+    for (int a = 0; a < 2; a++) {
+      mbar_init(b_sfull + 8 * a, 1);
+      mbar_init(b_pfull + 8 * a, 8);
+      mbar_init(b_ofull + 8 * a, 1);
+    }
+    for (int a = 0; a < 8; a++) mbar_init(b_max + 8 * a, 2);
+    for (int a = 0; a < 4; a++) mbar_init(b_sum + 8 * a, 2);
+    *abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  // Every role walks the same items in the same order and counts the key tiles (J) and the items (I) by itself; a barrier's phase
+  // follows from those counts, so nothing is set up again between items.
+  if (warp == 0) {
+    if (lane == 0) {
+      int J = 0, I = 0;
+      FtItem it;
+      bool ok = true;
+      for (int round = 0; ok && ft_item(p, round, it); round++) {
+        if (!it.valid) continue;
+        const int* bt = p.block_table + (size_t)it.b * p.max_pages;
+        if (!mbar_wait(b_qempty, (I & 1) ^ 1, abort)) break;      // the products of the last item that read Q are done
+        mbar_expect_tx(b_qfull, Q_BYTES);
+#pragma unroll
+        for (int a = 0; a < NK; a++) tma_load_2d(sQ + a * QA, &map_q, it.h * p.hd + 64 * a, it.row0 + it.r0, b_qfull);
+        I++;
+        for (int j = 0; j < it.n_tiles; j++, J++) {
+          const int s = J % FT_STAGES;
+          if (!mbar_wait(b_kvempty + 8 * s, ((J / FT_STAGES) & 1) ^ 1, abort)) { ok = false; break; }
+          const int krow = (bt[ft_tile(it, j)] * p.G + it.g) * FT_BK;
+          mbar_expect_tx(b_kvfull + 8 * s, K_BYTES + V_BYTES);
+#pragma unroll
+          for (int a = 0; a < NK; a++) tma_load_2d(sK + s * K_BYTES + a * KA, &map_k, 64 * a, krow, b_kvfull + 8 * s);
+#pragma unroll
+          for (int a = 0; a < NV; a++) tma_load_2d(sV + s * V_BYTES + a * KA, &map_v, 64 * a, krow, b_kvfull + 8 * s);
+        }
+      }
+      if (*abort) {              // let the copies that are under way land before the block leaves
+        volatile int never = 0;
+        if (I > 0) mbar_wait(b_qfull, (I - 1) & 1, &never);
+        for (int j = max(0, J - FT_STAGES); j < J; j++) mbar_wait(b_kvfull + 8 * (j % FT_STAGES), (j / FT_STAGES) & 1, &never);
+      }
+    }
+  } else if (warp == 1) {
+    {
+      const bool one = elect_one();
+      constexpr uint32_t idesc_s = umma_idesc_bf16(FT_BQ, FT_BK);          // S = Q K^T: both K-major
+      constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(FT_BQ, VD);         // O = P V: V is MN-major (dims contiguous)
+      int J0 = 0, I = 0;
+      FtItem it;
+      bool ok = true;
+      for (int round = 0; ok && ft_item(p, round, it); round++) {
+        if (!it.valid) continue;
+        const int n = it.n_tiles;
+        ok = mbar_wait(b_qfull, I & 1, abort);
+        I++;
+        // S of a tile takes the place of S two tiles before, which the softmax threads had in their registers when they announced
+        // its P, and that was waited for
+        auto issue_s = [&](int j) -> bool {
+          const int Jg = J0 + j, s = Jg % FT_STAGES;
+          if (!mbar_wait(b_kvfull + 8 * s, (Jg / FT_STAGES) & 1, abort)) return false;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int k = 0; k < KD / 16; k++)         // 16 dims a step: four steps in each 64-wide block
+            if (16 * k < p.hd && one)
+              umma_bf16(tmem_base + (Jg & 1) * 64, umma_desc_sw128(sQ + (k >> 2) * QA + (k & 3) * 32),
+                        umma_desc_sw128(sK + s * K_BYTES + (k >> 2) * KA + (k & 3) * 32), idesc_s, k ? 1u : 0u);
+          if (one) umma_commit(b_sfull + 8 * (Jg & 1));
+          if (one && j == n - 1) umma_commit(b_qempty);    // the item's last products that read Q
+          return true;
+        };
+        if (ok) ok = issue_s(0);
+        if (ok && n > 1) ok = issue_s(1);
+        for (int j = 0; j < n && ok; j++) {
+          const int Jg = J0 + j, s = Jg % FT_STAGES, a = Jg & 1;
+          ok = mbar_wait(b_pfull + 8 * a, (Jg >> 1) & 1, abort);   // P of this tile is written, and O has been rescaled if it had to be
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int part = 0; part < 3; part++)
+#pragma unroll
+            for (int k = 0; k < FT_BK / 16; k++)
+              if (one) umma_bf16_ta(tmem_base + O_COL, tmem_base + P_COL + a * P_STEP + part * 32 + k * 8,
+                           umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k | part) ? 1u : 0u);
+          if (one) {
+            umma_commit(b_ofull + 8 * a);
+            umma_commit(b_kvempty + 8 * s);
+          }
+          __syncwarp();
+          if (j + 2 < n) ok = issue_s(j + 2);
+        }
+        J0 += n;
+      }
+    }
+  } else {
+    const int x = (warp - 2) >> 2;                 // which half of a tile's keys, and of O's columns
+    const int q = warp & 3;                        // tensor-memory quarter of this warp
+    const int r = q * 32 + lane;                   // query row of this thread (and of the one with the other half) in the tile
+    const float sc = p.scale * FT_LOG2E;
+    const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16);
+    int J0 = 0, I = 0;
+    FtItem it;
+    bool ok = true;
+    for (int round = 0; ok && ft_item(p, round, it); round++) {
+      if (!it.valid) continue;
+      const int n = it.n_tiles, seq_end = it.pos0 + p.seq_start[it.b + 1] - it.row0 - 1;
+      const int qpos = it.pos0 + it.r0 + r, qfirst = first_seen(qpos, p.window);
+      float m_ref = -INFINITY, l = 0.f;            // reference maximum (raw score units) and the sum of this half's keys relative to it
+#pragma unroll 1
+      for (int j = 0; j < n; j++) {
+        const int Jg = J0 + j, a = Jg & 1, t = ft_tile(it, j);
+        uint32_t s[32];
+        ok = mbar_wait(b_sfull + 8 * a, (Jg >> 1) & 1, abort);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_ld32(t_lane + a * 64 + x * 32, s);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (p.softcap > 0.f) {
+          const float cap_out = p.softcap / p.scale, cap_in = p.scale / p.softcap;
+#pragma unroll
+          for (int i = 0; i < 32; i++) s[i] = ft_cap(s[i], cap_out, cap_in);
+        }
+        fe_mask(s, t * FT_BK + x * 32, qpos, qfirst, p.keep);
+        // the row's maximum over both halves
+        float mx = fe_rowmax(s);
+        row_max[(a * 2 + x) * FT_BQ + r] = mx;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_max + 16 * q + 8 * a);
+        ok = mbar_wait(b_max + 16 * q + 8 * a, (Jg >> 1) & 1, abort);
+        if (!ok) break;
+        mx = fmaxf(mx, row_max[(a * 2 + (x ^ 1)) * FT_BQ + r]);
+        // ---- move the reference maximum only when the row's maximum has outgrown it by 2^8
+        const bool grow = mx > m_ref && (m_ref == -INFINITY || (mx - m_ref) * sc > 8.0f);
+        if (__any_sync(0xffffffffu, grow)) {       // (the same rows in the warp with the other half: it answers alike)
+          const float factor = grow ? ((m_ref == -INFINITY) ? 0.f : ft_ex2((m_ref - mx) * sc)) : 1.f;
+          if (j >= 1) {
+            // O holds the products of tiles 0..j-1: they must be complete before it is rewritten
+            ok = mbar_wait(b_ofull + 8 * (a ^ 1), ((Jg - 1) >> 1) & 1, abort);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t v[32];
+#pragma unroll 1
+            for (int c0 = x * (VD / 2); c0 < (x + 1) * (VD / 2); c0 += 32) {
+              tmem_ld32(t_lane + O_COL + c0, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
+              tmem_st32(t_lane + O_COL + c0, v);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          }
+          l *= factor;
+          if (grow) m_ref = mx;
+        }
+        const float msc = (m_ref == -INFINITY) ? 0.f : m_ref * sc;
+        uint64_t rs2 = 0ull;                        // two partial sums side by side
+        const uint64_t sc2 = ft_pack2(sc, sc), nm2 = ft_pack2(-msc, -msc);
+        uint32_t p3[3][16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          float e0, e1;
+          ft_unpack2(ft_fma2(ft_pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), sc2, nm2), e0, e1);
+          e0 = ft_ex2(e0);
+          e1 = ft_ex2(e1);
+          rs2 = ft_add2(rs2, ft_pack2(e0, e1));
+          p3[0][i] = ft_cut_pair(e0, e1);
+          p3[1][i] = ft_cut_pair(e0, e1);
+          p3[2][i] = ft_cut_pair(e0, e1);
+        }
+        // P into tensor memory. The product that read this buffer's last P, two tiles ago, is complete: it was issued before S(Jg),
+        // and the commit that announced S(Jg) covers every product issued before it.
+#pragma unroll
+        for (int part = 0; part < 3; part++) tmem_st16(t_lane + P_COL + a * P_STEP + part * 32 + x * 16, p3[part]);
+        {
+          float ra, rb;
+          ft_unpack2(rs2, ra, rb);
+          l += ra + rb;
+        }
+        if (t * FT_BK + FT_BK - 1 > seq_end) {
+          // keys of the sequence's last page beyond its last position hold whatever the page held before: their probabilities are
+          // zero, but 0 * NaN is NaN, so their value rows are cleared
+          const int st = Jg % FT_STAGES, n_valid = max(0, seq_end + 1 - t * FT_BK);
+          ok = mbar_wait(b_kvfull + 8 * st, (Jg / FT_STAGES) & 1, abort);
+          if (!ok) break;
+          for (int e = x * 128 + r; e < (FT_BK - n_valid) * 8 * NV; e += 256) {
+            const int blk = e / ((FT_BK - n_valid) * 8), e1 = e % ((FT_BK - n_valid) * 8), row = n_valid + e1 / 8, c = e1 % 8;
+            *(uint4*)(smem + Q_BYTES + FT_STAGES * K_BYTES + st * V_BYTES + blk * KA + row * 128 + ((c ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_pfull + 8 * a);
+      }
+      // the row's sum over both halves
+      if (ok) {
+        row_sum[x * FT_BQ + r] = l;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_sum + 8 * q);
+        ok = mbar_wait(b_sum + 8 * q, I & 1, abort) && mbar_wait(b_ofull + 8 * ((J0 + n - 1) & 1), ((J0 + n - 1) >> 1) & 1, abort);
+      }
+      I++;
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      l = row_sum[r] + row_sum[FT_BQ + r];
+      if (p.sink != nullptr) l = (m_ref == -INFINITY) ? 1.f : l + ft_ex2(p.sink[it.h] * FT_LOG2E - m_ref * sc);
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const size_t row = (size_t)(it.row0 + it.r0 + r);
+      bf16* dst = p.out + row * ((size_t)p.H * p.vd) + (size_t)it.h * p.vd;
+#pragma unroll 1
+      for (int c0 = x * (VD / 2); c0 < (x + 1) * (VD / 2); c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(t_lane + O_COL + c0, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float any = 0.f;                            // (a sum l that is not finite has seen a score that is not)
+#pragma unroll
+        for (int k = 0; k < 32; k++) any = fmaf(__uint_as_float(v[k]), 0.f, any);
+        if (r < it.nq && any != 0.f && l < INFINITY && c0 < p.vd) {
+          float acc[32];
+          fp_sums_by_key(p, p.q + row * p.q_ld + (size_t)it.h * p.hd, p.block_table + (size_t)it.b * p.max_pages, it.g, qpos, qfirst,
+                         m_ref == -INFINITY ? 0.f : m_ref * sc, c0, acc);
+#pragma unroll
+          for (int k = 0; k < 32; k++) v[k] = __float_as_uint(acc[k]);
+        }
+        __syncwarp();
+        if (r < it.nq) {
+          if (p.gate != nullptr) ft_gate(v, p.gate + row * p.gate_ld + (size_t)it.h * p.vd + c0, p.vd - c0);
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            uint4 w;
+            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(v[8 * c]) * inv, __uint_as_float(v[8 * c + 1]) * inv);
+            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(v[8 * c + 2]) * inv, __uint_as_float(v[8 * c + 3]) * inv);
+            __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(v[8 * c + 4]) * inv, __uint_as_float(v[8 * c + 5]) * inv);
+            __nv_bfloat162 p3b = __floats2bfloat162_rn(__uint_as_float(v[8 * c + 6]) * inv, __uint_as_float(v[8 * c + 7]) * inv);
+            w.x = *(uint32_t*)&p0; w.y = *(uint32_t*)&p1; w.z = *(uint32_t*)&p2; w.w = *(uint32_t*)&p3b;
+            if (c0 + 8 * c < p.vd) *(uint4*)(dst + c0 + 8 * c) = w;
+          }
+        }
+      }
+      // the rows of O are read (the loads above were waited for) before this thread signals the next item's first P
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      J0 += n;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+  if (threadIdx.x == 0 && *abort) atomicExch(p.err, 2);
+}
+
+template <int KD, int VD, int STAGES>
+static int fe_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FtArgs& a, dim3 grid, cudaStream_t stream) {
+  constexpr size_t need = FT_BQ * KD * 2 + STAGES * FT_BK * (KD + VD) * 2 + 512 + 6 * FT_BQ * 4, smem = need + 1024;
+  static_assert(smem <= 232448, "the block of this head width does not fit an SM");
+  static bool raised = false;
+  if (!raised) {
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_exact_kernel<KD, VD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    raised = true;
+  }
+  attn_prefill_exact_kernel<KD, VD, STAGES><<<grid, FE_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
+  SLLM_RETURN_LAST();
+}
+
 template <int HD, int STAGES>
 static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FtArgs& a, dim3 grid,
                      cudaStream_t stream) {
@@ -952,7 +1236,7 @@ static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   SLLM_RETURN_LAST();
 }
 
-template <int KD, int VD, int STAGES, int PARTS>
+template <int KD, int VD, int STAGES>
 static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FtArgs& a, dim3 grid,
                      cudaStream_t stream) {
   // what the kernel lays out after aligning to 1 KB; one block on an SM
@@ -962,11 +1246,11 @@ static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   static_assert(need <= smem, "the block of this head width does not fit an SM");
   static bool raised = false;
   if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<KD, VD, STAGES, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<KD, VD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     raised = true;
   }
-  attn_prefill_pair_kernel<KD, VD, STAGES, PARTS><<<grid, FP_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
+  attn_prefill_pair_kernel<KD, VD, STAGES><<<grid, FP_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
   SLLM_RETURN_LAST();
 }
 
@@ -1008,28 +1292,25 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
     dim3 grid((unsigned)(n_items < 2LL * sm_count ? n_items : 2LL * sm_count));     // two blocks per SM that stay
     return ft_launch<64, 3>(mq, mk, mv, a, grid, stream);
   }
-  // A head by itself whose items are one wave (float weights, every earlier key seen): the wave lasts as long as its longest item,
-  // and neighbouring tiles at a prompt's end make that twice the average. Tiles from both ends make all items alike, though they
-  // share fewer pages. 16 heads of 192 / 128, one prompt of 2,048 tokens 97.5 -> 71.5 us, 1,100 tokens 50.7 -> 43.8, 500 tokens
-  // 27.3 -> 23.7, two of 900 tokens 48.5 -> 38.0. At five tiles a head both take 27; at three (15.9, 17.2 from both ends) the last tile is
-  // better alone. With several waves (three prompts of 900 tokens) the next item fills the gap, and neighbours share more.
-  int pair_heads = ((H / G) % 2 == 0) ? 1 : 0;
-  if (!pair_heads && weight_parts == 3 && window == 0 && n_qt >= 4 && (long long)H * ((n_qt + 1) / 2) * B <= sm_count) pair_heads = 2;
+  if (weight_parts == 3) {
+    FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, 0, softcap, sink,
+             (const bf16*)gate, gate_ld, (const bf16*)q, (const bf16*)kpages, (const bf16*)vpages, q_ld};
+    dim3 grid((unsigned)(n_items < (long long)sm_count ? n_items : (long long)sm_count));       // one block per SM that stays
+    if (vd <= 64) {
+      if (hd <= 64) return fe_launch<64, 64, 6>(mq, mk, mv, a, grid, stream);
+      if (hd <= 128) return fe_launch<128, 64, 6>(mq, mk, mv, a, grid, stream);
+      return fe_launch<192, 64, 5>(mq, mk, mv, a, grid, stream);
+    }
+    if (hd <= 64) return fe_launch<64, 128, 6>(mq, mk, mv, a, grid, stream);
+    if (hd <= 128) return fe_launch<128, 128, 5>(mq, mk, mv, a, grid, stream);
+    return fe_launch<192, 128, 4>(mq, mk, mv, a, grid, stream);
+  }
+  const int pair_heads = ((H / G) % 2 == 0) ? 1 : 0;
   n_items = pair_heads == 1 ? (long long)(H / 2) * n_qt * B : (long long)H * ((n_qt + 1) / 2) * B;
   FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, pair_heads, softcap, sink,
            (const bf16*)gate, gate_ld, (const bf16*)q, (const bf16*)kpages, (const bf16*)vpages, q_ld};
   dim3 grid((unsigned)(n_items < (long long)sm_count ? n_items : (long long)sm_count));       // one block per SM that stays
-  if (weight_parts == 3) {
-    if (vd <= 64) {
-      if (hd <= 64) return fp_launch<64, 64, 5, 3>(mq, mk, mv, a, grid, stream);
-      if (hd <= 128) return fp_launch<128, 64, 5, 3>(mq, mk, mv, a, grid, stream);
-      return fp_launch<192, 64, 4, 3>(mq, mk, mv, a, grid, stream);
-    }
-    if (hd <= 64) return fp_launch<64, 128, 5, 3>(mq, mk, mv, a, grid, stream);
-    if (hd <= 128) return fp_launch<128, 128, 4, 3>(mq, mk, mv, a, grid, stream);
-    return fp_launch<192, 128, 3, 3>(mq, mk, mv, a, grid, stream);
-  }
-  if (vd <= 64) return fp_launch<128, 64, 5, 1>(mq, mk, mv, a, grid, stream);
-  if (hd <= 64) return fp_launch<64, 128, 5, 1>(mq, mk, mv, a, grid, stream);
-  return fp_launch<128, 128, 4, 1>(mq, mk, mv, a, grid, stream);
+  if (vd <= 64) return fp_launch<128, 64, 5>(mq, mk, mv, a, grid, stream);
+  if (hd <= 64) return fp_launch<64, 128, 5>(mq, mk, mv, a, grid, stream);
+  return fp_launch<128, 128, 4>(mq, mk, mv, a, grid, stream);
 }

@@ -697,6 +697,33 @@ def test_attn_prefill_tcgen05_with_float_weights(kernel_sets, kd, vd, H, G, wind
     assert rel_err(out.cpu().float(), torch.cat(want)) < 2.0 ** -8 + 2e-5
 
 
+@pytest.mark.parametrize("kd, vd, H, G, window", [(64, 128, 48, 6, 300), (192, 128, 40, 40, 0), (128, 64, 64, 8, -128)])
+def test_attn_prefill_with_float_weights_many_items(kernel_sets, kd, vd, H, G, window):
+    """More work items than blocks that stay: a block's rings, accumulators and maxima go on from one item to the next, among them items of
+    one key tile and of two. Rows at the tiles' edges against 64 bits, to the output's rounding and float sums below it."""
+    fa, err = kernel_sets[torch.bfloat16].prefill_attention_tc, torch.zeros(1, dtype=torch.int32, device="cuda")
+    lens, pos0, g = [900, 40, 129], [0, 0, 500], torch.Generator().manual_seed(kd)
+    draw = lambda *s: torch.randn(*s, generator=g).bfloat16().float()      # noqa: E731
+    held = [p + n for p, n in zip(pos0, lens)]
+    kk, vv, qs = [draw(n, G, kd) for n in held], [draw(n, G, vd) for n in held], [draw(n, H, kd) for n in lens]
+    kp, _, bt = paged(kk, kk, held, dtype=torch.bfloat16)
+    vp, _, _ = paged(vv, vv, held, dtype=torch.bfloat16)
+    q, out = dev(torch.cat([t.reshape(t.shape[0], -1) for t in qs]), torch.bfloat16), torch.full((sum(lens), H * vd), 7.0, dtype=torch.bfloat16, device="cuda")
+    fa.attn(q, out, dev(np.concatenate([[0], np.cumsum(lens)]), torch.int32), dev(pos0, torch.int32), bt, kp, vp, len(lens), max(lens), H, G, kd, window,
+            kd ** -0.5, err, v_dim=vd, exact_weights=True)
+    row0 = 0
+    for b, (n, p) in enumerate(zip(lens, pos0)):
+        rows = torch.tensor(sorted({0, 1, 39, 63, 64, 127, 128, 255, 256, 700, n - 1} & set(range(n))))
+        at, key = (p + rows)[:, None], torch.arange(p + n)[None, :]
+        first = torch.zeros_like(at) if window == 0 else at - window + 1 if window > 0 else at - at % -window
+        k, v = (f64(t).repeat_interleave(H // G, 1) for t in (kk[b], vv[b]))
+        sc = (torch.einsum("qhd,khd->hqk", f64(qs[b][rows]), k) * kd ** -0.5).masked_fill((key > at) | (key < first), -math.inf).softmax(-1)
+        want = torch.einsum("hqk,khd->qhd", sc, v).reshape(len(rows), -1)
+        assert rel_err(out[row0 + rows].cpu().float(), want) < 2.0 ** -8 + 2e-5
+        row0 += n
+    assert int(err) == 0
+
+
 @pytest.mark.parametrize("hd, H, G, window", [(64, 40, 40, None), (64, 24, 6, 700), (128, 24, 6, None), (128, 15, 15, None), (128, 9, 3, 900)])
 def test_attn_prefill_tcgen05_long_prompts_many_items(kernel_sets, hd, H, G, window):
     """Prompts of a few thousand tokens and more work items than resident blocks: every block walks several
