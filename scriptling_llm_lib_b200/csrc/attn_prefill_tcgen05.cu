@@ -261,7 +261,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(FT_BQ, FT_BK);          // S = Q K^T: both K-major
       constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(FT_BQ, FT_HD);      // O = P V: V is MN-major (dims contiguous)
       int J0 = 0, I = 0;
@@ -279,10 +280,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
           for (int k = 0; k < FT_HD / 16; k++)      // 16 dims a step: four steps in each 64-wide block
-            if (16 * k < p.hd) umma_bf16(tmem_base + a * 64, umma_desc_sw128(sQ + (k >> 2) * QA + (k & 3) * 32),
+            if (16 * k < p.hd && one) umma_bf16(tmem_base + a * 64, umma_desc_sw128(sQ + (k >> 2) * QA + (k & 3) * 32),
                       umma_desc_sw128(sK + s * KV_BYTES + (k >> 2) * KA + (k & 3) * 32), idesc_s, k ? 1u : 0u);
-          umma_commit(b_sfull + 8 * a);
-          if (j == n_tiles - 1) umma_commit(b_qempty);     // the item's last product that reads Q
+          if (one) umma_commit(b_sfull + 8 * a);
+          if (one && j == n_tiles - 1) umma_commit(b_qempty);     // the item's last product that reads Q
           return true;
         };
         if (ok) ok = issue_s(0);
@@ -294,10 +295,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
           for (int k = 0; k < FT_BK / 16; k++)
-            umma_bf16_ta(tmem_base + 128, tmem_base + P_COL0 + a * P_STEP + k * 8, umma_desc_sw128_mn(sV + s * KV_BYTES + k * 2048, NA > 1 ? KA : 0),
+            if (one) umma_bf16_ta(tmem_base + 128, tmem_base + P_COL0 + a * P_STEP + k * 8, umma_desc_sw128_mn(sV + s * KV_BYTES + k * 2048, NA > 1 ? KA : 0),
                          idesc_o, (j | k) ? 1u : 0u);
-          umma_commit(b_ofull + 8 * a);
-          umma_commit(b_kvempty + 8 * s);
+          if (one) {
+            umma_commit(b_ofull + 8 * a);
+            umma_commit(b_kvempty + 8 * s);
+          }
         }
         J0 += n_tiles;
       }
@@ -687,7 +690,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         }
       }
     } else if (warp <= 2) {
-      if (lane == 0) {
+      {
+        const bool one = elect_one();
         const int x = warp - 1;                    // this thread issues the products of one tile of the pair
         constexpr uint32_t idesc_s = umma_idesc_bf16(FT_BQ, FT_BK);          // S = Q K^T: both K-major
         constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(FT_BQ, VD);         // O = P V: V is MN-major (dims contiguous)
@@ -711,12 +715,12 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
               for (int k = 0; k < KD / 16; k++)         // 16 dims a step: four steps in each 64-wide block
-                if (16 * k < p.hd)
+                if (16 * k < p.hd && one)
                   umma_bf16(tmem_base + x * SUB_COLS + sb * 64, umma_desc_sw128(sQ + x * Q_BYTES + (k >> 2) * QA + (k & 3) * 32),
                             umma_desc_sw128(sK + s * K_BYTES + (k >> 2) * KA + (k & 3) * 32), idesc_s, k ? 1u : 0u);
-              umma_commit(b_sub + SUB_BARS * x + 8 * sb);
+              if (one) umma_commit(b_sub + SUB_BARS * x + 8 * sb);
             }
-            if (u == n_union - 1) umma_commit(b_qempty);     // the item's last products that read Q
+            if (one && u == n_union - 1) umma_commit(b_qempty);     // the item's last products that read Q
             return true;
           };
           if (ok) ok = issue_s(0);
@@ -730,12 +734,12 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
               for (int k = 0; k < FT_BK / 16; k++)
-                umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + k * 8,
+                if (one) umma_bf16_ta(tmem_base + x * SUB_COLS + 128, tmem_base + x * SUB_COLS + P_COL0 + a * P_STEP + k * 8,
                              umma_desc_sw128_mn(sV + s * V_BYTES + k * 2048, NV > 1 ? KA : 0), idesc_o, (j | k) ? 1u : 0u);
-              umma_commit(b_sub + SUB_BARS * x + B_OFULL + 8 * a);
+              if (one) umma_commit(b_sub + SUB_BARS * x + B_OFULL + 8 * a);
             }
             if (!ok) break;
-            umma_commit(b_kvempty + 8 * s);
+            if (one) umma_commit(b_kvempty + 8 * s);
           }
           JU0 += n_union;
           if (sub.valid) J0 += sub.n_tiles;

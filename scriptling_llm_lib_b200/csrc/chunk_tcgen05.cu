@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
   __syncthreads();
   put_silu(ka, kr, scale);
   u.ready();
-  if (tid == 0) {
+  if (tid < 32) {
     product<true, true>(u.tmem, smem_u32(ka), smem_u32(va), (n + 15) / 16);
     u.commit();
   }
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   put_floats(xa, p.chunk_state + ((first_chunk(start, b) + blockIdx.x) * p.hs + hl) * (size_t)p.D * p.V + v0, p.V, p.D, vn, p.vec);
   u.ready();
   const int dsteps = (p.D + 15) / 16, rsteps = (n + 15) / 16;
-  if (tid == 0) {
+  if (tid < 32) {
     product<false, true>(u.tmem, smem_u32(qa), smem_u32(xa), dsteps);
     u.commit();
   }
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   u.done();
   put_silu(xa, raw, nullptr);
   u.ready();
-  if (tid == 0) {
+  if (tid < 32) {
     product<false, false>(u.tmem + 128, smem_u32(qa), smem_u32(xa), dsteps);
     u.commit();
   }
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
     for (int q = 0; q < 3; q++) tmem_st16(t_lane + 128 + q * 64 + c0 / 2, part[q]);
   }
   u.ready();
-  if (tid == 0) {
+  if (tid < 32) {
     product_ta<true>(u.tmem + 320, u.tmem + 128, smem_u32(xa), rsteps);
     u.commit();
   }
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   put_rows<false, BY_ROW>(xa, f, nullptr, &watch);
   u.ready();
   const int dsteps = (p.dk + 15) / 16;
-  if (tid == 0) {
+  if (tid < 32) {
     product<false, false>(u.tmem, smem_u32(xa), smem_u32(xa), dsteps);
     u.commit();
   }
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   put_rows<false>(ya, f, nullptr);
   u.done();
   u.ready();
-  if (tid == 0) {
+  if (tid < 32) {
     product<false, false>(u.tmem + 128, smem_u32(ya), smem_u32(xa), dsteps);
     u.commit();
   }
@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   const size_t unit = (first_chunk(start, b) + blockIdx.x) * p.hs + blockIdx.y, mat = unit * MAT;
   put_rows<true, BY_COLUMN>(ya, f, beta, &watch);
   u.ready();
-  if (tid == 0) {                                  // U0
+  if (tid < 32) {                                  // U0
     product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
     u.commit();
   }
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   take(t_lane + 384 + c0, w);
   put_lane(ya, i, c0, w);
   u.ready();
-  if (tid == 0) {                                  // P U0
+  if (tid < 32) {                                  // P U0
     product_ta<true>(u.tmem + 384, u.tmem + 192, smem_u32(ya), 8);
     u.commit();
   }
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   u.done();
   take(t_lane + 384 + c0, w);
   u.ready();                                       // the sums have been read
-  if (tid == 0) {                                  // K'^T U0
+  if (tid < 32) {                                  // K'^T U0
     product<true, true>(u.tmem + 384, smem_u32(xa), smem_u32(ya), 8);
     u.commit();
   }
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   put_rows<true>(ya, f, bfront);
   take(t_lane + 384 + c0, w);
   u.ready();
-  if (tid == 0) {                                  // W
+  if (tid < 32) {                                  // W
     product_ta<true>(u.tmem + 384, u.tmem, smem_u32(ya), 8);
     u.commit();
   }
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   take(t_lane + 384 + c0, w);
   put_lane(ya, i, c0, w);
   u.ready();
-  if (tid == 0) {                                  // P W and K'^T W
+  if (tid < 32) {                                  // P W and K'^T W
     product_ta<true>(u.tmem + 384, u.tmem + 192, smem_u32(ya), 8);
     product<true, true>(u.tmem, smem_u32(xa), smem_u32(ya), 8);
     u.commit();
@@ -808,7 +808,8 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
       }
     }
     u.ready();
-    if (tid == 0) {
+    if (tid < 32) {
+      const bool one = elect_one();
       if (!mbar_wait(full + 8 * (c & 1), (c >> 1) & 1, u.abort)) u.ok = false;
       const uint32_t m = smem_u32(ma + (c & 1) * TILE_BYTES), s = smem_u32(sa);
 #pragma unroll
@@ -816,7 +817,7 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
         const uint32_t pa = m + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = s + (TERM_B >> 2 * t & 3) * ST_PLANE;
 #pragma unroll
         for (int k = 0; k < 8; k++)
-          umma_bf16(u.tmem, desc_cols(pa, k), umma_desc_sw128(pb + (k >> 2) * ST_BLOCK + (k & 3) * 32), id, (t | k) ? 1u : 0u);
+          if (one) umma_bf16(u.tmem, desc_cols(pa, k), umma_desc_sw128(pb + (k >> 2) * ST_BLOCK + (k & 3) * 32), id, (t | k) ? 1u : 0u);
       }
       u.commit();
     }
@@ -870,7 +871,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_out_kernel(DeltaArgs p) {
   put_quads(xa, fq);
   put_quads(ya, fs);
   u.ready();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     product<false, true>(u.tmem, smem_u32(xa), smem_u32(ya), (p.dk + 15) / 16);
     u.commit();
   }

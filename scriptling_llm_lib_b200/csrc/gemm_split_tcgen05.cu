@@ -152,7 +152,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
+      const bool one = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(GS_BM, BN);
       int it = 0;
       bool ok = true;
@@ -167,7 +168,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const uint32_t a_addr = smem_base + sa * SLOT_BYTES, b_addr = smem_base + sb * SLOT_BYTES + A_BYTES;
 #pragma unroll
             for (int k = 0; k < GS_BK / 16; k++)
-              umma_bf16_pair(acc, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (first && k == 0) ? 0u : 1u);
+              if (one) umma_bf16_pair(acc, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (first && k == 0) ? 0u : 1u);
           };
           ok = mbar_wait_cluster(acc_empty0 + 8 * a, ph ^ 1, abort)        // both blocks have taken this accumulator's last sums
                && mbar_wait(full0 + 8 * s2, ph, abort) && mbar_wait(full0 + 8 * s0, ph, abort);
@@ -175,17 +176,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           term(s2, s0, true);
           term(s0, s2, false);
-          umma_commit_pair(empty0 + 8 * s2);
+          if (one) umma_commit_pair(empty0 + 8 * s2);
           ok = mbar_wait(full0 + 8 * s1, ph, abort);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           term(s1, s1, false);
           term(s1, s0, false);
           term(s0, s1, false);
-          umma_commit_pair(empty0 + 8 * s1);
+          if (one) umma_commit_pair(empty0 + 8 * s1);
           term(s0, s0, false);
-          umma_commit_pair(empty0 + 8 * s0);
-          umma_commit_pair(acc_full0 + 8 * a);
+          if (one) {
+            umma_commit_pair(empty0 + 8 * s0);
+            umma_commit_pair(acc_full0 + 8 * a);
+          }
         }
       }
     }

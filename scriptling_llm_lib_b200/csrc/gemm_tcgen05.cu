@@ -448,7 +448,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
       int it = 0, i = 0;
       bool ok = true;
@@ -467,10 +468,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           uint32_t a_addr = smem_base + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
 #pragma unroll
           for (int k = 0; k < TC_BK / 16; k++)
-            umma_bf16(acc, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
-          umma_commit(empty0 + 8 * s);
+            if (one) umma_bf16(acc, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (kb | k) ? 1u : 0u);
+          if (one) umma_commit(empty0 + 8 * s);
         }
-        if (ok) umma_commit(acc_full0 + 8 * a);
+        if (ok && one) umma_commit(acc_full0 + 8 * a);
       }
     }
   } else {
@@ -790,7 +791,8 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       const uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
       bool ok = true;
       uint32_t ph = 0;
@@ -801,11 +803,11 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const uint32_t a_addr = smem_base + s * STAGE_BYTES, b_addr = a_addr + A_BYTES;
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; k++)
-          umma_bf16(tmem_base, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (it | k) ? 1u : 0u);
-        umma_commit(empty0 + 8 * s);
+          if (one) umma_bf16(tmem_base, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc, (it | k) ? 1u : 0u);
+        if (one) umma_commit(empty0 + 8 * s);
         if (++s == stages) { s = 0; ph ^= 1; }
       }
-      if (ok) umma_commit(acc_full);
+      if (ok && one) umma_commit(acc_full);
     }
   } else if (mbar_wait(acc_full, 0, abort)) {
     // every product has read its operands: the ring's space takes the sums, a row's columns together (rows 16 bytes apart modulo
@@ -1179,7 +1181,8 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       constexpr uint32_t idesc = umma_idesc_bf16(128, BT);
       bool ok = true;
       for (int it = 0; it < nkb; it++) {
@@ -1190,10 +1193,10 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         uint32_t w_addr = smem_base + s * STAGE_BYTES, x_addr = w_addr + W_BYTES;
 #pragma unroll
         for (int k = 0; k < TC_BK / 16; k++)
-          umma_bf16(tmem_base, umma_desc_sw128(w_addr + k * 32), umma_desc_sw128(x_addr + k * 32), idesc, (it | k) ? 1u : 0u);
-        umma_commit(empty0 + 8 * s);
+          if (one) umma_bf16(tmem_base, umma_desc_sw128(w_addr + k * 32), umma_desc_sw128(x_addr + k * 32), idesc, (it | k) ? 1u : 0u);
+        if (one) umma_commit(empty0 + 8 * s);
       }
-      if (ok) umma_commit(acc_full);
+      if (ok && one) umma_commit(acc_full);
     }
   } else {
     const int q = warp & 3;                      // the quarter of tensor memory this warp may read

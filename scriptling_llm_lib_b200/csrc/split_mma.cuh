@@ -47,36 +47,39 @@ __host__ __device__ constexpr uint32_t idesc(bool a_rows, bool b_rows) {
 }
 // planes of the six terms' factors, smallest term first, two bits each
 constexpr uint32_t TERM_A = 2u | 0u << 2 | 1u << 4 | 1u << 6 | 0u << 8 | 0u << 10, TERM_B = 0u | 2u << 2 | 1u << 4 | 0u << 6 | 1u << 8 | 0u << 10;
-// D = A B, `steps` of 16 deep, both operands tiles in shared memory; one thread issues it. The loops stay loops: these kernels run
-// through their code once a block, so code is fetched, not found.
+// D = A B, `steps` of 16 deep, both operands tiles in shared memory; a converged warp issues it through one lane (in a
+// branch of one lane a product of 48 steps took some 85 clocks a step to issue, not the 64 it takes). The loops stay loops: these kernels run through their code once a block, so code is fetched, not found.
 template <bool A_ROWS, bool B_ROWS>
 __device__ __forceinline__ void product(uint32_t tmem_d, uint32_t a, uint32_t b, int steps) {
   constexpr uint32_t id = idesc(A_ROWS, B_ROWS);
+  const bool one = elect_one();
 #pragma unroll 1
   for (int t = 0; t < 6; t++) {
     const uint32_t pa = a + (TERM_A >> 2 * t & 3) * PLANE_BYTES, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
 #pragma unroll 4
     for (int k = 0; k < steps; k++)
-      umma_bf16(tmem_d, A_ROWS ? desc_rows(pa, k) : desc_cols(pa, k), B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k), id, (t | k) ? 1u : 0u);
+      if (one) umma_bf16(tmem_d, A_ROWS ? desc_rows(pa, k) : desc_cols(pa, k), B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k), id, (t | k) ? 1u : 0u);
   }
 }
 // the same with A in tensor memory: three planes of 64 columns (two bfloat16 of K each)
 template <bool B_ROWS>
 __device__ __forceinline__ void product_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b, int steps) {
   constexpr uint32_t id = idesc(false, B_ROWS);
+  const bool one = elect_one();
 #pragma unroll 1
   for (int t = 0; t < 6; t++) {
     const uint32_t pa = tmem_a + (TERM_A >> 2 * t & 3) * 64, pb = b + (TERM_B >> 2 * t & 3) * PLANE_BYTES;
 #pragma unroll 4
     for (int k = 0; k < steps; k++)
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                   ::"r"(tmem_d), "r"(pa + k * 8), "l"(B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k)), "r"(id), "r"((t | k) ? 1u : 0u) : "memory");
+      if (one)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                     ::"r"(tmem_d), "r"(pa + k * 8), "l"(B_ROWS ? desc_rows(pb, k) : desc_cols(pb, k)), "r"(id), "r"((t | k) ? 1u : 0u) : "memory");
   }
 }
 
 // What every block of these kernels has: all of tensor memory, one barrier for the products it waits for, a flag of waits given
-// up. Products are issued by thread 0 between `ready()` (operands written by all threads are visible to the tensor cores) and
+// up. Products are issued by warp 0 between `ready()` (operands written by all threads are visible to the tensor cores) and
 // `commit()`; `done()` lets every thread wait for them.
 struct Unit {
   uint32_t tmem, bar, phase;
@@ -110,7 +113,9 @@ struct Unit {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
-  __device__ __forceinline__ void commit() { umma_commit(bar); }
+  __device__ __forceinline__ void commit() {    // by the warp that issued the products
+    if (elect_one()) umma_commit(bar);
+  }
   __device__ __forceinline__ void done() {      // a wait given up is remembered; the block walks on to its end and raises the flag
     if (!mbar_wait(bar, phase & 1, abort)) ok = false;
     phase++;
