@@ -223,6 +223,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;          // columns: S0 0-63, S1 64-127, O 128-191 (one column per dim), P0 192-223, P1 224-255
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
 
   // Every role walks the same items in the same order and counts tiles (J) and items (I) by itself; a
   // barrier's phase follows from those counts, so nothing is set up again between items.
@@ -646,6 +648,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
 
   // Every role walks the same items in the same order and counts by itself the key tiles fetched (JU),
   // the tiles its query tile of the pair has taken (J) and the items (I); a barrier's phase follows from
@@ -967,6 +971,8 @@ attn_prefill_exact_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
 
   // Every role walks the same items in the same order and counts the key tiles (J) and the items (I) by itself; a barrier's phase
   // follows from those counts, so nothing is set up again between items.
@@ -1218,8 +1224,7 @@ static int fe_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     if (e != cudaSuccess) return (int)e;
     raised = true;
   }
-  attn_prefill_exact_kernel<KD, VD, STAGES><<<grid, FE_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
-  SLLM_RETURN_LAST();
+  return (int)sllm_launch(attn_prefill_exact_kernel<KD, VD, STAGES>, grid, dim3(FE_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
 template <int HD, int STAGES>
@@ -1236,8 +1241,7 @@ static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     if (e != cudaSuccess) return (int)e;
     raised = true;
   }
-  attn_prefill_tc_kernel<HD, STAGES><<<grid, FT_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
-  SLLM_RETURN_LAST();
+  return (int)sllm_launch(attn_prefill_tc_kernel<HD, STAGES>, grid, dim3(FT_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
 template <int KD, int VD, int STAGES>
@@ -1254,8 +1258,7 @@ static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
     if (e != cudaSuccess) return (int)e;
     raised = true;
   }
-  attn_prefill_pair_kernel<KD, VD, STAGES><<<grid, FP_THREADS, smem, stream>>>(mq, mk, mv, a, (uint32_t)smem);
-  SLLM_RETURN_LAST();
+  return (int)sllm_launch(attn_prefill_pair_kernel<KD, VD, STAGES>, grid, dim3(FP_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
 // q: [T, q_ld] rotated queries (head h at columns h*hd); out: [T, H*vd]; kpages [n_pages][G][64][hd], vpages

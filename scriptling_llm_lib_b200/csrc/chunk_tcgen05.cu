@@ -183,6 +183,7 @@ __device__ __forceinline__ uint8_t* aligned_smem(uint8_t* raw) { return (uint8_t
 constexpr uint32_t LIN_SMEM = 2 * TILE_BYTES + 2 * (Q + 4) * 4 + 16 + 1024;
 
 __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
   if (r0 >= len) return;
@@ -199,6 +200,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
   fill_powers(pw, p.decay[h]);
   Unit u;
   u.open((uint8_t*)(scale + Q + 4));
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   if (tid < Q) scale[tid] = tid < n ? pw[n - 1 - tid] : 0.f;
   put_silu(va, vr, nullptr);
   __syncthreads();
@@ -223,6 +225,8 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_states_kernel(LinArgs p) {
 // a thread (4 where they come in fours).
 template <int E>
 __global__ void __launch_bounds__(256) chunk_lin_pass_kernel(LinArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int b = blockIdx.z, h = p.h0 + blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
   const int DV = p.D * p.V, e0 = (blockIdx.x * 256 + threadIdx.x) * E;
   if (e0 >= DV || len <= 0) return;
@@ -268,6 +272,7 @@ __global__ void __launch_bounds__(256) chunk_lin_pass_kernel(LinArgs p) {
 // Tensor memory: q S in columns 0-127; q k^T in 128-255, whose place (and 64 columns more) its decayed lower triangle takes in
 // three planes; that times v in 320-447.
 __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
   if (r0 >= len) return;
@@ -284,6 +289,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_lin_scan_kernel(LinArgs p) {
   open_watch(watch);
   Unit u;
   u.open((uint8_t*)(pw + 2 * (Q + 4)));
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   put_silu(qa, raw, nullptr);
   put_floats(xa, p.chunk_state + ((first_chunk(start, b) + blockIdx.x) * p.hs + hl) * (size_t)p.D * p.V + v0, p.V, p.D, vn, p.vec);
   u.ready();
@@ -549,6 +555,7 @@ __device__ __forceinline__ void merge_level(float* t) {
 // once T is done with, in 0-127). VEC: 16-byte accesses are allowed everywhere.
 template <bool VEC>
 __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
   if (r0 >= len) return;
@@ -568,6 +575,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
   open_watch(watch);
   Unit u;
   u.open((uint8_t*)(bfront + Q));
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   // a thread a row: the running sum of log2 d, in double; a decay of 0 is far below what a float can hold from one row to the next
   double c = 0.0;
   float bt = 0.f;
@@ -759,6 +767,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_parts_kernel(DeltaArgs p) {
 constexpr int PV = 32;
 constexpr uint32_t ST_BLOCK = PV * 128, ST_PLANE = 2 * ST_BLOCK, PASS_SMEM = 2 * TILE_BYTES + 3 * ST_PLANE + 32 + 1024;
 __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ma = aligned_smem(smem_raw);
   uint8_t* sa = ma + 2 * TILE_BYTES;
@@ -775,6 +784,7 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
   if (tid == 0) { mbar_init(full, 1); mbar_init(full + 8, 1); }
   Unit u;
   u.open(head);
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   auto fetch_m = [&](int c) {
     const uint32_t bar = full + 8 * (c & 1);
     mbar_expect_tx(bar, TILE_BYTES);
@@ -856,6 +866,7 @@ __global__ void __launch_bounds__(256, 1) chunk_delta_pass_kernel(DeltaArgs p) {
 
 template <bool VEC>
 __global__ void __launch_bounds__(NT, 1) chunk_delta_out_kernel(DeltaArgs p) {
+  pdl_wait();
   extern __shared__ uint8_t smem_raw[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.x * Q;
   if (r0 >= len) return;
@@ -868,6 +879,7 @@ __global__ void __launch_bounds__(NT, 1) chunk_delta_out_kernel(DeltaArgs p) {
   fetch_quads(fs, p.n + mat);
   Unit u;
   u.open(ya + TILE_BYTES);
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
   put_quads(xa, fq);
   put_quads(ya, fs);
   u.ready();
@@ -921,10 +933,10 @@ SLLM_EXPORT int sllm_chunk_lin_attn_bf16(const void* proj, int ld, int q_col, in
     const int hs = H - h0 < heads_held ? H - h0 : heads_held;
     chunked::LinArgs p{(const bf16*)proj, ld, q_col, k_col, v_col, decay, state, seq_start, slots, chunk_state, o, H, D, V, h0, hs, err, vec};
     const dim3 grid(chunks, hs * vblocks, n_seqs);
-    chunked::chunk_lin_states_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
-    if (vec) chunked::chunk_lin_pass_kernel<4><<<dim3((DV / 4 + 255) / 256, hs, n_seqs), 256, 0, stream>>>(p);
-    else chunked::chunk_lin_pass_kernel<1><<<dim3((DV + 255) / 256, hs, n_seqs), 256, 0, stream>>>(p);
-    chunked::chunk_lin_scan_kernel<<<grid, chunked::NT, chunked::LIN_SMEM, stream>>>(p);
+    sllm_launch(chunked::chunk_lin_states_kernel, grid, dim3(chunked::NT), chunked::LIN_SMEM, stream, p);
+    if (vec) sllm_launch(chunked::chunk_lin_pass_kernel<4>, dim3((DV / 4 + 255) / 256, hs, n_seqs), dim3(256), 0, stream, p);
+    else sllm_launch(chunked::chunk_lin_pass_kernel<1>, dim3((DV + 255) / 256, hs, n_seqs), dim3(256), 0, stream, p);
+    sllm_launch(chunked::chunk_lin_scan_kernel, grid, dim3(chunked::NT), chunked::LIN_SMEM, stream, p);
   }
   SLLM_RETURN_LAST();
 }
@@ -954,9 +966,9 @@ SLLM_EXPORT int sllm_chunk_delta(const float* qk, int ld_qk, const float* v, int
     DeltaArgs p{qk, ld_qk, v, ld_v, bd, state, seq_start, slots, (uint8_t*)scratch, mats, mats + units * MAT, mats + 2 * units * MAT, o, H, G, dk, dv,
                 h0, hs, err};
     const dim3 grid((max_new + Q - 1) / Q, hs, n_seqs);
-    parts<<<grid, NT, DELTA_SMEM, stream>>>(p);
-    chunk_delta_pass_kernel<<<dim3((dv + PV - 1) / PV, hs, n_seqs), 256, PASS_SMEM, stream>>>(p);
-    out<<<grid, NT, DELTA_SMEM, stream>>>(p);
+    sllm_launch(parts, grid, dim3(NT), DELTA_SMEM, stream, p);
+    sllm_launch(chunk_delta_pass_kernel, dim3((dv + PV - 1) / PV, hs, n_seqs), dim3(256), PASS_SMEM, stream, p);
+    sllm_launch(out, grid, dim3(NT), DELTA_SMEM, stream, p);
   }
   SLLM_RETURN_LAST();
 }

@@ -28,6 +28,8 @@
 // One operand's floats as three planes [3][rows][cols] of bfloat16, eight elements a thread; both operands in one launch (blockIdx.y).
 struct GsSplit { const float* src; bf16* dst; int rows, cols, ld; };
 __global__ void __launch_bounds__(256) gemm_split_planes_kernel(const GsSplit sa, const GsSplit sb) {
+  pdl_launch_dependents();
+  pdl_wait();
   const GsSplit s = blockIdx.y ? sb : sa;
   const int groups = s.cols >> 3;
   const long long total = (long long)s.rows * groups, plane = (long long)s.rows * s.cols;
@@ -114,6 +116,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   cluster_sync_all();                   // the other block's barriers are set up before anything arrives on them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();               // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -283,7 +287,7 @@ static int gs_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GsArgs&
   const long long tiles = (long long)((g.N + BN - 1) / BN) * ((g.M + GS_BM - 1) / GS_BM) * g.parts * g.batch;
   if (tiles > 0x7fffffffLL) return SLLM_ERR_ARG;
   const dim3 grid(2 * (int)(tiles < pairs ? tiles : pairs));
-  gemm_split_kernel<BN><<<grid, GS_THREADS, smem, stream>>>(ma, mb, g, err);
+  sllm_launch(gemm_split_kernel<BN>, grid, dim3(GS_THREADS), smem, stream, ma, mb, g, err);
   SLLM_RETURN_LAST();
 }
 
@@ -337,7 +341,7 @@ SLLM_EXPORT int sllm_gemm_split_f32(const float* A, const float* B, float* C, in
       if (m0 > 0) sb.rows = 0;
       const long long most = ((long long)(sa.rows) * sa.cols > (long long)sb.rows * K ? (long long)sa.rows * sa.cols : (long long)sb.rows * K) / 8;
       const long long blocks = (most + 255) / 256;
-      gemm_split_planes_kernel<<<dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 2), 256, 0, stream>>>(sa, sb);
+      sllm_launch(gemm_split_planes_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 2), dim3(256), 0, stream, sa, sb);
       const GsArgs g{A + m0 * lda, B + n0 * ldb, C + m0 * ldc + n0, m, n, K, lda, ldb, ldc, parts, batch, kb_part, c_part, batch * n};
       const int rc = gs_product(g, pa, pb, gs_tile_n(m, n, parts * batch), err, stream);
       if (rc) return rc;

@@ -403,8 +403,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES, acc_full0 = empty0 + 8 * STAGES, acc_empty0 = acc_full0 + 16;
 
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (fd.m_used) M = min(M, *fd.m_used);     // the same number for every thread of every block: all walk the same tiles
-  const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
   const int nkb = (K + TC_BK - 1) / TC_BK;
 
   if (threadIdx.x == 0) {
@@ -422,6 +420,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                   // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
+  if (fd.m_used) M = min(M, *fd.m_used);     // the same number for every thread of every block: all walk the same tiles
+  const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -515,8 +517,7 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C, int 
   }
   int n_tiles = ((N + BN - 1) / BN) * ((M + TC_BM - 1) / TC_BM);
   dim3 grid(n_tiles < sms ? n_tiles : sms);
-  gemm_tc_kernel<BN, STAGES, EPI><<<grid, TC_THREADS, smem, stream>>>(ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
-  SLLM_RETURN_LAST();
+  return (int)sllm_launch(gemm_tc_kernel<BN, STAGES, EPI>, grid, dim3(TC_THREADS), smem, stream, ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
 }
 
 // ------------------------------------------------------------------ two SMs on one tile
@@ -563,8 +564,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  if (fd.m_used) M = min(M, *fd.m_used);     // the same number for every thread of every block: all walk the same tiles
-  const int tiles_m = (M + TC2_BM - 1) / TC2_BM, tiles_n = (N + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
   const int nkb = (K + TC_BK - 1) / TC_BK;
   // A read of tensor memory waits behind the products already queued, some thousands of clocks
   // each time, so with few k-blocks to a tile four warps would take longer over a tile's epilogue
@@ -590,6 +589,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   cluster_sync_all();                   // the other block's barriers are set up before anything arrives on them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                   // (behind the allocation: a dependent's block must not take the columns first)
+  pdl_wait();
+  if (fd.m_used) M = min(M, *fd.m_used);     // the same number for every thread of every block: all walk the same tiles
+  const int tiles_m = (M + TC2_BM - 1) / TC2_BM, tiles_n = (N + BN - 1) / BN, n_tiles = tiles_m * tiles_n;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -706,8 +709,7 @@ static int tc_pair_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C,
   }
   int n_tiles = ((N + TC2_BN - 1) / TC2_BN) * ((M + TC2_BM - 1) / TC2_BM);
   dim3 grid(2 * (n_tiles < pairs ? n_tiles : pairs));
-  gemm_tc_pair_kernel<STAGES, EPI><<<grid, TC2_THREADS, smem, stream>>>(ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
-  SLLM_RETURN_LAST();
+  return (int)sllm_launch(gemm_tc_pair_kernel<STAGES, EPI>, grid, dim3(TC2_THREADS), smem, stream, ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
 }
 
 // whether the two-SM kernel takes a product: more than one block's rows and wide enough for its tile

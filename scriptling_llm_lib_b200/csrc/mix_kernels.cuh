@@ -420,6 +420,10 @@ template <typename A>
 __global__ void __launch_bounds__(512) gated_row_rms_vec_kernel(const float* __restrict__ o, const A* __restrict__ g, int ldg,
                                                                 const void* __restrict__ w, int w_f32, A* __restrict__ y, int W,
                                                                 float eps, int gate_act) {
+  pdl_launch_dependents();
+  pdl_wait();
+  o = pdl_after(o);
+  g = pdl_after(g);
   __shared__ float red[32];
   const int t = blockIdx.x, j = threadIdx.x * 8;
   const bool live = j < W;
@@ -453,6 +457,10 @@ __global__ void latent_store_kernel(A* __restrict__ q, int ldq, int H, int D, co
                                     const void* __restrict__ nw, int nw_f32, float eps, const float2* __restrict__ cos_sin,
                                     int rot, int half, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                                     const int* __restrict__ block_table, int max_pages, A* __restrict__ pages, int R, int P) {
+  pdl_launch_dependents();
+  pdl_wait();
+  q = pdl_after(q);
+  dkv = pdl_after(dkv);
   __shared__ float red[32];
   int t = blockIdx.x;
   int pos = tok_pos[t];
@@ -494,6 +502,9 @@ __global__ void latent_store_kernel(A* __restrict__ q, int ldq, int H, int D, co
 template <typename A>
 __global__ void latent_gather_kernel(const A* __restrict__ pages, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                                      const int* __restrict__ block_table, int max_pages, A* __restrict__ dense, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
+  pages = pdl_after(pages);
   int t = blockIdx.x;
   int pos = tok_pos[t];
   const A* src = pages + ((size_t)block_table[(size_t)tok_seq[t] * max_pages + pos / SLLM_PAGE] * SLLM_PAGE + pos % SLLM_PAGE) * W;
@@ -510,6 +521,11 @@ __global__ void latent_heads_kernel(const A* __restrict__ q, int ldq, const A* _
                                     const A* __restrict__ dense, int ldd, int R, const int* __restrict__ tok_pos,
                                     const int* __restrict__ tok_seq, const int* __restrict__ table, int max_pages,
                                     A* __restrict__ kt, A* __restrict__ vt, A* __restrict__ qt, int H, int D, int P, int V, int kw, int vw) {
+  pdl_launch_dependents();
+  pdl_wait();
+  q = pdl_after(q);
+  kv = pdl_after(kv);
+  dense = pdl_after(dense);
   int t = blockIdx.x, h = blockIdx.y;
   int pos = tok_pos[t];
   size_t at = ((size_t)table[(size_t)tok_seq[t] * max_pages + pos / SLLM_PAGE] * H + h) * SLLM_PAGE + pos % SLLM_PAGE;
@@ -530,6 +546,11 @@ __global__ void __launch_bounds__(256) latent_heads_vec_kernel(const A* __restri
                                                                const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                                                                const int* __restrict__ table, int max_pages, A* __restrict__ kt,
                                                                A* __restrict__ vt, A* __restrict__ qt, int H, int D, int P, int V) {
+  pdl_launch_dependents();
+  pdl_wait();
+  q = pdl_after(q);
+  kv = pdl_after(kv);
+  dense = pdl_after(dense);
   constexpr int E = 16 / sizeof(A);               // elements an access
   const int t = blockIdx.x, pos = tok_pos[t];
   const int kc = (D + P) / E, dc = D / E, vc = V / E;
@@ -1185,6 +1206,8 @@ __device__ __forceinline__ bool scan_aligned(const void* p, size_t row_bytes) { 
 
 template <typename A, int NP>
 __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_piece_kernel(ScanArgs p, ScanPieces w) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
   if (r0 >= len) return;
@@ -1239,6 +1262,8 @@ __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_piece_kernel(Sc
 
 // a thread a state of a channel: over the sequence's pieces in order, what a piece adds is replaced by the state in front of it
 __global__ void __launch_bounds__(256) selective_scan_carry_kernel(ScanArgs p, ScanPieces w) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int b = blockIdx.y, start = p.seq_start[b], len = p.seq_start[b + 1] - start;
   const size_t e = (size_t)blockIdx.x * 256 + threadIdx.x, all = (size_t)p.I * p.N;
   if (e >= all || len <= 0) return;
@@ -1267,6 +1292,8 @@ __global__ void __launch_bounds__(256) selective_scan_carry_kernel(ScanArgs p, S
 
 template <typename A, int NP>
 __global__ void __launch_bounds__(MIX_SCAN_BLOCK) selective_scan_write_kernel(ScanArgs p, ScanPieces w) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int b = blockIdx.z, start = p.seq_start[b], len = p.seq_start[b + 1] - start, r0 = blockIdx.y * w.R;
   if (r0 >= len) return;
@@ -1330,6 +1357,9 @@ __global__ void __launch_bounds__(32 * MIX_ROUTE_WARPS) moe_route_kernel(const f
                                                                          int corr_f32, int* __restrict__ idx,
                                                                          float* __restrict__ wgt, int T, int E, int n_groups,
                                                                          int keep, int top, float scale, int mode) {
+  pdl_launch_dependents();
+  pdl_wait();
+  z = pdl_after(z);
   extern __shared__ __align__(16) float sm[];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int t = blockIdx.x * MIX_ROUTE_WARPS + wid;
@@ -1519,6 +1549,9 @@ __device__ __forceinline__ int moe_peer_count(const int* cnt, int e, uint32_t ra
 __global__ void __cluster_dims__(MOE_GROUP_BLOCKS, 1, 1) __launch_bounds__(MOE_GROUP_THREADS)
 moe_group_kernel(const int* __restrict__ idx, int n_pairs, int* __restrict__ offsets, int* __restrict__ pair_of_row, int* __restrict__ row_of_pair,
                  int* __restrict__ tile_group, int n_tiles, int E, int pad) {
+  pdl_launch_dependents();
+  pdl_wait();
+  idx = pdl_after(idx);
   extern __shared__ int sm_group[];
   int* cnt = sm_group;                    // [E] this block's pairs
   int* next = cnt + E;                    // [E] where this block's next pair of an expert goes
@@ -1584,6 +1617,10 @@ moe_group_kernel(const int* __restrict__ idx, int n_pairs, int* __restrict__ off
 template <typename A>
 __global__ void moe_gather_rows_kernel(const A* __restrict__ h, int ldh, const int* __restrict__ row_of_pair, int top,
                                        A* __restrict__ xs, int K, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  h = pdl_after(h);
+  row_of_pair = pdl_after(row_of_pair);
   const A* src = h + (size_t)blockIdx.x * ldh;
   const int* rows = row_of_pair + (size_t)blockIdx.x * top;
   if (vec) {                                      // 16 bytes a thread: K * sizeof(A), ldh * sizeof(A) and both starts are multiples
@@ -1612,6 +1649,11 @@ __global__ void moe_combine_kernel(const float* __restrict__ ys, const int* __re
 // the same, four columns a thread (N a multiple of four); the choices are added in the same order, four choices' loads at a time
 __global__ void moe_combine_vec_kernel(const float* __restrict__ ys, const int* __restrict__ row_of_pair,
                                        const float* __restrict__ wgt, float* __restrict__ out, int top, int N) {
+  pdl_launch_dependents();
+  pdl_wait();
+  ys = pdl_after(ys);
+  row_of_pair = pdl_after(row_of_pair);
+  wgt = pdl_after(wgt);
   const int t = blockIdx.x;
   const int* rows = row_of_pair + (size_t)t * top;
   const float* ws = wgt + (size_t)t * top;

@@ -196,6 +196,8 @@ __global__ void causal_conv_vec_kernel(ConvArgs p) {
 // 16 rows with four on their way 22: it waits more than it saves).
 template <typename A, int TAPS, int ROWS, bool XF, bool YF>      // inputs, results: floats or of type A
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int HIST = TAPS - 1;
   const int t0 = blockIdx.x * ROWS, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= p.C) return;
@@ -269,6 +271,8 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(ConvArgs p, int T
 // After the convolution of a step: the state becomes the last taps - 1 inputs of [state | step's rows].
 template <typename A>
 __global__ void conv_state_update_kernel(ConvArgs p, int n_seqs) {
+  pdl_launch_dependents();
+  pdl_wait();
   int b = blockIdx.x;
   int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.C || b >= n_seqs) return;
@@ -293,6 +297,9 @@ __global__ void kv_store_kernel(A* __restrict__ qkv, int ld, const int* __restri
                                 const int* __restrict__ block_table, int max_pages, const float2* __restrict__ cs,
                                 A* __restrict__ kpages, A* __restrict__ vpages, int H, int G, int hd, int vd, int rot,
                                 int interleaved, float v_eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  qkv = pdl_after(qkv);
   int t = blockIdx.x;
   int pos = tok_pos[t];
   int half = rot >> 1;
@@ -482,6 +489,10 @@ template <typename A>
 __global__ void delta_prepare_kernel(float* __restrict__ qk, int ld_qk, const float* __restrict__ ba, int ld_ba,
                                      const void* __restrict__ a_log, const void* __restrict__ dt_bias, int w_f32,
                                      float* __restrict__ bd, int H, int G, int dk, int vec) {
+  pdl_launch_dependents();
+  pdl_wait();
+  qk = pdl_after(qk);
+  ba = pdl_after(ba);
   int t = blockIdx.x;
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float qmult = rsqrtf((float)dk);
@@ -735,6 +746,10 @@ __global__ void __launch_bounds__(DR_THREADS + 32) delta_rule_kernel(const float
 template <typename A>
 __global__ void gated_unit_rms_kernel(const float* __restrict__ o, const A* __restrict__ gate, int ld_gate,
                                       const void* __restrict__ w, int w_f32, A* __restrict__ y, int T, int H, int dv, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  o = pdl_after(o);
+  gate = pdl_after(gate);
   int lane = threadIdx.x & 31;
   size_t idx = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (idx >= (size_t)T * H) return;
@@ -756,6 +771,10 @@ template <typename A>
 __global__ void __launch_bounds__(128) gated_unit_rms_vec_kernel(const float* __restrict__ o, const A* __restrict__ gate, int ld_gate,
                                                                  const void* __restrict__ w, int w_f32, A* __restrict__ y, int T, int H, int dv,
                                                                  float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  o = pdl_after(o);
+  gate = pdl_after(gate);
   const int j = (threadIdx.x & 31) * 4;
   const size_t i = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= (size_t)T * H) return;
@@ -835,6 +854,8 @@ __global__ void rglru_scan_kernel(LruArgs p) {
 #define LRU_ROWS 4
 template <typename A>
 __global__ void rglru_piece_kernel(LruArgs p, float* __restrict__ prod, float* __restrict__ end, int pieces) {
+  pdl_launch_dependents();
+  pdl_wait();
   int b = blockIdx.x / pieces, k = blockIdx.x % pieces;
   int c = blockIdx.y * blockDim.x + threadIdx.x;
   int t0 = p.seq_start[b] + k * LRU_PIECE, t1 = min(p.seq_start[b + 1], t0 + LRU_PIECE);
@@ -867,6 +888,10 @@ __global__ void rglru_piece_kernel(LruArgs p, float* __restrict__ prod, float* _
 }
 
 __global__ void rglru_carry_kernel(LruArgs p, const float* __restrict__ prod, float* __restrict__ end, int pieces) {
+  pdl_launch_dependents();
+  pdl_wait();
+  prod = pdl_after(prod);
+  end = pdl_after(end);
   int b = blockIdx.x;
   int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= p.W) return;
@@ -896,6 +921,9 @@ __global__ void rglru_carry_kernel(LruArgs p, const float* __restrict__ prod, fl
 
 template <typename A>
 __global__ void rglru_write_kernel(LruArgs p, const float* __restrict__ start, int pieces) {
+  pdl_launch_dependents();
+  pdl_wait();
+  start = pdl_after(start);
   int b = blockIdx.x / pieces, k = blockIdx.x % pieces;
   int c = blockIdx.y * blockDim.x + threadIdx.x;
   int t0 = p.seq_start[b] + k * LRU_PIECE, t1 = min(p.seq_start[b + 1], t0 + LRU_PIECE);
