@@ -96,7 +96,7 @@ class KernelSet:
             raise KernelError(f"embed_rows: a copy of {tuple(copy.shape)} for rows of {(T, d)}")
         _check(self._fn("embed_rows")(_ptr(ids, torch.int32, "ids"), _ptr(table, self.dtype, "table"),
                                       _ptr(out, torch.float32, "out"), _ptr(copy, torch.float32, "copy"), c_float(scale),
-                                      c_int(T), c_int(d), c_int(table.shape[0]), _ptr(err_flag, torch.int32, "err"), _stream()), "embed_rows")
+                                      T, d, table.shape[0], _ptr(err_flag, torch.int32, "err"), _stream()), "embed_rows")
 
     def embed_pair_rows(self, ids, ctx, table, pair_table, buckets, mul_prev, mul_cur, last, out, err_flag, scale=1.0, copy=None):
         """out float32 [T, d] = scale * table[ids[t]] + pair_table[(previous token * mul_prev + ids[t] * mul_cur) mod buckets], the
@@ -110,7 +110,7 @@ class KernelSet:
                                            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                                            _ptr(ctx.slots, torch.int32, "slots"), _ptr(table, self.dtype, "table"),
                                            _ptr(pair_table, self.dtype, "pair_table"), _ptr(out, torch.float32, "out"),
-                                           _ptr(copy, torch.float32, "copy"), c_float(scale), c_int(T), c_int(d), c_int(table.shape[0]), c_int(buckets), c_longlong(mul_prev), c_longlong(mul_cur),
+                                           _ptr(copy, torch.float32, "copy"), c_float(scale), T, d, table.shape[0], buckets, c_longlong(mul_prev), c_longlong(mul_cur),
                                            _ptr(last, torch.int32, "last"), _ptr(err_flag, torch.int32, "err"), _stream()),
                "embed_pair_rows")
 
@@ -123,8 +123,8 @@ class KernelSet:
             raise KernelError(f"embed_rows_sinusoid: tables {tuple(coarse.shape)}, {tuple(fine.shape)} for rows of {d}")
         _check(self._fn("embed_rows_sinusoid")(_ptr(ids, torch.int32, "ids"), _ptr(tok_pos, torch.int32, "tok_pos"),
                                                _ptr(table, self.dtype, "table"), _ptr(coarse, torch.float32, "coarse"),
-                                               _ptr(fine, torch.float32, "fine"), _ptr(out, torch.float32, "out"), c_int(T), c_int(d),
-                                               c_int(table.shape[0]), c_int(coarse.shape[0]), _ptr(err_flag, torch.int32, "err"),
+                                               _ptr(fine, torch.float32, "fine"), _ptr(out, torch.float32, "out"), T, d,
+                                               table.shape[0], coarse.shape[0], _ptr(err_flag, torch.int32, "err"),
                                                _stream()), "embed_rows_sinusoid")
 
     # ------------------------------------------------------------------ norm
@@ -142,10 +142,10 @@ class KernelSet:
             n_parts, stride = delta.shape[0], x.shape[0] * d
         elif delta is not None and (delta.dtype != self.dtype or tuple(delta.shape) != tuple(x.shape)):
             raise KernelError(f"addend must be {self.dtype} {tuple(x.shape)}, found {delta.dtype} {tuple(delta.shape)}")
-        _check(self._fn("add_rmsnorm")(_ptr(x, torch.float32, "x"), _ptr(delta, None, "delta"), c_int(n_parts),
+        _check(self._fn("add_rmsnorm")(_ptr(x, torch.float32, "x"), _ptr(delta, None, "delta"), n_parts,
                                        c_longlong(stride), _ptr(rows, torch.int32, "rows"), _ptr(weight, None, "weight"),
-                                       c_int(1 if weight.dtype == torch.float32 else 0), _ptr(y, self.dtype, "y"),
-                                       c_int(n), c_int(d), c_float(eps), _stream()), "add_rmsnorm")
+                                       1 if weight.dtype == torch.float32 else 0, _ptr(y, self.dtype, "y"),
+                                       n, d, c_float(eps), _stream()), "add_rmsnorm")
 
     # ------------------------------------------------------------------ matrix products
     def gemm_nt(self, a, w, out):
@@ -160,9 +160,9 @@ class KernelSet:
         if a.dtype != self.dtype or not a.is_cuda or a.stride(1) != 1:
             raise KernelError(f"gemm_nt: a must be {self.dtype} on a CUDA device with unit column stride")
         _check(self._fn("gemm_nt")(c_void_p(a.data_ptr()), _ptr(w, self.dtype, "w"),
-                                   _ptr(out, torch.float32 if out_f32 else self.dtype, "out"), c_int(M), c_int(N),
-                                   c_int(K), c_int(a.stride(0)), c_int(w.stride(0)), c_int(N), c_int(out_f32),
-                                   c_int(ksplit), _stream()), "gemm_nt")
+                                   _ptr(out, torch.float32 if out_f32 else self.dtype, "out"), M, N,
+                                   K, a.stride(0), w.stride(0), N, out_f32,
+                                   ksplit, _stream()), "gemm_nt")
 
     def gemm_nt_blocks_take(self, a, w) -> bool:
         """Whether `gemm_nt_blocks` runs these as one launch: the 32-bit set, more than 64 rows, 16-byte aligned pieces."""
@@ -176,9 +176,9 @@ class KernelSet:
         M = a.shape[0]
         if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or a.dtype != self.dtype or not a.is_cuda or a.stride(1) != 1:
             raise KernelError(f"gemm_nt_blocks: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)}")
-        _check(self._fn("gemm_nt_batched")(c_void_p(a.data_ptr()), _ptr(w, self.dtype, "w"), _ptr(out, self.dtype, "out"), c_int(M), c_int(N),
-                                           c_int(K), c_int(a.stride(0)), c_int(K), c_int(N), c_longlong(K), c_longlong(N * K),
-                                           c_longlong(M * N), c_int(nb), _stream()), "gemm_nt_batched")
+        _check(self._fn("gemm_nt_batched")(c_void_p(a.data_ptr()), _ptr(w, self.dtype, "w"), _ptr(out, self.dtype, "out"), M, N,
+                                           K, a.stride(0), K, N, c_longlong(K), c_longlong(N * K),
+                                           c_longlong(M * N), nb, _stream()), "gemm_nt_batched")
 
     @staticmethod
     def gemm_nt_split(m: int, n_out: int, k: int, sm_count: int) -> int:
@@ -196,14 +196,14 @@ class KernelSet:
     def rope_kv_write(self, qkv, tok_pos, tok_seq, block_table, cos_sin, kpages, vpages, n_heads, n_kv, head_dim, rot,
                       interleaved):
         T, ld = qkv.shape
-        _check(self._fn("rope_kv_write")(_ptr(qkv, self.dtype, "qkv"), c_int(ld), _ptr(tok_pos, torch.int32, "tok_pos"),
+        _check(self._fn("rope_kv_write")(_ptr(qkv, self.dtype, "qkv"), ld, _ptr(tok_pos, torch.int32, "tok_pos"),
                                          _ptr(tok_seq, torch.int32, "tok_seq"),
-                                         _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
+                                         _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
                                          _ptr(cos_sin, torch.float32, "cos_sin"),
                                          _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-                                         _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c_int(T),
-                                         c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(rot),
-                                         c_int(1 if interleaved else 0), _stream()), "rope_kv_write")
+                                         _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T,
+                                         n_heads, n_kv, head_dim, rot,
+                                         (1 if interleaved else 0), _stream()), "rope_kv_write")
 
     # ------------------------------------------------------------------ attention
     def attn_paged(self, q, out, seq_start, seq_pos0, block_table, kpages, vpages, n_seqs, max_new, n_heads, n_kv,
@@ -211,12 +211,12 @@ class KernelSet:
         """`softcap`: a score s becomes softcap * tanh(s / softcap) before the softmax; `sink` float32 [n_heads]:
         exp(sink[h]) joins head h's denominator with no key and no value. `v_dim`: the values' width where it is not
         the keys'; `keep`: the first positions of a sequence that stay visible behind the window."""
-        _check(self._fn("attn_paged")(_ptr(q, self.dtype, "q"), c_int(q.shape[1]), _ptr(out, self.dtype, "out"),
+        _check(self._fn("attn_paged")(_ptr(q, self.dtype, "q"), q.shape[1], _ptr(out, self.dtype, "out"),
                                       _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
-                                      _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
+                                      _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
                                       _ptr(kpages, self.dtype, "kpages"), _ptr(vpages, self.dtype, "vpages"),
-                                      c_int(n_seqs), c_int(max_new), c_int(n_heads), c_int(n_kv), c_int(head_dim),
-                                      c_int(v_dim or head_dim), c_int(window or 0), c_int(keep), c_float(scale),
+                                      n_seqs, max_new, n_heads, n_kv, head_dim,
+                                      (v_dim or head_dim), (window or 0), keep, c_float(scale),
                                       c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()), "attn_paged")
 
     def attn_decode_split(self, q, out, seq_pos0, block_table, kpages, vpages, part, n_seqs, n_heads, n_kv, head_dim,
@@ -229,13 +229,13 @@ class KernelSet:
         if need and (part is None or part.numel() < need):
             raise KernelError(f"attn_decode_split scratch holds {0 if part is None else part.numel()} floats, needs {need}")
         _check(self._fn("attn_decode_split")(_ptr(q, self.dtype, "q") if q.is_contiguous() else c_void_p(q.data_ptr()),
-                                             c_int(q.stride(0)), _ptr(out, self.dtype, "out"),
+                                             q.stride(0), _ptr(out, self.dtype, "out"),
                                              _ptr(seq_pos0, torch.int32, "seq_pos0"),
-                                             _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
+                                             _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
                                              _ptr(kpages, self.dtype, "kpages"), _ptr(vpages, self.dtype, "vpages"),
-                                             _ptr(part, torch.float32, "part"), c_int(n_seqs), c_int(n_heads), c_int(n_kv),
-                                             c_int(head_dim), c_int(v_dim), c_int(window or 0), c_int(keep), c_float(scale),
-                                             c_int(n_split), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()),
+                                             _ptr(part, torch.float32, "part"), n_seqs, n_heads, n_kv,
+                                             head_dim, v_dim, (window or 0), keep, c_float(scale),
+                                             n_split, c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()),
                "attn_decode_split")
 
     @staticmethod
@@ -256,8 +256,8 @@ class KernelSet:
         T, F = out.shape
         if tuple(gate_up.shape) != (T, 2 * F):
             raise KernelError(f"swiglu shapes: gate_up {tuple(gate_up.shape)}, out {tuple(out.shape)}")
-        _check(self._fn("swiglu")(_ptr(gate_up, self.dtype, "gate_up"), _ptr(out, self.dtype, "out"), c_int(T), c_int(F),
-                                  c_int(1 if tiled else 0), _stream()), "swiglu")
+        _check(self._fn("swiglu")(_ptr(gate_up, self.dtype, "gate_up"), _ptr(out, self.dtype, "out"), T, F,
+                                  (1 if tiled else 0), _stream()), "swiglu")
 
     @property
     def split(self) -> "SplitGemm":
@@ -360,8 +360,8 @@ class SplitGemm:
     def _run(self, a, w, out, M, N, K, ldb, parts, batch, apart, err_flag):
         scratch = torch.empty((min(6 * K * batch * (M + N), self.SCRATCH_BYTES),), dtype=torch.uint8, device=a.device)
         _check(self.lib.sllm_gemm_split_f32(
-            c_void_p(a.data_ptr()), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), c_int(M), c_int(N), c_int(K),
-            c_int(a.stride(0)), c_int(ldb), c_int(N), c_int(parts), c_int(batch), c_longlong(apart), _ptr(scratch),
+            c_void_p(a.data_ptr()), _ptr(w, torch.float32, "w"), _ptr(out, torch.float32, "out"), M, N, K,
+            a.stride(0), ldb, N, parts, batch, c_longlong(apart), _ptr(scratch),
             c_longlong(scratch.numel()), _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_split")
 
     def gemm(self, a, w, out, err_flag):
@@ -399,11 +399,11 @@ class TensorCoreGemm:
     @staticmethod
     def _owed_args(owed, M):
         if owed is None:
-            return c_void_p(None), c_int(0), c_int(0), c_float(0.0)
+            return c_void_p(None), 0, 0, c_float(0.0)
         sq, width, eps = owed
         if sq.dtype != torch.float32 or sq.dim() != 2 or sq.shape[1] != M or not sq.is_contiguous():
             raise KernelError(f"sums of squares {tuple(sq.shape)} {sq.dtype} for {M} rows")
-        return _ptr(sq, torch.float32, "sumsq"), c_int(sq.shape[0]), c_int(width), c_float(eps)
+        return _ptr(sq, torch.float32, "sumsq"), sq.shape[0], width, c_float(eps)
 
     FOLD_SPAN = 128      # columns to a partial sum of squares that a folded product leaves
     FOLD_MIN_M = 129     # the product that finishes a sublayer for a folded norm runs on the two-SM tiles only
@@ -428,8 +428,8 @@ class TensorCoreGemm:
                 raise KernelError(f"gemm_tc fold: residual {tuple(out.shape)} {out.dtype}, norm weight {tuple(norm_w.shape)}, "
                                   f"xb {tuple(xb.shape)}, sums {tuple(sq_out.shape)} for M={M}, N={N}")
             _check(self.lib.sllm_gemm_tc_fold_bf16(
-                c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M), c_int(N), c_int(K),
-                c_int(a.stride(0)), c_int(w.stride(0)), c_int(out.stride(0)), c_int(1), c_int(2), *self._owed_args(owed, M),
+                c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), M, N, K,
+                a.stride(0), w.stride(0), out.stride(0), 1, 2, *self._owed_args(owed, M),
                 _ptr(norm_w, torch.float32, "norm_w"), _ptr(xb, torch.bfloat16, "xb"), _ptr(sq_out, torch.float32, "sumsq_out"),
                 _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_tc")
             return
@@ -441,9 +441,9 @@ class TensorCoreGemm:
         if not (a.is_cuda and w.is_cuda and out.is_cuda):
             raise KernelError("gemm_tc runs on a CUDA device only")
         _check(self.lib.sllm_gemm_tc_fold_bf16(
-            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M), c_int(N), c_int(K),
-            c_int(a.stride(0)), c_int(w.stride(0)), c_int(out.stride(0)), c_int(1 if out.dtype == torch.float32 else 0),
-            c_int(1 if swiglu else 0), *self._owed_args(owed, M), c_void_p(None), c_void_p(None), c_void_p(None),
+            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), M, N, K,
+            a.stride(0), w.stride(0), out.stride(0), 1 if out.dtype == torch.float32 else 0,
+            (1 if swiglu else 0), *self._owed_args(owed, M), c_void_p(None), c_void_p(None), c_void_p(None),
             _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_tc")
 
 
@@ -466,11 +466,11 @@ class TensorCoreGemm:
         if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or qkv.dtype != torch.bfloat16:
             raise KernelError("gemm_qkv_rope works in bfloat16")
         _check(self.lib.sllm_gemm_tc_qkv_rope_fold_bf16(
-            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(qkv.data_ptr()), c_int(M), c_int(K), c_int(a.stride(0)),
-            c_int(w.stride(0)), c_int(qkv.stride(0)), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
-            _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]), _ptr(cos_sin, torch.float32, "cos_sin"),
-            _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), c_int(n_heads), c_int(n_kv),
-            c_int(head_dim), c_int(rot), c_int(1 if interleaved else 0), *self._owed_args(owed, M),
+            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(qkv.data_ptr()), M, K, a.stride(0),
+            w.stride(0), qkv.stride(0), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
+            _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(cos_sin, torch.float32, "cos_sin"),
+            _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), n_heads, n_kv,
+            head_dim, rot, (1 if interleaved else 0), *self._owed_args(owed, M),
             _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_qkv_rope")
 
     SKINNY_MAX_M = 128
@@ -494,10 +494,10 @@ class TensorCoreGemm:
             raise KernelError(f"gemm_grouped shapes: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}")
         fn = self.lib.sllm_gemm_tc_grouped_bf16
         fn.restype = c_int
-        _check(fn(_ptr(a, torch.bfloat16, "a"), _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), c_int(M), c_int(N), c_int(K),
-                  c_int(K), c_int(K), c_int(out.shape[1]), c_int(1 if out.dtype == torch.float32 else 0),
-                  _ptr(tile_group, torch.int32, "tile_group"), c_int(tile_rows), c_int(G), c_int(self.ACTS[act]), _ptr(rows_used, torch.int32, "rows_used"),
-                  c_int(0 if glu is None else 1), c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]),
+        _check(fn(_ptr(a, torch.bfloat16, "a"), _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K,
+                  K, K, out.shape[1], 1 if out.dtype == torch.float32 else 0,
+                  _ptr(tile_group, torch.int32, "tile_group"), tile_rows, G, self.ACTS[act], _ptr(rows_used, torch.int32, "rows_used"),
+                  (0 if glu is None else 1), c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]),
                   _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_grouped")
 
     def gemm_act(self, a, w, out, err_flag, act: str):
@@ -508,8 +508,8 @@ class TensorCoreGemm:
             raise KernelError(f"gemm_act shapes: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}")
         fn = self.lib.sllm_gemm_tc_act_bf16
         fn.restype = c_int
-        _check(fn(c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M), c_int(N), c_int(K),
-                  c_int(a.stride(0)), c_int(w.stride(0)), c_int(N), c_int(1 if out.dtype == torch.float32 else 0), c_int(self.ACTS[act]),
+        _check(fn(c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), M, N, K,
+                  a.stride(0), w.stride(0), N, 1 if out.dtype == torch.float32 else 0, self.ACTS[act],
                   _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_act")
 
     def gemm_skinny(self, a, w, out, err_flag, swiglu=False):
@@ -529,9 +529,9 @@ class TensorCoreGemm:
         if not (a.is_cuda and w.is_cuda and out.is_cuda):
             raise KernelError("gemm_skinny runs on a CUDA device only")
         _check(self.lib.sllm_gemm_tc_skinny_bf16(
-            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), c_int(M), c_int(N), c_int(K),
-            c_int(a.stride(0)), c_int(w.stride(0)), c_int(out.stride(-2)), c_int(1 if out.dtype == torch.float32 else 0),
-            c_int(1 if swiglu else 0), c_int(ksplit), _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_skinny")
+            c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), M, N, K,
+            a.stride(0), w.stride(0), out.stride(-2), 1 if out.dtype == torch.float32 else 0,
+            (1 if swiglu else 0), ksplit, _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_skinny")
 
     def prefers_skinny(self, a, w, kind: str, sm_count: int) -> bool:
         """True where the few-rows kernel is the fastest of the three products for a [M,K] x [N,K]^T
@@ -590,10 +590,10 @@ class PrefillAttentionTC:
 def _gate_args(gate, rows: int, cols: int):
     """Pointer and row stride of bfloat16 gate logits [rows, cols], a column slice of a wider buffer; (null, 0) without."""
     if gate is None:
-        return c_void_p(0), c_int(0)
+        return c_void_p(0), 0
     if not gate.is_cuda or gate.dtype != torch.bfloat16 or tuple(gate.shape) != (rows, cols) or gate.stride(1) != 1:
         raise KernelError(f"gate logits {tuple(gate.shape)} {gate.dtype} for an output of {(rows, cols)}")
-    return c_void_p(gate.data_ptr()), c_int(gate.stride(0))
+    return c_void_p(gate.data_ptr()), gate.stride(0)
 
 
 def gate_aligned(gate) -> bool:
@@ -630,11 +630,11 @@ class PrefillAttentionMMA:
         [T, n_heads * vd]): as for `PrefillAttentionTC.attn`."""
         gp, gl = _gate_args(gate, q.shape[0], n_heads * vd)
         _check(self.lib.sllm_attn_prefill_mma_bf16(
-            _ptr(q, torch.bfloat16, "q"), c_int(q.shape[1]), c_int(q_hw), _ptr(out, torch.bfloat16, "out"), c_int(out.shape[1]),
-            c_int(o_hw), _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
-            _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]), _ptr(kpages, torch.bfloat16, "kpages"),
-            c_int(kpages.shape[-1]), _ptr(vpages, torch.bfloat16, "vpages"), c_int(vpages.shape[-1]), c_int(n_seqs), c_int(max_new),
-            c_int(n_heads), c_int(n_kv), c_int(kd), c_int(vd), c_int(window or 0), c_int(keep), c_float(scale), c_float(softcap or 0.0),
+            _ptr(q, torch.bfloat16, "q"), q.shape[1], q_hw, _ptr(out, torch.bfloat16, "out"), out.shape[1],
+            o_hw, _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
+            _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"),
+            kpages.shape[-1], _ptr(vpages, torch.bfloat16, "vpages"), vpages.shape[-1], n_seqs, max_new,
+            n_heads, n_kv, kd, vd, (window or 0), keep, c_float(scale), c_float(softcap or 0.0),
             _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_prefill_mma")
 
 
@@ -684,7 +684,7 @@ class DecodeKernels:
         with 1,152 blocks against 74.6 with 768; 6 sequences 36.1 with 1,152 against 37.2 with 960;
         16 sequences 84.6 with 1,024 against 98.8 with 1,536)."""
         pairs = max(1, n_seqs * n_kv_heads)
-        if self.lib.sllm_attn_decode_uses_mma(c_int(n_seqs), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim)):
+        if self.lib.sllm_attn_decode_uses_mma(n_seqs, n_heads, n_kv_heads, head_dim):
             want, cap = ((4 if head_dim <= 64 else 2) * sm_count) // pairs, max(1, pages // 4)
         else:
             want, cap = ((39 if n_heads == n_kv_heads else 17) * sm_count) // (5 * pairs), pages
@@ -716,9 +716,9 @@ class DecodeKernels:
             raise KernelError(f"gemm_small_m output dtype {out.dtype}")
         _check(self.lib.sllm_gemm_small_m_bf16(
             _ptr(a, torch.bfloat16, "a") if a.is_contiguous() else c_void_p(a.data_ptr()),
-            _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-            c_int(w.stride(0)), c_int(out.stride(-2)), c_int(1 if out.dtype == torch.float32 else 0),
-            c_int(1 if swiglu else 0), c_int(ksplit), _stream()), "gemm_small_m")
+            _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K, a.stride(0),
+            w.stride(0), out.stride(-2), 1 if out.dtype == torch.float32 else 0,
+            (1 if swiglu else 0), ksplit, _stream()), "gemm_small_m")
 
     def gemm_small_m_act(self, a, w, out, act: str):
         """out[M, N] (bfloat16) = act(a @ w^T), the activation on the float sums (names as `TensorCoreGemm.ACTS`)."""
@@ -727,8 +727,8 @@ class DecodeKernels:
         if w.shape[1] != K or tuple(out.shape) != (M, N) or out.dtype != torch.bfloat16 or a.dtype != torch.bfloat16 or a.stride(1) != 1:
             raise KernelError(f"gemm_small_m_act shapes: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} {out.dtype}")
         _check(self.lib.sllm_gemm_small_m_act_bf16(
-            c_void_p(a.data_ptr()), _ptr(w, torch.bfloat16, "w"), _ptr(out, torch.bfloat16, "out"), c_int(M), c_int(N), c_int(K),
-            c_int(a.stride(0)), c_int(w.stride(0)), c_int(N), c_int(TensorCoreGemm.ACTS[act]), _stream()), "gemm_small_m_act")
+            c_void_p(a.data_ptr()), _ptr(w, torch.bfloat16, "w"), _ptr(out, torch.bfloat16, "out"), M, N, K,
+            a.stride(0), w.stride(0), N, TensorCoreGemm.ACTS[act], _stream()), "gemm_small_m_act")
 
     def _gemm_small_m_fold(self, a, w, out, swiglu, owed, fold):
         M, K = a.shape
@@ -759,27 +759,27 @@ class DecodeKernels:
             epilogue = 1 if swiglu else 0
         _check(self.lib.sllm_gemm_small_m_fold_bf16(
             _ptr(a, torch.bfloat16, "a") if a.is_contiguous() else c_void_p(a.data_ptr()),
-            _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-            c_int(w.stride(0)), c_int(out.stride(-2)), c_int(1 if out.dtype == torch.float32 else 0),
-            c_int(epilogue), c_int(1), sumsq_in, c_int(n_in), c_int(width), c_float(eps), *tail, _stream()), "gemm_small_m")
+            _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K, a.stride(0),
+            w.stride(0), out.stride(-2), 1 if out.dtype == torch.float32 else 0,
+            epilogue, 1, sumsq_in, n_in, width, c_float(eps), *tail, _stream()), "gemm_small_m")
 
     def attn_decode_rope(self, qkv, out, seq_pos0, block_table, kpages, vpages, scratch, tickets, cos_sin, rot,
                          interleaved, write_kv, n_seqs, n_heads, n_kv, head_dim, window, scale, n_split):
         """Rotary positions, cache write and attention of a decode step in one kernel: `qkv` holds the
         unrotated [q | k | v] rows of the step (only q when write_kv is false)."""
-        need = self.lib.sllm_attn_decode_scratch_bytes(c_int(n_seqs), c_int(n_heads), c_int(head_dim), c_int(n_split))
+        need = self.lib.sllm_attn_decode_scratch_bytes(n_seqs, n_heads, head_dim, n_split)
         if scratch.numel() * scratch.element_size() < need or tickets.numel() < n_seqs * n_kv:
             raise KernelError("attn_decode_rope: scratch or tickets too small")
         width = (n_heads + 2 * n_kv) * head_dim if write_kv else n_heads * head_dim
         if qkv.shape[1] < width:
             raise KernelError(f"attn_decode_rope: rows of {qkv.shape[1]} columns, need {width}")
         _check(self.lib.sllm_attn_decode_rope_bf16(
-            _ptr(qkv, torch.bfloat16, "qkv"), c_int(qkv.shape[1]), _ptr(out, torch.bfloat16, "out"),
+            _ptr(qkv, torch.bfloat16, "qkv"), qkv.shape[1], _ptr(out, torch.bfloat16, "out"),
             _ptr(seq_pos0, torch.int32, "seq_pos0"), _ptr(block_table, torch.int32, "block_table"),
-            c_int(block_table.shape[1]), _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
+            block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
             _ptr(scratch, torch.float32, "scratch"), _ptr(tickets, torch.int32, "tickets"),
-            _ptr(cos_sin, torch.float32, "cos_sin"), c_int(rot), c_int(1 if interleaved else 0), c_int(1 if write_kv else 0),
-            c_int(n_seqs), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(window or 0), c_float(scale), c_int(n_split),
+            _ptr(cos_sin, torch.float32, "cos_sin"), rot, (1 if interleaved else 0), (1 if write_kv else 0),
+            n_seqs, n_heads, n_kv, head_dim, (window or 0), c_float(scale), n_split,
             _stream()), "attn_decode_rope")
 
     def split_for(self, n_out: int, k: int, sm_count: int) -> int:
@@ -791,15 +791,15 @@ class DecodeKernels:
                     window, scale, n_split, tickets=None):
         """`tickets` (int32 [>= n_seqs * n_kv], zero before its first use, left zero): the last split
         to finish merges the partial results in the same kernel; without it a second kernel merges."""
-        need = self.lib.sllm_attn_decode_scratch_bytes(c_int(n_seqs), c_int(n_heads), c_int(head_dim), c_int(n_split))
+        need = self.lib.sllm_attn_decode_scratch_bytes(n_seqs, n_heads, head_dim, n_split)
         if scratch.numel() * scratch.element_size() < need:
             raise KernelError(f"attn_decode scratch holds {scratch.numel() * scratch.element_size()} bytes, needs {need}")
-        head = (_ptr(q, torch.bfloat16, "q"), c_int(q.shape[1]), _ptr(out, torch.bfloat16, "out"),
+        head = (_ptr(q, torch.bfloat16, "q"), q.shape[1], _ptr(out, torch.bfloat16, "out"),
                 _ptr(seq_pos0, torch.int32, "seq_pos0"), _ptr(block_table, torch.int32, "block_table"),
-                c_int(block_table.shape[1]), _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
+                block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
                 _ptr(scratch, torch.float32, "scratch"))
-        tail = (c_int(n_seqs), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(window or 0), c_float(scale),
-                c_int(n_split), _stream())
+        tail = (n_seqs, n_heads, n_kv, head_dim, (window or 0), c_float(scale),
+                n_split, _stream())
         if tickets is None:
             _check(self.lib.sllm_attn_decode_bf16(*head, *tail), "attn_decode")
         else:
@@ -829,11 +829,11 @@ class DecodeKernels:
             raise KernelError("attn_decode_general: scratch or tickets too small")
         gp, gl = _gate_args(gate, n_seqs, n_heads * v_dim)
         _check(self.lib.sllm_attn_decode_general_bf16(
-            _ptr(q, torch.bfloat16, "q"), c_int(q.shape[1]), _ptr(out, torch.bfloat16, "out"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
-            _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]), _ptr(kpages, torch.bfloat16, "kpages"),
+            _ptr(q, torch.bfloat16, "q"), q.shape[1], _ptr(out, torch.bfloat16, "out"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
+            _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"),
             _ptr(vpages, torch.bfloat16, "vpages"), _ptr(scratch, torch.float32, "scratch"), _ptr(tickets, torch.int32, "tickets"),
-            c_int(n_seqs), c_int(n_heads), c_int(n_kv), c_int(head_dim), c_int(v_dim), c_int(window or 0), c_int(keep), c_float(scale),
-            c_int(n_split), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_decode_general")
+            n_seqs, n_heads, n_kv, head_dim, v_dim, (window or 0), keep, c_float(scale),
+            n_split, c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_decode_general")
 
 
 class SequenceKernels:
@@ -894,10 +894,10 @@ class SequenceKernels:
         ptrs = (c_void_p * max(1, n))(*[t.data_ptr() for t, _ in addends])
         coefs = (c_float * max(1, n))(*[float(c) for _, c in addends])
         flags = (c_int * max(1, n))(*[self._flag(t, "addend") for t, _ in addends])
-        _check(self._fn("add_norm")(_ptr(x, torch.float32, "x"), ptrs, coefs, flags, c_int(n), _ptr(rows, torch.int32, "rows"),
-                                    _ptr(weight, None, "weight"), c_int(self._flag(weight, "weight")),
-                                    _ptr(y, None, "y"), c_int(self._flag(y, "y")), c_int(y.shape[0]), c_int(d), c_float(eps),
-                                    c_int(1 if center else 0), _stream()), "add_norm")
+        _check(self._fn("add_norm")(_ptr(x, torch.float32, "x"), ptrs, coefs, flags, n, _ptr(rows, torch.int32, "rows"),
+                                    _ptr(weight, None, "weight"), self._flag(weight, "weight"),
+                                    _ptr(y, None, "y"), self._flag(y, "y"), y.shape[0], d, c_float(eps),
+                                    (1 if center else 0), _stream()), "add_norm")
 
     def causal_conv(self, x, weight, state, ctx, y, taps, in_bias=None, out_bias=None, add_input=False, act=None, y2=None):
         """y[t] = act(sum_j weight[:, j] * in(t - taps + 1 + j) + out_bias (+ in(t))), in = x + in_bias, over the
@@ -911,13 +911,13 @@ class SequenceKernels:
             if b is not None:
                 b_f32 = self._flag(b, "bias")
         _check(self._fn("causal_conv")(
-            self._view(x, "x"), c_int(self._flag(x, "x")), c_int(x.stride(0)), _ptr(weight, None, "weight"),
-            c_int(self._flag(weight, "weight")), _ptr(in_bias, None, "in_bias"), _ptr(out_bias, None, "out_bias"), c_int(b_f32),
+            self._view(x, "x"), self._flag(x, "x"), x.stride(0), _ptr(weight, None, "weight"),
+            self._flag(weight, "weight"), _ptr(in_bias, None, "in_bias"), _ptr(out_bias, None, "out_bias"), b_f32,
             _ptr(state, torch.float32, "state") if taps > 1 else c_void_p(0), _ptr(ctx.seq_start, torch.int32, "seq_start"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), self._view(y, "y"),
-            c_int(self._flag(y, "y")), c_int(y.stride(0)), self._view(y2, "y2") if y2 is not None else c_void_p(0),
-            c_int(y2.stride(0) if y2 is not None else 0), c_int(T), c_int(ctx.n_seqs), c_int(C), c_int(taps),
-            c_int(1 if add_input else 0), c_int({None: 0, "silu": 1}[act]), _stream()), "causal_conv")
+            self._flag(y, "y"), y.stride(0), self._view(y2, "y2") if y2 is not None else c_void_p(0),
+            (y2.stride(0) if y2 is not None else 0), T, ctx.n_seqs, C, taps,
+            (1 if add_input else 0), {None: 0, "silu": 1}[act], _stream()), "causal_conv")
 
     def kv_store(self, qkv, tok_pos, tok_seq, block_table, cos_sin, kpages, vpages, n_heads, n_kv, head_dim, v_dim, rot,
                  interleaved, v_eps):
@@ -933,12 +933,12 @@ class SequenceKernels:
                                     c_float(-1.0 if v_eps is None else v_eps), _stream()), "kv_store")
 
     def attn_wide_value(self, q, out, tok_pos, tok_seq, block_table, kpages, vpages, n_heads, n_kv, head_dim, v_dim, window, scale):
-        _check(self._fn("attn_wide_value")(_ptr(q, self.dtype, "q"), c_int(q.shape[1]), _ptr(out, self.dtype, "out"),
-                                           c_int(out.shape[1]), _ptr(tok_pos, torch.int32, "tok_pos"),
+        _check(self._fn("attn_wide_value")(_ptr(q, self.dtype, "q"), q.shape[1], _ptr(out, self.dtype, "out"),
+                                           out.shape[1], _ptr(tok_pos, torch.int32, "tok_pos"),
                                            _ptr(tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"),
-                                           c_int(block_table.shape[1]), _ptr(kpages, self.dtype, "kpages"),
-                                           _ptr(vpages, self.dtype, "vpages"), c_int(q.shape[0]), c_int(n_heads), c_int(n_kv),
-                                           c_int(head_dim), c_int(v_dim), c_int(window or 0), c_float(scale), _stream()),
+                                           block_table.shape[1], _ptr(kpages, self.dtype, "kpages"),
+                                           _ptr(vpages, self.dtype, "vpages"), q.shape[0], n_heads, n_kv,
+                                           head_dim, v_dim, (window or 0), c_float(scale), _stream()),
                "attn_wide_value")
 
     def delta_prepare(self, qk, ba, a_log, dt_bias, bd, n_heads, n_kv, dk):
@@ -974,9 +974,9 @@ class SequenceKernels:
                                       n_kv, dk, dv, _stream()), "delta_rule")
 
     def gated_unit_rms(self, o, gate, weight, y, n_heads, dv, eps):
-        _check(self._fn("gated_unit_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), c_int(gate.stride(0)),
-                                          _ptr(weight, None, "weight"), c_int(self._flag(weight, "weight")),
-                                          _ptr(y, self.dtype, "y"), c_int(o.shape[0]), c_int(n_heads), c_int(dv), c_float(eps),
+        _check(self._fn("gated_unit_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), gate.stride(0),
+                                          _ptr(weight, None, "weight"), self._flag(weight, "weight"),
+                                          _ptr(y, self.dtype, "y"), o.shape[0], n_heads, dv, c_float(eps),
                                           _stream()), "gated_unit_rms")
 
     SCAN_WALK_MAX = 4     # rows of a sequence in one step up to which a thread walks them one after the other
@@ -992,12 +992,12 @@ class SequenceKernels:
             piece = self._fn("rglru_piece_rows")()
             scratch = torch.empty((2 * ctx.n_seqs * -(-ctx.max_new // piece) * W,), dtype=torch.float32, device=u.device)
         _check(self._fn("rglru_scan")(_ptr(gates, torch.float32, "gates"), _ptr(u, torch.float32, "u"), self._view(yraw, "yraw"),
-                                      c_int(yraw.stride(0)), _ptr(ra_b, None, "ra_b"), _ptr(ri_b, None, "ri_b"),
-                                      _ptr(lam, None, "lam"), _ptr(y_b, None, "y_b"), c_int(self._flag(lam, "lam")),
+                                      yraw.stride(0), _ptr(ra_b, None, "ra_b"), _ptr(ri_b, None, "ri_b"),
+                                      _ptr(lam, None, "lam"), _ptr(y_b, None, "y_b"), self._flag(lam, "lam"),
                                       _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                                       _ptr(ctx.slots, torch.int32, "slots"), _ptr(out, self.dtype, "out"),
-                                      _ptr(scratch, torch.float32, "scratch"), c_int(max(1, ctx.max_new)), c_int(T),
-                                      c_int(ctx.n_seqs), c_int(W), c_int(block_size), _stream()), "rglru_scan")
+                                      _ptr(scratch, torch.float32, "scratch"), max(1, ctx.max_new), T,
+                                      ctx.n_seqs, W, block_size, _stream()), "rglru_scan")
 
 
 class ChunkKernels:
@@ -1062,10 +1062,10 @@ class ChunkKernels:
         held = self.heads_held(n, n_heads, self.DELTA_BYTES)
         scratch = torch.empty((n * held * self.DELTA_BYTES,), dtype=torch.uint8, device=o.device)
         _check(self.lib.sllm_chunk_delta(
-            SequenceKernels._view(qk, "qk"), c_int(qk.stride(0)), SequenceKernels._view(v, "v"), c_int(v.stride(0)),
+            SequenceKernels._view(qk, "qk"), qk.stride(0), SequenceKernels._view(v, "v"), v.stride(0),
             _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), c_int(held), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
-            c_int(ctx.max_new), c_int(n_heads), c_int(n_kv), c_int(dk), c_int(dv),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), held, _ptr(o, torch.float32, "o"), ctx.n_seqs,
+            ctx.max_new, n_heads, n_kv, dk, dv,
             _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "chunk_delta")
 
     def lin_attn(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
@@ -1074,10 +1074,10 @@ class ChunkKernels:
         held = self.heads_held(n, n_heads, 4 * dk * dv)
         chunk_state = torch.empty((n, held, dk, dv), dtype=torch.float32, device=o.device)
         _check(self.lib.sllm_chunk_lin_attn_bf16(
-            _ptr(proj, torch.bfloat16, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
+            _ptr(proj, torch.bfloat16, "proj"), proj.shape[1], q_col, k_col, v_col,
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), c_int(held), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs),
-            c_int(ctx.max_new), c_int(n_heads), c_int(dk), c_int(dv), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), held, _ptr(o, torch.float32, "o"), ctx.n_seqs,
+            ctx.max_new, n_heads, dk, dv, _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
             "chunk_lin_attn")
 
 
@@ -1130,14 +1130,14 @@ class MixKernels:
             y_f32 = self._flag(addend, "addend")
         pw, pb, pa = post if post is not None else (None, None, 0.0)
         _check(self._fn("dyt_add_norm")(
-            _ptr(x, torch.float32, "x"), _ptr(addend, None, "addend"), c_int(y_f32), c_int(n_parts), c_longlong(stride),
+            _ptr(x, torch.float32, "x"), _ptr(addend, None, "addend"), y_f32, n_parts, c_longlong(stride),
             _ptr(pw, torch.float32, "post weight"), _ptr(pb, torch.float32, "post bias"), c_float(pa),
-            c_int(1 if post is not None else 0), c_int(1), _ptr(rows, torch.int32, "rows"), _ptr(weight, torch.float32, "weight"),
-            _ptr(bias, torch.float32, "bias"), c_float(alpha), c_int(1), _ptr(out, None, "out"), c_int(self._flag(out, "out")),
-            c_int(out.shape[0]), c_int(d), _stream()), "dyt_add_norm")
+            (1 if post is not None else 0), 1, _ptr(rows, torch.int32, "rows"), _ptr(weight, torch.float32, "weight"),
+            _ptr(bias, torch.float32, "bias"), c_float(alpha), 1, _ptr(out, None, "out"), self._flag(out, "out"),
+            out.shape[0], d, _stream()), "dyt_add_norm")
 
     def act_inplace(self, x, kind: str):
-        _check(self._fn("act_inplace")(_ptr(x, self.dtype, "x"), c_longlong(x.numel()), c_int(self.ACTS[kind]), _stream()),
+        _check(self._fn("act_inplace")(_ptr(x, self.dtype, "x"), c_longlong(x.numel()), self.ACTS[kind], _stream()),
                "act_inplace")
 
     def lin_attn_decay(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
@@ -1152,29 +1152,29 @@ class MixKernels:
         # general kernel), 8 6.0 (19.6), 32 15.2 (62.6), 512 251 (1,062); of 16 x 16 1 sequence 4.3 (9.9), 512 59 (175); 8 heads of
         # 256 x 64 1 sequence 5.6 (13.6); float32 the same. Better at every size of 1 x 16 to 256 x 64 and 128 x 128 measured: widths alone decide.
         if (ctx.max_new == 1 and proj.shape[0] == ctx.n_seqs and state.data_ptr() % 16 == 0
-                and self._fn("lin_attn_step_takes")(c_int(dk), c_int(dv))):
+                and self._fn("lin_attn_step_takes")(dk, dv)):
             _check(self._fn("lin_attn_step")(
-                _ptr(proj, self.dtype, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
+                _ptr(proj, self.dtype, "proj"), proj.shape[1], q_col, k_col, v_col,
                 _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-                _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(n_heads), c_int(dk), c_int(dv),
-                c_int(ctx.engine.sm_count), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "lin_attn_step")
+                _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), ctx.n_seqs, n_heads, dk, dv,
+                ctx.engine.sm_count, _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "lin_attn_step")
             return
         self.lin_attn_walk(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
 
     def lin_attn_walk(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
         """`lin_attn_decay` in pieces of up to 32 rows one after the other."""
         _check(self._fn("lin_attn_decay")(
-            _ptr(proj, self.dtype, "proj"), c_int(proj.shape[1]), c_int(q_col), c_int(k_col), c_int(v_col),
+            _ptr(proj, self.dtype, "proj"), proj.shape[1], q_col, k_col, v_col,
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)),
-            c_int(n_heads), c_int(dk), c_int(dv), c_int(ctx.engine.sm_count), _stream()), "lin_attn_decay")
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), ctx.n_seqs, max(1, ctx.max_new),
+            n_heads, dk, dv, ctx.engine.sm_count, _stream()), "lin_attn_decay")
 
     chunk = SequenceKernels.chunk
 
     def gated_row_rms(self, o, gate, weight, y, eps, gate_act: str):
-        _check(self._fn("gated_row_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), c_int(gate.stride(0)),
-                                         _ptr(weight, torch.float32, "weight"), c_int(1), _ptr(y, self.dtype, "y"),
-                                         c_int(o.shape[0]), c_int(o.shape[1]), c_float(eps), c_int(self.GATES[gate_act]), _stream()),
+        _check(self._fn("gated_row_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), gate.stride(0),
+                                         _ptr(weight, torch.float32, "weight"), 1, _ptr(y, self.dtype, "y"),
+                                         o.shape[0], o.shape[1], c_float(eps), self.GATES[gate_act], _stream()),
                "gated_row_rms")
 
     def latent_store(self, q, n_heads, dim, dkv, norm_w, eps, cos_sin, rot, ctx, block_table, pages, rank, rot_dim, half=False):
@@ -1183,31 +1183,31 @@ class MixKernels:
         `pages`, stores [dkv[:rank] / rms * norm_w | rotated dkv[rank:]] at the rows' places. q and dkv may be
         column slices of one buffer."""
         _check(self._fn("latent_store")(
-            self._view(q, "q"), c_int(q.stride(0)), c_int(n_heads), c_int(dim),
-            self._view(dkv, "dkv") if dkv is not None else c_void_p(0), c_int(dkv.stride(0) if dkv is not None else 0),
-            _ptr(norm_w, torch.float32, "norm weight"), c_int(1), c_float(eps),
-            _ptr(cos_sin, torch.float32, "cos_sin"), c_int(rot), c_int(1 if half else 0), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
-            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
-            _ptr(pages, self.dtype if pages is not None else None, "pages"), c_int(q.shape[0]), c_int(rank), c_int(rot_dim),
+            self._view(q, "q"), q.stride(0), n_heads, dim,
+            self._view(dkv, "dkv") if dkv is not None else c_void_p(0), (dkv.stride(0) if dkv is not None else 0),
+            _ptr(norm_w, torch.float32, "norm weight"), 1, c_float(eps),
+            _ptr(cos_sin, torch.float32, "cos_sin"), rot, (1 if half else 0), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
+            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
+            _ptr(pages, self.dtype if pages is not None else None, "pages"), q.shape[0], rank, rot_dim,
             _stream()), "latent_store")
 
     def latent_gather(self, pages, ctx, block_table, dense):
         """dense[t] = the cached vector at row t's (sequence, position)."""
         _check(self._fn("latent_gather")(_ptr(pages, self.dtype, "pages"), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
                                          _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"),
-                                         c_int(block_table.shape[1]), _ptr(dense, self.dtype, "dense"), c_int(dense.shape[0]),
-                                         c_int(dense.shape[1]), _stream()), "latent_gather")
+                                         block_table.shape[1], _ptr(dense, self.dtype, "dense"), dense.shape[0],
+                                         dense.shape[1], _stream()), "latent_gather")
 
     def latent_heads(self, q, kv, dense, rank, ctx, table, kt, vt, qt, n_heads, dim, rot_dim, v_dim):
         """Keys [Wuk c | rotated part | 0] and values [Wuv c | 0] per head, as wide as kt's and vt's rows, into pages of their
         own by `table` (a prompt step from position 0), and queries [q | 0] as wide as the keys into qt (None: they stay)."""
-        _check(self._fn("latent_heads")(self._view(q, "q"), c_int(q.stride(0)), self._view(kv, "kv"), c_int(kv.stride(0)),
-                                        self._view(dense, "dense"), c_int(dense.stride(0)), c_int(rank),
+        _check(self._fn("latent_heads")(self._view(q, "q"), q.stride(0), self._view(kv, "kv"), kv.stride(0),
+                                        self._view(dense, "dense"), dense.stride(0), rank,
                                         _ptr(ctx.tok_pos, torch.int32, "tok_pos"), _ptr(ctx.tok_seq, torch.int32, "tok_seq"),
-                                        _ptr(table, torch.int32, "table"), c_int(table.shape[1]), _ptr(kt, self.dtype, "kt"),
+                                        _ptr(table, torch.int32, "table"), table.shape[1], _ptr(kt, self.dtype, "kt"),
                                         _ptr(vt, self.dtype, "vt"), _ptr(qt, self.dtype if qt is not None else None, "qt"),
-                                        c_int(q.shape[0]), c_int(n_heads), c_int(dim), c_int(rot_dim), c_int(v_dim), c_int(kt.shape[-1]),
-                                        c_int(vt.shape[-1]), _stream()), "latent_heads")
+                                        q.shape[0], n_heads, dim, rot_dim, v_dim, kt.shape[-1],
+                                        vt.shape[-1], _stream()), "latent_heads")
 
     @property
     def latent(self) -> "LatentKernels | None":
@@ -1227,13 +1227,13 @@ class MixKernels:
             raise KernelError(f"latent_absorb: q has dtype {q.dtype}, expected {self.dtype}")
         lat = self.latent
         if lat is not None and lat.takes(dim, rot_dim, 8, rank) and q.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0 and wuk.data_ptr() % 16 == 0:
-            _check(lat.lib.sllm_latent_absorb_mma(self._view(q, "q"), c_int(q.stride(0)), _ptr(wuk, self.dtype, "wuk"),
-                                                  _ptr(qa, torch.float32, "qa"), c_int(q.shape[0]), c_int(n_heads), c_int(dim),
-                                                  c_int(rot_dim), c_int(rank), c_float(scale), _stream()), "latent_absorb_mma")
+            _check(lat.lib.sllm_latent_absorb_mma(self._view(q, "q"), q.stride(0), _ptr(wuk, self.dtype, "wuk"),
+                                                  _ptr(qa, torch.float32, "qa"), q.shape[0], n_heads, dim,
+                                                  rot_dim, rank, c_float(scale), _stream()), "latent_absorb_mma")
             return
-        _check(self._fn("latent_absorb")(self._view(q, "q"), c_int(q.stride(0)), _ptr(wuk, self.dtype, "wuk"),
-                                         _ptr(qa, torch.float32, "qa"), c_int(q.shape[0]), c_int(n_heads), c_int(dim),
-                                         c_int(rot_dim), c_int(rank), c_float(scale), _stream()), "latent_absorb")
+        _check(self._fn("latent_absorb")(self._view(q, "q"), q.stride(0), _ptr(wuk, self.dtype, "wuk"),
+                                         _ptr(qa, torch.float32, "qa"), q.shape[0], n_heads, dim,
+                                         rot_dim, rank, c_float(scale), _stream()), "latent_absorb")
 
     def latent_attn(self, qa, pages, ctx, block_table, part, n_heads, rank, rot_dim, n_split, window=0):
         """`window` > 0: a row sees its own position and the window - 1 before it; 0: every earlier one."""
@@ -1241,9 +1241,9 @@ class MixKernels:
         fn = lat.lib.sllm_latent_attn_mma if lat is not None and lat.takes(8, rot_dim, 8, rank) and pages.data_ptr() % 16 == 0 else self._fn("latent_attn")
         _check(fn(
             _ptr(qa, torch.float32, "qa"), _ptr(pages, self.dtype, "pages"), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
-            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1]),
-            _ptr(part, torch.float32, "part"), c_int(qa.shape[0]), c_int(n_heads), c_int(rank), c_int(rot_dim), c_int(n_split),
-            c_int(window), _stream()), "latent_attn")
+            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
+            _ptr(part, torch.float32, "part"), qa.shape[0], n_heads, rank, rot_dim, n_split,
+            window, _stream()), "latent_attn")
 
     def latent_expand(self, part, olat, wuv, out, n_heads, v_dim, rank, n_split, sink=None, gate=None):
         """Merges the splits of `part` into olat float32 [T, H, rank] (scratch), then out[t, h] = Wuv_h olat[t, h]. `sink` float32
@@ -1258,10 +1258,10 @@ class MixKernels:
         mma = lat is not None and lat.takes(8, 0, v_dim, rank) and n_split <= 64 and wuv.data_ptr() % 16 == 0
         fn = lat.lib.sllm_latent_expand_mma if mma else self._fn("latent_expand")
         _check(fn(_ptr(part, torch.float32, "part"), _ptr(olat, torch.float32, "olat"),
-                                         _ptr(wuv, self.dtype, "wuv"), _ptr(out, self.dtype, "out"), c_int(out.shape[1]),
-                                         c_int(out.shape[0]), c_int(n_heads), c_int(v_dim), c_int(rank), c_int(n_split),
+                                         _ptr(wuv, self.dtype, "wuv"), _ptr(out, self.dtype, "out"), out.shape[1],
+                                         out.shape[0], n_heads, v_dim, rank, n_split,
                                          _ptr(sink, torch.float32, "sink"), self._view(gate, "gate") if gate is not None else c_void_p(0),
-                                         c_int(gate.stride(0) if gate is not None else 0), c_int(mode), _stream()), "latent_expand")
+                                         (gate.stride(0) if gate is not None else 0), mode, _stream()), "latent_expand")
         LAUNCHES[0] += 1
 
     @staticmethod
@@ -1297,17 +1297,17 @@ class MixKernels:
         for t, name in ((x, "x"), (z, "z"), (bc, "bc"), (out, "out")):
             if t.dtype != self.dtype:
                 raise KernelError(f"selective_scan: {name} has dtype {t.dtype}, expected {self.dtype}")
-        args = (self._view(x, "x"), c_int(x.stride(0)), _ptr(dt_raw, torch.float32, "dt_raw"), c_int(dt_raw.shape[1]),
+        args = (self._view(x, "x"), x.stride(0), _ptr(dt_raw, torch.float32, "dt_raw"), dt_raw.shape[1],
                 _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"),
-                c_int(1), self._view(bc, "bc"), c_int(bc.stride(0)), c_int(b_col), c_int(c_col), self._view(z, "z"),
-                c_int(z.stride(0)), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-                _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), c_int(out.stride(0)))
-        tail = (c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)), c_int(inner), c_int(n_state), _stream())
+                1, self._view(bc, "bc"), bc.stride(0), b_col, c_col, self._view(z, "z"),
+                z.stride(0), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+                _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), out.stride(0))
+        tail = (ctx.n_seqs, max(1, ctx.max_new), inner, n_state, _stream())
         if self.scan_pays(x.shape[0], ctx.n_seqs, ctx.max_new, inner, n_state, ctx.engine.sm_count):
             T, rows = x.shape[0], self.scan_piece_rows(x.shape[0], inner, ctx.engine.sm_count)
             n = T // rows + ctx.n_seqs
             scratch = [torch.empty(shape, dtype=torch.float32, device=x.device) for shape in ((T, inner), (n, n_state, inner), (n, inner))]
-            _check(self._fn("selective_scan_pieces")(*args, *(_ptr(t) for t in scratch), c_int(rows), *tail), "selective_scan_pieces")
+            _check(self._fn("selective_scan_pieces")(*args, *(_ptr(t) for t in scratch), rows, *tail), "selective_scan_pieces")
             return
         _check(self._fn("selective_scan")(*args, *tail), "selective_scan")
 
@@ -1321,9 +1321,9 @@ class MixKernels:
         that only enters the picking, runs of experts rated by their best two."""
         T, E = z.shape
         mode = self.ROUTERS[router] if router is not None else (1 if top_softmax else 0)
-        _check(self._fn("moe_route")(_ptr(z, torch.float32, "z"), _ptr(correction, torch.float32, "correction"), c_int(1),
-                                     _ptr(idx, torch.int32, "idx"), _ptr(wgt, torch.float32, "wgt"), c_int(T), c_int(E),
-                                     c_int(n_groups), c_int(keep), c_int(top), c_float(scale), c_int(mode),
+        _check(self._fn("moe_route")(_ptr(z, torch.float32, "z"), _ptr(correction, torch.float32, "correction"), 1,
+                                     _ptr(idx, torch.int32, "idx"), _ptr(wgt, torch.float32, "wgt"), T, E,
+                                     n_groups, keep, top, c_float(scale), mode,
                                      _stream()), "moe_route")
 
     def moe_pairs(self, h, wup, wdown, idx, wgt, hid, out, glu=None, tiled=False):
@@ -1333,10 +1333,10 @@ class MixKernels:
         T, K = h.shape
         top = idx.shape[1]
         F = wdown.shape[2]
-        _check(self._fn("moe_pairs")(self._view(h, "h"), c_int(h.stride(0)), _ptr(wup, self.dtype, "wup"),
+        _check(self._fn("moe_pairs")(self._view(h, "h"), h.stride(0), _ptr(wup, self.dtype, "wup"),
                                      _ptr(wdown, self.dtype, "wdown"), _ptr(idx, torch.int32, "idx"), _ptr(wgt, torch.float32, "wgt"),
-                                     _ptr(hid, self.dtype, "hid"), _ptr(out, torch.float32, "out"), c_int(T), c_int(top), c_int(K),
-                                     c_int(F), c_int(wdown.shape[1]), c_int(0 if glu is None else 2 if tiled else 1),
+                                     _ptr(hid, self.dtype, "hid"), _ptr(out, torch.float32, "out"), T, top, K,
+                                     F, wdown.shape[1], (0 if glu is None else 2 if tiled else 1),
                                      c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]), _stream()),
                "moe_pairs")
 
@@ -1344,9 +1344,9 @@ class MixKernels:
         """out [rows, F] = the clamped gate of gu [rows, 2 F] (F gate sums, then F up sums a row; `tiled`: 8 and 8 in turn):
         g' * sigmoid(alpha g') * (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit). `rows_used`: an int32 on the
         device, rows from there on stay."""
-        _check(self._fn("glu_clamp")(_ptr(gu, self.dtype, "gu"), _ptr(out, self.dtype, "out"), c_int(out.shape[0]),
-                                     c_int(out.shape[1]), c_float(limit), c_float(alpha), _ptr(rows_used, torch.int32, "rows_used"),
-                                     c_int(1 if tiled else 0), _stream()), "glu_clamp")
+        _check(self._fn("glu_clamp")(_ptr(gu, self.dtype, "gu"), _ptr(out, self.dtype, "out"), out.shape[0],
+                                     out.shape[1], c_float(limit), c_float(alpha), _ptr(rows_used, torch.int32, "rows_used"),
+                                     (1 if tiled else 0), _stream()), "glu_clamp")
 
     def moe_group_rows(self, idx, n_experts, offsets, pair_of_row=None, row_of_pair=None, tile_group=None, pad=1):
         """Groups the (token, expert) pairs of idx [T, top] by expert. offsets int32 [E + 1]: the experts' first rows; pair_of_row
@@ -1358,8 +1358,8 @@ class MixKernels:
             raise KernelError(f"moe_group_rows: offsets {tuple(offsets.shape)} for {n_experts} experts, {rows} rows")
         _check(self._fn("moe_group_rows")(_ptr(idx, torch.int32, "idx"), _ptr(offsets, torch.int32, "offsets"),
                                           _ptr(pair_of_row, torch.int32, "pair_of_row"), _ptr(row_of_pair, torch.int32, "row_of_pair"),
-                                          _ptr(tile_group, torch.int32, "tile_group"), c_int(T), c_int(top), c_int(n_experts), c_int(pad),
-                                          c_int(rows), _stream()), "moe_group_rows")
+                                          _ptr(tile_group, torch.int32, "tile_group"), T, top, n_experts, pad,
+                                          rows, _stream()), "moe_group_rows")
 
     def moe_grouped(self, h, wup, wdown, wgt, offsets, pair_of_row, hid, out, glu=None, raw=None, tiled=False):
         """The experts' products over rows grouped without padding (`moe_group_rows` with pad 1), float32 sums on
@@ -1367,12 +1367,12 @@ class MixKernels:
         (`tiled` as for `moe_pairs`)."""
         T, K = h.shape
         top = wgt.shape[1]
-        _check(self._fn("moe_grouped")(self._view(h, "h"), c_int(h.stride(0)), _ptr(wup, self.dtype, "wup"),
+        _check(self._fn("moe_grouped")(self._view(h, "h"), h.stride(0), _ptr(wup, self.dtype, "wup"),
                                        _ptr(wdown, self.dtype, "wdown"), _ptr(wgt, torch.float32, "wgt"),
                                        _ptr(offsets, torch.int32, "offsets"), _ptr(pair_of_row, torch.int32, "pair_of_row"),
-                                       _ptr(hid, self.dtype, "hid"), _ptr(out, torch.float32, "out"), c_int(T), c_int(top),
-                                       c_int(wup.shape[0]), c_int(K), c_int(wdown.shape[2]), c_int(wdown.shape[1]),
-                                       c_int(0 if glu is None else 2 if tiled else 1), c_float(0.0 if glu is None else glu[0]),
+                                       _ptr(hid, self.dtype, "hid"), _ptr(out, torch.float32, "out"), T, top,
+                                       wup.shape[0], K, wdown.shape[2], wdown.shape[1],
+                                       (0 if glu is None else 2 if tiled else 1), c_float(0.0 if glu is None else glu[0]),
                                        c_float(0.0 if glu is None else glu[1]), _ptr(raw, self.dtype, "raw"), _stream()),
                "moe_grouped")
         LAUNCHES[0] += 1
@@ -1381,16 +1381,16 @@ class MixKernels:
         """xs[row_of_pair[t * top + k]] = h[t]; other rows of xs stay."""
         if row_of_pair.numel() != h.shape[0] * top:
             raise KernelError(f"moe_gather_rows: {row_of_pair.numel()} pairs of {h.shape[0]} rows, {top} each")
-        _check(self._fn("moe_gather_rows")(self._view(h, "h"), c_int(h.stride(0)), _ptr(row_of_pair, torch.int32, "row_of_pair"),
-                                           c_int(top), _ptr(xs, self.dtype, "xs"), c_int(h.shape[0]), c_int(xs.shape[1]), _stream()),
+        _check(self._fn("moe_gather_rows")(self._view(h, "h"), h.stride(0), _ptr(row_of_pair, torch.int32, "row_of_pair"),
+                                           top, _ptr(xs, self.dtype, "xs"), h.shape[0], xs.shape[1], _stream()),
                "moe_gather_rows")
 
     def moe_combine(self, ys, row_of_pair, wgt, out):
         """out[t] = sum_k wgt[t, k] * ys[row_of_pair[t * top + k]], float32 [T, N]."""
         T, top = wgt.shape
         _check(self._fn("moe_combine")(_ptr(ys, torch.float32, "ys"), _ptr(row_of_pair, torch.int32, "row_of_pair"),
-                                       _ptr(wgt, torch.float32, "wgt"), _ptr(out, torch.float32, "out"), c_int(T), c_int(top),
-                                       c_int(out.shape[1]), _stream()), "moe_combine")
+                                       _ptr(wgt, torch.float32, "wgt"), _ptr(out, torch.float32, "out"), T, top,
+                                       out.shape[1], _stream()), "moe_combine")
 
 
 class SsdKernels:
@@ -1436,13 +1436,13 @@ class SsdKernels:
             chunked = self.dtype == torch.bfloat16 and ctx.max_new >= self.CHUNK_MIN_ROWS
         chunked = chunked and n_state <= self.CHUNK_MAX_STATE
         if (not chunked and weight is None and ctx.max_new == 1 and T == ctx.n_seqs and T * n_heads >= self.STEP_MIN_UNITS
-                and head_dim >= self.STEP_MIN_COLS and state.data_ptr() % 16 == 0 and self._fn("ssd_step_takes")(c_int(head_dim), c_int(n_state))):
+                and head_dim >= self.STEP_MIN_COLS and state.data_ptr() % 16 == 0 and self._fn("ssd_step_takes")(head_dim, n_state)):
             _check(self._fn("ssd_step")(
-                self._view(xbc, "xbc"), c_int(xbc.stride(0)), self._view(dt, "dt"), c_int(dt.stride(0)), _ptr(dt_bias, torch.float32, "dt_bias"),
-                _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), c_int(z.stride(0)),
+                self._view(xbc, "xbc"), xbc.stride(0), self._view(dt, "dt"), dt.stride(0), _ptr(dt_bias, torch.float32, "dt_bias"),
+                _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), z.stride(0),
                 _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
-                self._view(out, "out"), c_int(out.stride(0)), c_int(T), c_int(n_heads), c_int(n_groups), c_int(head_dim), c_int(n_state),
-                c_int(self._sms(out.device)), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "ssd_step")
+                self._view(out, "out"), out.stride(0), T, n_heads, n_groups, head_dim, n_state,
+                self._sms(out.device), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "ssd_step")
             return None
         states = decays = sums = sumsq = None
         if chunked:
@@ -1453,12 +1453,12 @@ class SsdKernels:
         if weight is not None:
             sumsq = torch.empty((n_heads * -(-head_dim // (64 if chunked else 32)), T), dtype=torch.float32, device=out.device)
         _check(self._fn("ssd")(
-            self._view(xbc, "xbc"), c_int(xbc.stride(0)), self._view(dt, "dt"), c_int(dt.stride(0)), _ptr(dt_bias, torch.float32, "dt_bias"),
-            _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), c_int(z.stride(0)),
+            self._view(xbc, "xbc"), xbc.stride(0), self._view(dt, "dt"), dt.stride(0), _ptr(dt_bias, torch.float32, "dt_bias"),
+            _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), z.stride(0),
             _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
-            self._view(out, "out"), c_int(out.stride(0)), _ptr(weight, torch.float32, "weight"), _ptr(sumsq, torch.float32, "sumsq"),
-            _ptr(states, torch.float32, "states"), _ptr(decays, torch.float32, "decays"), _ptr(sums, torch.float32, "sums"), c_int(ctx.n_seqs), c_int(max(1, ctx.max_new)),
-            c_int(T), c_int(n_heads), c_int(n_groups), c_int(head_dim), c_int(n_state), _stream()), "ssd")
+            self._view(out, "out"), out.stride(0), _ptr(weight, torch.float32, "weight"), _ptr(sumsq, torch.float32, "sumsq"),
+            _ptr(states, torch.float32, "states"), _ptr(decays, torch.float32, "decays"), _ptr(sums, torch.float32, "sums"), ctx.n_seqs, max(1, ctx.max_new),
+            T, n_heads, n_groups, head_dim, n_state, _stream()), "ssd")
         if chunked:
             LAUNCHES[0] += 2
         return sumsq
@@ -1468,7 +1468,7 @@ class SsdKernels:
         if tuple(u.shape) != tuple(y.shape) or weight.numel() != u.shape[1] or u.shape[1] % groups:
             raise KernelError(f"group_norm shapes: u {tuple(u.shape)}, weight {tuple(weight.shape)}, {groups} groups")
         _check(self._fn("group_norm")(_ptr(u, self.dtype, "u"), _ptr(weight, torch.float32, "weight"), _ptr(y, self.dtype, "y"),
-                                      c_int(u.shape[0]), c_int(u.shape[1]), c_int(groups), c_float(eps), _stream()), "group_norm")
+                                      u.shape[0], u.shape[1], groups, c_float(eps), _stream()), "group_norm")
 
 
 class GateKernels:
@@ -1511,14 +1511,14 @@ class GateKernels:
             if w is not None:
                 w_f32 = self._flag(w, "norm weight")
         _check(self._fn("qk_norm_store")(
-            self._view(c, "c"), c_int(self._flag(c, "c")), c_int(c.stride(0)), _ptr(bias, torch.float32, "bias"),
-            self._view(q_out, "q_out"), c_int(q_out.stride(0)), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
-            _ptr(block_table, torch.int32, "block_table"), c_int(block_table.shape[1] if block_table is not None else 0),
+            self._view(c, "c"), self._flag(c, "c"), c.stride(0), _ptr(bias, torch.float32, "bias"),
+            self._view(q_out, "q_out"), q_out.stride(0), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
+            _ptr(block_table, torch.int32, "block_table"), (block_table.shape[1] if block_table is not None else 0),
             _ptr(cos_sin, torch.float32, "cos_sin"), _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c_int(c.shape[0]), c_int(n_heads), c_int(n_kv),
-            c_int(head_dim), c_int(v_dim), c_int(rot), c_int(1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
-            _ptr(k_weight, None, "k_weight"), c_int(w_f32), c_int(1 if per_head else 0), c_float(eps),
-            _ptr(kept, self.dtype if kept is not None else None, "kept"), c_int(mode), c_float(lam), c_int(1 if norm_after else 0),
+            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c.shape[0], n_heads, n_kv,
+            head_dim, v_dim, rot, (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
+            _ptr(k_weight, None, "k_weight"), w_f32, (1 if per_head else 0), c_float(eps),
+            _ptr(kept, self.dtype if kept is not None else None, "kept"), mode, c_float(lam), (1 if norm_after else 0),
             _stream()), "qk_norm_store")
 
     FUSED_CONV_MAX_WIDTH = 200 * 1024 // 4      # the row stays in shared memory as floats
@@ -1538,23 +1538,23 @@ class GateKernels:
             if w is not None:
                 w_f32 = self._flag(w, "norm weight")
         _check(self._fn("conv_qk_norm_store")(
-            self._view(y, "y"), c_int(y.stride(0)), _ptr(conv_weight, None, "conv_weight"), c_int(self._flag(conv_weight, "conv_weight")),
-            c_int(taps), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), c_int(ctx.n_seqs),
-            c_int(1 if ctx.is_decode else 0), self._view(q_out, "q_out"), c_int(q_out.stride(0)),
+            self._view(y, "y"), y.stride(0), _ptr(conv_weight, None, "conv_weight"), self._flag(conv_weight, "conv_weight"),
+            taps, _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), ctx.n_seqs,
+            (1 if ctx.is_decode else 0), self._view(q_out, "q_out"), q_out.stride(0),
             _ptr(ctx.tok_pos, torch.int32, "tok_pos"), _ptr(block_table, torch.int32, "block_table"),
-            c_int(block_table.shape[1] if block_table is not None else 0), _ptr(cos_sin, torch.float32, "cos_sin"),
+            (block_table.shape[1] if block_table is not None else 0), _ptr(cos_sin, torch.float32, "cos_sin"),
             _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c_int(T), c_int(n_heads), c_int(n_kv),
-            c_int(head_dim), c_int(v_dim), c_int(rot), c_int(1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
-            _ptr(k_weight, None, "k_weight"), c_int(w_f32), c_float(eps), _stream()), "conv_qk_norm_store")
+            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, n_heads, n_kv,
+            head_dim, v_dim, rot, (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
+            _ptr(k_weight, None, "k_weight"), w_f32, c_float(eps), _stream()), "conv_qk_norm_store")
         if not ctx.is_decode:
             LAUNCHES[0] += 1
 
     def head_gate(self, o, g, n_heads, v_dim):
         """o [T, n_heads * v_dim] (element type) *= sigmoid(g [T, n_heads]) per head; g a view, float32 or element type."""
-        _check(self._fn("head_gate")(self._view(o, "o"), c_int(o.stride(0)), self._view(g, "g"), c_int(self._flag(g, "g")),
-                                     c_int(g.stride(0)), c_int(o.shape[0]), c_int(n_heads), c_int(v_dim), _stream()), "head_gate")
+        _check(self._fn("head_gate")(self._view(o, "o"), o.stride(0), self._view(g, "g"), self._flag(g, "g"),
+                                     g.stride(0), o.shape[0], n_heads, v_dim, _stream()), "head_gate")
 
     def add_cast(self, x, delta, xb):
         """x float32 [T, d] += delta (None, [T, d] float32 or element type, or float32 [P, T, d] partial sums);
@@ -1563,7 +1563,7 @@ class GateKernels:
         if delta is not None and (tuple(delta.shape[-2:]) != tuple(x.shape) or not delta.is_contiguous()):
             raise KernelError(f"addend {tuple(delta.shape)} does not fit the stream {tuple(x.shape)}")
         _check(self._fn("add_cast")(_ptr(x, torch.float32, "x"), _ptr(delta, None, "delta"),
-                                    c_int(self._flag(delta, "delta") if delta is not None else 0), c_int(P),
+                                    (self._flag(delta, "delta") if delta is not None else 0), P,
                                     _ptr(xb, self.dtype, "xb"), ctypes.c_longlong(x.numel()), _stream()), "add_cast")
 
     def add_list_cast(self, x, addends, xb=None, vec=None):
@@ -1578,15 +1578,15 @@ class GateKernels:
         ptrs = (c_void_p * max(n, 1))(*[a.data_ptr() for a in addends])
         f32 = (c_int * max(n, 1))(*[self._flag(a, "addend") for a in addends])
         parts = (c_int * max(n, 1))(*[a.shape[0] if a.dim() == 3 else 1 for a in addends])
-        _check(self._fn("add_list_cast")(_ptr(x, torch.float32, "x"), ptrs, f32, parts, c_int(n), _ptr(vec, torch.float32, "vec"),
-                                         c_int(x.shape[1]), _ptr(xb, self.dtype if xb is not None else None, "xb"),
+        _check(self._fn("add_list_cast")(_ptr(x, torch.float32, "x"), ptrs, f32, parts, n, _ptr(vec, torch.float32, "vec"),
+                                         x.shape[1], _ptr(xb, self.dtype if xb is not None else None, "xb"),
                                          ctypes.c_longlong(x.numel()), _stream()), "add_list_cast")
 
     def gelu_mul_rows(self, a, ids, table, col0, out):
         """out [T, D] = gelu_tanh(a [T, D]) * table[ids[t], col0 : col0 + D]."""
-        _check(self._fn("gelu_mul_rows")(self._view(a, "a"), c_int(a.stride(0)), _ptr(ids, torch.int32, "ids"),
-                                         _ptr(table, self.dtype, "table"), c_int(table.shape[1]), c_int(col0),
-                                         _ptr(out, self.dtype, "out"), c_int(a.shape[0]), c_int(a.shape[1]), _stream()),
+        _check(self._fn("gelu_mul_rows")(self._view(a, "a"), a.stride(0), _ptr(ids, torch.int32, "ids"),
+                                         _ptr(table, self.dtype, "table"), table.shape[1], col0,
+                                         _ptr(out, self.dtype, "out"), a.shape[0], a.shape[1], _stream()),
                "gelu_mul_rows")
 
     def add_rms_normed(self, x, y, weight, eps, norm=None, rows=None, vec=None, dyt=None, y_bias=None, copy=None):
@@ -1620,10 +1620,10 @@ class GateKernels:
         if norm is not None and (tuple(out.shape) != (n_out, x.shape[1]) or not out.is_contiguous()
                                  or (w2 is not None and w2.shape[0] != x.shape[1])):
             raise KernelError(f"the norm's output {tuple(out.shape)} does not fit {n_out} rows of the stream {tuple(x.shape)}")
-        _check(self._fn("add_rms_normed")(_ptr(x, torch.float32, "x"), _ptr(y, None, "y"), c_int(self._flag(y, "y")), c_int(P),
-                                          c_int(x.shape[0]), _ptr(y_bias, torch.float32, "y_bias"),
-                                          _ptr(weight, None, "weight"), c_int(self._flag(weight, "weight")), c_int(x.shape[1]), c_float(eps), _ptr(rows, torch.int32, "rows"), c_int(n_out),
-                                          _ptr(w2, None, "weight2"), c_int(self._flag(w2, "weight2") if w2 is not None else 0),
+        _check(self._fn("add_rms_normed")(_ptr(x, torch.float32, "x"), _ptr(y, None, "y"), self._flag(y, "y"), P,
+                                          x.shape[0], _ptr(y_bias, torch.float32, "y_bias"),
+                                          _ptr(weight, None, "weight"), self._flag(weight, "weight"), x.shape[1], c_float(eps), _ptr(rows, torch.int32, "rows"), n_out,
+                                          _ptr(w2, None, "weight2"), (self._flag(w2, "weight2") if w2 is not None else 0),
                                           c_float(eps2), _ptr(out, self.dtype if out is not None else None, "out"),
                                           _ptr(vec, torch.float32, "vec"), _ptr(b2, torch.float32, "bias2"), c_float(alpha2), _stream()),
                "add_rms_normed")
@@ -1664,7 +1664,7 @@ class RandomKernels:
     def fill_normal(self, out, seed: int, index: int, mean: float, std: float):
         if out.dtype not in (torch.float32, torch.bfloat16):
             raise KernelError(f"fill_normal writes float32 or bfloat16, not {out.dtype}")
-        _check(self.lib.sllm_fill_normal(_ptr(out, None, "out"), c_int(0 if out.dtype == torch.float32 else 1),
+        _check(self.lib.sllm_fill_normal(_ptr(out, None, "out"), (0 if out.dtype == torch.float32 else 1),
                                          c_longlong(out.numel()), ctypes.c_ulonglong(seed & (2 ** 64 - 1)),
                                          ctypes.c_uint(index), ctypes.c_double(mean), ctypes.c_double(std), _stream()),
                "fill_normal")
@@ -1691,7 +1691,7 @@ class ProbeKernels:
         for i in range(repeats + 1):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            _check(self.lib.sllm_fma_loop(_ptr(out, torch.float32, "out"), c_int(blocks), c_int(iters), _stream()), "fma_loop")
+            _check(self.lib.sllm_fma_loop(_ptr(out, torch.float32, "out"), blocks, iters, _stream()), "fma_loop")
             e1.record()
             e1.synchronize()
             if i:
@@ -1715,7 +1715,7 @@ class SamplingKernels:
         fn.restype = c_int
         if not logits.is_cuda or logits.dtype != torch.float32:
             raise KernelError("logits must be float32 on a CUDA device")
-        _check(fn(c_void_p(logits.data_ptr()), c_int(logits.stride(0)), c_int(n), c_int(V),
+        _check(fn(c_void_p(logits.data_ptr()), logits.stride(0), n, V,
                   _ptr(params, torch.int32, "params"), _ptr(out, torch.int32, "out"), _stream()), "sample_rows")
 
     STATE_WORDS = 8   # int32 words of a sequence's state record: pos, generated, last token, flags, key x2, counter x2
@@ -1730,15 +1730,15 @@ class SamplingKernels:
             raise KernelError("sample_rows_state: state must be [slots, 8] and slots/out must cover every row")
         fn = self.lib.sllm_sample_rows_state
         fn.restype = c_int
-        _check(fn(c_void_p(logits.data_ptr()), c_int(logits.stride(0)), c_int(n), c_int(V), _ptr(options, torch.int32, "options"),
+        _check(fn(c_void_p(logits.data_ptr()), logits.stride(0), n, V, _ptr(options, torch.int32, "options"),
                   _ptr(state, torch.int32, "state"), _ptr(slots, torch.int32, "slots"), _ptr(pos_after, torch.int32, "pos_after"),
-                  _ptr(stop_ids, torch.int32, "stop_ids"), c_int(0 if stop_ids is None else stop_ids.numel()),
+                  _ptr(stop_ids, torch.int32, "stop_ids"), (0 if stop_ids is None else stop_ids.numel()),
                   _ptr(out, torch.int32, "out"), _stream()), "sample_rows_state")
 
     def repeat_penalty(self, logits, recent, counts, penalty, last_n):
         n, V = logits.shape
         fn = self.lib.sllm_repeat_penalty
         fn.restype = c_int
-        _check(fn(c_void_p(logits.data_ptr()), c_int(logits.stride(0)), c_int(n), c_int(V),
-                  _ptr(recent, torch.int32, "recent"), c_int(recent.shape[1]), _ptr(counts, torch.int32, "counts"),
-                  _ptr(penalty, torch.float32, "penalty"), c_int(last_n), _stream()), "repeat_penalty")
+        _check(fn(c_void_p(logits.data_ptr()), logits.stride(0), n, V,
+                  _ptr(recent, torch.int32, "recent"), recent.shape[1], _ptr(counts, torch.int32, "counts"),
+                  _ptr(penalty, torch.float32, "penalty"), last_n, _stream()), "repeat_penalty")
