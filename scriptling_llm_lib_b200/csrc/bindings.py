@@ -500,6 +500,26 @@ class TensorCoreGemm:
                   (0 if glu is None else 1), c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]),
                   _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_grouped")
 
+    @classmethod
+    def takes_blocks(cls, a, w) -> bool:
+        """Whether `gemm_blocks` takes a block-diagonal product of `a` [M, b K] with `w` [b, N, K] as one launch: tiles of 256 columns
+        that lie in one block, copies of 64 that end with it (one block alone is a plain product, which other kernels split better:
+        33 rows by 5,120 x 2,560 10.7 us, 15.5 here)."""
+        return (w.shape[0] > 1 and a.dtype == w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 256 == 0
+                and w.shape[2] % 64 == 0 and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0
+                and w.data_ptr() % 16 == 0)
+
+    def gemm_blocks(self, a, w, out, err_flag):
+        """out[b] (float32 [b, M, N]) = a[:, b K:(b + 1) K] @ w[b]^T, every block in one launch."""
+        nb, N, K = w.shape
+        M = a.shape[0]
+        if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or not self.takes_blocks(a, w) or not a.is_cuda:
+            raise KernelError(f"gemm_blocks: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)}")
+        fn = self.lib.sllm_gemm_tc_blocks_bf16
+        fn.restype = c_int
+        _check(fn(c_void_p(a.data_ptr()), _ptr(w, torch.bfloat16, "w"), _ptr(out, torch.float32, "out"), M, N, K, nb, a.stride(0),
+                  _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_blocks")
+
     def gemm_act(self, a, w, out, err_flag, act: str):
         """out[M, N] = act(a @ w^T): the activation on the float sums, in the product's epilogue."""
         M, K = a.shape
@@ -719,6 +739,24 @@ class DecodeKernels:
             _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K, a.stride(0),
             w.stride(0), out.stride(-2), 1 if out.dtype == torch.float32 else 0,
             (1 if swiglu else 0), ksplit, _stream()), "gemm_small_m")
+
+    BLOCKS_MAX_M = 32    # rows up to which a block-diagonal product is taken here
+
+    @classmethod
+    def takes_blocks(cls, a, w) -> bool:
+        """Whether `gemm_small_m_blocks` takes a block-diagonal product of `a` [M, b K] with `w` [b, N, K]."""
+        return (a.shape[0] <= cls.BLOCKS_MAX_M and a.dtype == w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[2] % 8 == 0
+                and w.shape[0] <= 65535 and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+    def gemm_small_m_blocks(self, a, w, out):
+        """out[b] (float32 [b, M, N]) = a[:, b K:(b + 1) K] @ w[b]^T, every block in one launch, up to BLOCKS_MAX_M rows."""
+        nb, N, K = w.shape
+        M = a.shape[0]
+        if a.shape[1] != nb * K or tuple(out.shape) != (nb, M, N) or not self.takes_blocks(a, w) or not a.is_cuda:
+            raise KernelError(f"gemm_small_m_blocks: a {tuple(a.shape)} {a.dtype}, w {tuple(w.shape)} {w.dtype}, out {tuple(out.shape)}")
+        _check(self.lib.sllm_gemm_small_m_blocks_bf16(
+            c_void_p(a.data_ptr()), _ptr(w, torch.bfloat16, "w"), _ptr(out, torch.float32, "out"), M, N, K, nb, a.stride(0),
+            _stream()), "gemm_small_m_blocks")
 
     def gemm_small_m_act(self, a, w, out, act: str):
         """out[M, N] (bfloat16) = act(a @ w^T), the activation on the float sums (names as `TensorCoreGemm.ACTS`)."""

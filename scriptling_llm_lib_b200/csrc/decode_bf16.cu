@@ -52,6 +52,7 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 #define SM_EPI_STORE 0
 #define SM_EPI_SWIGLU 1
 #define SM_EPI_RESID 2
+#define SM_EPI_BLOCKS 3      // the float store of a block-diagonal product: a template's case, so that the others keep their code
 
 // The two halves of a norm folded into its neighbours (all pointers null: nothing folded).
 struct SmFold {
@@ -67,6 +68,7 @@ struct SmFold {
   bf16* xb;
   float* sumsq_out;
   int act;              // of the plain epilogue with bfloat16 output (common.cuh: act_of)
+  int blocks;           // SM_EPI_BLOCKS: blockIdx.z is the block, W[b][N][K], x's columns from b K on, y[b][M][ldy]
 };
 
 __device__ __forceinline__ float ld_dep_f32(const float* p) {      // of data an earlier kernel of the stream wrote
@@ -83,6 +85,11 @@ gemm_small_m_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, void
   __shared__ float row_scale[NT * 8];
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   int n0 = blockIdx.x * 16;
+  if constexpr (EPI == SM_EPI_BLOCKS) {
+    W += (size_t)blockIdx.z * N * ldw;
+    x += (size_t)blockIdx.z * K;
+    y = (float*)y + (size_t)blockIdx.z * M * ldy;
+  }
   const bf16* w0 = W + (size_t)min(n0 + g, N - 1) * ldw;
   const bf16* w1 = W + (size_t)min(n0 + g + 8, N - 1) * ldw;
   float acc[NT][4];
@@ -201,7 +208,9 @@ gemm_small_m_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, void
     for (int w = 0; w < WARPS; w++) s += red[w][i][r][ln];
     const int feat = n0 + (ln >> 2) + 8 * (r >> 1), tok = 8 * i + 2 * (ln & 3) + (r & 1);
     if (f.sumsq_in != nullptr && tok < M) s *= row_scale[tok];
-    if (EPI == SM_EPI_STORE) {
+    if (EPI == SM_EPI_BLOCKS) {
+      if (feat < N && tok < M) ((float*)y)[(size_t)tok * ldy + feat] = s;
+    } else if (EPI == SM_EPI_STORE) {
       if (feat < N && tok < M) {
         if (out_f32) ((float*)y)[((size_t)blockIdx.y * M + tok) * ldy + feat] = s;
         else ((bf16*)y)[(size_t)tok * ldy + feat] = __float2bfloat16_rn(act_of(f.act, s));
@@ -260,7 +269,7 @@ static int sllm_sm_count() {
 template <int NT, int WARPS, int EPI>
 static int small_m_launch_w(const bf16* x, const bf16* W, void* y, int M, int N, int K, int ldx, int ldw, int ldy,
                             int out_f32, int ksplit, const SmFold& f, cudaStream_t stream) {
-  dim3 grid((N + 15) / 16, ksplit);
+  dim3 grid((N + 15) / 16, ksplit, EPI == SM_EPI_BLOCKS ? f.blocks : 1);
   constexpr int UN = NT <= 2 ? 2 : 1;
   if constexpr (NT <= 2 && WARPS == 4) {
     // Blocks are equal pieces of work, so a last wave that is nearly empty costs a whole one. With one chunk
@@ -270,7 +279,7 @@ static int small_m_launch_w(const bf16* x, const bf16* W, void* y, int M, int N,
     // times the blocks a wave holds. Measured at 8 rows: 1,024 blocks 13.4 -> 12.3 us, 1,792 blocks 43.7 ->
     // 41.3 us, 3,072 blocks 35.5 -> 34.4 us; at 16 rows: 512 blocks of K 8,192 13.1 -> 10.2 us, 1,024 blocks
     // 18.1 -> 15.4 us.
-    const long long blocks = (long long)grid.x * grid.y, sms = sllm_sm_count();
+    const long long blocks = (long long)grid.x * grid.y * grid.z, sms = sllm_sm_count();
     auto cost = [&](int per_sm) { const long long wave = per_sm * sms; return (blocks + wave - 1) / wave * wave; };
     const long long usual = cost(NT == 1 ? 4 : 3);
     static const bool usual_only = getenv("SLLM_SMALL_M_USUAL") != nullptr;   // for comparisons
@@ -340,6 +349,21 @@ SLLM_EXPORT int sllm_gemm_small_m_fold_bf16(const void* x, const void* W, void* 
                                             cudaStream_t stream) {
   return gemm_small_m_dispatch(x, W, y, M, N, K, ldx, ldw, ldy, out_f32, epilogue, ksplit, sumsq_in, n_in, width_in, eps_in, norm_w,
                                xb, sumsq_out, 0, stream);
+}
+
+// y[b][M][N] = x[:, b K : (b + 1) K] W[b][N][K]^T (float out) for every block b in one launch. Each block's products are those of a
+// launch of its own, bit for bit; ten of those (512 x 256) were ten launches of 32 blocks, each a launch's latency: 1 row 14.4 us,
+// 2.2 here; 16 rows 16.2, 2.3; 32 rows 18.1, 2.5; two of 2,560 x 1,280 8.2, 4.5 (16 rows).
+SLLM_EXPORT int sllm_gemm_small_m_blocks_bf16(const void* x, const void* W, float* y, int M, int N, int K, int blocks, int ldx,
+                                              cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || blocks <= 0) return 0;
+  if (M > 32 || K <= 0 || (K & 7) || (ldx & 7) || blocks > 65535 || ((uintptr_t)x & 15) || ((uintptr_t)W & 15)) return SLLM_ERR_ARG;
+  SmFold f{};
+  f.blocks = blocks;
+  const bf16 *xp = (const bf16*)x, *wp = (const bf16*)W;
+  return M <= 8    ? small_m_launch<1, SM_EPI_BLOCKS>(xp, wp, y, M, N, K, ldx, K, N, 1, 1, f, stream)
+         : M <= 16 ? small_m_launch<2, SM_EPI_BLOCKS>(xp, wp, y, M, N, K, ldx, K, N, 1, 1, f, stream)
+                   : small_m_launch<4, SM_EPI_BLOCKS>(xp, wp, y, M, N, K, ldx, K, N, 1, 1, f, stream);
 }
 
 // y[M,N] = act(x W^T) in bfloat16, the activation (common.cuh: act_of) on the float sums

@@ -50,6 +50,9 @@ struct TcFold {
   const int* tile_group;
   int group_rows;
   const int* m_used;      // (or null) on the device: the rows of A that hold anything; tiles behind them are not worked
+  // block-diagonal (the plain store, float out): columns come in `block_cols` (a multiple of the tile's) to a block, block b
+  // multiplies A's columns from b * K on and is stored as a matrix of its own, C[b][M][block_cols]. 0: one matrix.
+  int block_cols;
   // an activation applied to the float sums before they are stored (the plain store only): 0 none, 1 the tanh form of
   // gelu, 2 the square of relu, 3 silu
   int act;
@@ -432,6 +435,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
         int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * BN;
         int b_row = n0 + (fd.tile_group ? fd.tile_group[tile % tiles_m] * fd.group_rows : 0);     // the row tile's own matrix
+        int k_own = 0;                  // where the tile's own columns of A begin
+        if constexpr (EPI == TC_EPI_STORE) k_own = fd.block_cols ? n0 / fd.block_cols * K : 0;
         for (int kb = 0; kb < nkb; kb++, it++) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
@@ -439,7 +444,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (!ok) break;
           mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
           uint32_t a_dst = smem_base + s * STAGE_BYTES;
-          tma_load_2d(a_dst, &map_a, kb * TC_BK, m0, full0 + 8 * s);
+          tma_load_2d(a_dst, &map_a, k_own + kb * TC_BK, m0, full0 + 8 * s);
           tma_load_2d(a_dst + A_BYTES, &map_b, kb * TC_BK, b_row, full0 + 8 * s);
         }
       }
@@ -484,7 +489,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int a = i & 1;
       if (!mbar_wait(acc_full0 + 8 * a, (i >> 1) & 1, abort)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0, 0, BN, C, M, N, ldc, out_f32, rp, fd);
+      if (EPI == TC_EPI_STORE && fd.block_cols)
+        tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0 % fd.block_cols, 0, BN,
+                              (float*)C + (size_t)(n0 / fd.block_cols) * M * fd.block_cols, M, fd.block_cols, ldc, out_f32, rp, fd);
+      else tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0, 0, BN, C, M, N, ldc, out_f32, rp, fd);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * a) : "memory");
@@ -603,6 +611,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         tc2_tile_origin(tile, tiles_m, tiles_n, tm, tn);
         const int m0 = tm * TC2_BM + (int)rank * 128;
         const int b_row = tn * BN + (int)rank * 128 + (fd.tile_group ? fd.tile_group[tm] * fd.group_rows : 0);     // the row tile's own matrix
+        int k_own = 0;
+        if constexpr (EPI == TC_EPI_STORE) k_own = fd.block_cols ? tn * BN / fd.block_cols * K : 0;
         for (int kb = 0; kb < nkb; kb++, it++) {
           int s = it % STAGES;
           uint32_t ph = (it / STAGES) & 1;
@@ -611,7 +621,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);     // both blocks' bytes
           uint32_t full_lead = mapa_shared(full0 + 8 * s, 0);
           uint32_t a_dst = smem_base + s * STAGE_BYTES;
-          tma_load_2d_pair(a_dst, &map_a, kb * TC_BK, m0, full_lead);
+          tma_load_2d_pair(a_dst, &map_a, k_own + kb * TC_BK, m0, full_lead);
           tma_load_2d_pair(a_dst + A_BYTES, &map_b, kb * TC_BK, b_row, full_lead);
         }
       }
@@ -668,7 +678,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       } else {
         if (!mbar_wait(acc_full0 + 8 * a, (i >> 1) & 1, abort)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0, c_lo, c_hi, C, M, N, ldc, out_f32, rp, fd);
+        if (EPI == TC_EPI_STORE && fd.block_cols)
+          tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0 % fd.block_cols, c_lo, c_hi,
+                                (float*)C + (size_t)(n0 / fd.block_cols) * M * fd.block_cols, M, fd.block_cols, ldc, out_f32, rp, fd);
+        else tc_epilogue_tile<EPI>(tmem_base + (uint32_t)(a * BN), q, lane, m0, n0, c_lo, c_hi, C, M, N, ldc, out_f32, rp, fd);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -1037,6 +1050,27 @@ SLLM_EXPORT int sllm_gemm_tc_grouped_bf16(const void* A, const void* B, void* C,
                : tc_launch<128, 6, TC_EPI_SWIGLU>(ma, mb, C, M, N, K, ldc, 0, err, stream, rp, fd);
   return big ? tc_launch<256, 4, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd)
              : tc_launch<128, 6, TC_EPI_STORE>(ma, mb, C, M, N, K, ldc, out_f32, err, stream, rp, fd);
+}
+
+// Block-diagonal: C[b][M][N] = A[:, b K : (b + 1) K] B[b][N][K]^T for every block b in one launch (float out; N a multiple of 256, so
+// that no tile has columns of two blocks, K of 64, so that no copy reads into the next block's columns of A). A launch a block
+// filled 32 of 148 SMs with 2,048 rows by 512 x 256, for four k-blocks and a latency each: ten of those 84.7 us, 19.9 here (42 MB of
+// float sums to write, 6.5); 129 rows 75.2, 8.8; 33 rows 36.8, 5.3; two of 2,560 x 1,280 39.6, 28.2 (2,048 rows), 98 and 92 (8,192).
+SLLM_EXPORT int sllm_gemm_tc_blocks_bf16(const void* A, const void* B, float* C, int M, int N, int K, int blocks, int lda, int* err,
+                                         cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || blocks <= 0) return 0;
+  if (K <= 0 || (K & 63) || (N & 255) || (lda & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15)) return SLLM_ERR_ARG;
+  if ((long long)blocks * N > 0x7fffffffLL || (long long)blocks * K > 0x7fffffffLL) return SLLM_ERR_ARG;
+  TcFold fd{};
+  fd.block_cols = N;
+  CUtensorMap ma, mb;
+  const bool pair = tc_use_pair(M, blocks * N);
+  int rc = tc_make_map(&ma, A, M, blocks * K, lda, TC_BM);
+  if (rc) return rc;
+  rc = tc_make_map(&mb, B, blocks * N, K, K, pair ? 128 : 256);
+  if (rc) return rc;
+  return pair ? tc_pair_launch<6, TC_EPI_STORE>(ma, mb, C, M, blocks * N, K, N, 1, err, stream, TcRope{}, fd)
+              : tc_launch<256, 4, TC_EPI_STORE>(ma, mb, C, M, blocks * N, K, N, 1, err, stream, TcRope{}, fd);
 }
 
 // C[M,N] = act(A[M,K] B[N,K]^T): the plain store with an activation on the float sums (1 the tanh form of gelu, 2 the

@@ -78,6 +78,10 @@ class RGLRU(Mixer):
             ctx.kernels.split.blocks(src, self.gate_w, gates, ctx.err_flag)    # every block's product in one launch
         elif src.dtype == torch.float32 == self.gate_w.dtype and ctx.kernels.gemm_nt_blocks_take(src, self.gate_w):
             ctx.kernels.gemm_nt_blocks(src, self.gate_w, gates)
+        elif src.dtype == torch.bfloat16 and ctx.kernels.decode.takes_blocks(src, self.gate_w):
+            ctx.kernels.decode.gemm_small_m_blocks(src, self.gate_w, gates)
+        elif src.dtype == torch.bfloat16 and ctx.kernels.tensor_core.takes_blocks(src, self.gate_w):
+            ctx.kernels.tensor_core.gemm_blocks(src, self.gate_w, gates, ctx.err_flag)
         else:
             for b, lin in enumerate(self.gates):
                 lin.forward(src[:, b * bs:(b + 1) * bs], ctx, out_dtype=torch.float32, out=gates[b])

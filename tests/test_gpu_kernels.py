@@ -1124,3 +1124,31 @@ def test_a_value_that_is_not_finite_is_seen_by_the_queries_that_see_it(kernel_se
             hit[row0:row0 + lens[b], (G - 1) * (H // G):, 9] = sees[:, None]
         assert int(err) == 0 and bool(hit.any()) and torch.equal(~hit, out.isfinite())
         assert float((out - plain_out)[~hit].abs().max()) <= 2.0 ** -7 * float(plain_out.abs().max())
+
+
+@pytest.mark.parametrize("blocks, M, N, K", [(10, 1, 512, 256), (5, 8, 20, 24), (3, 17, 256, 72), (2, 32, 512, 256),
+                                             (5, 33, 512, 256), (3, 128, 256, 64), (10, 129, 512, 256), (2, 700, 256, 128)])
+def test_bfloat16_block_diagonal_products(kernel_sets, blocks, M, N, K):
+    """One launch for every block, on a column slice of a wider buffer, from one row to several row tiles: each sum within what K
+    additions of exact products can lose, and with few rows the bits of a launch a block."""
+    ks, bf = kernel_sets[torch.bfloat16], torch.bfloat16
+    wide, w = dev(rand(M, blocks * K + 8, seed=3), bf), dev(rand(blocks, N, K, seed=4), bf)
+    a = wide[:, 8:]
+    out = torch.full((blocks, M, N), float("nan"), device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    few = ks.decode.takes_blocks(a, w)
+    assert few == (M <= 32) and not ks.decode.takes_blocks(wide[:, 1:1 + blocks * K], w)
+    if few:
+        ks.decode.gemm_small_m_blocks(a, w, out)
+        each = torch.empty_like(out)
+        for b in range(blocks):
+            ks.decode.gemm_small_m(a[:, b * K:(b + 1) * K], w[b], each[b])
+        assert torch.equal(out, each)
+    else:
+        assert ks.tensor_core.takes_blocks(a, w) and not ks.tensor_core.takes_blocks(wide[:, 1:1 + blocks * K], w)
+        assert not ks.tensor_core.takes_blocks(a, w[:, :N - 16].contiguous())
+        ks.tensor_core.gemm_blocks(a, w, out, err)
+    x = f64(a).view(M, blocks, K)
+    want = torch.einsum("mbk,bnk->bmn", x, f64(w))
+    room = torch.einsum("mbk,bnk->bmn", x.abs(), f64(w).abs()) * (K + 4) * 2.0 ** -23      # an addition cuts at most its last bit
+    assert ((f64(out) - want).abs() <= room).all() and err.item() == 0
