@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
+from operator import index as as_int      # a caller's number as the int it stands for; what is none (None, a float) is refused
 
 import torch
 
@@ -110,7 +111,7 @@ class KernelSet:
                                            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                                            _ptr(ctx.slots, torch.int32, "slots"), _ptr(table, self.dtype, "table"),
                                            _ptr(pair_table, self.dtype, "pair_table"), _ptr(out, torch.float32, "out"),
-                                           _ptr(copy, torch.float32, "copy"), c_float(scale), T, d, table.shape[0], buckets, c_longlong(mul_prev), c_longlong(mul_cur),
+                                           _ptr(copy, torch.float32, "copy"), c_float(scale), T, d, table.shape[0], as_int(buckets), c_longlong(mul_prev), c_longlong(mul_cur),
                                            _ptr(last, torch.int32, "last"), _ptr(err_flag, torch.int32, "err"), _stream()),
                "embed_pair_rows")
 
@@ -202,7 +203,7 @@ class KernelSet:
                                          _ptr(cos_sin, torch.float32, "cos_sin"),
                                          _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
                                          _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T,
-                                         n_heads, n_kv, head_dim, rot,
+                                         as_int(n_heads), as_int(n_kv), as_int(head_dim), as_int(rot),
                                          (1 if interleaved else 0), _stream()), "rope_kv_write")
 
     # ------------------------------------------------------------------ attention
@@ -215,8 +216,8 @@ class KernelSet:
                                       _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
                                       _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
                                       _ptr(kpages, self.dtype, "kpages"), _ptr(vpages, self.dtype, "vpages"),
-                                      n_seqs, max_new, n_heads, n_kv, head_dim,
-                                      (v_dim or head_dim), (window or 0), keep, c_float(scale),
+                                      as_int(n_seqs), as_int(max_new), as_int(n_heads), as_int(n_kv), as_int(head_dim),
+                                      as_int(v_dim or head_dim), as_int(window or 0), as_int(keep), c_float(scale),
                                       c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()), "attn_paged")
 
     def attn_decode_split(self, q, out, seq_pos0, block_table, kpages, vpages, part, n_seqs, n_heads, n_kv, head_dim,
@@ -233,9 +234,9 @@ class KernelSet:
                                              _ptr(seq_pos0, torch.int32, "seq_pos0"),
                                              _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
                                              _ptr(kpages, self.dtype, "kpages"), _ptr(vpages, self.dtype, "vpages"),
-                                             _ptr(part, torch.float32, "part"), n_seqs, n_heads, n_kv,
-                                             head_dim, v_dim, (window or 0), keep, c_float(scale),
-                                             n_split, c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()),
+                                             _ptr(part, torch.float32, "part"), as_int(n_seqs), as_int(n_heads), as_int(n_kv),
+                                             as_int(head_dim), as_int(v_dim), as_int(window or 0), as_int(keep), c_float(scale),
+                                             as_int(n_split), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), _stream()),
                "attn_decode_split")
 
     @staticmethod
@@ -403,7 +404,7 @@ class TensorCoreGemm:
         sq, width, eps = owed
         if sq.dtype != torch.float32 or sq.dim() != 2 or sq.shape[1] != M or not sq.is_contiguous():
             raise KernelError(f"sums of squares {tuple(sq.shape)} {sq.dtype} for {M} rows")
-        return _ptr(sq, torch.float32, "sumsq"), sq.shape[0], width, c_float(eps)
+        return _ptr(sq, torch.float32, "sumsq"), sq.shape[0], as_int(width), c_float(eps)
 
     FOLD_SPAN = 128      # columns to a partial sum of squares that a folded product leaves
     FOLD_MIN_M = 129     # the product that finishes a sublayer for a folded norm runs on the two-SM tiles only
@@ -469,8 +470,8 @@ class TensorCoreGemm:
             c_void_p(a.data_ptr()), c_void_p(w.data_ptr()), c_void_p(qkv.data_ptr()), M, K, a.stride(0),
             w.stride(0), qkv.stride(0), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
             _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(cos_sin, torch.float32, "cos_sin"),
-            _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), n_heads, n_kv,
-            head_dim, rot, (1 if interleaved else 0), *self._owed_args(owed, M),
+            _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), as_int(n_heads), as_int(n_kv),
+            as_int(head_dim), as_int(rot), (1 if interleaved else 0), *self._owed_args(owed, M),
             _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_qkv_rope")
 
     SKINNY_MAX_M = 128
@@ -496,7 +497,7 @@ class TensorCoreGemm:
         fn.restype = c_int
         _check(fn(_ptr(a, torch.bfloat16, "a"), _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K,
                   K, K, out.shape[1], 1 if out.dtype == torch.float32 else 0,
-                  _ptr(tile_group, torch.int32, "tile_group"), tile_rows, G, self.ACTS[act], _ptr(rows_used, torch.int32, "rows_used"),
+                  _ptr(tile_group, torch.int32, "tile_group"), as_int(tile_rows), G, self.ACTS[act], _ptr(rows_used, torch.int32, "rows_used"),
                   (0 if glu is None else 1), c_float(0.0 if glu is None else glu[0]), c_float(0.0 if glu is None else glu[1]),
                   _ptr(err_flag, torch.int32, "err_flag"), _stream()), "gemm_grouped")
 
@@ -603,7 +604,7 @@ class PrefillAttentionTC:
             _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
             _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
             _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"), c_longlong(kpages.shape[0]),
-            n_seqs, max_new, n_heads, n_kv, head_dim, v_dim, window or 0, keep, c_float(scale), c_float(softcap or 0.0),
+            as_int(n_seqs), as_int(max_new), as_int(n_heads), as_int(n_kv), as_int(head_dim), as_int(v_dim), as_int(window or 0), as_int(keep), c_float(scale), c_float(softcap or 0.0),
             _ptr(sink, torch.float32, "sink"), gp, gl, 3 if exact_weights else 1, _ptr(err_flag, torch.int32, "err_flag"), _stream()), "attn_prefill_tc")
 
 
@@ -650,11 +651,11 @@ class PrefillAttentionMMA:
         [T, n_heads * vd]): as for `PrefillAttentionTC.attn`."""
         gp, gl = _gate_args(gate, q.shape[0], n_heads * vd)
         _check(self.lib.sllm_attn_prefill_mma_bf16(
-            _ptr(q, torch.bfloat16, "q"), q.shape[1], q_hw, _ptr(out, torch.bfloat16, "out"), out.shape[1],
-            o_hw, _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
+            _ptr(q, torch.bfloat16, "q"), q.shape[1], as_int(q_hw), _ptr(out, torch.bfloat16, "out"), out.shape[1],
+            as_int(o_hw), _ptr(seq_start, torch.int32, "seq_start"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
             _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"),
-            kpages.shape[-1], _ptr(vpages, torch.bfloat16, "vpages"), vpages.shape[-1], n_seqs, max_new,
-            n_heads, n_kv, kd, vd, (window or 0), keep, c_float(scale), c_float(softcap or 0.0),
+            kpages.shape[-1], _ptr(vpages, torch.bfloat16, "vpages"), vpages.shape[-1], as_int(n_seqs), as_int(max_new),
+            as_int(n_heads), as_int(n_kv), as_int(kd), as_int(vd), as_int(window or 0), as_int(keep), c_float(scale), c_float(softcap or 0.0),
             _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_prefill_mma")
 
 
@@ -704,7 +705,7 @@ class DecodeKernels:
         with 1,152 blocks against 74.6 with 768; 6 sequences 36.1 with 1,152 against 37.2 with 960;
         16 sequences 84.6 with 1,024 against 98.8 with 1,536)."""
         pairs = max(1, n_seqs * n_kv_heads)
-        if self.lib.sllm_attn_decode_uses_mma(n_seqs, n_heads, n_kv_heads, head_dim):
+        if self.lib.sllm_attn_decode_uses_mma(as_int(n_seqs), as_int(n_heads), as_int(n_kv_heads), as_int(head_dim)):
             want, cap = ((4 if head_dim <= 64 else 2) * sm_count) // pairs, max(1, pages // 4)
         else:
             want, cap = ((39 if n_heads == n_kv_heads else 17) * sm_count) // (5 * pairs), pages
@@ -799,13 +800,13 @@ class DecodeKernels:
             _ptr(a, torch.bfloat16, "a") if a.is_contiguous() else c_void_p(a.data_ptr()),
             _ptr(w, torch.bfloat16, "w"), _ptr(out, None, "out"), M, N, K, a.stride(0),
             w.stride(0), out.stride(-2), 1 if out.dtype == torch.float32 else 0,
-            epilogue, 1, sumsq_in, n_in, width, c_float(eps), *tail, _stream()), "gemm_small_m")
+            epilogue, 1, sumsq_in, n_in, as_int(width), c_float(eps), *tail, _stream()), "gemm_small_m")
 
     def attn_decode_rope(self, qkv, out, seq_pos0, block_table, kpages, vpages, scratch, tickets, cos_sin, rot,
                          interleaved, write_kv, n_seqs, n_heads, n_kv, head_dim, window, scale, n_split):
         """Rotary positions, cache write and attention of a decode step in one kernel: `qkv` holds the
         unrotated [q | k | v] rows of the step (only q when write_kv is false)."""
-        need = self.lib.sllm_attn_decode_scratch_bytes(n_seqs, n_heads, head_dim, n_split)
+        need = self.lib.sllm_attn_decode_scratch_bytes(as_int(n_seqs), as_int(n_heads), as_int(head_dim), as_int(n_split))
         if scratch.numel() * scratch.element_size() < need or tickets.numel() < n_seqs * n_kv:
             raise KernelError("attn_decode_rope: scratch or tickets too small")
         width = (n_heads + 2 * n_kv) * head_dim if write_kv else n_heads * head_dim
@@ -816,8 +817,8 @@ class DecodeKernels:
             _ptr(seq_pos0, torch.int32, "seq_pos0"), _ptr(block_table, torch.int32, "block_table"),
             block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
             _ptr(scratch, torch.float32, "scratch"), _ptr(tickets, torch.int32, "tickets"),
-            _ptr(cos_sin, torch.float32, "cos_sin"), rot, (1 if interleaved else 0), (1 if write_kv else 0),
-            n_seqs, n_heads, n_kv, head_dim, (window or 0), c_float(scale), n_split,
+            _ptr(cos_sin, torch.float32, "cos_sin"), as_int(rot), (1 if interleaved else 0), (1 if write_kv else 0),
+            as_int(n_seqs), as_int(n_heads), as_int(n_kv), as_int(head_dim), as_int(window or 0), c_float(scale), as_int(n_split),
             _stream()), "attn_decode_rope")
 
     def split_for(self, n_out: int, k: int, sm_count: int) -> int:
@@ -829,15 +830,15 @@ class DecodeKernels:
                     window, scale, n_split, tickets=None):
         """`tickets` (int32 [>= n_seqs * n_kv], zero before its first use, left zero): the last split
         to finish merges the partial results in the same kernel; without it a second kernel merges."""
-        need = self.lib.sllm_attn_decode_scratch_bytes(n_seqs, n_heads, head_dim, n_split)
+        need = self.lib.sllm_attn_decode_scratch_bytes(as_int(n_seqs), as_int(n_heads), as_int(head_dim), as_int(n_split))
         if scratch.numel() * scratch.element_size() < need:
             raise KernelError(f"attn_decode scratch holds {scratch.numel() * scratch.element_size()} bytes, needs {need}")
         head = (_ptr(q, torch.bfloat16, "q"), q.shape[1], _ptr(out, torch.bfloat16, "out"),
                 _ptr(seq_pos0, torch.int32, "seq_pos0"), _ptr(block_table, torch.int32, "block_table"),
                 block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"), _ptr(vpages, torch.bfloat16, "vpages"),
                 _ptr(scratch, torch.float32, "scratch"))
-        tail = (n_seqs, n_heads, n_kv, head_dim, (window or 0), c_float(scale),
-                n_split, _stream())
+        tail = (as_int(n_seqs), as_int(n_heads), as_int(n_kv), as_int(head_dim), as_int(window or 0), c_float(scale),
+                as_int(n_split), _stream())
         if tickets is None:
             _check(self.lib.sllm_attn_decode_bf16(*head, *tail), "attn_decode")
         else:
@@ -870,8 +871,8 @@ class DecodeKernels:
             _ptr(q, torch.bfloat16, "q"), q.shape[1], _ptr(out, torch.bfloat16, "out"), _ptr(seq_pos0, torch.int32, "seq_pos0"),
             _ptr(block_table, torch.int32, "block_table"), block_table.shape[1], _ptr(kpages, torch.bfloat16, "kpages"),
             _ptr(vpages, torch.bfloat16, "vpages"), _ptr(scratch, torch.float32, "scratch"), _ptr(tickets, torch.int32, "tickets"),
-            n_seqs, n_heads, n_kv, head_dim, v_dim, (window or 0), keep, c_float(scale),
-            n_split, c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_decode_general")
+            as_int(n_seqs), as_int(n_heads), as_int(n_kv), as_int(head_dim), as_int(v_dim), as_int(window or 0), as_int(keep), c_float(scale),
+            as_int(n_split), c_float(softcap or 0.0), _ptr(sink, torch.float32, "sink"), gp, gl, _stream()), "attn_decode_general")
 
 
 class SequenceKernels:
@@ -954,7 +955,7 @@ class SequenceKernels:
             _ptr(state, torch.float32, "state") if taps > 1 else c_void_p(0), _ptr(ctx.seq_start, torch.int32, "seq_start"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), self._view(y, "y"),
             self._flag(y, "y"), y.stride(0), self._view(y2, "y2") if y2 is not None else c_void_p(0),
-            (y2.stride(0) if y2 is not None else 0), T, ctx.n_seqs, C, taps,
+            (y2.stride(0) if y2 is not None else 0), T, as_int(ctx.n_seqs), C, as_int(taps),
             (1 if add_input else 0), {None: 0, "silu": 1}[act], _stream()), "causal_conv")
 
     def kv_store(self, qkv, tok_pos, tok_seq, block_table, cos_sin, kpages, vpages, n_heads, n_kv, head_dim, v_dim, rot,
@@ -966,8 +967,8 @@ class SequenceKernels:
                                     _ptr(tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"),
                                     block_table.shape[1], _ptr(cos_sin, torch.float32, "cos_sin"),
                                     _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-                                    _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, n_heads,
-                                    n_kv, head_dim, v_dim, rot, (1 if interleaved else 0),
+                                    _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, as_int(n_heads),
+                                    as_int(n_kv), as_int(head_dim), as_int(v_dim), as_int(rot), (1 if interleaved else 0),
                                     c_float(-1.0 if v_eps is None else v_eps), _stream()), "kv_store")
 
     def attn_wide_value(self, q, out, tok_pos, tok_seq, block_table, kpages, vpages, n_heads, n_kv, head_dim, v_dim, window, scale):
@@ -975,8 +976,8 @@ class SequenceKernels:
                                            out.shape[1], _ptr(tok_pos, torch.int32, "tok_pos"),
                                            _ptr(tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"),
                                            block_table.shape[1], _ptr(kpages, self.dtype, "kpages"),
-                                           _ptr(vpages, self.dtype, "vpages"), q.shape[0], n_heads, n_kv,
-                                           head_dim, v_dim, (window or 0), c_float(scale), _stream()),
+                                           _ptr(vpages, self.dtype, "vpages"), q.shape[0], as_int(n_heads), as_int(n_kv),
+                                           as_int(head_dim), as_int(v_dim), as_int(window or 0), c_float(scale), _stream()),
                "attn_wide_value")
 
     def delta_prepare(self, qk, ba, a_log, dt_bias, bd, n_heads, n_kv, dk):
@@ -988,7 +989,7 @@ class SequenceKernels:
         _check(self._fn("delta_prepare")(self._view(qk, "qk"), qk.stride(0), self._view(ba, "ba"), ba.stride(0),
                                          _ptr(a_log, None, "a_log"), _ptr(dt_bias, None, "dt_bias"),
                                          self._flag(a_log, "a_log"), _ptr(bd, torch.float32, "bd"), qk.shape[0],
-                                         n_heads, n_kv, dk, _stream()), "delta_prepare")
+                                         as_int(n_heads), as_int(n_kv), as_int(dk), _stream()), "delta_prepare")
 
     def delta_rule(self, qk, v, bd, state, ctx, o, n_heads, n_kv, dk, dv):
         """qk float32 rows [G dk queries | G dk keys] (unit vectors), v float32 [T, H dv], bd float32 [T, 2H + G]
@@ -1008,13 +1009,13 @@ class SequenceKernels:
         _check(self._fn("delta_rule")(self._view(qk, "qk"), qk.stride(0), self._view(v, "v"), v.stride(0),
                                       _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"),
                                       _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
-                                      _ptr(o, torch.float32, "o"), ctx.n_seqs, max(1, ctx.max_new), n_heads,
-                                      n_kv, dk, dv, _stream()), "delta_rule")
+                                      _ptr(o, torch.float32, "o"), as_int(ctx.n_seqs), as_int(max(1, ctx.max_new)), as_int(n_heads),
+                                      as_int(n_kv), as_int(dk), as_int(dv), _stream()), "delta_rule")
 
     def gated_unit_rms(self, o, gate, weight, y, n_heads, dv, eps):
         _check(self._fn("gated_unit_rms")(_ptr(o, torch.float32, "o"), self._view(gate, "gate"), gate.stride(0),
                                           _ptr(weight, None, "weight"), self._flag(weight, "weight"),
-                                          _ptr(y, self.dtype, "y"), o.shape[0], n_heads, dv, c_float(eps),
+                                          _ptr(y, self.dtype, "y"), o.shape[0], as_int(n_heads), as_int(dv), c_float(eps),
                                           _stream()), "gated_unit_rms")
 
     SCAN_WALK_MAX = 4     # rows of a sequence in one step up to which a thread walks them one after the other
@@ -1034,8 +1035,8 @@ class SequenceKernels:
                                       _ptr(lam, None, "lam"), _ptr(y_b, None, "y_b"), self._flag(lam, "lam"),
                                       _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                                       _ptr(ctx.slots, torch.int32, "slots"), _ptr(out, self.dtype, "out"),
-                                      _ptr(scratch, torch.float32, "scratch"), max(1, ctx.max_new), T,
-                                      ctx.n_seqs, W, block_size, _stream()), "rglru_scan")
+                                      _ptr(scratch, torch.float32, "scratch"), as_int(max(1, ctx.max_new)), T,
+                                      as_int(ctx.n_seqs), W, as_int(block_size), _stream()), "rglru_scan")
 
 
 class ChunkKernels:
@@ -1102,8 +1103,8 @@ class ChunkKernels:
         _check(self.lib.sllm_chunk_delta(
             SequenceKernels._view(qk, "qk"), qk.stride(0), SequenceKernels._view(v, "v"), v.stride(0),
             _ptr(bd, torch.float32, "bd"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), held, _ptr(o, torch.float32, "o"), ctx.n_seqs,
-            ctx.max_new, n_heads, n_kv, dk, dv,
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(scratch), c_longlong(n), held, _ptr(o, torch.float32, "o"), as_int(ctx.n_seqs),
+            as_int(ctx.max_new), as_int(n_heads), as_int(n_kv), as_int(dk), as_int(dv),
             _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "chunk_delta")
 
     def lin_attn(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
@@ -1112,10 +1113,10 @@ class ChunkKernels:
         held = self.heads_held(n, n_heads, 4 * dk * dv)
         chunk_state = torch.empty((n, held, dk, dv), dtype=torch.float32, device=o.device)
         _check(self.lib.sllm_chunk_lin_attn_bf16(
-            _ptr(proj, torch.bfloat16, "proj"), proj.shape[1], q_col, k_col, v_col,
+            _ptr(proj, torch.bfloat16, "proj"), proj.shape[1], as_int(q_col), as_int(k_col), as_int(v_col),
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), held, _ptr(o, torch.float32, "o"), ctx.n_seqs,
-            ctx.max_new, n_heads, dk, dv, _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(chunk_state), held, _ptr(o, torch.float32, "o"), as_int(ctx.n_seqs),
+            as_int(ctx.max_new), as_int(n_heads), as_int(dk), as_int(dv), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()),
             "chunk_lin_attn")
 
 
@@ -1192,20 +1193,20 @@ class MixKernels:
         if (ctx.max_new == 1 and proj.shape[0] == ctx.n_seqs and state.data_ptr() % 16 == 0
                 and self._fn("lin_attn_step_takes")(dk, dv)):
             _check(self._fn("lin_attn_step")(
-                _ptr(proj, self.dtype, "proj"), proj.shape[1], q_col, k_col, v_col,
+                _ptr(proj, self.dtype, "proj"), proj.shape[1], as_int(q_col), as_int(k_col), as_int(v_col),
                 _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-                _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), ctx.n_seqs, n_heads, dk, dv,
-                ctx.engine.sm_count, _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "lin_attn_step")
+                _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), as_int(ctx.n_seqs), as_int(n_heads), as_int(dk), as_int(dv),
+                as_int(ctx.engine.sm_count), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "lin_attn_step")
             return
         self.lin_attn_walk(proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv)
 
     def lin_attn_walk(self, proj, q_col, k_col, v_col, decay, state, ctx, o, n_heads, dk, dv):
         """`lin_attn_decay` in pieces of up to 32 rows one after the other."""
         _check(self._fn("lin_attn_decay")(
-            _ptr(proj, self.dtype, "proj"), proj.shape[1], q_col, k_col, v_col,
+            _ptr(proj, self.dtype, "proj"), proj.shape[1], as_int(q_col), as_int(k_col), as_int(v_col),
             _ptr(decay, torch.float32, "decay"), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), ctx.n_seqs, max(1, ctx.max_new),
-            n_heads, dk, dv, ctx.engine.sm_count, _stream()), "lin_attn_decay")
+            _ptr(ctx.slots, torch.int32, "slots"), _ptr(o, torch.float32, "o"), as_int(ctx.n_seqs), as_int(max(1, ctx.max_new)),
+            as_int(n_heads), as_int(dk), as_int(dv), as_int(ctx.engine.sm_count), _stream()), "lin_attn_decay")
 
     chunk = SequenceKernels.chunk
 
@@ -1221,12 +1222,12 @@ class MixKernels:
         `pages`, stores [dkv[:rank] / rms * norm_w | rotated dkv[rank:]] at the rows' places. q and dkv may be
         column slices of one buffer."""
         _check(self._fn("latent_store")(
-            self._view(q, "q"), q.stride(0), n_heads, dim,
+            self._view(q, "q"), q.stride(0), as_int(n_heads), as_int(dim),
             self._view(dkv, "dkv") if dkv is not None else c_void_p(0), (dkv.stride(0) if dkv is not None else 0),
             _ptr(norm_w, torch.float32, "norm weight"), 1, c_float(eps),
-            _ptr(cos_sin, torch.float32, "cos_sin"), rot, (1 if half else 0), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
+            _ptr(cos_sin, torch.float32, "cos_sin"), as_int(rot), (1 if half else 0), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
-            _ptr(pages, self.dtype if pages is not None else None, "pages"), q.shape[0], rank, rot_dim,
+            _ptr(pages, self.dtype if pages is not None else None, "pages"), q.shape[0], as_int(rank), as_int(rot_dim),
             _stream()), "latent_store")
 
     def latent_gather(self, pages, ctx, block_table, dense):
@@ -1240,11 +1241,11 @@ class MixKernels:
         """Keys [Wuk c | rotated part | 0] and values [Wuv c | 0] per head, as wide as kt's and vt's rows, into pages of their
         own by `table` (a prompt step from position 0), and queries [q | 0] as wide as the keys into qt (None: they stay)."""
         _check(self._fn("latent_heads")(self._view(q, "q"), q.stride(0), self._view(kv, "kv"), kv.stride(0),
-                                        self._view(dense, "dense"), dense.stride(0), rank,
+                                        self._view(dense, "dense"), dense.stride(0), as_int(rank),
                                         _ptr(ctx.tok_pos, torch.int32, "tok_pos"), _ptr(ctx.tok_seq, torch.int32, "tok_seq"),
                                         _ptr(table, torch.int32, "table"), table.shape[1], _ptr(kt, self.dtype, "kt"),
                                         _ptr(vt, self.dtype, "vt"), _ptr(qt, self.dtype if qt is not None else None, "qt"),
-                                        q.shape[0], n_heads, dim, rot_dim, v_dim, kt.shape[-1],
+                                        q.shape[0], as_int(n_heads), as_int(dim), as_int(rot_dim), as_int(v_dim), kt.shape[-1],
                                         vt.shape[-1], _stream()), "latent_heads")
 
     @property
@@ -1266,12 +1267,12 @@ class MixKernels:
         lat = self.latent
         if lat is not None and lat.takes(dim, rot_dim, 8, rank) and q.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0 and wuk.data_ptr() % 16 == 0:
             _check(lat.lib.sllm_latent_absorb_mma(self._view(q, "q"), q.stride(0), _ptr(wuk, self.dtype, "wuk"),
-                                                  _ptr(qa, torch.float32, "qa"), q.shape[0], n_heads, dim,
-                                                  rot_dim, rank, c_float(scale), _stream()), "latent_absorb_mma")
+                                                  _ptr(qa, torch.float32, "qa"), q.shape[0], as_int(n_heads), as_int(dim),
+                                                  as_int(rot_dim), as_int(rank), c_float(scale), _stream()), "latent_absorb_mma")
             return
         _check(self._fn("latent_absorb")(self._view(q, "q"), q.stride(0), _ptr(wuk, self.dtype, "wuk"),
-                                         _ptr(qa, torch.float32, "qa"), q.shape[0], n_heads, dim,
-                                         rot_dim, rank, c_float(scale), _stream()), "latent_absorb")
+                                         _ptr(qa, torch.float32, "qa"), q.shape[0], as_int(n_heads), as_int(dim),
+                                         as_int(rot_dim), as_int(rank), c_float(scale), _stream()), "latent_absorb")
 
     def latent_attn(self, qa, pages, ctx, block_table, part, n_heads, rank, rot_dim, n_split, window=0):
         """`window` > 0: a row sees its own position and the window - 1 before it; 0: every earlier one."""
@@ -1280,8 +1281,8 @@ class MixKernels:
         _check(fn(
             _ptr(qa, torch.float32, "qa"), _ptr(pages, self.dtype, "pages"), _ptr(ctx.tok_pos, torch.int32, "tok_pos"),
             _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(block_table, torch.int32, "block_table"), block_table.shape[1],
-            _ptr(part, torch.float32, "part"), qa.shape[0], n_heads, rank, rot_dim, n_split,
-            window, _stream()), "latent_attn")
+            _ptr(part, torch.float32, "part"), qa.shape[0], as_int(n_heads), as_int(rank), as_int(rot_dim), as_int(n_split),
+            as_int(window), _stream()), "latent_attn")
 
     def latent_expand(self, part, olat, wuv, out, n_heads, v_dim, rank, n_split, sink=None, gate=None):
         """Merges the splits of `part` into olat float32 [T, H, rank] (scratch), then out[t, h] = Wuv_h olat[t, h]. `sink` float32
@@ -1297,7 +1298,7 @@ class MixKernels:
         fn = lat.lib.sllm_latent_expand_mma if mma else self._fn("latent_expand")
         _check(fn(_ptr(part, torch.float32, "part"), _ptr(olat, torch.float32, "olat"),
                                          _ptr(wuv, self.dtype, "wuv"), _ptr(out, self.dtype, "out"), out.shape[1],
-                                         out.shape[0], n_heads, v_dim, rank, n_split,
+                                         out.shape[0], as_int(n_heads), as_int(v_dim), as_int(rank), as_int(n_split),
                                          _ptr(sink, torch.float32, "sink"), self._view(gate, "gate") if gate is not None else c_void_p(0),
                                          (gate.stride(0) if gate is not None else 0), mode, _stream()), "latent_expand")
         LAUNCHES[0] += 1
@@ -1337,15 +1338,15 @@ class MixKernels:
                 raise KernelError(f"selective_scan: {name} has dtype {t.dtype}, expected {self.dtype}")
         args = (self._view(x, "x"), x.stride(0), _ptr(dt_raw, torch.float32, "dt_raw"), dt_raw.shape[1],
                 _ptr(dt_bias, torch.float32, "dt_bias"), _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"),
-                1, self._view(bc, "bc"), bc.stride(0), b_col, c_col, self._view(z, "z"),
+                1, self._view(bc, "bc"), bc.stride(0), as_int(b_col), as_int(c_col), self._view(z, "z"),
                 z.stride(0), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
                 _ptr(ctx.slots, torch.int32, "slots"), self._view(out, "out"), out.stride(0))
-        tail = (ctx.n_seqs, max(1, ctx.max_new), inner, n_state, _stream())
+        tail = (as_int(ctx.n_seqs), as_int(max(1, ctx.max_new)), as_int(inner), as_int(n_state), _stream())
         if self.scan_pays(x.shape[0], ctx.n_seqs, ctx.max_new, inner, n_state, ctx.engine.sm_count):
             T, rows = x.shape[0], self.scan_piece_rows(x.shape[0], inner, ctx.engine.sm_count)
             n = T // rows + ctx.n_seqs
             scratch = [torch.empty(shape, dtype=torch.float32, device=x.device) for shape in ((T, inner), (n, n_state, inner), (n, inner))]
-            _check(self._fn("selective_scan_pieces")(*args, *(_ptr(t) for t in scratch), rows, *tail), "selective_scan_pieces")
+            _check(self._fn("selective_scan_pieces")(*args, *(_ptr(t) for t in scratch), as_int(rows), *tail), "selective_scan_pieces")
             return
         _check(self._fn("selective_scan")(*args, *tail), "selective_scan")
 
@@ -1361,7 +1362,7 @@ class MixKernels:
         mode = self.ROUTERS[router] if router is not None else (1 if top_softmax else 0)
         _check(self._fn("moe_route")(_ptr(z, torch.float32, "z"), _ptr(correction, torch.float32, "correction"), 1,
                                      _ptr(idx, torch.int32, "idx"), _ptr(wgt, torch.float32, "wgt"), T, E,
-                                     n_groups, keep, top, c_float(scale), mode,
+                                     as_int(n_groups), as_int(keep), as_int(top), c_float(scale), as_int(mode),
                                      _stream()), "moe_route")
 
     def moe_pairs(self, h, wup, wdown, idx, wgt, hid, out, glu=None, tiled=False):
@@ -1396,8 +1397,8 @@ class MixKernels:
             raise KernelError(f"moe_group_rows: offsets {tuple(offsets.shape)} for {n_experts} experts, {rows} rows")
         _check(self._fn("moe_group_rows")(_ptr(idx, torch.int32, "idx"), _ptr(offsets, torch.int32, "offsets"),
                                           _ptr(pair_of_row, torch.int32, "pair_of_row"), _ptr(row_of_pair, torch.int32, "row_of_pair"),
-                                          _ptr(tile_group, torch.int32, "tile_group"), T, top, n_experts, pad,
-                                          rows, _stream()), "moe_group_rows")
+                                          _ptr(tile_group, torch.int32, "tile_group"), T, top, as_int(n_experts), as_int(pad),
+                                          as_int(rows), _stream()), "moe_group_rows")
 
     def moe_grouped(self, h, wup, wdown, wgt, offsets, pair_of_row, hid, out, glu=None, raw=None, tiled=False):
         """The experts' products over rows grouped without padding (`moe_group_rows` with pad 1), float32 sums on
@@ -1420,7 +1421,7 @@ class MixKernels:
         if row_of_pair.numel() != h.shape[0] * top:
             raise KernelError(f"moe_gather_rows: {row_of_pair.numel()} pairs of {h.shape[0]} rows, {top} each")
         _check(self._fn("moe_gather_rows")(self._view(h, "h"), h.stride(0), _ptr(row_of_pair, torch.int32, "row_of_pair"),
-                                           top, _ptr(xs, self.dtype, "xs"), h.shape[0], xs.shape[1], _stream()),
+                                           as_int(top), _ptr(xs, self.dtype, "xs"), h.shape[0], xs.shape[1], _stream()),
                "moe_gather_rows")
 
     def moe_combine(self, ys, row_of_pair, wgt, out):
@@ -1479,7 +1480,7 @@ class SsdKernels:
                 self._view(xbc, "xbc"), xbc.stride(0), self._view(dt, "dt"), dt.stride(0), _ptr(dt_bias, torch.float32, "dt_bias"),
                 _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), z.stride(0),
                 _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
-                self._view(out, "out"), out.stride(0), T, n_heads, n_groups, head_dim, n_state,
+                self._view(out, "out"), out.stride(0), T, as_int(n_heads), as_int(n_groups), as_int(head_dim), as_int(n_state),
                 self._sms(out.device), _ptr(getattr(ctx, "err_flag", None), torch.int32, "err_flag"), _stream()), "ssd_step")
             return None
         states = decays = sums = sumsq = None
@@ -1495,8 +1496,8 @@ class SsdKernels:
             _ptr(a_log, torch.float32, "a_log"), _ptr(dskip, torch.float32, "dskip"), self._view(z, "z"), z.stride(0),
             _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"), _ptr(ctx.slots, torch.int32, "slots"),
             self._view(out, "out"), out.stride(0), _ptr(weight, torch.float32, "weight"), _ptr(sumsq, torch.float32, "sumsq"),
-            _ptr(states, torch.float32, "states"), _ptr(decays, torch.float32, "decays"), _ptr(sums, torch.float32, "sums"), ctx.n_seqs, max(1, ctx.max_new),
-            T, n_heads, n_groups, head_dim, n_state, _stream()), "ssd")
+            _ptr(states, torch.float32, "states"), _ptr(decays, torch.float32, "decays"), _ptr(sums, torch.float32, "sums"), as_int(ctx.n_seqs), as_int(max(1, ctx.max_new)),
+            T, as_int(n_heads), as_int(n_groups), as_int(head_dim), as_int(n_state), _stream()), "ssd")
         if chunked:
             LAUNCHES[0] += 2
         return sumsq
@@ -1506,7 +1507,7 @@ class SsdKernels:
         if tuple(u.shape) != tuple(y.shape) or weight.numel() != u.shape[1] or u.shape[1] % groups:
             raise KernelError(f"group_norm shapes: u {tuple(u.shape)}, weight {tuple(weight.shape)}, {groups} groups")
         _check(self._fn("group_norm")(_ptr(u, self.dtype, "u"), _ptr(weight, torch.float32, "weight"), _ptr(y, self.dtype, "y"),
-                                      u.shape[0], u.shape[1], groups, c_float(eps), _stream()), "group_norm")
+                                      u.shape[0], u.shape[1], as_int(groups), c_float(eps), _stream()), "group_norm")
 
 
 class GateKernels:
@@ -1553,8 +1554,8 @@ class GateKernels:
             self._view(q_out, "q_out"), q_out.stride(0), _ptr(tok_pos, torch.int32, "tok_pos"), _ptr(tok_seq, torch.int32, "tok_seq"),
             _ptr(block_table, torch.int32, "block_table"), (block_table.shape[1] if block_table is not None else 0),
             _ptr(cos_sin, torch.float32, "cos_sin"), _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c.shape[0], n_heads, n_kv,
-            head_dim, v_dim, rot, (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
+            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), c.shape[0], as_int(n_heads), as_int(n_kv),
+            as_int(head_dim), as_int(v_dim), as_int(rot), (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
             _ptr(k_weight, None, "k_weight"), w_f32, (1 if per_head else 0), c_float(eps),
             _ptr(kept, self.dtype if kept is not None else None, "kept"), mode, c_float(lam), (1 if norm_after else 0),
             _stream()), "qk_norm_store")
@@ -1577,14 +1578,14 @@ class GateKernels:
                 w_f32 = self._flag(w, "norm weight")
         _check(self._fn("conv_qk_norm_store")(
             self._view(y, "y"), y.stride(0), _ptr(conv_weight, None, "conv_weight"), self._flag(conv_weight, "conv_weight"),
-            taps, _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
-            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), ctx.n_seqs,
+            as_int(taps), _ptr(state, torch.float32, "state"), _ptr(ctx.seq_start, torch.int32, "seq_start"),
+            _ptr(ctx.tok_seq, torch.int32, "tok_seq"), _ptr(ctx.slots, torch.int32, "slots"), as_int(ctx.n_seqs),
             (1 if ctx.is_decode else 0), self._view(q_out, "q_out"), q_out.stride(0),
             _ptr(ctx.tok_pos, torch.int32, "tok_pos"), _ptr(block_table, torch.int32, "block_table"),
             (block_table.shape[1] if block_table is not None else 0), _ptr(cos_sin, torch.float32, "cos_sin"),
             _ptr(kpages, self.dtype if kpages is not None else None, "kpages"),
-            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, n_heads, n_kv,
-            head_dim, v_dim, rot, (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
+            _ptr(vpages, self.dtype if vpages is not None else None, "vpages"), T, as_int(n_heads), as_int(n_kv),
+            as_int(head_dim), as_int(v_dim), as_int(rot), (1 if interleaved else 0), _ptr(q_weight, None, "q_weight"),
             _ptr(k_weight, None, "k_weight"), w_f32, c_float(eps), _stream()), "conv_qk_norm_store")
         if not ctx.is_decode:
             LAUNCHES[0] += 1
@@ -1592,7 +1593,7 @@ class GateKernels:
     def head_gate(self, o, g, n_heads, v_dim):
         """o [T, n_heads * v_dim] (element type) *= sigmoid(g [T, n_heads]) per head; g a view, float32 or element type."""
         _check(self._fn("head_gate")(self._view(o, "o"), o.stride(0), self._view(g, "g"), self._flag(g, "g"),
-                                     g.stride(0), o.shape[0], n_heads, v_dim, _stream()), "head_gate")
+                                     g.stride(0), o.shape[0], as_int(n_heads), as_int(v_dim), _stream()), "head_gate")
 
     def add_cast(self, x, delta, xb):
         """x float32 [T, d] += delta (None, [T, d] float32 or element type, or float32 [P, T, d] partial sums);
@@ -1623,7 +1624,7 @@ class GateKernels:
     def gelu_mul_rows(self, a, ids, table, col0, out):
         """out [T, D] = gelu_tanh(a [T, D]) * table[ids[t], col0 : col0 + D]."""
         _check(self._fn("gelu_mul_rows")(self._view(a, "a"), a.stride(0), _ptr(ids, torch.int32, "ids"),
-                                         _ptr(table, self.dtype, "table"), table.shape[1], col0,
+                                         _ptr(table, self.dtype, "table"), table.shape[1], as_int(col0),
                                          _ptr(out, self.dtype, "out"), a.shape[0], a.shape[1], _stream()),
                "gelu_mul_rows")
 
@@ -1729,7 +1730,7 @@ class ProbeKernels:
         for i in range(repeats + 1):
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            _check(self.lib.sllm_fma_loop(_ptr(out, torch.float32, "out"), blocks, iters, _stream()), "fma_loop")
+            _check(self.lib.sllm_fma_loop(_ptr(out, torch.float32, "out"), as_int(blocks), as_int(iters), _stream()), "fma_loop")
             e1.record()
             e1.synchronize()
             if i:
@@ -1779,4 +1780,4 @@ class SamplingKernels:
         fn.restype = c_int
         _check(fn(c_void_p(logits.data_ptr()), logits.stride(0), n, V,
                   _ptr(recent, torch.int32, "recent"), recent.shape[1], _ptr(counts, torch.int32, "counts"),
-                  _ptr(penalty, torch.float32, "penalty"), last_n, _stream()), "repeat_penalty")
+                  _ptr(penalty, torch.float32, "penalty"), as_int(last_n), _stream()), "repeat_penalty")
