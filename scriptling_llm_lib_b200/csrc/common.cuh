@@ -180,7 +180,8 @@ __device__ __forceinline__ void st4(bf16* p, float4 v) {
   r.y = *(uint32_t*)&hi;
   *(uint2*)p = r;
 }
-// two neighbouring floats as three packed pairs of bfloat16 that add up to them
+// two neighbouring floats as three packed pairs of bfloat16 that add up to them (from 2^-110 on; below, the last bits lie under the smallest
+// bfloat16)
 __device__ __forceinline__ void split_pair(float u, float v, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
   const __nv_bfloat162 a = __floats2bfloat162_rn(u, v);
   p0 = *(const uint32_t*)&a;

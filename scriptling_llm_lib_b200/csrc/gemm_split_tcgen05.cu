@@ -1,8 +1,10 @@
 // Products of float matrices on the 5th-generation tensor cores: C[M,N] = A[M,K] * B[N,K]^T.
 //
-// A float is the sum of three bfloat16 numbers (see split_mma.cuh: 8 + 8 + 8 bits). A first kernel writes both operands as three
-// planes of bfloat16, a second one multiplies the planes: the six largest terms (2,0) (0,2) (1,1) (1,0) (0,1) (0,0) of a product of
-// two such sums, smallest first; what is left out comes to 2^-24 of the product at most.
+// A float of 2^-110 or more is the sum of three bfloat16 numbers (see split_mma.cuh: 8 + 8 + 8 bits); below, its last bits lie under
+// the smallest bfloat16. So a first kernel writes both operands times 2^24 as three planes of bfloat16: exact for every float up to
+// 2^104, subnormal ones included. A second one multiplies the planes: the six largest terms (2,0) (0,2) (1,1) (1,0) (0,1) (0,0) of a
+// product of two such sums, smallest first; what is left out comes to 2^-24 of the product at most. Results are scaled back by 2^-48; what
+// overflows under way, a float above 2^104 or a sum of 2^80 or more, goes the way of what is not finite (below).
 //
 // Sums in tensor memory cut what does not fit their 24 bits at every step, which a long sum cannot afford (8,192 terms in one
 // accumulator: 9.1e-6 off, a chain of FMA 1.6e-6). So a sum ends after 64 terms of K: the epilogue's warps keep the tile's outputs as
@@ -23,6 +25,7 @@
 #define GS_BK 64
 #define GS_BM 256
 #define GS_THREADS 320            // a warp of copies, a warp of products, eight of sums
+#define GS_SCALE 0x1p24f          // of either operand in its planes
 #define GS_SLOTS 6                // three parts of a k-block, two k-blocks
 
 // One operand's floats as three planes [3][rows][cols] of bfloat16, eight elements a thread; both operands in one launch (blockIdx.y).
@@ -35,7 +38,9 @@ __global__ void __launch_bounds__(256) gemm_split_planes_kernel(const GsSplit sa
   const long long total = (long long)s.rows * groups, plane = (long long)s.rows * s.cols;
   for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
     const int row = (int)(i / groups), c = (int)(i - (long long)row * groups) << 3;
-    const F8 f = ld8(s.src + (size_t)row * s.ld + c);
+    F8 f = ld8(s.src + (size_t)row * s.ld + c);
+#pragma unroll
+    for (int e = 0; e < 8; e++) f.f[e] *= GS_SCALE;
     uint4 q[3];
     split_pair(f.f[0], f.f[1], q[0].x, q[1].x, q[2].x);
     split_pair(f.f[2], f.f[3], q[0].y, q[1].y, q[2].y);
@@ -225,6 +230,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (lane == 0) mbar_arrive_cluster(mapa_shared(acc_empty0 + 8 * a, 0));
       }
       if (!ok) break;
+#pragma unroll
+      for (int j = 0; j < OWN; j++) sum[j] *= 1.0f / (GS_SCALE * GS_SCALE);
       const int row = m0 + (int)rank * 128 + q * 32 + lane, col = n0 + c_lo;
       if (row < g.M && col < g.N) {
         float* dst = g.c + (g.parts > 1 || g.batch > 1 ? z * g.c_part : 0) + (size_t)row * g.ldc + col;

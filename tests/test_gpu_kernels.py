@@ -526,6 +526,22 @@ def test_gemm_split_is_at_least_as_exact_as_the_chain(kernel_sets, M, N, K):
     assert torch.equal(again, out) and int(flag) == 0
 
 
+@pytest.mark.parametrize("ea, ew", [(-115, 0), (-125, 0), (0, -120), (-140, 20), (-100, 90), (100, -140), (-60, -50), (70, 40), (110, -60)])
+def test_gemm_split_keeps_small_and_large_operands(kernel_sets, ea, ew):
+    """Operands as small as floats go, subnormal ones included, keep their 24 bits, also beside larger ones that meet a zero; sums that leave
+    the scaled range come out as the chain of multiply-adds has them."""
+    ks, M, N, K = kernel_sets[torch.float32], 129, 40, 200
+    a, w = dev(torch.ldexp(rand(M, K, seed=3), torch.tensor(ea))), dev(torch.ldexp(rand(N, K, seed=4), torch.tensor(ew)))
+    a[:, 0], w[:, 0], w[:, 1], a[:, 1] = 1.0, 0.0, 1.0, 0.0
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want, tol = f64(a) @ f64(w).T, 2.0 ** -23 * (1 + 0.25 * math.sqrt(K / 64))
+    off = lambda got: ((got.cpu().double() - want).norm() / want.norm()).item()                  # noqa: E731
+    out, chain = (torch.full((M, N), float("nan"), device="cuda") for _ in range(2))
+    ks.split.gemm(a, w, out, flag)
+    ks.gemm_nt(a, w, chain)
+    assert off(out) <= min(tol, 1.05 * off(chain)) and int(flag) == 0
+
+
 def test_gemm_split_blocks_and_what_is_not_finite(kernel_sets):
     """A block-diagonal product in one launch; infinities, NaN and values whose first part rounds up to an infinity come out as the
     chain of multiply-adds has them."""
