@@ -20,6 +20,7 @@ from ..cache import PAGE, SequenceCache, pages_for
 from ..config.registry import architecture_for, architecture_name, load_config
 from ..csrc.bindings import CastKernels, KernelSet, SplitGemm
 from ..parts.base import Part
+from ..parts.linear import linears
 from ..weights.loader import load_weights, stored_to_kept
 from .graphs import DecodeGraphs
 from .layout import ModelLayout
@@ -352,11 +353,14 @@ class Engine:
 
     def activation_reserve_bytes(self) -> int:
         """A generous bound on what a prompt step of PROMPT_TOKENS_PER_STEP rows allocates beside
-        weights and cache (residual, products' outputs, the planes of a 32-bit product), plus the logits of
-        the captured decode steps: what the cache must leave free."""
+        weights and cache (residual, products' outputs), plus the logits of the captured decode steps: what the
+        cache must leave free. Where a matrix is kept in 32-bit, the planes of its product count too, and once more
+        for captured decode steps of many rows, whose graphs hold theirs beside what prompts allocate."""
         width = 64 * self.layout.hidden_size                        # bytes a row, all buffers of a layer alive at once
         scratch = max(p.scratch_bytes(self.PROMPT_TOKENS_PER_STEP) for p in self.model.parts() if isinstance(p, Part))
-        return self.PROMPT_TOKENS_PER_STEP * width + scratch + SplitGemm.SCRATCH_BYTES + 4 * self.layout.vocab_size * 4 * 1024
+        if any(lin.weight is not None and lin.weight.dtype == torch.float32 for p in self.model.parts() for lin in linears(p)):
+            scratch += (2 if getattr(self, "use_graphs", False) else 1) * SplitGemm.SCRATCH_BYTES
+        return self.PROMPT_TOKENS_PER_STEP * width + scratch + 4 * self.layout.vocab_size * 4 * 1024
 
     def check_errors(self) -> None:
         """Raises if a kernel of an earlier step reported an error (a wait on the device that ran out

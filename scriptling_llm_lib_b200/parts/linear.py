@@ -10,7 +10,7 @@ import torch
 
 from ..csrc.bindings import SplitGemm
 from ..weights.spec import TensorSpec
-from .base import Folded, FoldRequest
+from .base import Folded, FoldRequest, Part
 
 
 class Linear:
@@ -137,3 +137,13 @@ class Linear:
             ctx.casts.to_bf16(out32, out)
             return out
         raise ValueError(f"weight {self.names} is {w.dtype} but the engine runs in {x.dtype}")
+
+
+def linears(part):
+    """Every product that a part holds: in its attributes, in lists of them, and in the parts inside it."""
+    for v in list(getattr(part, "__dict__", {}).values()):
+        for x in v if isinstance(v, (list, tuple)) else (v,):
+            if isinstance(x, Linear):
+                yield x
+            elif isinstance(x, Part):
+                yield from linears(x)

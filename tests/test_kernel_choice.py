@@ -180,3 +180,23 @@ def test_a_decode_step_of_unequal_widths_splits_its_keys(D, V, decode, want):
     x, kp = torch.empty((3, 128), dtype=torch.float32, device="meta"), torch.empty((9, G, 64, D), dtype=torch.float32, device="meta")
     layer._attend(torch.empty((3, H * D + G * (D + V)), dtype=torch.float32, device="meta"), x, ctx, kp, kp, None, False, None, True, 0)
     assert ran == [want]
+
+
+@pytest.mark.parametrize("dtype, graphs, times", [(torch.bfloat16, True, 0), (torch.float32, False, 1), (torch.float32, True, 2)])
+def test_the_reserve_counts_the_planes_where_a_matrix_is_kept_in_32_bit(dtype, graphs, times):
+    """A bfloat16 engine's cache does not give way to products that it does not run; a captured decode step holds its own planes."""
+    from scriptling_llm_lib_b200.csrc.bindings import SplitGemm
+    from scriptling_llm_lib_b200.engine import Engine
+    from scriptling_llm_lib_b200.parts.base import FeedForward, Norm
+    from scriptling_llm_lib_b200.parts.linear import Linear
+
+    def reserve(parts):
+        return Engine.activation_reserve_bytes(SimpleNamespace(layout=SimpleNamespace(hidden_size=1024, vocab_size=512), use_graphs=graphs,
+                                                               model=SimpleNamespace(parts=lambda: parts),
+                                                               PROMPT_TOKENS_PER_STEP=Engine.PROMPT_TOKENS_PER_STEP))
+
+    plain, outer, inner, lin = reserve([Norm(), object()]), FeedForward(), FeedForward(), Linear(["w"], [64], 128)
+    outer.shared, inner.gates = inner, [Linear(["v"], [8], 8), lin]
+    assert reserve([outer]) == plain == Engine.PROMPT_TOKENS_PER_STEP * 64 * 1024 + 4 * 512 * 4 * 1024      # (its weights are not bound yet)
+    lin.bind({"w": torch.zeros(64, 128, dtype=dtype)}, dtype, "cpu")
+    assert reserve([Norm(), outer]) == plain + times * SplitGemm.SCRATCH_BYTES
