@@ -163,6 +163,22 @@ class RoutedExperts(FeedForward):
         if self.w_up.dtype != dtype:
             raise ValueError(f"the experts' matrices are {self.w_up.dtype}, the engine runs in {dtype}")
 
+    def scratch_bytes(self, rows: int) -> int:
+        """The grouped rows: inputs, hidden rows and float sums of every pair and of what pads the experts to whole tiles, and the sums of
+        their choices; on the FMA kernels hidden rows, the gate's raw rows and a sum a choice."""
+        pairs, w = rows * self.top, getattr(self, "w_up", None)
+        size = 4 if w is not None and w.dtype == torch.float32 else 2
+        if size == 2 and self.hidden % 8 == 0 and self.F % 8 == 0:
+            own = self._grouped_rows(pairs) * (2 * self.hidden + 2 * self.F + 4 * self.hidden) + 4 * rows * self.hidden
+        else:
+            own = pairs * (size * self.F * (1 if self.glu is None else 3) + 4 * self.hidden)
+        return own + (self.shared.scratch_bytes(rows) if self.shared is not None else 0)
+
+    def _grouped_rows(self, pairs: int) -> int:
+        """The most rows that so many pairs take with every expert's rounded up to whole tiles."""
+        tile = self._tile_rows(pairs)
+        return -(-(pairs + self.E * (tile - 1)) // tile) * tile
+
     def _on_tensor_cores(self, x) -> bool:
         """The grouped products can run on the tensor-core kernel: bfloat16, and the contraction widths (hidden for the
         experts' first product, their own width for the second) multiples of 8 elements (16 bytes for its copies)."""
@@ -206,7 +222,7 @@ class RoutedExperts(FeedForward):
             return out
         # every expert's rows from a multiple of a tile on, so that a tile of the tensor-core product has one expert
         tile = self._tile_rows(pairs)
-        rows = -(-(pairs + self.E * (tile - 1)) // tile) * tile
+        rows = self._grouped_rows(pairs)
         row_of_pair = torch.empty((pairs,), dtype=torch.int32, device=dev)
         tile_group = torch.empty((rows // tile,), dtype=torch.int32, device=dev)
         k.moe_group_rows(idx, self.E, offsets, None, row_of_pair, tile_group, pad=tile)

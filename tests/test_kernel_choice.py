@@ -200,3 +200,18 @@ def test_the_reserve_counts_the_planes_where_a_matrix_is_kept_in_32_bit(dtype, g
     assert reserve([outer]) == plain == Engine.PROMPT_TOKENS_PER_STEP * 64 * 1024 + 4 * 512 * 4 * 1024      # (its weights are not bound yet)
     lin.bind({"w": torch.zeros(64, 128, dtype=dtype)}, dtype, "cpu")
     assert reserve([Norm(), outer]) == plain + times * SplitGemm.SCRATCH_BYTES
+
+
+@pytest.mark.parametrize("hidden, F, E, top, act, tile", [(2048, 1024, 256, 8, "silu_glu", 256), (2048, 512, 1024, 8, "relu_squared", 256),
+                                                          (1024, 704, 32, 4, "silu_glu", 256), (1024, 704, 700, 1, "clamped_glu", 128)])
+def test_the_reserve_counts_the_grouped_rows_of_routed_experts(hidden, F, E, top, act, tile):
+    """Inputs, hidden rows and sums of every pair and of the rows that pad each expert to whole tiles; a wrapped part counts them too."""
+    from scriptling_llm_lib_b200.parts.experts import RoutedExperts
+    gated = dict(gate_names=[f"g{j}" for j in range(E)], limit=7.0 if act == "clamped_glu" else None) if act != "relu_squared" else {}
+    part = RoutedExperts(hidden, F, E, top, 1, 1, 1.0, "r", "c", [f"u{j}" for j in range(E)], [f"d{j}" for j in range(E)], act=act, **gated)
+    rows = 16384
+    padded = -(-(rows * top + E * (tile - 1)) // tile) * tile
+    assert part._tile_rows(rows * top) == tile
+    assert part.scratch_bytes(rows) == padded * (6 * hidden + 2 * F) + 4 * rows * hidden
+    part.w_up = torch.empty((1, 1, 1))                      # kept in 32-bit: the FMA kernels' buffers
+    assert part.scratch_bytes(rows) == rows * top * (4 * F * (3 if gated else 1) + 4 * hidden)
