@@ -19,7 +19,9 @@
 // 5.7e-7 / 1.1e-7, 8,192 1.6e-6 / 2.2e-7, 64 1.4e-7 / 7.8e-8; of positive ones 4.9e-7 / 1.1e-7, 1.4e-6 / 2.0e-7, 1.2e-7 / 9.2e-8.
 //
 // What is not finite comes out not finite of any term it meets (a head that rounds up to infinity included), so an output that is not
-// finite is computed again by its chain of FMA, from the floats.
+// finite is computed again by its chain of FMA, from the floats: by the warp that stored it, when its tiles are done and nothing waits
+// for it, rows that hold one eight at a time. 1,000 rows by 2,560 x 2,048 84 us, with a row of NaN 246, all NaN 1,950 (FMA kernel 393; an
+// output a thread at a time, in front of waiting tiles: the one row 5,665).
 #include "tcgen05.cuh"
 
 #define GS_BK 64
@@ -64,10 +66,86 @@ struct GsArgs {
   int b_rows;                      // rows of a plane of B
 };
 
-__device__ __noinline__ float gs_dot(const float* a, const float* b, int k0, int k1) {
-  float s = 0.f;
-  for (int k = k0; k < k1; k++) s = fmaf(a[k], b[k], s);
-  return s;
+// The outputs of a warp's 32 rows and OWN columns that are not finite, by their chains of multiply-adds from k0 to k1 (in multiples of
+// 8). A lane takes every 32nd column, ROWS of the rows marked in `rows` at a time, so that a column's weights are read once for them.
+template <int OWN, int ROWS>
+__device__ __forceinline__ void gs_rows_again(const float* a, int lda, const float* b, int ldb, float* c, int ldc, int n, uint32_t rows, int k0, int k1) {
+  constexpr int COLS = OWN / 32;
+  const int lane = threadIdx.x & 31;
+  const float* bc[COLS];
+#pragma unroll
+  for (int i = 0; i < COLS; i++) bc[i] = b + (size_t)min(lane + 32 * i, n - 1) * ldb;
+  while (rows) {
+    const float* ar[ROWS];
+    float* cr[ROWS];
+    float s[ROWS][COLS];
+    int r = 0, there = 0;
+#pragma unroll
+    for (int u = 0; u < ROWS; u++) {          // (past the last marked row: that row again, not written)
+      if (rows) { r = __ffs(rows) - 1; there++; }
+      rows &= rows - 1;
+      ar[u] = a + (size_t)r * lda;
+      cr[u] = c + (size_t)r * ldc;
+#pragma unroll
+      for (int i = 0; i < COLS; i++) s[u][i] = 0.f;
+    }
+#pragma unroll 2
+    for (int k = k0; k < k1; k += 4) {
+      float4 w[COLS];
+#pragma unroll
+      for (int i = 0; i < COLS; i++) w[i] = *(const float4*)(bc[i] + k);
+#pragma unroll
+      for (int u = 0; u < ROWS; u++) {
+        const float4 x = *(const float4*)(ar[u] + k);
+#pragma unroll
+        for (int i = 0; i < COLS; i++) s[u][i] = fmaf(x.w, w[i].w, fmaf(x.z, w[i].z, fmaf(x.y, w[i].y, fmaf(x.x, w[i].x, s[u][i]))));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < ROWS; u++)
+#pragma unroll
+      for (int i = 0; i < COLS; i++) {
+        const int col = lane + 32 * i;
+        if (u < there && col < n && !(fabsf(cr[u][col]) <= 3.402823466e+38f)) cr[u][col] = s[u][i];
+      }
+  }
+}
+
+// Tile number: z slowest, then columns, rows fastest (tiles that run side by side share B). k-blocks kb0 .. kb0 + nkb - 1
+template <int BN>
+__device__ __forceinline__ void gs_tile(const GsArgs& g, int tile, int& z, int& m0, int& n0, int& kb0, int& nkb) {
+  const int tiles_m = (g.M + GS_BM - 1) / GS_BM, per_z = tiles_m * ((g.N + BN - 1) / BN);
+  z = tile / per_z;
+  const int r = tile - z * per_z;
+  m0 = (r % tiles_m) * GS_BM;
+  n0 = (r / tiles_m) * BN;
+  kb0 = g.batch > 1 ? 0 : z * g.kb_part;
+  nkb = max(0, min(g.kb_part, (g.K + GS_BK - 1) / GS_BK - kb0));
+}
+
+// Behind a warp's last tile (its first row and column of a tile at `dm`, `dn`): the tiles in which it stored something not finite, the
+// i-th if bit i % 32 of `marked` says so.
+template <int BN>
+__device__ __noinline__ void gs_again(const GsArgs& g, int tile, int n_pairs, int n_tiles, int dm, int dn, uint32_t marked) {
+  constexpr int OWN = BN / 2;
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  for (int i = 0; tile < n_tiles; tile += n_pairs, i++) {
+    if (!(marked >> (i & 31) & 1)) continue;
+    int z, m0, n0, kb0, nkb;
+    gs_tile<BN>(g, tile, z, m0, n0, kb0, nkb);
+    const int row0 = m0 + dm, col = n0 + dn, n = min(OWN, g.N - col), k0 = kb0 * GS_BK, k1 = min(g.K, (kb0 + nkb) * GS_BK);
+    float* c = g.c + (g.parts > 1 || g.batch > 1 ? z * g.c_part : 0) + (size_t)row0 * g.ldc + col;
+    bool bad = false;
+    if (row0 + lane < g.M)
+      for (int j = 0; j < n; j++) bad |= !(fabsf(c[(size_t)lane * g.ldc + j]) <= 3.402823466e+38f);
+    const uint32_t rows = __ballot_sync(0xffffffffu, bad);
+    if (!rows) continue;
+    const float* a = g.a + (size_t)row0 * g.lda + (g.batch > 1 ? (size_t)z * g.K : 0);
+    const float* b = g.b + ((g.batch > 1 ? (size_t)z * g.N : 0) + col) * g.ldb;
+    if (__popc(rows) > 1) gs_rows_again<OWN, 8>(a, g.lda, b, g.ldb, c, g.ldc, n, rows, k0, k1);
+    else gs_rows_again<OWN, 1>(a, g.lda, b, g.ldb, c, g.ldc, n, rows, k0, k1);
+  }
 }
 
 __device__ __forceinline__ void gs_store8(float* p, const float* v) {
@@ -77,7 +155,8 @@ __device__ __forceinline__ void gs_store8(float* p, const float* v) {
 
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GS_THREADS, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GsArgs g, int* __restrict__ err) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ GsArgs g,
+                  int* __restrict__ err) {
   constexpr uint32_t A_BYTES = 128 * GS_BK * 2, B_BYTES = (BN / 2) * GS_BK * 2, SLOT_BYTES = A_BYTES + B_BYTES;
   constexpr int OWN = BN / 2;                                   // columns of an epilogue warp
   extern __shared__ uint8_t smem_raw[];
@@ -91,17 +170,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int tiles_m = (g.M + GS_BM - 1) / GS_BM, tiles_n = (g.N + BN - 1) / BN, per_z = tiles_m * tiles_n;
-  const int n_tiles = per_z * g.parts * g.batch, nkb_all = (g.K + GS_BK - 1) / GS_BK;
-  // tile number: z slowest, then columns, rows fastest (tiles that run side by side share B). k-blocks kb0 .. kb0 + nkb - 1
-  auto tile_at = [&](int tile, int& z, int& m0, int& n0, int& kb0, int& nkb) {
-    z = tile / per_z;
-    const int r = tile - z * per_z;
-    m0 = (r % tiles_m) * GS_BM;
-    n0 = (r / tiles_m) * BN;
-    kb0 = g.batch > 1 ? 0 : z * g.kb_part;
-    nkb = max(0, min(g.kb_part, nkb_all - kb0));
-  };
+  const int n_tiles = (g.M + GS_BM - 1) / GS_BM * ((g.N + BN - 1) / BN) * g.parts * g.batch;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GS_SLOTS; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
@@ -130,7 +199,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         int z, m0, n0, kb0, nkb;
-        tile_at(tile, z, m0, n0, kb0, nkb);
+        gs_tile<BN>(g, tile, z, m0, n0, kb0, nkb);
         const int am = m0 + (int)rank * 128, bn = (g.batch > 1 ? z * g.N : 0) + n0 + (int)rank * (BN / 2), ak = g.batch > 1 ? z * g.K : 0;
         for (int kb = 0; kb < nkb && ok; kb++, it++) {
           for (int part = 0; part < 3; part++) {                // plane 2 - part of both operands into slot 2 part + (it & 1)
@@ -168,7 +237,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         int z, m0, n0, kb0, nkb;
-        tile_at(tile, z, m0, n0, kb0, nkb);
+        gs_tile<BN>(g, tile, z, m0, n0, kb0, nkb);
         for (int kb = 0; kb < nkb; kb++, it++) {
           const int a = it & 1;
           const uint32_t ph = (it >> 1) & 1, acc = tmem_base + (uint32_t)(a * BN);
@@ -204,11 +273,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   } else {
     const int q = warp & 3, c_lo = warp < 6 ? 0 : OWN;
     const uint32_t trow = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c_lo;
-    int it = 0;
+    int it = 0, i = 0;
+    uint32_t marked = 0;                // of the tiles, by their number modulo 32: something not finite was stored
     bool ok = true;
-    for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+    for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, i++) {
       int z, m0, n0, kb0, nkb;
-      tile_at(tile, z, m0, n0, kb0, nkb);
+      gs_tile<BN>(g, tile, z, m0, n0, kb0, nkb);
       float sum[OWN];
 #pragma unroll
       for (int j = 0; j < OWN; j++) sum[j] = 0.f;
@@ -233,10 +303,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
       for (int j = 0; j < OWN; j++) sum[j] *= 1.0f / (GS_SCALE * GS_SCALE);
       const int row = m0 + (int)rank * 128 + q * 32 + lane, col = n0 + c_lo;
+      bool bad = false;
       if (row < g.M && col < g.N) {
         float* dst = g.c + (g.parts > 1 || g.batch > 1 ? z * g.c_part : 0) + (size_t)row * g.ldc + col;
         const bool vec = ((uintptr_t)dst & 31) == 0;
-        bool bad = false;
 #pragma unroll
         for (int j = 0; j < OWN; j += 8) {
           if (vec && col + j + 8 <= g.N) {
@@ -249,16 +319,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
           for (int e = 0; e < 8; e++) bad |= !(fabsf(sum[j + e]) <= 3.402823466e+38f);
         }
-        if (bad) {
-          const float* ar = g.a + (size_t)row * g.lda + (g.batch > 1 ? (size_t)z * g.K : 0);
-          const float* br = g.b + (size_t)(g.batch > 1 ? (size_t)z * g.N : 0) * g.ldb;
-          const int k0 = kb0 * GS_BK, k1 = min(g.K, (kb0 + nkb) * GS_BK);
-          for (int j = 0; j < OWN && col + j < g.N; j++)
-            if (!(fabsf(dst[j]) <= 3.402823466e+38f)) dst[j] = gs_dot(ar, br + (size_t)(col + j) * g.ldb, k0, k1);
-        }
       }
-      __syncwarp();
+      if (__any_sync(0xffffffffu, bad)) marked |= 1u << (i & 31);
     }
+    if (ok && marked) gs_again<BN>(g, pair, n_pairs, n_tiles, (int)rank * 128 + q * 32, c_lo, marked);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

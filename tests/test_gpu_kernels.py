@@ -526,10 +526,11 @@ def test_gemm_split_is_at_least_as_exact_as_the_chain(kernel_sets, M, N, K):
     assert torch.equal(again, out) and int(flag) == 0
 
 
-@pytest.mark.parametrize("ea, ew", [(-115, 0), (-125, 0), (0, -120), (-140, 20), (-100, 90), (100, -140), (-60, -50), (70, 40), (110, -60)])
-def test_gemm_split_keeps_small_and_large_operands(kernel_sets, ea, ew):
-    """Operands as small as floats go, subnormal ones included, keep their 24 bits, also beside larger ones that meet a zero; sums that leave
-    the scaled range come out as the chain of multiply-adds has them."""
+@pytest.mark.parametrize("ea, ew, chained", [(-115, 0, False), (-125, 0, False), (0, -120, False), (-140, 20, False), (-100, 90, False),
+                                             (100, -140, False), (-60, -50, False), (70, 40, True), (110, -60, True)])
+def test_gemm_split_keeps_small_and_large_operands(kernel_sets, ea, ew, chained):
+    """Operands as small as floats go, subnormal ones included, keep their 24 bits, also beside larger ones that meet a zero; what leaves the
+    scaled range (operands above 2^104, sums from 2^80 on) comes out as the chain of multiply-adds has it."""
     ks, M, N, K = kernel_sets[torch.float32], 129, 40, 200
     a, w = dev(torch.ldexp(rand(M, K, seed=3), torch.tensor(ea))), dev(torch.ldexp(rand(N, K, seed=4), torch.tensor(ew)))
     a[:, 0], w[:, 0], w[:, 1], a[:, 1] = 1.0, 0.0, 1.0, 0.0
@@ -539,7 +540,45 @@ def test_gemm_split_keeps_small_and_large_operands(kernel_sets, ea, ew):
     out, chain = (torch.full((M, N), float("nan"), device="cuda") for _ in range(2))
     ks.split.gemm(a, w, out, flag)
     ks.gemm_nt(a, w, chain)
-    assert off(out) <= min(tol, 1.05 * off(chain)) and int(flag) == 0
+    assert int(flag) == 0 and (torch.equal(out[:, 1:], chain[:, 1:]) if chained else off(out) <= min(tol, 1.05 * off(chain)))
+
+
+@pytest.mark.parametrize("M, N, K, parts", [(300, 200, 1032, 1), (300, 200, 1032, 3), (20, 129, 4096, 1), (6500, 12800, 64, 1)])
+def test_gemm_split_sums_again_what_is_not_finite(kernel_sets, M, N, K, parts):
+    """Rows, columns and single outputs that are not finite, in a block's first tiles and past its thirty-second, have the chain's values and
+    the others keep theirs."""
+    ks, flag = kernel_sets[torch.float32], torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, w = dev(rand(M, K, seed=3)), dev(rand(N, K, seed=4))
+    plain, out, chain = (torch.full((parts, M, N) if parts > 1 else (M, N), 7.0, device="cuda") for _ in range(3))
+    ks.split.gemm(a, w, plain, flag)
+    a[0], a[3, 1], a[M // 2, K - 1], a[M - 9:, 5], w[N - 1, 2] = math.nan, math.inf, -math.inf, 3.4e38, math.inf
+    ks.split.gemm(a, w, out, flag)
+    ks.gemm_nt(a, w, chain)
+    bad = ~chain.isfinite()
+    assert torch.equal(bad, ~out.isfinite()) and torch.equal(chain[bad].nan_to_num(1.5, 2.5, 3.5), out[bad].nan_to_num(1.5, 2.5, 3.5))
+    touched = torch.zeros(M, N, dtype=torch.bool, device="cuda")
+    touched[[0, 3, M // 2]], touched[M - 9:], touched[:, N - 1] = True, True, True
+    assert torch.equal(out[..., ~touched], plain[..., ~touched]) and int(flag) == 0 and int(bad.sum()) >= parts * N
+    assert rel_err(out[chain.abs() > 1e30].nan_to_num(0, 0, 0).cpu(), f64(chain[chain.abs() > 1e30].nan_to_num(0, 0, 0))) < 1e-6
+
+
+def test_gemm_split_of_a_diverged_operand_is_no_hang(kernel_sets):
+    """Every output not finite: a few times the chains' own kernel, and no wait near its limit. (An output a thread at a time took 100
+    times as long.)"""
+    ks, flag = kernel_sets[torch.float32], torch.zeros(1, dtype=torch.int32, device="cuda")
+    a, w, out = torch.full((1000, 2048), math.nan, device="cuda"), dev(rand(2560, 2048, seed=4)), torch.empty((1000, 2560), device="cuda")
+
+    def us(run):
+        run()
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        for _ in range(3):
+            run()
+        end.record()
+        torch.cuda.synchronize()
+        return start.elapsed_time(end) / 3
+
+    assert us(lambda: ks.split.gemm(a, w, out, flag)) < 25 * us(lambda: ks.gemm_nt(a, w, out)) and bool(out.isnan().all()) and int(flag) == 0
 
 
 def test_gemm_split_blocks_and_what_is_not_finite(kernel_sets):
