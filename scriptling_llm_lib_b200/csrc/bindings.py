@@ -245,12 +245,28 @@ class KernelSet:
 
     @staticmethod
     def attn_decode_splits(n_seqs: int, n_heads: int, n_kv: int, pages: int, sm_count: int) -> int:
-        """Blocks per (sequence, key/value head, pass over the keys; a pass serves up to four of the
-        query heads that share the key/value head): enough for about six blocks of four warps per SM,
-        at most one per page."""
-        passes = -(-(n_heads // n_kv) // 4)       # (wide heads, above 128: two heads a pass; the estimate stays)
+        """Blocks per (sequence, up to four of the query heads that share a key/value head): enough for
+        about six blocks of four warps per SM, at most one per page."""
+        passes = -(-(n_heads // n_kv) // 4)       # (wide heads, above 128: two heads a block; the estimate stays)
         want = -(-6 * sm_count // max(1, n_seqs * n_kv * passes))
         return max(1, min(want, pages, 64))
+
+    @staticmethod
+    def attn_decode_split_pays(dtype, n_seqs: int, n_heads: int, n_kv: int, head_dim: int, v_dim: int, pages: int) -> bool:
+        """Whether a decode step of unequal widths takes less by `attn_decode_split` than by the kernel with a block a row and head, which
+        walks its keys 32 at a time: with three pages and more; with fewer in bfloat16 while the blocks are few (a block costs about
+        4 us, once for each that an SM holds in turn) and in 32-bit, where that kernel's walk is twice as fast, only where two pages meet many
+        blocks or a block has one head. A block a row and head / keys split, us: bfloat16 64 / 128, 16 heads on 4, 16 sequences of 20
+        keys 9.2 / 6.5, of 64 11.8 / 8.7, of 400 35 / 18; 256 sequences of 8 8.3 / 10.3, of 128 51 / 37; 64 heads on one, 64 of 8
+        6.7 / 9.9; 32-bit 64 / 128 one of 40 6.9 / 7.7, of 128 7.3 / 11.5, of 200 11.2 / 11.2, of 1,000 36 / 13; 256 of 65 37 / 24;
+        192 / 128, 16 heads, one of 40 8.7 / 5.9, of 65 8.8 / 9.6."""
+        rep = n_heads // n_kv
+        blocks = n_seqs * n_kv * -(-rep // (2 if max(head_dim, v_dim) > 128 else 4))
+        if pages > 2:
+            return True
+        if blocks >= 1024:
+            return pages == 2
+        return dtype != torch.float32 or (pages == 1 and rep == 1)
 
     # ------------------------------------------------------------------ feed-forward
     def swiglu(self, gate_up, out, tiled=False):

@@ -1056,12 +1056,13 @@ __global__ void __launch_bounds__(256) attn_paged_tiled_kernel(AttnArgs p) {
 }
 
 // ------------------------------------------------------------------ one query per sequence, keys split over blocks
-// The decode step of the generic path: block (split, key/value head, sequence) streams its share of
-// the sequence's pages once for up to NREP of the query heads that share the key/value head (more
-// heads: once per NREP of them), LPK lanes per key with 4 dims each per pass (NV passes for wide
+// The decode step of the generic path: block (split, up to NREP of the query heads that share a key/value head,
+// sequence) streams its share of the sequence's pages once for its heads, LPK lanes per key with 4 dims each per pass (NV passes for wide
 // heads), online softmax per lane group and head in float (exponentials as 2^x of scores scaled by
 // log2 e), folded over the warp and the block. With one split the block writes the output row; otherwise it leaves
 // (unnormalised sum, maximum, sum) in `part` [B][H][n_split][vd + 2] for the merge kernel below.
+// Bound by a block's chain over its keys. One block for all of a group's heads, NREP after NREP, took that chain once for each: 64 heads
+// of 32 / 64 on one key/value head, one sequence of 64 keys 60 us, 6.3 with a block for each NREP; 4,096 keys 107, 29.
 // Keys and values may have different widths, both up to LPK * 4 * NV.
 struct AttnSplitArgs {
   const void* q;        // [B, q_ld] rotated queries of this step
@@ -1086,8 +1087,8 @@ __global__ void __launch_bounds__(128) attn_decode_split_generic_kernel(AttnSpli
   constexpr int UN = NV == 1 ? 4 : (NV == 2 ? 2 : 1);   // loads in flight per lane group
   extern __shared__ __align__(16) float ad_sm[];        // [4 warps][NREP][vd] partial outputs, then [4][NREP][2] (m, l)
   const int hd = p.hd, vd = p.vd;
-  const int split = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
-  const int nrep = p.H / p.G;                   // query heads that share this key/value head: served NREP at a time
+  const int nrep = p.H / p.G;                   // query heads that share a key/value head: NREP of them a block
+  const int split = blockIdx.x, g = blockIdx.y / ((nrep + NREP - 1) / NREP), r0 = blockIdx.y % ((nrep + NREP - 1) / NREP) * NREP, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slot = lane / LPK, dl = (lane % LPK) * 4;
   const int pos = p.seq_pos0[b];
@@ -1102,131 +1103,128 @@ __global__ void __launch_bounds__(128) attn_decode_split_generic_kernel(AttnSpli
   float* sm_acc = ad_sm;                        // [4][NREP][vd]
   float* sm_ml = ad_sm + 4 * NREP * vd;         // [4][NREP][2]
 
-  for (int r0 = 0; r0 < nrep; r0 += NREP) {
-    float qv[NREP][NV][4], acc[NREP][NV][4], m[NREP], l[NREP];
+  float qv[NREP][NV][4], acc[NREP][NV][4], m[NREP], l[NREP];
 #pragma unroll
-    for (int r = 0; r < NREP; r++) {
-      const int h = g * nrep + min(r0 + r, nrep - 1);           // heads past the group's last repeat it (not stored)
-      const A* qrow = (const A*)p.q + (size_t)b * p.q_ld + (size_t)h * hd;
+  for (int r = 0; r < NREP; r++) {
+    const int h = g * nrep + min(r0 + r, nrep - 1);           // heads past the group's last repeat it (not stored)
+    const A* qrow = (const A*)p.q + (size_t)b * p.q_ld + (size_t)h * hd;
+#pragma unroll
+    for (int v = 0; v < NV; v++) {
+      int d = dl + v * LPK * 4;
+      float4 t = d < hd ? ld4(qrow + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float sc = p.softcap > 0.f ? p.scale : p.scale * ATT_LOG2E;   // a capped score is brought to base 2 after the cap
+      qv[r][v][0] = t.x * sc; qv[r][v][1] = t.y * sc; qv[r][v][2] = t.z * sc; qv[r][v][3] = t.w * sc;
+      acc[r][v][0] = acc[r][v][1] = acc[r][v][2] = acc[r][v][3] = 0.f;
+    }
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+  }
+  for (int kb = x_lo + warp * KPW * UN; kb < x_hi; kb += 4 * KPW * UN) {
+    {                                         // keys no query sees: the ends of the kept and of the window's first page
+      const int f = seen_keys.key(kb);
+      if (f > pos || (f >= p.keep && f + KPW * UN <= k_begin)) continue;
+    }
+    float4 kr[UN][NV], vr[UN][NV];
+    bool ok[UN];
+#pragma unroll
+    for (int u = 0; u < UN; u++) {
+      int key = seen_keys.key(kb + u * KPW + slot);
+      ok[u] = key_seen(key, pos, k_begin, p.keep);
+      int kk = ok[u] ? key : pos;
+      int page = bt[kk / SLLM_PAGE];
+      size_t row = ((size_t)page * p.G + g) * SLLM_PAGE + (kk % SLLM_PAGE);
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         int d = dl + v * LPK * 4;
-        float4 t = d < hd ? ld4(qrow + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float sc = p.softcap > 0.f ? p.scale : p.scale * ATT_LOG2E;   // a capped score is brought to base 2 after the cap
-        qv[r][v][0] = t.x * sc; qv[r][v][1] = t.y * sc; qv[r][v][2] = t.z * sc; qv[r][v][3] = t.w * sc;
-        acc[r][v][0] = acc[r][v][1] = acc[r][v][2] = acc[r][v][3] = 0.f;
-      }
-      m[r] = -INFINITY;
-      l[r] = 0.f;
-    }
-    for (int kb = x_lo + warp * KPW * UN; kb < x_hi; kb += 4 * KPW * UN) {
-      {                                         // keys no query sees: the ends of the kept and of the window's first page
-        const int f = seen_keys.key(kb);
-        if (f > pos || (f >= p.keep && f + KPW * UN <= k_begin)) continue;
-      }
-      float4 kr[UN][NV], vr[UN][NV];
-      bool ok[UN];
-#pragma unroll
-      for (int u = 0; u < UN; u++) {
-        int key = seen_keys.key(kb + u * KPW + slot);
-        ok[u] = key_seen(key, pos, k_begin, p.keep);
-        int kk = ok[u] ? key : pos;
-        int page = bt[kk / SLLM_PAGE];
-        size_t row = ((size_t)page * p.G + g) * SLLM_PAGE + (kk % SLLM_PAGE);
-#pragma unroll
-        for (int v = 0; v < NV; v++) {
-          int d = dl + v * LPK * 4;
-          kr[u][v] = d < hd ? ld4(kp + row * hd + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-          vr[u][v] = d < vd ? ld4(vp + row * vd + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < NREP; r++) {
-        float s[UN], m_new = m[r];
-#pragma unroll
-        for (int u = 0; u < UN; u++) {
-          float d = 0.f;
-#pragma unroll
-          for (int v = 0; v < NV; v++) {
-            d = fmaf(qv[r][v][0], kr[u][v].x, d); d = fmaf(qv[r][v][1], kr[u][v].y, d);
-            d = fmaf(qv[r][v][2], kr[u][v].z, d); d = fmaf(qv[r][v][3], kr[u][v].w, d);
-          }
-#pragma unroll
-          for (int o = 1; o < LPK; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-          if (p.softcap > 0.f) d = p.softcap * ATT_LOG2E * tanhf(d / p.softcap);
-          s[u] = ok[u] ? d : -INFINITY;
-          m_new = fmaxf(m_new, s[u]);
-        }
-        if (m_new == -INFINITY) continue;
-        float corr = exp2f(m[r] - m_new);
-        m[r] = m_new;
-        l[r] *= corr;
-#pragma unroll
-        for (int v = 0; v < NV; v++) { acc[r][v][0] *= corr; acc[r][v][1] *= corr; acc[r][v][2] *= corr; acc[r][v][3] *= corr; }
-#pragma unroll
-        for (int u = 0; u < UN; u++) {
-          float pr = exp2f(s[u] - m_new);
-          l[r] += pr;
-#pragma unroll
-          for (int v = 0; v < NV; v++) {
-            acc[r][v][0] = fmaf(pr, vr[u][v].x, acc[r][v][0]); acc[r][v][1] = fmaf(pr, vr[u][v].y, acc[r][v][1]);
-            acc[r][v][2] = fmaf(pr, vr[u][v].z, acc[r][v][2]); acc[r][v][3] = fmaf(pr, vr[u][v].w, acc[r][v][3]);
-          }
-        }
+        kr[u][v] = d < hd ? ld4(kp + row * hd + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        vr[u][v] = d < vd ? ld4(vp + row * vd + d) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    // fold the key slots of the warp, then the warps
 #pragma unroll
     for (int r = 0; r < NREP; r++) {
+      float s[UN], m_new = m[r];
 #pragma unroll
-      for (int o = LPK; o < 32; o <<= 1) {
-        float mo = __shfl_xor_sync(0xffffffffu, m[r], o), lo = __shfl_xor_sync(0xffffffffu, l[r], o);
-        float mn = fmaxf(m[r], mo);
-        float c1 = mn == -INFINITY ? 0.f : exp2f(m[r] - mn), c2 = mn == -INFINITY ? 0.f : exp2f(mo - mn);
-        l[r] = l[r] * c1 + lo * c2;
-        m[r] = mn;
-#pragma unroll
-        for (int v = 0; v < NV; v++)
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            float ao = __shfl_xor_sync(0xffffffffu, acc[r][v][c], o);
-            acc[r][v][c] = acc[r][v][c] * c1 + ao * c2;
-          }
-      }
-      if (lane < LPK) {
+      for (int u = 0; u < UN; u++) {
+        float d = 0.f;
 #pragma unroll
         for (int v = 0; v < NV; v++) {
-          int d = dl + v * LPK * 4;
-          if (d < vd) *(float4*)(sm_acc + (warp * NREP + r) * vd + d) = make_float4(acc[r][v][0], acc[r][v][1], acc[r][v][2], acc[r][v][3]);
+          d = fmaf(qv[r][v][0], kr[u][v].x, d); d = fmaf(qv[r][v][1], kr[u][v].y, d);
+          d = fmaf(qv[r][v][2], kr[u][v].z, d); d = fmaf(qv[r][v][3], kr[u][v].w, d);
         }
-        if (lane == 0) { sm_ml[(warp * NREP + r) * 2] = m[r]; sm_ml[(warp * NREP + r) * 2 + 1] = l[r]; }
+#pragma unroll
+        for (int o = 1; o < LPK; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (p.softcap > 0.f) d = p.softcap * ATT_LOG2E * tanhf(d / p.softcap);
+        s[u] = ok[u] ? d : -INFINITY;
+        m_new = fmaxf(m_new, s[u]);
+      }
+      if (m_new == -INFINITY) continue;
+      float corr = exp2f(m[r] - m_new);
+      m[r] = m_new;
+      l[r] *= corr;
+#pragma unroll
+      for (int v = 0; v < NV; v++) { acc[r][v][0] *= corr; acc[r][v][1] *= corr; acc[r][v][2] *= corr; acc[r][v][3] *= corr; }
+#pragma unroll
+      for (int u = 0; u < UN; u++) {
+        float pr = exp2f(s[u] - m_new);
+        l[r] += pr;
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+          acc[r][v][0] = fmaf(pr, vr[u][v].x, acc[r][v][0]); acc[r][v][1] = fmaf(pr, vr[u][v].y, acc[r][v][1]);
+          acc[r][v][2] = fmaf(pr, vr[u][v].z, acc[r][v][2]); acc[r][v][3] = fmaf(pr, vr[u][v].w, acc[r][v][3]);
+        }
       }
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < NREP * vd; e += 128) {
-      const int r = e / vd, dd = e % vd;
-      if (r0 + r >= nrep) continue;
-      const int h = g * nrep + r0 + r;
-      float mn = -INFINITY;
+  }
+  // fold the key slots of the warp, then the warps
 #pragma unroll
-      for (int w = 0; w < 4; w++) mn = fmaxf(mn, sm_ml[(w * NREP + r) * 2]);
-      float a = 0.f, ls = 0.f;
+  for (int r = 0; r < NREP; r++) {
 #pragma unroll
-      for (int w = 0; w < 4; w++) {
-        float cw = mn == -INFINITY ? 0.f : exp2f(sm_ml[(w * NREP + r) * 2] - mn);
-        a += sm_acc[(w * NREP + r) * vd + dd] * cw;
-        ls += sm_ml[(w * NREP + r) * 2 + 1] * cw;
-      }
-      if (p.n_split == 1) {
-        if (p.sink) ls = mn == -INFINITY ? 1.0f : ls + exp2f(p.sink[h] * ATT_LOG2E - mn);
-        ((A*)p.out)[((size_t)b * p.H + h) * vd + dd] = from_f32<A>(ls > 0.f ? a / ls : 0.f);
-      } else {
-        float* dst = p.part + (((size_t)b * p.H + h) * p.n_split + split) * (vd + 2);
-        dst[dd] = a;
-        if (dd == 0) { dst[vd] = mn; dst[vd + 1] = ls; }
-      }
+    for (int o = LPK; o < 32; o <<= 1) {
+      float mo = __shfl_xor_sync(0xffffffffu, m[r], o), lo = __shfl_xor_sync(0xffffffffu, l[r], o);
+      float mn = fmaxf(m[r], mo);
+      float c1 = mn == -INFINITY ? 0.f : exp2f(m[r] - mn), c2 = mn == -INFINITY ? 0.f : exp2f(mo - mn);
+      l[r] = l[r] * c1 + lo * c2;
+      m[r] = mn;
+#pragma unroll
+      for (int v = 0; v < NV; v++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          float ao = __shfl_xor_sync(0xffffffffu, acc[r][v][c], o);
+          acc[r][v][c] = acc[r][v][c] * c1 + ao * c2;
+        }
     }
-    __syncthreads();
+    if (lane < LPK) {
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        int d = dl + v * LPK * 4;
+        if (d < vd) *(float4*)(sm_acc + (warp * NREP + r) * vd + d) = make_float4(acc[r][v][0], acc[r][v][1], acc[r][v][2], acc[r][v][3]);
+      }
+      if (lane == 0) { sm_ml[(warp * NREP + r) * 2] = m[r]; sm_ml[(warp * NREP + r) * 2 + 1] = l[r]; }
+    }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < NREP * vd; e += 128) {
+    const int r = e / vd, dd = e % vd;
+    if (r0 + r >= nrep) continue;
+    const int h = g * nrep + r0 + r;
+    float mn = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < 4; w++) mn = fmaxf(mn, sm_ml[(w * NREP + r) * 2]);
+    float a = 0.f, ls = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+      float cw = mn == -INFINITY ? 0.f : exp2f(sm_ml[(w * NREP + r) * 2] - mn);
+      a += sm_acc[(w * NREP + r) * vd + dd] * cw;
+      ls += sm_ml[(w * NREP + r) * 2 + 1] * cw;
+    }
+    if (p.n_split == 1) {
+      if (p.sink) ls = mn == -INFINITY ? 1.0f : ls + exp2f(p.sink[h] * ATT_LOG2E - mn);
+      ((A*)p.out)[((size_t)b * p.H + h) * vd + dd] = from_f32<A>(ls > 0.f ? a / ls : 0.f);
+    } else {
+      float* dst = p.part + (((size_t)b * p.H + h) * p.n_split + split) * (vd + 2);
+      dst[dd] = a;
+      if (dd == 0) { dst[vd] = mn; dst[vd + 1] = ls; }
+    }
   }
 }
 

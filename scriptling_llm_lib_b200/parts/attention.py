@@ -13,7 +13,7 @@ before it is cached. Either sends the step's keys and values through a store ker
 rotation, value norm and cache write in one pass (`kv_store`); values as wide as keys then still
 use the attention kernels below, other widths kernels that take both (in a bfloat16 prompt step with widths in
 multiples of 8 the tcgen05 kernel with float32 weights, in a decode step with widths in multiples of 4 the one that
-splits the keys over blocks, else `attn_wide_value`).
+splits the keys over blocks where that pays, else `attn_wide_value`).
 
 Four more options, none in the reference. `chunk`: a query sees the earlier keys of its own chunk of that many
 positions only, chunks counted from position 0 of the sequence (not from where a step begins); the cache
@@ -64,7 +64,7 @@ import math
 import torch
 
 from ..cache.needs import CacheNeed
-from ..csrc.bindings import DecodeKernels, PrefillAttentionMMA, PrefillAttentionTC, gate_aligned
+from ..csrc.bindings import DecodeKernels, KernelSet, PrefillAttentionMMA, PrefillAttentionTC, gate_aligned
 from ..cache.needs import StateNeed
 from ..weights.spec import TensorSpec
 from .base import MIXERS, POSITION_ENCODINGS, Folded, Mixer, PartSpec
@@ -312,7 +312,9 @@ class Attention(Mixer):
             ctx.kernels.prefill_attention_tc.attn(qkv, attn, ctx.seq_start, ctx.seq_pos0, block_table, kpages, vpages, ctx.n_seqs,
                                                   ctx.max_new, self.n_heads, self.n_kv_heads, self.head_dim, self.span, self.scale,
                                                   ctx.err_flag, v_dim=self.v_dim, exact_weights=True)
-        elif self.other_widths and ctx.is_decode and ctx.kernels.attn_decode_split_takes(self.head_dim, qkv.stride(0), self.v_dim):
+        elif (self.other_widths and ctx.is_decode and ctx.kernels.attn_decode_split_takes(self.head_dim, qkv.stride(0), self.v_dim)
+              and KernelSet.attn_decode_split_pays(x.dtype, ctx.n_seqs, self.n_heads, self.n_kv_heads, self.head_dim, self.v_dim,
+                                                   ctx.pages_seen(unit))):
             # keys split over blocks, read once for up to four of a group's heads (8 sequences of 16 heads, keys 64 and values 128, 500
             # keys each: 12.9 us with the merge, 36.4 with a block a row and head)
             n_split = ctx.kernels.attn_decode_splits(ctx.n_seqs, self.n_heads, self.n_kv_heads, ctx.pages_seen(unit), ctx.engine.sm_count)

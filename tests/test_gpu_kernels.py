@@ -955,6 +955,45 @@ def test_attn_decode_split_generic(kernel_sets, dtype, H, G, hd, window, n_split
     assert rel_err(out.cpu().float(), want) < TOL[dtype]
 
 
+@pytest.mark.parametrize("H, G, hd, vd, n_split", [(9, 1, 32, 64, 1), (14, 2, 24, 40, 3), (64, 1, 32, 64, 2), (6, 2, 64, 256, 2), (10, 2, 320, 64, 1)])
+def test_attn_decode_split_of_groups_of_any_size(kernel_sets, H, G, hd, vd, n_split):
+    """Groups that fill no block's heads, unequal widths: the attention of every head; and many heads on one key/value head, a block for
+    every few of them, take no longer than a block a row and head (one block for all of them took ten times that)."""
+    ks, pos0, g = kernel_sets[torch.float32], [0, 63, 130], torch.Generator().manual_seed(H)
+    held = [p + 1 for p in pos0]
+    kk, vv = [torch.randn(n, G, hd, generator=g) for n in held], [torch.randn(n, G, vd, generator=g) for n in held]
+    kp, _, bt = paged(kk, kk, held)
+    vp, _, _ = paged(vv, vv, held)
+    q = torch.randn(3, H, hd, generator=g)
+    out, part = torch.full((3, H * vd), float("nan"), device="cuda"), torch.full((3 * H * n_split * (vd + 2),), float("nan"), device="cuda")
+    qd, pd = dev(q.view(3, -1)), dev(pos0, torch.int32)
+    split = lambda: ks.attn_decode_split(qd, out, pd, bt, kp, vp, part, 3, H, G, hd, 0, hd ** -0.5, n_split, v_dim=vd)      # noqa: E731
+    split()
+    want = []
+    for b in range(3):
+        k, v = (f64(t).repeat_interleave(H // G, 1) for t in (kk[b], vv[b]))
+        sc = (torch.einsum("hd,khd->hk", f64(q[b]), k) * hd ** -0.5).softmax(-1)
+        want.append(torch.einsum("hk,khd->hd", sc, v).reshape(-1))
+    assert rel_err(out.cpu(), torch.stack(want)) < TOL[torch.float32]
+    if H // G > 32:
+        wide = lambda: ks.seq.attn_wide_value(qd, out, pd, torch.arange(3, dtype=torch.int32, device="cuda"), bt, kp, vp, H, G, hd, vd, 0, hd ** -0.5)      # noqa: E731
+
+        def us(run):
+            run()
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                for _ in range(20):
+                    run()
+            start.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            return start.elapsed_time(end)
+
+        assert us(split) < 3 * us(wide)
+
+
 FAR_CASES = [(3, None, True), (517, None, True), (899 - 199, 200, True), (899 - 200, 200, False),
              (640, 260, True), (639, 260, False)]     # the last two: the window's edge (key 640) on a page and tile boundary
 

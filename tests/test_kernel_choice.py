@@ -215,3 +215,15 @@ def test_the_reserve_counts_the_grouped_rows_of_routed_experts(hidden, F, E, top
     assert part.scratch_bytes(rows) == padded * (6 * hidden + 2 * F) + 4 * rows * hidden
     part.w_up = torch.empty((1, 1, 1))                      # kept in 32-bit: the FMA kernels' buffers
     assert part.scratch_bytes(rows) == rows * top * (4 * F * (3 if gated else 1) + 4 * hidden)
+
+
+@pytest.mark.parametrize("dtype, n_seqs, H, G, D, V, pages, want", [
+    (torch.bfloat16, 1, 16, 4, 64, 128, 1, True), (torch.bfloat16, 255, 16, 4, 64, 128, 1, True), (torch.bfloat16, 256, 16, 4, 64, 128, 1, False),
+    (torch.bfloat16, 256, 16, 4, 64, 128, 2, True), (torch.bfloat16, 64, 64, 1, 32, 64, 1, False), (torch.bfloat16, 64, 64, 1, 32, 64, 3, True),
+    (torch.float32, 1, 16, 4, 64, 128, 1, False), (torch.float32, 1, 16, 4, 64, 128, 2, False), (torch.float32, 1, 16, 4, 64, 128, 3, True),
+    (torch.float32, 256, 16, 4, 64, 128, 2, True), (torch.float32, 1, 16, 16, 192, 128, 1, True), (torch.float32, 1, 16, 16, 192, 128, 2, False),
+    (torch.float32, 128, 16, 2, 128, 256, 2, True), (torch.float32, 127, 16, 2, 128, 256, 2, False)])
+def test_short_contexts_of_unequal_widths_keep_a_block_a_row_and_head(dtype, n_seqs, H, G, D, V, pages, want):
+    """Two heads a block from 129 columns on, else four; the line lies at 1,024 blocks."""
+    from scriptling_llm_lib_b200.csrc.bindings import KernelSet
+    assert KernelSet.attn_decode_split_pays(dtype, n_seqs, H, G, D, V, pages) == want
