@@ -230,11 +230,10 @@ __global__ void __launch_bounds__(128) attn_prefill_mma_kernel(PmArgs p) {
 template <int KD, int VD>
 static int pm_launch(const PmArgs& a, int B, int max_new, cudaStream_t stream) {
   size_t smem = (size_t)2 * PM_BK * ((KD + 8) + (VD + 8)) * sizeof(bf16);
-  static bool raised = false;
-  if (smem > 48 * 1024 && !raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_mma_kernel<KD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SllmPerDevice allowed;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = sllm_allow_smem(allowed, attn_prefill_mma_kernel<KD, VD>, smem);
     if (e != cudaSuccess) return (int)e;
-    raised = true;
   }
   dim3 grid((max_new + PM_BQ - 1) / PM_BQ, a.H, B);
   attn_prefill_mma_kernel<KD, VD><<<grid, 128, smem, stream>>>(a);

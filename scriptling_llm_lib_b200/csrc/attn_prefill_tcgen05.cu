@@ -1218,12 +1218,9 @@ template <int KD, int VD, int STAGES>
 static int fe_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const FtArgs& a, dim3 grid, cudaStream_t stream) {
   constexpr size_t need = FT_BQ * KD * 2 + STAGES * FT_BK * (KD + VD) * 2 + 512 + 6 * FT_BQ * 4, smem = need + 1024;
   static_assert(smem <= 232448, "the block of this head width does not fit an SM");
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_exact_kernel<KD, VD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, attn_prefill_exact_kernel<KD, VD, STAGES>, smem);
+  if (e != cudaSuccess) return (int)e;
   return (int)sllm_launch(attn_prefill_exact_kernel<KD, VD, STAGES>, grid, dim3(FE_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
@@ -1235,12 +1232,9 @@ static int ft_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   constexpr size_t room = (233472 / 2 - 1024);
   constexpr size_t smem = need + 1024 <= room ? need + 1024 : room;     // the slack for the alignment, as far as it fits
   static_assert(need <= smem, "two blocks of this head width do not fit an SM");
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, attn_prefill_tc_kernel<HD, STAGES>, smem);
+  if (e != cudaSuccess) return (int)e;
   return (int)sllm_launch(attn_prefill_tc_kernel<HD, STAGES>, grid, dim3(FT_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
@@ -1252,12 +1246,9 @@ static int fp_launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
   constexpr size_t room = 232448;
   constexpr size_t smem = need + 1024 <= room ? need + 1024 : room;     // the slack for the alignment, as far as it fits
   static_assert(need <= smem, "the block of this head width does not fit an SM");
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<KD, VD, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, attn_prefill_pair_kernel<KD, VD, STAGES>, smem);
+  if (e != cudaSuccess) return (int)e;
   return (int)sllm_launch(attn_prefill_pair_kernel<KD, VD, STAGES>, grid, dim3(FP_THREADS), smem, stream, mq, mk, mv, a, (uint32_t)smem);
 }
 
@@ -1286,13 +1277,7 @@ SLLM_EXPORT int sllm_attn_prefill_tc_bf16(const void* q, int q_ld, int T, void* 
   int n_qt = (max_new + FT_BQ - 1) / FT_BQ;
   long long n_items = (long long)H * n_qt * B;
   if (n_items > 0x7fffffffLL) return SLLM_ERR_ARG;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return (int)e;
-  }
+  const int sm_count = sllm_sm_count();
   if (hd <= 64 && vd <= 64 && weight_parts == 1) {
     FtArgs a{(bf16*)out, seq_start, seq_pos0, block_table, max_pages, H, G, hd, vd, window, keep, scale, err, n_qt, B, (int)n_items, 0, softcap, sink,
              (const bf16*)gate, gate_ld, (const bf16*)q, (const bf16*)kpages, (const bf16*)vpages, q_ld};

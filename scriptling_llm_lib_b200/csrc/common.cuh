@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <atomic>
 
 #define SLLM_PAGE 64  // tokens per cache page; the Python side asserts the same number
 
@@ -18,6 +19,36 @@ SLLM_EXPORT int sllm_page_tokens(void) { return SLLM_PAGE; }
 #define SLLM_RETURN_LAST() return (int)cudaGetLastError()
 
 typedef __nv_bfloat16 bf16;
+
+// What a launcher finds out or sets up once for each device, as a static of its own: a kernel's limit of shared memory, how many of its
+// blocks fit. 0: not yet. (A process may run engines on several devices; a kernel's attributes are each device's own.)
+struct SllmPerDevice {
+  std::atomic<int> of[64] = {};
+  std::atomic<int>& here() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return of[dev & 63];
+  }
+};
+// the current device lets `kernel` have `bytes` of dynamic shared memory
+template <typename K>
+static inline cudaError_t sllm_allow_smem(SllmPerDevice& allowed, K kernel, size_t bytes) {
+  std::atomic<int>& now = allowed.here();
+  if ((size_t)now.load() >= bytes) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) now.store((int)bytes);
+  return e;
+}
+static inline int sllm_sm_count() {
+  static SllmPerDevice sms;
+  std::atomic<int>& n = sms.here();
+  if (!n.load()) {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    n.store(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 1);
+  }
+  return n.load();
+}
 
 // Which of the keys at or before its own position a query sees, as the one number every attention
 // kernel takes under the name `window`: 0 all of them; w > 0 the last w (a sliding window); w < 0

@@ -256,16 +256,6 @@ gemm_small_m_kernel(const bf16* __restrict__ x, const bf16* __restrict__ W, void
   }
 }
 
-static int sllm_sm_count() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-  }
-  return sms;
-}
-
 template <int NT, int WARPS, int EPI>
 static int small_m_launch_w(const bf16* x, const bf16* W, void* y, int M, int N, int K, int ldx, int ldw, int ldy,
                             int out_f32, int ksplit, const SmFold& f, cudaStream_t stream) {

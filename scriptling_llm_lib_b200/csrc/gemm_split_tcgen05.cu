@@ -337,13 +337,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 template <int BN>
 static int gs_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GsArgs& g, int* err, cudaStream_t stream) {
   constexpr size_t smem = GS_SLOTS * (128 + BN / 2) * GS_BK * 2 + 1024 + 256;
-  static int pairs = 0;                  // how many pairs of blocks the GPU holds at once
-  if (!pairs) {
+  static SllmPerDevice held;             // how many pairs of blocks the GPU holds at once
+  std::atomic<int>& pairs = held.here();
+  if (!pairs.load()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 2) return SLLM_ERR_ARG - 3;
+    const int sms = sllm_sm_count();
+    if (sms < 2) return SLLM_ERR_ARG - 3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms & ~1);
     cfg.blockDim = dim3(GS_THREADS);
@@ -353,11 +353,11 @@ static int gs_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GsArgs&
       cudaGetLastError();
       n = sms / 2;
     }
-    pairs = n < sms / 2 ? n : sms / 2;
+    pairs.store(n < sms / 2 ? n : sms / 2);
   }
   const long long tiles = (long long)((g.N + BN - 1) / BN) * ((g.M + GS_BM - 1) / GS_BM) * g.parts * g.batch;
   if (tiles > 0x7fffffffLL) return SLLM_ERR_ARG;
-  const dim3 grid(2 * (int)(tiles < pairs ? tiles : pairs));
+  const dim3 grid(2 * (int)(tiles < pairs.load() ? tiles : pairs.load()));
   sllm_launch(gemm_split_kernel<BN>, grid, dim3(GS_THREADS), smem, stream, ma, mb, g, err);
   SLLM_RETURN_LAST();
 }

@@ -511,18 +511,10 @@ template <int BN, int STAGES, int EPI>
 static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C, int M, int N, int K, int ldc, int out_f32,
                      int* err, cudaStream_t stream, const TcRope& rp = TcRope{}, const TcFold& fd = TcFold{}) {
   constexpr size_t smem = STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024 + 256;
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 1;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, gemm_tc_kernel<BN, STAGES, EPI>, smem);
+  if (e != cudaSuccess) return (int)e;
+  const int sms = sllm_sm_count();
   int n_tiles = ((N + BN - 1) / BN) * ((M + TC_BM - 1) / TC_BM);
   dim3 grid(n_tiles < sms ? n_tiles : sms);
   return (int)sllm_launch(gemm_tc_kernel<BN, STAGES, EPI>, grid, dim3(TC_THREADS), smem, stream, ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
@@ -702,13 +694,13 @@ static int tc_pair_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C,
                           int* err, cudaStream_t stream, const TcRope& rp = TcRope{}, const TcFold& fd = TcFold{}) {
   // (the residual epilogue stages its chunks through 4 KB a warp behind the barriers)
   constexpr size_t smem = STAGES * (2 * 128 * TC_BK * 2) + 1024 + 256 + (EPI == TC_EPI_RESID ? 8 * 4096 : 0);
-  static int pairs = 0;                  // how many pairs of blocks the GPU holds at once
-  if (!pairs) {
+  static SllmPerDevice held;             // how many pairs of blocks the GPU holds at once
+  std::atomic<int>& pairs = held.here();
+  if (!pairs.load()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 2) return SLLM_ERR_ARG - 3;
+    const int sms = sllm_sm_count();
+    if (sms < 2) return SLLM_ERR_ARG - 3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sms & ~1);
     cfg.blockDim = dim3(TC2_THREADS);
@@ -718,10 +710,10 @@ static int tc_pair_launch(const CUtensorMap& ma, const CUtensorMap& mb, void* C,
       cudaGetLastError();
       n = sms / 2;
     }
-    pairs = n < sms / 2 ? n : sms / 2;
+    pairs.store(n < sms / 2 ? n : sms / 2);
   }
   int n_tiles = ((N + TC2_BN - 1) / TC2_BN) * ((M + TC2_BM - 1) / TC2_BM);
-  dim3 grid(2 * (n_tiles < pairs ? n_tiles : pairs));
+  dim3 grid(2 * (n_tiles < pairs.load() ? n_tiles : pairs.load()));
   return (int)sllm_launch(gemm_tc_pair_kernel<STAGES, EPI>, grid, dim3(TC2_THREADS), smem, stream, ma, mb, C, M, N, K, ldc, out_f32, err, rp, fd);
 }
 
@@ -939,12 +931,9 @@ static int tc_cluster_run(const void* A, const void* B, void* C, int M, int N, i
   stages = stages < per ? stages : per;
   const int sums = TC_BM * (tile_n + 4) * 4;
   const int smem = (stages * stage > sums ? stages * stage : sums) + 1024;
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_cluster_kernel<SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, gemm_tc_cluster_kernel<SPLIT>, 202 * 1024);
+  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(SPLIT * ((M + TC_BM - 1) / TC_BM) * ((N + tile_n - 1) / tile_n));
   cfg.blockDim = dim3(TC_THREADS);
@@ -1291,12 +1280,9 @@ template <int BT, int STAGES, int EPI>
 static int tc_skinny_launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int M, int N, int K, int ldc, int out_f32,
                             int ksplit, int* err, cudaStream_t stream) {
   constexpr size_t smem = STAGES * (128 * TC_BK * 2 + BT * TC_BK * 2) + 1024 + 256;
-  static bool raised = false;
-  if (!raised) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_skinny_kernel<BT, STAGES, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    raised = true;
-  }
+  static SllmPerDevice allowed;
+  const cudaError_t e = sllm_allow_smem(allowed, gemm_tc_skinny_kernel<BT, STAGES, EPI>, smem);
+  if (e != cudaSuccess) return (int)e;
   dim3 grid((N + 127) / 128, ksplit);
   return (int)sllm_launch(gemm_tc_skinny_kernel<BT, STAGES, EPI>, grid, dim3(TC_THREADS), smem, stream, mw, mx, C, M, N, K, ldc,
                           out_f32, err);

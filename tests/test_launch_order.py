@@ -47,3 +47,9 @@ def test_tensor_memory_is_taken_before_dependents_may_start():
         taken = max(body.find("tcgen05.alloc"), body.find("u.open("))
         if taken >= 0 and "pdl_launch_dependents()" in body:
             assert body.find("pdl_launch_dependents()") > taken, name
+
+
+def test_what_a_launcher_sets_up_is_kept_for_each_device():
+    """A kernel's limit of shared memory and the blocks that fit are a device's own: a process may run engines on several."""
+    for name, text in FILES.items():
+        assert not re.findall(r"static (?:bool|int) \w+(?:\[\d+\])? = (?:false|0|\{)[^;]*;", text), name
