@@ -16,8 +16,8 @@ def _closing(s, i, pair):
     raise ValueError("unbalanced")
 
 
-def _bodies():
-    """Kernel name -> body, of every __global__ definition."""
+def _bodies(heads=False):
+    """Kernel name -> body (or list of parameters), of every __global__ definition."""
     out = {}
     for text in FILES.values():
         for m in re.finditer(r"__global__", text):
@@ -27,18 +27,47 @@ def _bodies():
             close = _closing(text, head.end() - 1, "()")
             brace = text.find("{", close)
             if text[close + 1:brace].strip() == "":
-                out[head.group(1)] = text[brace:_closing(text, brace, "{}") + 1]
+                out[head.group(1)] = text[head.end():close] if heads else text[brace:_closing(text, brace, "{}") + 1]
     return out
 
 
-def test_every_kernel_launched_ahead_waits_for_the_one_in_front():
-    bodies, ahead = _bodies(), set()
+def _ahead():
+    names = set()
     for text in FILES.values():
-        ahead |= set(re.findall(r"sllm_launch\(\s*(?:\w+::)*(\w+_kernel)\b", text))
-        ahead |= set(re.findall(r"cudaLaunchKernelEx\(&cfg, (\w+_kernel)\b", text))
-    ahead |= {"chunk_delta_parts_kernel", "chunk_delta_out_kernel"}             # launched through a pointer
+        names |= set(re.findall(r"sllm_launch\(\s*(?:\w+::)*(\w+_kernel)\b", text))
+        names |= set(re.findall(r"cudaLaunchKernelEx\(&cfg, (\w+_kernel)\b", text))
+    return names | {"chunk_delta_parts_kernel", "chunk_delta_out_kernel"}             # launched through a pointer
+
+
+def _read_in_front_of_the_wait(head, body):
+    """Parameters (pointers, tensor maps, a struct's pointers) that the text in front of the first wait reads through."""
+    before = re.sub(r"//[^\n]*", "", body).split("pdl_wait()")[0]
+    params = [(a.split()[-1].lstrip("*&"), "*" in a) for a in head.replace("\n", " ").split(",")]
+    pointers, others = {n for n, p in params if p}, {n for n, p in params if not p}
+    read = pointers & set(re.findall(r"(?<![\w.>])(\w+)\[", before) + re.findall(r"\(\s*\(?[^()]*\*\)\s*\(?(\w+)", before)
+                          + re.findall(r"\bld\w*\(\s*(\w+)", before) + re.findall(r"(?<![\w)\]] )\*(\w+)", before))
+    read |= {f"{s}.{f}" for s, f in re.findall(r"\b(\w+)\.(\w+)\[", before) if s in others}
+    return read | set(re.findall(r"tma_load\w*\([^;]*?&(\w+)", before)) | ({"?"} if re.search(r"\b(ld_dep|ld_stream|load_w|__ldg)\w*\s*\(", before) else set())
+
+
+# what is read in front of the wait on purpose: weights, which no kernel of a step writes (the few-rows product's lambdas that read
+# its input stand in front of the wait and run behind it)
+WEIGHTS = {"gemm_small_m_kernel": {"?", "y"}, "gemm_tc_cluster_kernel": {"map_b"}, "gemm_tc_skinny_kernel": {"map_w"}, "add_rms_normed_reg_kernel": {"?"}}
+
+
+def test_every_kernel_launched_ahead_waits_for_the_one_in_front():
+    bodies, heads, ahead = _bodies(), _bodies(heads=True), _ahead()
     assert len(ahead) > 40 and ahead <= set(bodies)
     assert not [k for k in sorted(ahead) if "pdl_wait()" not in bodies[k]]
+    early = {k: _read_in_front_of_the_wait(heads[k], bodies[k]) - WEIGHTS.get(k, set()) for k in sorted(ahead)}
+    assert not {k: v for k, v in early.items() if v}
+
+
+def test_a_read_in_front_of_the_wait_is_found():
+    for read in ("float v = x[threadIdx.x];", "float4 v = *(const float4*)(x + 4);", "float v = ld4(x + 3);", "int v = p.rows[0];",
+                 "tma_load_2d(dst, &map, 0, 0, bar);", "int n = *count;"):
+        head = "const float* __restrict__ x, const int* count, Args p, const __grid_constant__ CUtensorMap map"
+        assert _read_in_front_of_the_wait(head, "{ " + read + " pdl_wait(); }") and not _read_in_front_of_the_wait(head, "{ pdl_wait(); " + read + " }")
 
 
 def test_tensor_memory_is_taken_before_dependents_may_start():
