@@ -363,11 +363,14 @@ class SplitGemm:
     def takes(cls, a, w, parts: int = 1) -> bool:
         """Whether a product of `a` [M, K] with `w` [N, K], or with blocks [b, N, K] of a's columns, goes here and not to the FMA kernels:
         widths and places that the copies take, sums of at least 64 terms (shorter ones can come out less exact than a chain of FMA: 48
-        terms of very unequal rows 1.11e-7, 1.10e-7), and sizes where it is faster, which is from 65 rows on everywhere (weights out
+        terms of very unequal rows 1.11e-7, 1.10e-7), and sizes where it is faster, which is from 65 rows on nearly everywhere (weights out
         of memory, FMA / here, us: 65 rows 2,048 x 8,192 909 / 202, in 16 parts 103 / 71; 6,144 x 2,048 234 / 67; 2,048 x 64 9.4 / 8.2) and
         from 17 on where K is one part and not tiny (17 rows 1,024 x 1,024 76 / 27, 64 x 2,048 129 / 45; but 2,048 x 64 6.4 / 7.8, 6,144 x
-        2,048 in 6 parts 50 / 51)."""
+        2,048 in 6 parts 50 / 51). Up to 128 rows by many columns with short sums stay, for the planes of the weights weigh more than
+        the weights: 12,288 x 64 11.8 / 13.9 (128 rows), 32,768 x 80 18.5 / 21.6 (65 rows), x 112 25.7 / 26.2 (128); x 128 28.7 / 26.5."""
         M, K, N = a.shape[0], w.shape[-1], w.numel() // w.shape[-1]
+        if M <= 128 and K < 120 and N > 8192:
+            return False
         if not (M > 64 or (M > 16 and K >= 128 and parts == 1 and 6 * K * N + 6 * M * a.shape[1] <= cls.FEW_ROWS_BYTES)):
             return False
         return (a.dtype == w.dtype == torch.float32 and K % 8 == 0 and 64 <= K <= 32768 and 6 * a.shape[1] * 512 <= cls.SCRATCH_BYTES

@@ -227,3 +227,9 @@ def test_short_contexts_of_unequal_widths_keep_a_block_a_row_and_head(dtype, n_s
     """Two heads a block from 129 columns on, else four; the line lies at 1,024 blocks."""
     from scriptling_llm_lib_b200.csrc.bindings import KernelSet
     assert KernelSet.attn_decode_split_pays(dtype, n_seqs, H, G, D, V, pages) == want
+
+
+@pytest.mark.parametrize("M, N, K, want", [(65, 8192, 64, True), (65, 8200, 64, False), (128, 32768, 112, False), (128, 32768, 120, True), (129, 32768, 64, True)])
+def test_few_rows_by_many_columns_with_short_sums_keep_the_chains(M, N, K, want):
+    from scriptling_llm_lib_b200.csrc.bindings import SplitGemm
+    assert SplitGemm.takes(torch.empty((M, K), device="meta"), torch.empty((N, K), device="meta")) == want
