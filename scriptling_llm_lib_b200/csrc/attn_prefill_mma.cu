@@ -231,7 +231,7 @@ template <int KD, int VD>
 static int pm_launch(const PmArgs& a, int B, int max_new, cudaStream_t stream) {
   size_t smem = (size_t)2 * PM_BK * ((KD + 8) + (VD + 8)) * sizeof(bf16);
   static SllmPerDevice allowed;
-  if (smem > 48 * 1024) {
+  if (smem > SLLM_SMEM_UNASKED) {
     const cudaError_t e = sllm_allow_smem(allowed, attn_prefill_mma_kernel<KD, VD>, smem);
     if (e != cudaSuccess) return (int)e;
   }

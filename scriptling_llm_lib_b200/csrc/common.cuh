@@ -30,6 +30,8 @@ struct SllmPerDevice {
     return of[dev & 63];
   }
 };
+// Dynamic shared memory that any kernel here may have without asking for it: 48 KB, less what it has of its own.
+#define SLLM_SMEM_UNASKED (47 * 1024)
 // the current device lets `kernel` have `bytes` of dynamic shared memory
 template <typename K>
 static inline cudaError_t sllm_allow_smem(SllmPerDevice& allowed, K kernel, size_t bytes) {

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(128) latent_expand_mma_kernel(const float* __r
 
 template <typename K>
 static cudaError_t allow_smem(K kernel, size_t smem) {
-  return smem <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return smem <= SLLM_SMEM_UNASKED ? cudaSuccess : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 static inline bool al(const void* p, size_t bytes) { return ((uintptr_t)p % bytes) == 0; }
 

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) state_step_kernel(Job job, int units, int
 template <typename Job>
 static int launch(const Job& job, int rows, int cols, int units, int sm_count, int* err, cudaStream_t stream) {
   const size_t smem = smem_bytes(rows, cols);
-  cudaError_t e = smem <= 48 * 1024 ? cudaSuccess : cudaFuncSetAttribute(state_step_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  cudaError_t e = smem <= SLLM_SMEM_UNASKED ? cudaSuccess : cudaFuncSetAttribute(state_step_kernel<Job>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   if (e != cudaSuccess) return (int)e;
   const int most = (smem <= 112 * 1024 ? 2 : 1) * sm_count;
   state_step_kernel<Job><<<units < most ? units : most, 256, smem, stream>>>(job, units, err);

@@ -125,6 +125,20 @@ def test_add_rmsnorm_many_rows_of_any_width(kernel_sets, dtype, d):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [12032, 12256, 12257, 12288, 12292])
+def test_norms_of_rows_that_nearly_fill_what_a_block_may_have_unasked(kernel_sets, dtype, d):
+    """A row of 12,288 floats is 48 KB, and the kernel has some shared memory of its own besides."""
+    ks, T = kernel_sets[dtype], 3
+    x, w = dev(rand(T, d, seed=1)), dev(rand(d, seed=3) + 1.0, dtype)
+    y = torch.full((T, d), float("nan"), dtype=dtype, device="cuda")
+    ks.add_rmsnorm(x, None, None, w, y, 1e-5)
+    assert rel_err(y.cpu().float(), plain.rms_norm(f64(x), f64(w), 1e-5)) < TOL[dtype]
+    y.fill_(float("nan"))
+    ks.seq.add_norm(x, [], None, w, y, 1e-5, center=False)
+    assert rel_err(y.cpu().float(), plain.rms_norm(f64(x), f64(w), 1e-5)) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("dv", [4, 100, 127, 128, 132])
 def test_unit_norms_of_heads(kernel_sets, dtype, dv):
     """The gated norm behind the delta rule and the unit keys and queries in front of it: heads of up to 128 by four elements, others."""
