@@ -891,7 +891,8 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // 128 columns and 4.7 beyond, two-SM tiles 6.2) and takes 0.28 a k-block. Measured, there / here: 300 rows by 64 x 1,024 8.1 / 4.6, 300 by
 // 1,024 x 1,024 11.2 / 8.9, 300 by 2,048 x 2,048 15.8 / 10.9, 2,048 by 576 x 2,048 15.7 / 15.0 (the seventh asked of two blocks); but
 // 512 by 2,560 x 1,024 11.0 / 12.5, 300 by 4,096 x 128 7.0 / 10.1. Clusters beyond the first wave double it (512 rows by 1,024 x 1,024
-// on 16 clusters of 8 17.2, on 4 9.0): 14 of 8, 32 of 4 and 72 of 2 stand side by side, twice as many where two blocks fit an SM.
+// on 16 clusters of 8 17.2, on 4 9.0): 14 of 8, 32 of 4 and 72 of 2 stand side by side, twice as many where two blocks fit an SM. On 1,456
+// shapes of 33 to 4,000 rows, 8 to 4,096 columns and K 64 to 8,192 that had no part in the fit, none is slower than without clusters.
 static int tc_cluster_split(int M, int N, int K, float start, int* tile_n) {
   const int nkb = (K + TC_BK - 1) / TC_BK, tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + 255) / 256;
   *tile_n = ((N + tiles_n - 1) / tiles_n + 15) / 16 * 16;
@@ -912,10 +913,15 @@ static int tc_cluster_choice(int M, int N, int K, int* tile_n) {
   if (tc_one_sm_forced()) return 1;
   return tc_cluster_split(M, N, K, tc_use_pair(M, N) ? 6.2f : N > 128 ? 4.7f : 3.6f, tile_n);
 }
-// the blocks that the plain product of these sizes puts on a tile's K (1: a kernel that walks all of it)
-SLLM_EXPORT int sllm_gemm_tc_cluster_split(int M, int N, int K) {
+// the same where the other choice is the few-rows kernel, which has more of the SMs on few rows
+static int tc_skinny_cluster_choice(int M, int N, int K, int* tile_n) {
+  if (M <= 32 || tc_one_sm_forced()) return 1;
+  return tc_cluster_split(M, N, K, 3.6f, tile_n);
+}
+// the blocks that the plain product of these sizes, or that of the few-rows kernel, puts on a tile's K (1: a kernel that walks all of it)
+SLLM_EXPORT int sllm_gemm_tc_cluster_split(int M, int N, int K, int few_rows) {
   int tile_n;
-  return tc_cluster_choice(M, N, K, &tile_n);
+  return few_rows ? tc_skinny_cluster_choice(M, N, K, &tile_n) : tc_cluster_choice(M, N, K, &tile_n);
 }
 
 template <int SPLIT>
@@ -1297,9 +1303,9 @@ SLLM_EXPORT int sllm_gemm_tc_skinny_bf16(const void* A, const void* B, void* C, 
   if (epilogue != TC_EPI_STORE && epilogue != TC_EPI_SWIGLU) return SLLM_ERR_ARG;
   if (epilogue == TC_EPI_SWIGLU && ((N & 15) || out_f32 || ksplit != 1)) return SLLM_ERR_ARG;
   if (ksplit < 1 || ksplit > (K + TC_BK - 1) / TC_BK || (ksplit > 1 && !out_f32)) return SLLM_ERR_ARG;
-  if (epilogue == TC_EPI_STORE && ksplit == 1 && M > 32 && !tc_one_sm_forced()) {
+  if (epilogue == TC_EPI_STORE && ksplit == 1) {
     int tile_n;
-    const int split = tc_cluster_split(M, N, K, 3.6f, &tile_n);
+    const int split = tc_skinny_cluster_choice(M, N, K, &tile_n);
     if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, err, stream);
   }
   int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
