@@ -375,7 +375,8 @@ static int gs_product(const GsArgs& g, const bf16* planes_a, const bf16* planes_
 // twice as often, lose.
 static int gs_tile_n(int M, int N, int z) {
   const long long rows = (M + GS_BM - 1) / GS_BM * (long long)z, wide = rows * ((N + 255) / 256), narrow = rows * ((N + 127) / 128);
-  return (narrow + 73) / 74 * 11 < (wide + 73) / 74 * 20 ? 128 : 256;
+  const int pairs = sllm_sm_count() / 2 > 0 ? sllm_sm_count() / 2 : 1;
+  return (narrow + pairs - 1) / pairs * 11 < (wide + pairs - 1) / pairs * 20 ? 128 : 256;
 }
 
 // C[M,N] = A[M,K] B[N,K]^T, floats. parts > 1: K is cut into that many runs and C receives their partial sums, c_part apart. batch > 1:
@@ -400,7 +401,7 @@ SLLM_EXPORT int sllm_gemm_split_f32(const float* A, const float* B, float* C, in
     if (np < N) np = np / 256 * 256;
     if (mp < 1 || np < 1 || (batch > 1 && np < N)) return SLLM_ERR_ARG;      // (a batch's columns are not cut)
   }
-  const int nkb = (K + GS_BK - 1) / GS_BK, kb_part = (nkb + parts - 1) / parts;
+  const int nkb = (K + GS_BK - 1) / GS_BK, kb_part = (nkb + parts - 1) / parts, at_once = sllm_sm_count() * 8;
   bf16* pa = (bf16*)scratch;
   bf16* pb = (bf16*)((char*)scratch + mp * a_row);
   for (long long n0 = 0; n0 < N; n0 += np) {
@@ -412,7 +413,7 @@ SLLM_EXPORT int sllm_gemm_split_f32(const float* A, const float* B, float* C, in
       if (m0 > 0) sb.rows = 0;
       const long long most = ((long long)(sa.rows) * sa.cols > (long long)sb.rows * K ? (long long)sa.rows * sa.cols : (long long)sb.rows * K) / 8;
       const long long blocks = (most + 255) / 256;
-      sllm_launch(gemm_split_planes_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 2), dim3(256), 0, stream, sa, sb);
+      sllm_launch(gemm_split_planes_kernel, dim3((unsigned)(blocks < at_once ? blocks : at_once), 2), dim3(256), 0, stream, sa, sb);
       const GsArgs g{A + m0 * lda, B + n0 * ldb, C + m0 * ldc + n0, m, n, K, lda, ldb, ldc, parts, batch, kb_part, c_part, batch * n};
       const int rc = gs_product(g, pa, pb, gs_tile_n(m, n, parts * batch), err, stream);
       if (rc) return rc;
