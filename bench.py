@@ -936,8 +936,8 @@ def mix_kernels_alone(args):
             out = torch.empty(T, W, device=dev)
             err = torch.zeros(1, dtype=torch.int32, device=dev)
             tc = ks.tensor_core
-            us = timed(lambda i: (k.moe_group_rows(idx, E, offsets, None, rop, tg, pad=128), k.moe_gather_rows(h, rop, top, xs2)), 1)
-            report(f"moe_group_rows + moe_gather_rows ({label})", T, us, nbytes=(T + pairs) * W * esz)
+            us = timed(lambda i: (k.moe_group_rows(idx, E, offsets, None, rop, tg, pad=128), k.moe_spread_rows(h, rop, top, xs2)), 1)
+            report(f"moe_group_rows + moe_spread_rows ({label})", T, us, nbytes=(T + pairs) * W * esz)
             us = timed(lambda i: tc.gemm_grouped(xs2, w_up, hid, tg, err, act="relu_squared", rows_used=offsets[E:]), 1)
             report(f"gemm_grouped up, {rows} rows for {pairs} pairs ({label})", T, us, flops=2 * pairs * F * W, tensor=True)
             us = timed(lambda i: tc.gemm_grouped(hid, w_down, ys2, tg, err, rows_used=offsets[E:]), 1)
@@ -1094,7 +1094,7 @@ def gate_kernels_alone(args):
             out = torch.empty(T, W, device=dev)
             tc = ks.tensor_core
             ks.mix.moe_group_rows(idx, E, offsets, None, rop, tg, pad=128)
-            ks.mix.moe_gather_rows(h, rop, top, xs2)
+            ks.mix.moe_spread_rows(h, rop, top, xs2)
             us = timed(lambda i: tc.gemm_grouped(xs2, w_gu, hid, tg, err, rows_used=offsets[E:], glu=(7.0, 1.702)), 1)
             report(f"gemm_grouped gate|up with the clamped gate, {rows} rows for {pairs} pairs ({label})", T, us, flops=4 * pairs * F * W)
             us = timed(lambda i: (tc.gemm_grouped(xs2, w_gu, raw, tg, err, rows_used=offsets[E:]),

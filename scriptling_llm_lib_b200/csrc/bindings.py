@@ -1435,13 +1435,13 @@ class MixKernels:
                "moe_grouped")
         LAUNCHES[0] += 1
 
-    def moe_gather_rows(self, h, row_of_pair, top, xs):
+    def moe_spread_rows(self, h, row_of_pair, top, xs):
         """xs[row_of_pair[t * top + k]] = h[t]; other rows of xs stay."""
         if row_of_pair.numel() != h.shape[0] * top:
-            raise KernelError(f"moe_gather_rows: {row_of_pair.numel()} pairs of {h.shape[0]} rows, {top} each")
-        _check(self._fn("moe_gather_rows")(self._view(h, "h"), h.stride(0), _ptr(row_of_pair, torch.int32, "row_of_pair"),
+            raise KernelError(f"moe_spread_rows: {row_of_pair.numel()} pairs of {h.shape[0]} rows, {top} each")
+        _check(self._fn("moe_spread_rows")(self._view(h, "h"), h.stride(0), _ptr(row_of_pair, torch.int32, "row_of_pair"),
                                            as_int(top), _ptr(xs, self.dtype, "xs"), h.shape[0], xs.shape[1], _stream()),
-               "moe_gather_rows")
+               "moe_spread_rows")
 
     def moe_combine(self, ys, row_of_pair, wgt, out):
         """out[t] = sum_k wgt[t, k] * ys[row_of_pair[t * top + k]], float32 [T, N]."""

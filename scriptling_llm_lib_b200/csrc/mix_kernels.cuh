@@ -1615,7 +1615,7 @@ moe_group_kernel(const int* __restrict__ idx, int n_pairs, int* __restrict__ off
 // each of its choices; rows that pad keep what they hold (nobody reads what becomes of them). 2,048 rows of 2,048, six choices:
 // 10 us; by rows of the result, zeros in those that pad, 19.
 template <typename A>
-__global__ void moe_gather_rows_kernel(const A* __restrict__ h, int ldh, const int* __restrict__ row_of_pair, int top,
+__global__ void moe_spread_rows_kernel(const A* __restrict__ h, int ldh, const int* __restrict__ row_of_pair, int top,
                                        A* __restrict__ xs, int K, int vec) {
   pdl_launch_dependents();
   pdl_wait();

@@ -227,7 +227,7 @@ class RoutedExperts(FeedForward):
         tile_group = torch.empty((rows // tile,), dtype=torch.int32, device=dev)
         k.moe_group_rows(idx, self.E, offsets, None, row_of_pair, tile_group, pad=tile)
         xs = torch.empty((rows, self.hidden), dtype=x.dtype, device=dev)
-        k.moe_gather_rows(x, row_of_pair, self.top, xs)
+        k.moe_spread_rows(x, row_of_pair, self.top, xs)
         tc = ctx.kernels.tensor_core
         hid = torch.empty((rows, self.F), dtype=x.dtype, device=dev)
         if self.glu is not None:      # `tiled` holds here: its conditions are those of the tensor-core path

@@ -817,7 +817,7 @@ def test_moe_grouping_gives_every_pair_its_row(T, top, E, pad):
     K, N, tc, flag = 72, 264, k.tensor_core, torch.zeros(1, dtype=torch.int32, device="cuda")
     h, w = torch.randn(T, K, generator=g).bfloat16().cuda(), (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16().cuda()
     xs = torch.full((rows, K), float("nan"), dtype=torch.bfloat16, device="cuda")
-    k.mix.moe_gather_rows(h, rop, top, xs)
+    k.mix.moe_spread_rows(h, rop, top, xs)
     assert torch.equal(xs[rop.long()], h.repeat_interleave(top, 0))
     out = torch.full((rows, N), 7.0, device="cuda")
     tc.gemm_grouped(xs, w, out, tiles, flag, rows_used=offsets[E:], tile_rows=pad)

@@ -233,3 +233,8 @@ def test_short_contexts_of_unequal_widths_keep_a_block_a_row_and_head(dtype, n_s
 def test_few_rows_by_many_columns_with_short_sums_keep_the_chains(M, N, K, want):
     from scriptling_llm_lib_b200.csrc.bindings import SplitGemm
     assert SplitGemm.takes(torch.empty((M, K), device="meta"), torch.empty((N, K), device="meta")) == want
+
+
+def test_the_map_of_pairs_to_rows_has_a_name_of_its_own():
+    """Rows used to be gathered by the inverse map, as many int32 as this one where nothing pads: a call by the old name must not pass."""
+    assert hasattr(MixKernels, "moe_spread_rows") and not hasattr(MixKernels, "moe_gather_rows")
