@@ -554,7 +554,8 @@ class TensorCoreGemm:
 
     def gemm_skinny(self, a, w, out, err_flag, swiglu=False):
         """The same product for at most 128 rows of `a`, with the weights as the tensor cores' 128-row
-        operand and a grid over (128 weight rows, K splits). out [M,N] bfloat16 or float32, or
+        operand and a grid over (128 weight rows, K splits). `w` is read while kernels in front may still run: weights, not what
+        one of them writes. out [M,N] bfloat16 or float32, or
         [M,N/2] with swiglu; float32 [P,M,N]: K split P ways, out receives the partial sums."""
         M, K = a.shape
         N = w.shape[0]

@@ -729,9 +729,10 @@ static bool tc_use_pair(int M, int N) { return !tc_one_sm_forced() && M > 128 &&
 // Products whose output is a handful of tiles (a router's 64 columns, step sizes and decays, low ranks, short prompts) leave most SMs
 // idle and walk all of K on the others, a serial chain of copies and products. Here a cluster of 2, 4 or 8 blocks takes one tile of 128 x
 // BN outputs (BN a multiple of 16 up to 256, as the host cuts N), each block its share of K; the accumulators meet in shared memory,
-// where every block adds up its share of the tile's rows, the blocks' sums in their order, and stores whole rows. Weights are fetched
-// before the kernel in front has finished. Bound by latency: a copy's way, the cluster's two barriers. 2,048 rows by 64 x 2,048 13.8 us
-// on 16 one-SM tiles, 6.6 here; by 160 x 4,096 24.2 on 8 two-SM tiles, 11.9 here.
+// where every block adds up its share of the tile's rows, the blocks' sums in their order, and stores whole rows. Where it stands in for
+// the few-rows kernel (`b_ahead`), B holds weights and is fetched before the kernel in front has finished, as that one does (33 rows by 1,536 x
+// 2,048 7.6 us, 8.5 behind the wait); the plain product's B may be what the kernel in front writes. Bound by latency: a copy's way, the
+// cluster's two barriers. 2,048 rows by 64 x 2,048 14.0 us on 16 one-SM tiles, 6.7 here; by 160 x 4,096 27.9 on 8 two-SM tiles, 10.7 here.
 __device__ __forceinline__ float4 tc_cluster_float4(uint32_t cluster_addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
@@ -740,7 +741,7 @@ __device__ __forceinline__ float4 tc_cluster_float4(uint32_t cluster_addr) {
 template <int SPLIT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, void* __restrict__ C, int M,
-                       int N, int K, int ldc, int out_f32, int BN, int stages, int act, int* __restrict__ err) {
+                       int N, int K, int ldc, int out_f32, int BN, int stages, int act, int b_ahead, int* __restrict__ err) {
   const uint32_t A_BYTES = TC_BM * TC_BK * 2, STAGE_BYTES = A_BYTES + BN * TC_BK * 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -777,6 +778,7 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   if (warp == 0) {
     if (lane == 0) {
       const int pre = min(nkb, stages);
+      if (!b_ahead) pdl_wait();
       for (int i = 0; i < pre; i++) {
         mbar_expect_tx(full0 + 8 * i, STAGE_BYTES);
         tma_load_2d(smem_base + i * STAGE_BYTES + A_BYTES, &map_b, (kb0 + i) * TC_BK, n0, full0 + 8 * i);
@@ -891,8 +893,9 @@ gemm_tc_cluster_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 // 128 columns and 4.7 beyond, two-SM tiles 6.2) and takes 0.28 a k-block. Measured, there / here: 300 rows by 64 x 1,024 8.1 / 4.6, 300 by
 // 1,024 x 1,024 11.2 / 8.9, 300 by 2,048 x 2,048 15.8 / 10.9, 2,048 by 576 x 2,048 15.7 / 15.0 (the seventh asked of two blocks); but
 // 512 by 2,560 x 1,024 11.0 / 12.5, 300 by 4,096 x 128 7.0 / 10.1. Clusters beyond the first wave double it (512 rows by 1,024 x 1,024
-// on 16 clusters of 8 17.2, on 4 9.0): 14 of 8, 32 of 4 and 72 of 2 stand side by side, twice as many where two blocks fit an SM. On 1,456
-// shapes of 33 to 4,000 rows, 8 to 4,096 columns and K 64 to 8,192 that had no part in the fit, none is slower than without clusters.
+// on 16 clusters of 8 17.2, on 4 9.0): 14 of 8, 32 of 4 and 72 of 2 stand side by side, twice as many where two blocks fit an SM. Of 1,456
+// shapes of 33 to 4,000 rows, 8 to 4,096 columns and K 64 to 8,192, few of which had a part in the fit, 16 are slower by more than 3% than without
+// clusters (4,000 rows by 160 x 512 8.1 / 9.5, 33 by 2,560 x 1,024 6.9 / 7.8), 725 faster.
 static int tc_cluster_split(int M, int N, int K, float start, int* tile_n) {
   const int nkb = (K + TC_BK - 1) / TC_BK, tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + 255) / 256;
   *tile_n = ((N + tiles_n - 1) / tiles_n + 15) / 16 * 16;
@@ -926,7 +929,7 @@ SLLM_EXPORT int sllm_gemm_tc_cluster_split(int M, int N, int K, int few_rows) {
 
 template <int SPLIT>
 static int tc_cluster_run(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int out_f32, int act,
-                          int tile_n, int* err, cudaStream_t stream) {
+                          int tile_n, int b_ahead, int* err, cudaStream_t stream) {
   CUtensorMap ma, mb;
   int rc = tc_make_map(&ma, A, M, K, lda, TC_BM);
   if (!rc) rc = tc_make_map(&mb, B, N, K, ldb, tile_n);
@@ -953,13 +956,13 @@ static int tc_cluster_run(const void* A, const void* B, void* C, int M, int N, i
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = sllm_pdl_off() ? 1 : 2;
-  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<SPLIT>, ma, mb, C, M, N, K, ldc, out_f32, tile_n, stages, act, err);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_tc_cluster_kernel<SPLIT>, ma, mb, C, M, N, K, ldc, out_f32, tile_n, stages, act, b_ahead, err);
 }
 static int tc_cluster_launch(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, int out_f32, int act,
-                             int split, int tile_n, int* err, cudaStream_t stream) {
-  return split == 8   ? tc_cluster_run<8>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream)
-         : split == 4 ? tc_cluster_run<4>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream)
-                      : tc_cluster_run<2>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, err, stream);
+                             int split, int tile_n, int b_ahead, int* err, cudaStream_t stream) {
+  return split == 8   ? tc_cluster_run<8>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, b_ahead, err, stream)
+         : split == 4 ? tc_cluster_run<4>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, b_ahead, err, stream)
+                      : tc_cluster_run<2>(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, tile_n, b_ahead, err, stream);
 }
 
 // C[M,N] = A[M,K] B[N,K]^T. epilogue 0: C bfloat16 (or float when out_f32), row stride ldc;
@@ -984,7 +987,7 @@ SLLM_EXPORT int sllm_gemm_tc_fold_bf16(const void* A, const void* B, void* C, in
   if (epilogue == TC_EPI_STORE && !sumsq_in) {
     int tile_n;
     const int split = tc_cluster_choice(M, N, K, &tile_n);
-    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, err, stream);
+    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, 0, err, stream);
   }
   CUtensorMap ma, mb;
   int big = N > 128;
@@ -1076,7 +1079,7 @@ SLLM_EXPORT int sllm_gemm_tc_act_bf16(const void* A, const void* B, void* C, int
   if (K <= 0 || (K & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || act < 1 || act > 3) return SLLM_ERR_ARG;
   int tile_n;
   const int split = tc_cluster_choice(M, N, K, &tile_n);
-  if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, split, tile_n, err, stream);
+  if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, act, split, tile_n, 0, err, stream);
   TcFold fd{};
   fd.act = act;
   const TcRope rp{};
@@ -1306,7 +1309,7 @@ SLLM_EXPORT int sllm_gemm_tc_skinny_bf16(const void* A, const void* B, void* C, 
   if (epilogue == TC_EPI_STORE && ksplit == 1) {
     int tile_n;
     const int split = tc_skinny_cluster_choice(M, N, K, &tile_n);
-    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, err, stream);
+    if (split > 1) return tc_cluster_launch(A, B, C, M, N, K, lda, ldb, ldc, out_f32, 0, split, tile_n, 1, err, stream);
   }
   int bt = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   CUtensorMap mw, mx;

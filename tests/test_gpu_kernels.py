@@ -514,6 +514,22 @@ def test_few_tiles_share_their_k_among_a_cluster(kernel_sets, M, N, K, split):
     assert rel_err(act.cpu().float(), want.clamp(min=0) ** 2) < TOL[torch.bfloat16] and int(flag) == 0
 
 
+def test_a_product_of_what_the_kernel_in_front_writes(kernel_sets):
+    """Both operands of a plain product may come out of the launch before it, also where a cluster shares its K."""
+    tc, flag = kernel_sets[torch.bfloat16].tensor_core, torch.zeros(1, dtype=torch.int32, device="cuda")
+    x, y, a = dev(rand(256, 8192, seed=1), torch.bfloat16), dev(rand(2048, 8192, seed=2, scale=8192 ** -0.5), torch.bfloat16), dev(rand(300, 2048, seed=3), torch.bfloat16)
+    w, out, settled = (torch.zeros(s, device="cuda", dtype=t) for s, t in (((256, 2048), torch.bfloat16), ((300, 256), torch.float32), ((300, 256), torch.float32)))
+    assert tc.lib.sllm_gemm_tc_cluster_split(300, 256, 2048, 0) > 1
+    tc.gemm(x, y, w, flag)
+    torch.cuda.synchronize()
+    tc.gemm(a, w, settled, flag)
+    for _ in range(5):
+        w.zero_()
+        tc.gemm(x, y, w, flag)
+        tc.gemm(a, w, out, flag)
+        assert torch.equal(out, settled) and int(flag) == 0
+
+
 @pytest.mark.parametrize("M, N, K", [(17, 1, 128), (65, 7, 64), (128, 256, 72), (129, 129, 1000), (256, 128, 264), (257, 300, 4096), (700, 520, 136)])
 def test_gemm_split_is_at_least_as_exact_as_the_chain(kernel_sets, M, N, K):
     """Products in three bfloat16 parts on the tensor cores: ragged tiles and k-blocks, K in parts (more than there are k-blocks among

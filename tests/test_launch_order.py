@@ -63,6 +63,20 @@ def test_every_kernel_launched_ahead_waits_for_the_one_in_front():
     assert not {k: v for k, v in early.items() if v}
 
 
+def test_only_the_few_rows_product_reads_its_second_operand_ahead():
+    """The plain product's may be what the kernel in front writes: where a cluster shares its K it waits first, too."""
+    text = FILES["gemm_tcgen05.cu"]
+    body = _bodies()["gemm_tc_cluster_kernel"]
+    assert 0 < body.find("if (!b_ahead) pdl_wait();") < body.find("tma_load_2d(")
+    calls = re.findall(r"(sllm_gemm_tc_\w+)\(|return tc_cluster_launch\(A, B, [^;]*tile_n, ([01]), err", text)
+    ahead, fn = {}, None
+    for name, flag in calls:
+        fn = name or fn
+        if flag:
+            ahead[fn] = int(flag)
+    assert ahead == {"sllm_gemm_tc_fold_bf16": 0, "sllm_gemm_tc_act_bf16": 0, "sllm_gemm_tc_skinny_bf16": 1}
+
+
 def test_a_read_in_front_of_the_wait_is_found():
     for read in ("float v = x[threadIdx.x];", "float4 v = *(const float4*)(x + 4);", "float v = ld4(x + 3);", "int v = p.rows[0];",
                  "tma_load_2d(dst, &map, 0, 0, bar);", "int n = *count;"):
